@@ -87,6 +87,26 @@ struct BlockMap {
 
 __device__ __forceinline__ int sar(int x, int s) { return x >> s; }
 
+// Approximate reciprocal square root, division and cosine without the steps
+// that keep subnormal operands (none occurs where they are used): rsqrt of 0 is
+// infinite, and for normal operands the results are rsqrtf's, __fdividef's and
+// __cosf's.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float div_approx(float a, float b) {
+  float y;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float cos_approx(float x) {
+  float y;
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // ---------------------------------------------------------------- Saru
 // Saru(seed1, seed2, seed3) and u32() (saruprng.hpp:239-255, 322-333); the
 // constants are the generator's definition and must match bit for bit.
@@ -139,7 +159,7 @@ __device__ __forceinline__ float saru_nrml_f32(Saru& s) {
   const int dbl = M < 0xB504F334u ? 1 : 0;  // f < 1/sqrt 2 (0xB504F334 = 2^32 / sqrt 2)
   const uint32_t Md = M << dbl;             // f' 2^32, modulo 2^32 when doubled
   const float c = __int2float_rn((int)(0u - Md)) * two_m32;  // 1 - f'
-  const float z = __fdividef(c, 2.0f - c);
+  const float z = div_approx(c, 2.0f - c);
   const float z2 = z * z;
   float p = 1.0f / 9.0f;
   p = fmaf(p, z2, 1.0f / 7.0f);
@@ -148,9 +168,9 @@ __device__ __forceinline__ float saru_nrml_f32(Saru& s) {
   p = fmaf(p, z2, 1.0f);
   const float nlog = fmaf(__int2float_rn(j + dbl), 0.69314718055994531f, 2.0f * (z * p));
   // cos(2 pi u2) = cos(2 pi (u2 - 1)): the signed draw gives the argument in [-pi, pi)
-  const float cs = __cosf(__int2float_rn((int)m2) * (6.28318530717958647692f * two_m32));
+  const float cs = cos_approx(__int2float_rn((int)m2) * (6.28318530717958647692f * two_m32));
   const float r2 = 2.0f * nlog;
-  return r2 * rsqrtf(r2) * cs;  // nlog > 0 for every odd m1
+  return r2 * rsqrt_approx(r2) * cs;  // nlog > 0 for every odd m1
 }
 
 // FP64 normal exactly as the reference computes it (plain FP64 arm).

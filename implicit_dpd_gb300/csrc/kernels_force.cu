@@ -91,60 +91,67 @@ __device__ __forceinline__ void fill_off_table(OffTable& T, const RepDev& R, int
   T.o[c] = make_float4(dx * R.cs_f[0], dy * R.cs_f[1], dz * R.cs_f[2], 0.0f);
 }
 
-// A lane's share of the owner's fixed-point sums of pass 2, kept as the sums
-// of the fix_force_parts of its terms. A list holds at most kNbrCap terms, so
-// the parts' totals over a half warp stay below 2^30 and reduce in 32 bits.
-struct PartSums {
-  int hi[6], lo[6];
-};
-static_assert((long long)kNbrCap * (1 << 21) <= (1ll << 30), "32-bit totals of the fixed-point parts");
-
-// The total of parts c over the lanes of half warp h (lanes 16 h .. 16 h + 15).
-__device__ __forceinline__ long long half_total(const PartSums& P, int c, int h) {
-  const int hi0 = __reduce_add_sync(0xffffffffu, h ? 0 : P.hi[c]);
-  const int hi1 = __reduce_add_sync(0xffffffffu, h ? P.hi[c] : 0);
-  const int lo0 = __reduce_add_sync(0xffffffffu, h ? 0 : P.lo[c]);
-  const int lo1 = __reduce_add_sync(0xffffffffu, h ? P.lo[c] : 0);
-  return ((long long)(h ? hi1 : hi0) << 21) + (long long)(h ? lo1 : lo0);
+// The terms of the four pairs of a quad of lanes (4 q .. 4 q + 3, one particle's)
+// turned from one pair per lane to one component per lane: on return w[j] of
+// lane 4 q + c is component c (x, y, z; nothing for c = 3) of lane 4 q + j's pair.
+// Two butterfly exchanges; every lane of the warp takes part.
+__device__ __forceinline__ void quad_components(float x, float y, float z, int c, float w[4]) {
+  const bool odd = c & 1, up = c & 2;
+  float r = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+  const float a0 = odd ? r : x, a1 = odd ? y : r;   // component c & 1 of the even, odd lane's pair
+  const float a3 = __shfl_xor_sync(0xffffffffu, z, 1);  // even lanes: z of the odd lane's pair
+  r = __shfl_xor_sync(0xffffffffu, up ? a0 : z, 2);
+  w[0] = up ? r : a0;
+  w[2] = up ? z : r;
+  r = __shfl_xor_sync(0xffffffffu, up ? a1 : a3, 2);
+  w[1] = up ? r : a1;
+  w[3] = up ? a3 : r;
 }
 
-// One component v of a pair term, converted to fixed point once for both
-// particles: the owner subtracts its parts (its term is -v), the other
-// particle's sum receives round(v 2^26) (NEG: -round(v 2^26)) by atomic add.
-// A term beyond +-65536 goes to the other particle exactly (bit-level
-// conversion) and marks the owner for the 64-bit sums.
-template <bool NEG>
-__device__ __forceinline__ void part_both(float v, int& hi, int& lo, long long* q, bool& range) {
-  int h, l;
-  fix_force_parts(v, h, l);
-  hi -= h;
-  lo -= l;
-  long long x = (long long)h * 2097152ll + (long long)l;
-  if (!(fabsf(v) < 65536.0f)) {
-    x = fix_from_float(v, kForceBits);
-    range = false;
+// Component c of the terms of a quad's four pairs, converted to fixed point
+// once for both particles: the owner's 64-bit sum S takes -x (the virial, the
+// same for both, +x) and the sum of the other particle of pair j, row t[j], x by
+// atomic add. The three lanes of a quad that hold x, y and z address one row at a
+// time, so a row's three adds leave the SM as one access of its 32-byte sector.
+// BIG: some term of the warp may reach +-65536 (the bit-level conversion).
+// lim: pairs of the quad that exist (0 on the lane without a component); sums
+// points at component c of row 0.
+template <bool VIRIAL, bool BIG>
+__device__ __forceinline__ void quad_both(const float w[4], const int t[4], int lim,
+                                          long long* sums, long long& S) {
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    long long x;
+    if (BIG) {
+      x = fix_force(w[j]);
+    } else {
+      int h, l;
+      fix_force_parts(w[j], h, l);
+      x = mad_wide(h, 1 << 21, (long long)l);
+    }
+    S = VIRIAL ? S + x : S - x;
+    red_add_if(j < lim, sums + 4 * (size_t)t[j], x);
   }
-  red_add(q, NEG ? -x : x);
 }
 
 // One owned pair of a pass-1 list (fast path of pass 2), given the other
-// particle's three rows (posf, velf, densf): the pair arithmetic runs in FP32
-// (the compensated forms near the cutoff and for close pairs), and the term
-// is split between the owner's 32-bit parts and the other particle's sums.
-// A pair of equal ids contributes nothing (nbdf_calculator.hpp:84).
+// particle's three rows (posf, velf, densf): the force on the other particle
+// over the pair vector, and the pair vector. The pair arithmetic runs in FP32
+// (the compensated forms near the cutoff and for close pairs). A pair of equal
+// ids contributes nothing (nbdf_calculator.hpp:84), nor does a lane without a pair.
 template <bool PRESS, int FORM>
-__device__ __forceinline__ void owned_pair(const DevState& d, const RepDev* R, const PairTables& T,
-                                           const OffTable& OT, const PairI& I, uint32_t e,
-                                           float4 pj, float4 vj, float4 dj, PartSums& P,
-                                           bool& range) {
+__device__ __forceinline__ float owned_pair(const DevState& d, const RepDev* R, const PairTables& T,
+                                            const OffTable& OT, const PairI& I, uint32_t e,
+                                            bool valid, float4 pj, float4 vj, float4 dj, float& ex,
+                                            float& ey, float& ez) {
   const int t = (int)(e & kRowMask);
   const float4 o = OT.o[e >> kRowBits];
-  float ex = (I.pi.x - o.x) - pj.x;
-  float ey = (I.pi.y - o.y) - pj.y;
-  float ez = (I.pi.z - o.z) - pj.z;
-  float dr2 = ex * ex + ey * ey + ez * ez;
+  ex = (I.pi.x - o.x) - pj.x;
+  ey = (I.pi.y - o.y) - pj.y;
+  ez = (I.pi.z - o.z) - pj.z;
+  float dr2 = dist2(ex, ey, ez);
   float inv_dr, dr, w;
-  if (dr2 < kCloseCut2 || dr2 > kNearCut2) {  // rare: the compensated forms
+  if (valid && (dr2 < kCloseCut2 || dr2 > kNearCut2)) {  // rare: the compensated forms
     int tt, dx, dy, dz;
     read_entry(e, tt, dx, dy, dz);
     const float4 li = __ldg(d.poslo + I.row), lj = __ldg(d.poslo + t);
@@ -152,37 +159,26 @@ __device__ __forceinline__ void owned_pair(const DevState& d, const RepDev* R, c
       close_pair_vector(I.pi, li, pj, lj, dx, dy, dz, R, ex, ey, ez);
       dr2 = ex * ex + ey * ey + ez * ez;
     }
-    inv_dr = rsqrtf(dr2);
+    inv_dr = rsqrt_approx(dr2);
     dr = dr2 * inv_dr;
     w = 1.0f - dr;
     if (dr2 > kNearCut2)  // admitted pairs have 1 - r >= 0 up to ~1e-13
       w = fmaxf(near_cut_w(I.pi, li, pj, lj, dx, dy, dz, R, dr), 0.0f);
   } else {
-    inv_dr = rsqrtf(dr2);
+    inv_dr = rsqrt_approx(dr2);
     dr = dr2 * inv_dr;
     w = 1.0f - dr;
   }
   const uint32_t idj = fbits(vj.w);
-  const float a = pair_cf<FORM>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
+  const float a = pair_cf<FORM, PRESS>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
                                 I.di, dj, I.idi, idj, I.seed);
-  const float an = idj == I.idi ? 0.0f : -a;  // the other particle's force is -a e
-  const float gx = an * ex, gy = an * ey, gz = an * ez;
-  long long* q = d.fq + 4 * (size_t)t;
-  part_both<false>(gx, P.hi[0], P.lo[0], q, range);
-  part_both<false>(gy, P.hi[1], P.lo[1], q + 1, range);
-  part_both<false>(gz, P.hi[2], P.lo[2], q + 2, range);
-  if (PRESS) {  // the virial a e e, the same for both particles
-    long long* pq = d.pq + 4 * (size_t)t;
-    part_both<true>(gx * ex, P.hi[3], P.lo[3], pq, range);
-    part_both<true>(gy * ey, P.hi[4], P.lo[4], pq + 1, range);
-    part_both<true>(gz * ez, P.hi[5], P.lo[5], pq + 2, range);
-  }
+  return valid && idj != I.idi ? -a : 0.0f;  // the other particle's force is -a e
 }
 
 // The force and virial terms of one pair (the pair arithmetic of pass 2),
 // from the side of the particle that owns the pair (a pair of equal ids is
 // skipped, nbdf_calculator.hpp:84); 64-bit path.
-template <bool PRESS, bool CHECK, int FORM>
+template <bool PRESS, int FORM>
 __device__ __forceinline__ bool pair_terms(const DevState& d, const RepDev* R, const PairTables& T,
                                            const PairI& I, int t, int dx, int dy, int dz,
                                            float g[6]) {
@@ -200,17 +196,15 @@ __device__ __forceinline__ bool pair_terms(const DevState& d, const RepDev* R, c
                       ez);
     dr2 = ex * ex + ey * ey + ez * ez;
   }
-  const float inv_dr = rsqrtf(dr2);
+  const float inv_dr = rsqrt_approx(dr2);
   const float dr = dr2 * inv_dr;
   float w = 1.0f - dr;
   if (dr2 > kNearCut2)  // admitted pairs have 1 - r >= 0 up to ~1e-13
     w = fmaxf(near_cut_w(I.pi, __ldg(d.poslo + I.row), pj, __ldg(d.poslo + t), dx, dy, dz, R, dr),
               0.0f);
-  const float a = pair_cf<FORM>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
+  const float a = pair_cf<FORM, PRESS>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
                                 I.di, dj, I.idi, idj, I.seed);
-  // a non-finite term reports itself here (the fast path sends its particle
-  // to this path through the range test of its parts)
-  if (CHECK && !isfinite(a)) atomicCAS(d.err, 0, kErrNonFinite);
+  if (!isfinite(a)) atomicCAS(d.err, 0, kErrNonFinite);
   g[0] = a * ex;
   g[1] = a * ey;
   g[2] = a * ez;
@@ -238,13 +232,13 @@ __device__ __forceinline__ void add_to_other(const DevState& d, int t, const flo
   }
 }
 
-// One owned pair added to the owner's 64-bit sums (the lane's share) and,
-// with OTHER, to the other particle's sums in memory.
-template <bool PRESS, int FORM, bool OTHER>
+// One owned pair added to the owner's 64-bit sums (the lane's share) and to
+// the other particle's sums in memory.
+template <bool PRESS, int FORM>
 __device__ __forceinline__ void eval_pair(const DevState& d, const RepDev* R, const PairTables& T,
                                           PairI& I, int t, int dx, int dy, int dz) {
   float g[6];
-  if (!pair_terms<PRESS, true, FORM>(d, R, T, I, t, dx, dy, dz, g)) return;
+  if (!pair_terms<PRESS, FORM>(d, R, T, I, t, dx, dy, dz, g)) return;
   I.fx += fix_force(g[0]);
   I.fy += fix_force(g[1]);
   I.fz += fix_force(g[2]);
@@ -253,21 +247,16 @@ __device__ __forceinline__ void eval_pair(const DevState& d, const RepDev* R, co
     I.py += fix_force(g[4]);
     I.pz += fix_force(g[5]);
   }
-  if (OTHER) add_to_other<PRESS>(d, t, g);
+  add_to_other<PRESS>(d, t, g);
 }
 
-// The total of parts c over the LP lanes of group g (lanes LP g .. LP g + LP - 1).
+// A component's total over the lanes of its group that hold it (every fourth
+// lane of the LP).
 template <int LP>
-__device__ __forceinline__ long long group_total(const PartSums& P, int c, int g) {
-  constexpr int G = 32 / LP;
-  long long out = 0;
+__device__ __forceinline__ long long group_total(long long v) {
 #pragma unroll
-  for (int q = 0; q < G; q++) {
-    const int hi = __reduce_add_sync(0xffffffffu, g == q ? P.hi[c] : 0);
-    const int lo = __reduce_add_sync(0xffffffffu, g == q ? P.lo[c] : 0);
-    if (g == q) out = ((long long)hi << 21) + (long long)lo;
-  }
-  return out;
+  for (int o = 4; o < LP; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
 // Shared memory of pass 2 (dynamic, sized by the launch): per 128-row block
@@ -289,125 +278,97 @@ size_t force_smem_bytes(int fb) { return (size_t)fb * sizeof(ForceBlockSmem); }
 // Each pair is evaluated once, by the particle that owns it (owns()), and
 // its term goes to both particles (Newton's third law in exact fixed point: the
 // sums equal those of the reference's two evaluations up to the FP32
-// rounding of one of them). A warp takes the 32 particles of its chunk 32 / LP
+// rounding of one of them). A warp takes the particles of its chunk 32 / LP
 // at a time, LP lanes each, over their pass-1 lists (owned pairs only),
 // grouped by list length (the chunk sorted by length, neighbours in that
 // order share a warp) so that the groups run about as long; each lane reads
 // its next list entry one round ahead. The sums start at zero (launch_force)
-// and every term arrives by atomic add. A particle with a term outside the
-// 32-bit parts' range is summed again in 64 bits (its own side only). A
-// particle whose list overflowed is left to k_force_walk, so that this pass
-// keeps no walk state: no spills at 64 registers, and only the replica
-// tables in shared memory, which leaves the SM's L1 the room to cache the
-// other particles' rows (with the walk's 7.6 KB of shared memory per CTA in
+// and every term arrives by atomic add. A particle whose list overflowed is
+// left to k_force_walk, so that this pass keeps no walk state, and only the
+// replica tables in shared memory, which leaves the SM's L1 the room to cache
+// the other particles' rows (with the walk's 7.6 KB of shared memory per CTA in
 // the same kernel the pass took 1.15 ms instead of 1.08 on membrane_1m).
 // One launch per pair form present: a warp whose replica has another form
 // returns at once.
 //
-// Pass 2 over the rows s0 .. s0 + 31 of replica r (one warp's chunk), the
-// particles whose pass-1 list fit: G particles at a time, LP lanes each.
-template <int REACH, bool PRESS, int FORM, int LP>
-__device__ __forceinline__ void force_rows(const DevState& d, int s0, int r, const RepDev* R,
-                                           const PairTables& T, const OffTable& OT, int lane) {
+// What bounds it: instruction issue (70 % of the slots, ~340 instructions per 32
+// pairs) with the other particles' row loads behind it. The three adds to the other
+// particle bound it before: a lane that adds x, y and z of its own pair sends three
+// instructions of 32 scattered sectors each, which kept the L2's atomic unit 50 % and
+// L1 76 % busy. With the terms turned inside each quad of lanes (quad_components), one
+// instruction adds x, y and z of eight rows in eight sectors: a third of the sectors,
+// atomic unit 16 %, long-scoreboard stalls 4.3 -> 2.4 per issue, L1 hit rate 22 -> 39 %;
+// 984k-bead membrane 976 -> 836 us, 998k-particle liquid 248 -> 207 us. A register cap
+// of 72 or 92 instead of 64 (7 or 5 CTAs per SM) gave 852 and 935 us on that membrane.
+//
+// Pass 2 over the rows s0 .. s0 + rows - 1 of replica r (one warp's chunk, rows
+// <= 32), the particles whose pass-1 list fit: G particles at a time, LP lanes each.
+template <bool PRESS, int FORM, int LP>
+__device__ __forceinline__ void force_rows(const DevState& d, int s0, int rows, int r,
+                                           const RepDev* R, const PairTables& T,
+                                           const OffTable& OT, int lane) {
   constexpr int G = 32 / LP;  // particles per warp at a time
-  const int h = lane / LP, sl = lane % LP;
-  const int s_end = min(s0 + 32, R->row_off + R->n);
-  if (s0 >= s_end) return;
+  const int h = lane / LP, sl = lane % LP, c = lane & 3;
+  const int nrow = min(rows, R->row_off + R->n - s0);
+  if (nrow <= 0) return;
   PairI I;
   I.seed = R->seed + d.rep_time[r];
   constexpr uint32_t group_mask = LP == 32 ? 0xffffffffu : ((1u << LP) - 1u);
-  // the chunk's rows sorted by the length of their lists (rows past the end
-  // and overflowed lists count 0): key = length << 5 | row - s0
-  uint32_t key;
-  {
-    const int sk = s0 + lane;
-    const uint32_t c = sk < s_end ? (uint32_t)d.nbn[sk] : 0u;
-    key = ((c != kNbrFallback ? c : 0u) << 5) | (uint32_t)lane;
-    key = warp_sort_asc(key, lane);
+  // the chunk's rows sorted by the length of their lists (overflowed lists
+  // count 0, lanes without a row come last): key = length << 5 | row - s0
+  uint32_t key = 0xffffffffu;
+  if (lane < nrow) {
+    const uint32_t n = (uint32_t)d.nbn[s0 + lane];
+    key = ((n != kNbrFallback ? n : 0u) << 5) | (uint32_t)lane;
   }
-  for (int i2 = 0; i2 < 32; i2 += G) {
+  key = warp_sort_asc(key, lane);
+  for (int i2 = 0; i2 < nrow; i2 += G) {
     // ---- G particles, LP lanes each: the owned pairs of the lists
-    const int s2 = s0 + (int)(__shfl_sync(0xffffffffu, key, i2 + h) & 31u);
-    const bool act = s2 < s_end;
-    const int s = act ? s2 : s0;
+    const uint32_t ki = __shfl_sync(0xffffffffu, key, i2 + h);
+    const bool act = i2 + h < nrow;
+    const int s = act ? s0 + (int)(ki & 31u) : s0;
+    const int nu = act ? (int)(ki >> 5) : 0;
+    const int nmax = (int)(__shfl_sync(0xffffffffu, key, min(i2 + G, nrow) - 1) >> 5);
     load_row(I, d, s);
-    const uint32_t cnt = act ? (uint32_t)d.nbn[s] : 0u;
-    const int nu = cnt != kNbrFallback ? (int)cnt : 0;
     const uint32_t* list = d.nbl + (size_t)s * kNbrCap;
-    PartSums P;
-#pragma unroll
-    for (int c = 0; c < 6; c++) P.hi[c] = P.lo[c] = 0;
-    bool range = true;
-    uint32_t e_next = sl < nu ? __ldg(list + sl) : 0u;  // one round ahead
-    for (int k = sl; k < nu; k += LP) {
-      const uint32_t e = e_next;
+    long long F = 0, V = 0;
+    uint32_t e_next = sl < nu ? __ldg(list + sl) : make_entry(s, 0, 0, 0);  // one round ahead
+    for (int k0 = 0; k0 < nmax; k0 += LP) {
+      const int k = k0 + sl;
+      const bool valid = k < nu;
+      const uint32_t e = valid ? e_next : make_entry(s, 0, 0, 0);
       if (k + LP < nu) e_next = __ldg(list + k + LP);
       const int t = (int)(e & kRowMask);
-      owned_pair<PRESS, FORM>(d, R, T, OT, I, e, __ldg(d.posf + t), __ldg(d.velf + t),
-                              __ldg(d.densf + t), P, range);
-    }
-    __syncwarp();
-    const uint32_t bad = __ballot_sync(0xffffffffu, !range);
-    const bool ok = ((bad >> (LP * h)) & group_mask) == 0u;
-    {
-      const long long fx = group_total<LP>(P, 0, h), fy = group_total<LP>(P, 1, h),
-                      fz = group_total<LP>(P, 2, h);
-      long long px = 0, py = 0, pz = 0;
-      if (PRESS) {
-        px = group_total<LP>(P, 3, h);
-        py = group_total<LP>(P, 4, h);
-        pz = group_total<LP>(P, 5, h);
+      float ex, ey, ez;
+      const float an = owned_pair<PRESS, FORM>(d, R, T, OT, I, e, valid, __ldg(d.posf + t),
+                                        __ldg(d.velf + t), __ldg(d.densf + t), ex, ey, ez);
+      const float gx = an * ex, gy = an * ey, gz = an * ez;
+      int tq[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) tq[j] = __shfl_sync(0xffffffffu, t, j, 4);
+      const int lim = c < 3 ? nu - (k - c) : 0;
+      // |e| <= 1 up to rounding: below this no component reaches 65536
+      const bool big = __any_sync(0xffffffffu, !(fabsf(an) < 60000.0f));
+      float w[4];
+      quad_components(gx, gy, gz, c, w);
+      if (!big) {
+        quad_both<false, false>(w, tq, lim, d.fq + c, F);
+      } else {
+        if (!isfinite(an)) atomicCAS(d.err, 0, kErrNonFinite);
+        quad_both<false, true>(w, tq, lim, d.fq + c, F);
       }
-      if (sl == 0 && act && cnt != kNbrFallback && ok) {
-        long long* q = d.fq + 4 * (size_t)s;
-        red_add(q, fx);
-        red_add(q + 1, fy);
-        red_add(q + 2, fz);
-        if (PRESS) {
-          long long* pq = d.pq + 4 * (size_t)s;
-          red_add(pq, px);
-          red_add(pq + 1, py);
-          red_add(pq + 2, pz);
-        }
+      if (PRESS) {  // the virial a e e, the same for both particles
+        quad_components(-gx * ex, -gy * ey, -gz * ez, c, w);
+        if (!big)
+          quad_both<true, false>(w, tq, lim, d.pq + c, V);
+        else
+          quad_both<true, true>(w, tq, lim, d.pq + c, V);
       }
     }
-    // ---- a term outside the parts' range: the particle's own side again in
-    // 64 bits, one particle at a time, whole warp (the other particles'
-    // shares are already in memory)
-    uint32_t slow = __ballot_sync(0xffffffffu, sl == 0 && act && cnt != kNbrFallback && !ok);
-    while (slow) {
-      const int hs = (__ffs(slow) - 1) / LP;
-      slow &= slow - 1;
-      const int ss = __shfl_sync(0xffffffffu, s, LP * hs);
-      load_row(I, d, ss);
-      I.fx = I.fy = I.fz = I.px = I.py = I.pz = 0;
-      const uint32_t* l2 = d.nbl + (size_t)ss * kNbrCap;
-      const int n2 = (int)d.nbn[ss];
-      for (int k = lane; k < n2; k += 32) {
-        int t, dx, dy, dz;
-        read_entry(l2[k], t, dx, dy, dz);
-        eval_pair<PRESS, FORM, false>(d, R, T, I, t, dx, dy, dz);
-      }
-      const long long fx = warp_sum_ll(I.fx), fy = warp_sum_ll(I.fy), fz = warp_sum_ll(I.fz);
-      long long px = 0, py = 0, pz = 0;
-      if (PRESS) {
-        px = warp_sum_ll(I.px);
-        py = warp_sum_ll(I.py);
-        pz = warp_sum_ll(I.pz);
-      }
-      if (lane == 0) {
-        long long* q = d.fq + 4 * (size_t)ss;
-        red_add(q, fx);
-        red_add(q + 1, fy);
-        red_add(q + 2, fz);
-        if (PRESS) {
-          long long* pq = d.pq + 4 * (size_t)ss;
-          red_add(pq, px);
-          red_add(pq + 1, py);
-          red_add(pq + 2, pz);
-        }
-      }
-    }
+    F = group_total<LP>(F);
+    if (PRESS) V = group_total<LP>(V);
+    red_add_if(sl < 3 && nu > 0, d.fq + 4 * (size_t)s + c, F);
+    if (PRESS) red_add_if(sl < 3 && nu > 0, d.pq + 4 * (size_t)s + c, V);
   }
 }
 
@@ -484,7 +445,7 @@ __device__ __forceinline__ void force_walk_rows(const DevState& d, int kept, int
         if (qn >= 32) {
           __syncwarp();
           const PairCode pc = unpack_code(QC[lane]);
-          eval_pair<PRESS, FORM, true>(d, R, T, I, (int)QT[lane], pc.dx, pc.dy, pc.dz);
+          eval_pair<PRESS, FORM>(d, R, T, I, (int)QT[lane], pc.dx, pc.dy, pc.dz);
           __syncwarp();
           if (lane < qn - 32) {
             QT[lane] = QT[32 + lane];
@@ -498,7 +459,7 @@ __device__ __forceinline__ void force_walk_rows(const DevState& d, int kept, int
     __syncwarp();
     if (lane < qn) {
       const PairCode pc = unpack_code(QC[lane]);
-      eval_pair<PRESS, FORM, true>(d, R, T, I, (int)QT[lane], pc.dx, pc.dy, pc.dz);
+      eval_pair<PRESS, FORM>(d, R, T, I, (int)QT[lane], pc.dx, pc.dy, pc.dz);
     }
     __syncwarp();
     const long long fx = warp_sum_ll(I.fx), fy = warp_sum_ll(I.fy), fz = warp_sum_ll(I.fz);
@@ -527,8 +488,8 @@ __device__ __forceinline__ void force_walk_rows(const DevState& d, int kept, int
 // per 32-row chunk. Its shared memory is the replica tables only (1.2 KB per
 // row block), which leaves most of the SM's 256 KB of L1 and shared memory
 // to the L1 that caches the other particles' rows.
-template <int REACH, bool PRESS, int FORM, int LP>
-__global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk) {
+template <bool PRESS, int FORM, int LP>
+__global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk, int rows) {
   extern __shared__ __align__(16) unsigned char force_smem[];
   ForceBlockSmem* BS = reinterpret_cast<ForceBlockSmem*>(force_smem);
   const int fb = blockDim.x >> 7;  // 128-row blocks of this CTA
@@ -544,8 +505,8 @@ __global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk) {
   }
   __syncthreads();
   if (rb >= nblk || R->form != FORM) return;
-  force_rows<REACH, PRESS, FORM, LP>(d, d.blk_row[rb] + 32 * (wid % kWarps), r, R, BS[rbl].T,
-                                     BS[rbl].OT, lane);
+  force_rows<PRESS, FORM, LP>(d, d.blk_row[rb] + 32 * (wid % kWarps) + rows * blockIdx.y,
+                                     rows, r, R, BS[rbl].T, BS[rbl].OT, lane);
 }
 
 // Pass 2 of the particles whose list overflowed (force_walk_rows), one warp
@@ -565,13 +526,35 @@ __global__ void __launch_bounds__(kRowBlock) k_force_walk(DevState d, int kept, 
   force_walk_rows<REACH, PRESS, FORM>(d, kept, d.blk_row[rb] + 32 * wid, r, R, B.T, W[wid], lane);
 }
 
+// Rows of one warp's chunk (32 at most, at least one group of 32 / LP). Whole
+// 128-row blocks per CTA of 32-row warps leave a small system on a few SMs, and a
+// mid-sized one with a last wave that runs as long as its longest lists, so the chunk
+// is halved while the launch has fewer than kForceWarps warps (five waves of the 4,864
+// a GB300 holds at 64 registers), but not below two groups, whose setup (the sort of
+// the rows, the tables) is then a large part of the warp's work, unless even one wave
+// is not full. Measured at 32 / 16 / 8 / 4 / 2 rows: membranes at 16 lanes, 984k beads
+// 888 / 880 / 900 / 968 / 1098 us, 250k 283 / 254 / 247 / 254 / 274, 131k 168 / 157 /
+// 145 / 143 / 154, 62k 117 / 87 / 85 / 80 / 82, 8k 98 / 59 / 39 / 28 / 27; liquids at 4
+// lanes (32 / 16 / 8 rows), 998k 213 / 227 / 266, 200k 59 / 57 / 61, 24k 24 / 20 / 18.
+constexpr int kForceWarps = 24000, kWaveWarps = 4864;
+static int force_chunk_rows(int nblk, int lp) {
+  const int g = 32 / lp;
+  const long long n = (long long)nblk * kRowBlock;
+  int rows = 32;
+  while (rows > 2 * g && n < (long long)rows * kForceWarps) rows >>= 1;
+  if (rows == 2 * g && n < (long long)rows * kWaveWarps) rows = g;
+  return rows;
+}
+
 // Pass 2 of one pair form: the shape of the tuning (lanes per particle,
 // row blocks per CTA); the observation steps (PRESS) run 16 lanes, one row
 // block per CTA.
 template <int REACH, int FORM, bool PRESS, int LP>
 void launch_force_kernel(const DevState& d, int nblk, int kept, int fb, cudaStream_t st) {
-  k_force_f32<REACH, PRESS, FORM, LP>
-      <<<(nblk + fb - 1) / fb, kRowBlock * fb, force_smem_bytes(fb), st>>>(d, nblk);
+  const int rows = force_chunk_rows(nblk, LP);
+  k_force_f32<PRESS, FORM, LP>
+      <<<dim3((nblk + fb - 1) / fb, 32 / rows), kRowBlock * fb, force_smem_bytes(fb), st>>>(d, nblk,
+                                                                                        rows);
   k_force_walk<REACH, PRESS, FORM><<<nblk, kRowBlock, 0, st>>>(d, kept, nblk);
 }
 

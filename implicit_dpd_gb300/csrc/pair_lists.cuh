@@ -208,20 +208,17 @@ __device__ __forceinline__ void red_add(long long* p, long long v) {
   atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
 }
 
-// 16-byte asynchronous copy global -> shared (cp.async, kept in L1 and L2),
-// and its group commit / wait: a lane's copies of one round form one group.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+// The same where the predicate holds, without a branch.
+__device__ __forceinline__ void red_add_if(bool p, long long* a, long long v) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p red.global.add.u64 [%0], %1;\n}\n"
+               ::"l"(a), "l"(v), "r"((int)p) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_prev() {  // all groups but the newest done
-  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+
+// a b + c in 64 bits.
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
 }
 
 }  // namespace idpd

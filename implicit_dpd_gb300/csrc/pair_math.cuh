@@ -10,7 +10,7 @@ namespace idpd {
 // mantissa of 1 + w * pre (w * pre in [0, 1]).
 __device__ __forceinline__ uint32_t dens_weight(float dr2, bool warren, float inv_rd, float wnorm,
                                                 float pre) {
-  const float dr = dr2 * rsqrtf(dr2);
+  const float dr = dr2 * rsqrt_approx(dr2);
   float w = warren ? 1.0f - dr * inv_rd : 1.0f - dr;
   w = warren ? wnorm * (w * w) : w * w;
   return (uint32_t)(__float_as_int(fmaf(w, pre, 1.0f)) - 0x3f800000);
@@ -29,15 +29,22 @@ __host__ __device__ __forceinline__ void fill_pair_table(PairTables& T, const Re
   T.b[k] = make_float2(R.cf_m[3 * k + 1], R.cf_m[3 * k + 2]);
 }
 
+// Squared length, the products and sums rounded in one fixed order (written
+// out, so that every kernel that takes a pair gets the same bits).
+__device__ __forceinline__ float dist2(float ex, float ey, float ez) {
+  return fmaf(ez, ez, fmaf(ex, ex, __fmul_rn(ey, ey)));
+}
+
 // Conservative + random + dissipative magnitude over dr for one pair
 // (nbdf_calculator.hpp:108-132), FP32, for the pair-force form FORM. dr, 1/dr
-// and w = 1 - dr are passed in.
-template <int FORM>
+// and w = 1 - dr are passed in. YFIRST: the order in which e . dv is rounded
+// (the passes that also sum the virial round the y product first).
+template <int FORM, bool YFIRST>
 __device__ __forceinline__ float pair_cf(const PairTables& T, const RepDev* R, uint32_t pri,
                                          uint32_t prj, float dr, float inv_dr, float w, float ex,
                                          float ey, float ez, float4 vi, float4 vj, float4 di,
                                          float4 dj, uint32_t idi, uint32_t idj, uint32_t seed) {
-  const float sqw = w > 0.0f ? w * rsqrtf(w) : 0.0f;  // sqrt(1 - r), 2 ulp
+  const float sqw = w > 0.0f ? w * rsqrt_approx(w) : 0.0f;  // sqrt(1 - r), 2 ulp
   const int k = pri * 3 + prj;
   const float4 ta = T.a[k];
   float cons;
@@ -55,7 +62,9 @@ __device__ __forceinline__ float pair_cf(const PairTables& T, const RepDev* R, u
   }
   Saru sr(idi < idj ? idi : idj, idi < idj ? idj : idi, seed);
   const float rnd = saru_nrml_f32(sr);
-  const float ddv = ex * (vi.x - vj.x) + ey * (vi.y - vj.y) + ez * (vi.z - vj.z);
+  const float dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
+  const float ddv = fmaf(ez, dvz, YFIRST ? fmaf(ex, dvx, __fmul_rn(ey, dvy))
+                                         : fmaf(ey, dvy, __fmul_rn(ex, dvx)));
   return (cons + ta.y * sqw * rnd - ta.z * w * ddv * inv_dr) * inv_dr;
 }
 
@@ -66,12 +75,12 @@ __device__ __forceinline__ float pair_all_cf(const PairTables& T, const RepDev* 
                                              float4 vj, float4 di, float4 dj, uint32_t idi,
                                              uint32_t idj, uint32_t seed) {
   if (form == IDPD_FORM_PAIRWISE_K)
-    return pair_cf<IDPD_FORM_PAIRWISE_K>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di,
+    return pair_cf<IDPD_FORM_PAIRWISE_K, true>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di,
                                          dj, idi, idj, seed);
   if (form == IDPD_FORM_WARREN_K)
-    return pair_cf<IDPD_FORM_WARREN_K>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di, dj,
+    return pair_cf<IDPD_FORM_WARREN_K, true>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di, dj,
                                        idi, idj, seed);
-  return pair_cf<IDPD_FORM_MDPD_K>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di, dj, idi,
+  return pair_cf<IDPD_FORM_MDPD_K, true>(T, R, pri, prj, dr, inv_dr, w, ex, ey, ez, vi, vj, di, dj, idi,
                                    idj, seed);
 }
 
