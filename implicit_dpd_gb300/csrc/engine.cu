@@ -320,6 +320,7 @@ int ensure_capacity(idpd_handle* h, int rows, int ncell, int nblk, int namp) {
   AL(d.fq, 4 * (size_t)cap);
   AL(d.nbl, (size_t)kNbrCap * cap); AL(d.nbn, cap);
   AL(d.dsum, 4 * (size_t)cap);
+  d.dstride = (size_t)cap;
   AL(d.topol, 4 * ac);
   AL(d.cf_bend, ac);
   AL(d.reps, h->R);
@@ -767,7 +768,7 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
     end_if(h, c);
     launch_pack(d, h->nblk, h->st, gate);  // every step: the positions changed
     c = begin_if(h, rebuild);
-    launch_verlet_build(d, h->nblk, h->tune.reach, c.st);
+    launch_verlet_build(d, h->nblk, c.st);
     end_if(h, c);
   } else {
     launch_drift_bin(d, h->nblk, true, h->st);
@@ -776,7 +777,8 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
     launch_scatter_sort_pack(d, h->nblk, h->ncell_tot, true, h->st);
   }
   const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
-  launch_density(d, h->nblk, mode, h->tune.reach, verlet, marks, h->cap, h->st, h->tune.dlanes);
+  launch_density(d, h->nblk, mode, h->tune.reach, verlet, marks, h->cap,
+                 form_mask(h), h->st, h->tune.dlanes);
   launch_force(d, h->nblk, mode, observe, verlet, h->tune, form_mask(h), h->cap, h->st);
   if (h->prec_any) {
     d.prec_count = h->prec_dev;
@@ -1346,7 +1348,8 @@ int idpd_density(idpd_handle* h) {
   if (rc) return rc;
   if ((rc = ensure_aux(h))) return rc;
   enqueue_cells(h, false);
-  launch_density(h->d, h->nblk, pair_mode(h), h->tune.reach, false, false, h->cap, h->st);
+  launch_density(h->d, h->nblk, pair_mode(h), h->tune.reach, false, false, h->cap,
+                 form_mask(h), h->st);
   launch_com(h->d, h->nblk, h->cm64, h->cm_cnt, h->st);
   h->density_valid = true;
   h->pairs_valid = true;
@@ -1803,10 +1806,11 @@ int idpd_profile_step(idpd_handle* h, char* names, size_t names_len, float* ms, 
   CK(cudaEventRecord(ev[2], h->st));
   launch_scatter_sort_pack(d, h->nblk, h->ncell_tot, true, h->st, gate);
   CK(cudaEventRecord(ev[3], h->st));
-  if (verlet) launch_verlet_build(d, h->nblk, h->tune.reach, h->st);
+  if (verlet) launch_verlet_build(d, h->nblk, h->st);
   CK(cudaEventRecord(ev[4], h->st));
   h->pairs_valid = true;
-  launch_density(d, h->nblk, mode, h->tune.reach, verlet, false, h->cap, h->st, h->tune.dlanes);
+  launch_density(d, h->nblk, mode, h->tune.reach, verlet, false, h->cap, form_mask(h), h->st,
+                 h->tune.dlanes);
   CK(cudaEventRecord(ev[5], h->st));
   launch_force(d, h->nblk, mode, false, verlet, h->tune, form_mask(h), h->cap, h->st);
   CK(cudaEventRecord(ev[6], h->st));

@@ -76,21 +76,6 @@ __device__ __forceinline__ void load_row(PairI& I, const DevState& d, int s) {
   I.pri = fbits(I.pi.w);
 }
 
-// Frame-cell offsets (dx cs_x, dy cs_y, dz cs_z) of the 64 codes of a list
-// entry's top bits (dx + 1 | (dy + 1) << 2 | (dz + 1) << 4): one shared load
-// gives the shift of the other particle's cell-local coordinates. Each
-// product is exact (dx in {-1, 0, 1}), so (x_i - off) - x_j rounds as the
-// fused x_i - dx cs - x_j does.
-struct OffTable {
-  float4 o[64];
-};
-
-__device__ __forceinline__ void fill_off_table(OffTable& T, const RepDev& R, int c) {
-  const float dx = (float)((c & 3) - 1), dy = (float)(((c >> 2) & 3) - 1),
-              dz = (float)(((c >> 4) & 3) - 1);
-  T.o[c] = make_float4(dx * R.cs_f[0], dy * R.cs_f[1], dz * R.cs_f[2], 0.0f);
-}
-
 // The terms of the four pairs of a quad of lanes (4 q .. 4 q + 3, one particle's)
 // turned from one pair per lane to one component per lane: on return w[j] of
 // lane 4 q + c is component c (x, y, z; nothing for c = 3) of lane 4 q + j's pair.
@@ -526,32 +511,12 @@ __global__ void __launch_bounds__(kRowBlock) k_force_walk(DevState d, int kept, 
   force_walk_rows<REACH, PRESS, FORM>(d, kept, d.blk_row[rb] + 32 * wid, r, R, B.T, W[wid], lane);
 }
 
-// Rows of one warp's chunk (32 at most, at least one group of 32 / LP). Whole
-// 128-row blocks per CTA of 32-row warps leave a small system on a few SMs, and a
-// mid-sized one with a last wave that runs as long as its longest lists, so the chunk
-// is halved while the launch has fewer than kForceWarps warps (five waves of the 4,864
-// a GB300 holds at 64 registers), but not below two groups, whose setup (the sort of
-// the rows, the tables) is then a large part of the warp's work, unless even one wave
-// is not full. Measured at 32 / 16 / 8 / 4 / 2 rows: membranes at 16 lanes, 984k beads
-// 888 / 880 / 900 / 968 / 1098 us, 250k 283 / 254 / 247 / 254 / 274, 131k 168 / 157 /
-// 145 / 143 / 154, 62k 117 / 87 / 85 / 80 / 82, 8k 98 / 59 / 39 / 28 / 27; liquids at 4
-// lanes (32 / 16 / 8 rows), 998k 213 / 227 / 266, 200k 59 / 57 / 61, 24k 24 / 20 / 18.
-constexpr int kForceWarps = 24000, kWaveWarps = 4864;
-static int force_chunk_rows(int nblk, int lp) {
-  const int g = 32 / lp;
-  const long long n = (long long)nblk * kRowBlock;
-  int rows = 32;
-  while (rows > 2 * g && n < (long long)rows * kForceWarps) rows >>= 1;
-  if (rows == 2 * g && n < (long long)rows * kWaveWarps) rows = g;
-  return rows;
-}
-
 // Pass 2 of one pair form: the shape of the tuning (lanes per particle,
 // row blocks per CTA); the observation steps (PRESS) run 16 lanes, one row
 // block per CTA.
 template <int REACH, int FORM, bool PRESS, int LP>
 void launch_force_kernel(const DevState& d, int nblk, int kept, int fb, cudaStream_t st) {
-  const int rows = force_chunk_rows(nblk, LP);
+  const int rows = chunk_rows(nblk, LP);
   k_force_f32<PRESS, FORM, LP>
       <<<dim3((nblk + fb - 1) / fb, 32 / rows), kRowBlock * fb, force_smem_bytes(fb), st>>>(d, nblk,
                                                                                         rows);

@@ -3,11 +3,7 @@
 //   pass 2, CalcForceEpEpDPD::operator() (nbdf_calculator.hpp:63-145).
 //
 // FP32 passes (the engine): each pair is taken once, by the particle that
-// owns it (owns()), and its term goes to both particles. Pass 1 runs one warp
-// per particle over its kept list or its cells (the neighbour-cell segments
-// cached in shared memory, swept 32 candidates at a time with coalesced
-// float4 loads) and writes the owned pairs within the cutoff as the list of
-// pass 2, which runs two particles per warp, 16 lanes each. Pair vectors come
+// owns it (owns()), and its term goes to both particles. Pair vectors come
 // from cell-local FP32 coordinates; cutoff decisions within kGuard of the
 // cutoff are re-taken in FP64 from the FP64 positions as the reference takes
 // them; pairs within 0.01 of the cutoff take 1 - r from the compensated
@@ -17,39 +13,154 @@
 //
 // FP64 passes (the plain single-system baseline): one thread per particle,
 // FP64 throughout, FP64 sums in cell order.
+#include <algorithm>
+
 #include "pair_lists.cuh"
 
 namespace idpd {
 
-// One warp per particle, over the pairs it owns (owns(); the other particle
-// gets the same weight by atomic add). Without kept lists: phase A sweeps the
-// neighbour segments 32 candidates at a time and appends the owned pairs
-// within the cutoff 1 to a list in shared memory; phase B takes the density
-// weights from that list with every lane busy and copies the list out for
-// pass 2 (a particle whose list overflows takes its weights during a second
-// sweep). With kept lists (VERLET, owned candidates only): one pass over the
-// particle's kept list tests each candidate, adds its weight and appends it
-// to the list of pass 2. Each particle's own total is added to its sums in
-// dsum as well; k_dens_finalize turns them into the FP32 densities.
-// With MARKS, the precursor conversion's marks (phit): a pair of prop_from
-// and prop_near within the cutoff marks the prop_from particle.
+// ------------------------------------------------------------- pass 1
+// Two kernels. k_pair_build finds each particle's owned candidates (owns()) from the
+// cells: the kept lists on rebuild steps, or, without kept lists, on every step the
+// owned pairs within the cutoff themselves, straight into the lists of pass 2.
+// k_density_list goes over those lists: it takes each pair's density weight to both
+// particles and, over kept lists, tests each candidate and writes the pairs within the
+// cutoff as the list of pass 2. k_dens_finalize turns the fixed-point sums into the
+// FP32 densities. The rows whose list overflowed are swept by k_density_over.
+
+// The lists' densities, LP lanes per particle (LP 4, 8, 16 or 32). The warp sorts the
+// rows of its chunk by list length and takes them 32 / LP at a time, so that short
+// lists (a liquid at density 6 keeps ~20 owned candidates per particle) do not leave
+// lanes idle and neighbours in that order run about as long; every LP gives the same
+// densities and pass-2 lists bit for bit. KNOWN: the lists hold the pairs within the
+// cutoff 1 already (pass 2's own, no kept lists). MARKS: the precursor conversion's
+// marks (phit): a pair of prop_from and prop_near within the cutoff marks the
+// prop_from particle. Rows whose list overflowed are left to k_density_over; a replica
+// of another form (WARREN or not) to the other launch.
 //
-// Three forms (MODE): kDensSweep sweeps the cells of every row (no kept
-// lists); kDensKept takes the rows whose kept list fit and uses no shared
-// memory, which leaves the SM's L1 the room to cache the candidates' rows;
-// kDensKeptOver takes the rows whose kept list did not fit and sweeps their
-// cells (the ownership of the kept lists). The two kept-list forms run one
-// after the other (with the sweep's 13.8 KB of shared memory per CTA in the
-// kept-list kernel, pass 1 took 0.70 ms instead of 0.65 on membrane_1m). The sweeping forms keep per warp the neighbour segments
-// and a list buffer in dynamic shared memory (dens_sweep_smem_bytes).
-enum { kDensSweep = 0, kDensKept = 1, kDensKeptOver = 2 };
+// What bounds it: instruction issue and the latency of the candidates' rows. The sums
+// lie per property, so that the weights a group's lanes send to neighbouring rows share
+// 32-byte sectors (one sector of four sums per row before, the SM's request port 50 %
+// busy); frame offsets come from a table, the form is a template argument and a lane
+// without a candidate needs no test of its own. 984k-bead membrane (8 lanes) 510 -> 407
+// us, 998k-particle liquid (4 lanes) 197 -> 173 us.
+template <bool MARKS, bool WARREN, bool KNOWN, int LP>
+__global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int rows) {
+  constexpr int G = 32 / LP;  // particles per warp at a time
+  __shared__ OffTable OT;
+  const int r = d.blk_rep[blockIdx.x];
+  const RepDev* R = d.reps + r;
+  if ((R->form == IDPD_FORM_WARREN_K) != WARREN) return;
+  if (threadIdx.x < 64) fill_off_table(OT, *R, threadIdx.x);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int h = lane / LP, sl = lane % LP;
+  const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
+  const int nrow = min(rows, R->row_off + R->n - s0);
+  if (nrow <= 0) return;
+  const float cutd2 = WARREN ? R->wrd * R->wrd : 1.0f;  // density cutoff^2
+  const float inv_rd = R->winv_rd, wnorm = R->wnorm, pre = R->dens_prescale;
+  const bool prec = MARKS && R->prec_on;
+  const uint32_t gmask = (LP == 32 ? 0xffffffffu : ((1u << LP) - 1u)) << (LP * h);
+  const uint32_t group_lt = ((1u << lane) - 1u) & gmask;
+  const uint16_t* len = KNOWN ? d.nbn : d.vn;
+  // the chunk's rows sorted by list length, those without one (overflowed, or past the
+  // end) last: key = length << 5 | row - s0
+  uint32_t key = 0xffffffffu;
+  if (lane < nrow) {
+    const uint32_t n = (uint32_t)len[s0 + lane];
+    if (n != kNbrFallback) key = (n << 5) | (uint32_t)lane;
+  }
+  const int nact = __popc(__ballot_sync(0xffffffffu, key != 0xffffffffu));
+  key = warp_sort_asc(key, lane);
+  for (int i2 = 0; i2 < nact; i2 += G) {
+    const uint32_t ki = __shfl_sync(0xffffffffu, key, i2 + h);
+    const bool act = i2 + h < nact;
+    const int s = act ? s0 + (int)(ki & 31u) : s0;
+    const int nv = act ? (int)(ki >> 5) : 0;
+    const int nmax = (int)(__shfl_sync(0xffffffffu, key, min(i2 + G, nact) - 1) >> 5);
+    const float4 pi = d.posf[s];
+    const uint32_t pri = fbits(pi.w);
+    const uint32_t none = (uint32_t)s | (kOffNone << kRowBits);
+    unsigned long long* other = d.dsum + (pri & 3u) * d.dstride;
+    int nl = 0;  // owned pairs within the cutoff
+    bool hit = false;
+    uint32_t q0 = 0, q1 = 0, q2 = 0;
+    const uint32_t* list = KNOWN ? d.nbl + (size_t)s * kNbrCap : d.vl + (size_t)s * kVerletCap;
+    uint32_t* out = d.nbl + (size_t)s * kNbrCap;
+    uint32_t e_next = sl < nv ? list[sl] : none;  // one round ahead
+    for (int k0 = 0; k0 < nmax; k0 += LP) {
+      const uint32_t e = e_next;
+      e_next = k0 + LP + sl < nv ? list[k0 + LP + sl] : none;
+      const int t = (int)(e & kRowMask);
+      const float4 pj = __ldg(d.posf + t);
+      const float4 o = OT.o[e >> kRowBits];  // far away on a lane without a candidate
+      const float dr2 = dist2((pi.x - o.x) - pj.x, (pi.y - o.y) - pj.y, (pi.z - o.z) - pj.z);
+      bool in1 = dr2 < (KNOWN ? 4.0f : 1.0f);
+      bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
+      const bool near1 = !KNOWN && fabsf(dr2 - 1.0f) <= kGuard;
+      const bool near2 = dr2 < 1.0e-10f || (WARREN && fabsf(dr2 - cutd2) <= kGuard);
+      // rare: the FP64 decisions of the reference near the cutoffs and at
+      // coincident positions
+      if (__any_sync(0xffffffffu, near1 || near2)) {
+        if (near1 || near2) {
+          const double e2 = exact_dr2(d, R, d.perm[s], d.perm[t]);
+          const double cutd2d = WARREN ? (double)R->wrd * (double)R->wrd : 1.0;
+          if (near1) in1 = e2 < 1.0;
+          ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
+        }
+      }
+      const uint32_t prj = fbits(pj.w);
+      const uint32_t w = ind ? dens_weight(dr2, WARREN, inv_rd, wnorm, pre) : 0u;
+      add_weight(q0, q1, q2, prj, w);
+      red_add_if(ind, reinterpret_cast<long long*>(other + t), (long long)w);
+      if (MARKS && prec && in1) {
+        hit |= pri == R->prec_from && prj == R->prec_near;
+        if (prj == R->prec_from && pri == R->prec_near) d.phit[t] = 1;
+      }
+      if (!KNOWN) {
+        const uint32_t mask = __ballot_sync(0xffffffffu, in1);
+        const int pos = nl + __popc(mask & group_lt);
+        if (in1 && pos < kNbrCap) out[pos] = e;
+        nl += __popc(mask & gmask);
+      }
+    }
+    if (KNOWN) nl = nv;
+    // the totals of each group's lanes: a list holds at most 512 entries and each
+    // weight is below 2^23, so a total is below 2^32
+#pragma unroll
+    for (int o = 1; o < LP; o <<= 1) {
+      q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+      q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+      q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    }
+    const uint32_t q = sl == 0 ? q0 : (sl == 1 ? q1 : q2);
+    red_add_if(act && sl < 3 && q != 0u,
+               reinterpret_cast<long long*>(d.dsum + (sl < 3 ? sl : 0) * d.dstride + s), (long long)q);
+    if (MARKS) hit = (__ballot_sync(0xffffffffu, hit) & gmask) != 0u;
+    if (sl == 0 && act) {
+      if (!KNOWN) d.nbn[s] = nl <= kNbrCap ? (uint16_t)nl : (uint16_t)kNbrFallback;
+      d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
+      if (MARKS && hit) d.phit[s] = 1;
+    }
+  }
+}
+static_assert((long long)kVerletCap * (1ll << 23) <= (1ll << 32) &&
+              (long long)kNbrCap * (1ll << 23) <= (1ll << 32), "32-bit totals of pass 1");
+
+// Pass 1 of the rows whose list overflowed (VERLET: the kept list, with the ownership
+// of its build; else the pass-2 list), one warp per 32-row chunk, a row at a time:
+// phase A sweeps the neighbour segments 32 candidates at a time and appends the owned
+// pairs within the cutoff 1 to a list in shared memory; phase B takes the density
+// weights from that list with every lane busy and copies the list out for pass 2 (a
+// particle whose list overflows takes its weights during a second sweep). Shared
+// memory: per warp the neighbour segments and the list (dens_sweep_smem_bytes).
 constexpr size_t dens_sweep_smem_bytes() {
   return kWarps * (sizeof(SegTable) + kNbrCap * sizeof(uint32_t));
 }
 
-template <int REACH, int MODE, bool MARKS>
-__global__ void __launch_bounds__(kRowBlock, (MODE != kDensSweep && (REACH == 2 || MARKS)) ? 8 : 10) k_density_f32(DevState d) {
-  constexpr bool VERLET = MODE != kDensSweep;
+template <int REACH, bool VERLET, bool MARKS>
+__global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d) {
   extern __shared__ __align__(16) unsigned char dens_smem[];
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
@@ -58,6 +169,8 @@ __global__ void __launch_bounds__(kRowBlock, (MODE != kDensSweep && (REACH == 2 
   uint32_t* L = reinterpret_cast<uint32_t*>(dens_smem + kWarps * sizeof(SegTable)) + wid * kNbrCap;
   const int s0 = d.blk_row[blockIdx.x] + 32 * wid;
   const int s_end = min(s0 + 32, R->row_off + R->n);
+  const uint16_t* len = VERLET ? d.vn : d.nbn;
+  uint32_t todo = __ballot_sync(0xffffffffu, s0 + lane < s_end && len[s0 + lane] == kNbrFallback);
   const bool warren = R->form == IDPD_FORM_WARREN_K;
   const float cutd2 = R->wrd * R->wrd;  // density cutoff^2 (1 unless Warren)
   const double cutd2d = (double)R->wrd * (double)R->wrd;
@@ -67,29 +180,26 @@ __global__ void __launch_bounds__(kRowBlock, (MODE != kDensSweep && (REACH == 2 
   constexpr int nseg = 2 * (2 * REACH + 1) * (2 * REACH + 1);
   const uint32_t lt_mask = (1u << lane) - 1u;
   int cached = -1;
-  auto row = [&](const int s) {
+  for (; todo; todo &= todo - 1) {
+    const int s = s0 + __ffs(todo) - 1;
     const float4 pi = d.posf[s];
     const uint32_t si = d.perm[s], pri = fbits(pi.w);
     const float ki = VERLET ? d.okey[s] : pi.x;  // the ownership key of the step
     int nl = 0;  // owned pairs within the cutoff
-    int nw = 0;  // bound on the weighted pairs
     bool hit = false;
     uint32_t q0 = 0, q1 = 0, q2 = 0;
     // weight of one owned candidate, to both particles; called by every lane
     // together (valid = false for lanes without one) so that the rare FP64
-    // recheck is warp-uniform. Returns whether the pair lies within the cutoff 1.
+    // recheck is warp-uniform
     auto test = [&](bool valid, int t, int dx, int dy, int dz, float4 pj, bool list_known) {
       const float ex = (pi.x - (float)dx * csx) - pj.x;
       const float ey = (pi.y - (float)dy * csy) - pj.y;
       const float ez = (pi.z - (float)dz * csz) - pj.z;
-      const float dr2 = ex * ex + ey * ey + ez * ez;
+      const float dr2 = dist2(ex, ey, ez);
       bool in1 = valid && (list_known || dr2 < 1.0f);
       bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
       const bool near1 = valid && !list_known && fabsf(dr2 - 1.0f) <= kGuard;
       const bool near2 = valid && ((warren && fabsf(dr2 - cutd2) <= kGuard) || dr2 < 1.0e-10f);
-      // rare: the FP64 decisions of the reference near the cutoffs and at
-      // coincident positions (a warp-uniform branch keeps them out of the
-      // common path)
       if (__any_sync(0xffffffffu, near1 || near2)) {
         if (near1 || near2) {
           const double e2 = exact_dr2(d, R, si, d.perm[t]);
@@ -101,52 +211,72 @@ __global__ void __launch_bounds__(kRowBlock, (MODE != kDensSweep && (REACH == 2 
       if (ind) {
         const uint32_t w = dens_weight(dr2, warren, inv_rd, wnorm, pre);
         add_weight(q0, q1, q2, prj, w);
-        atomicAdd(d.dsum + 4 * (size_t)t + (pri & 3u), (unsigned long long)w);
+        atomicAdd(d.dsum + (pri & 3u) * d.dstride + t, (unsigned long long)w);
       }
       if (MARKS && prec && in1) {
         hit |= pri == R->prec_from && prj == R->prec_near;
         if (prj == R->prec_from && pri == R->prec_near) d.phit[t] = 1;
       }
-      return in1;
     };
-    const uint32_t nv = VERLET ? (uint32_t)d.vn[s] : kNbrFallback;
-    bool fits = true;
-    bool swept = true;  // the pairs came from a sweep of the cells (list out below)
-    if constexpr (MODE == kDensKept) {
-      // ---- the particle's kept list: test, weight and list out in one pass
-      swept = false;
-      const uint32_t* vl = d.vl + (size_t)s * kVerletCap;
-      uint32_t* out = d.nbl + (size_t)s * kNbrCap;
-      uint32_t e_next = lane < (int)nv ? vl[lane] : 0u;  // one round ahead
-      for (int k0 = 0; k0 < (int)nv; k0 += 32) {
-        const int k = k0 + lane;
-        const bool valid = k < (int)nv;
-        const uint32_t e = e_next;
-        if (k + 32 < (int)nv) e_next = vl[k + 32];
-        int t, dx, dy, dz;
-        read_entry(e, t, dx, dy, dz);
-        if (!valid) t = s;
-        const bool in1 = test(valid, t, dx, dy, dz, __ldg(d.posf + t), false);
+    const int cell = (int)d.scell[s];
+    if (cell != cached) {
+      int cx, cy, cz;
+      cell_xyz(cell - R->cell_off, R->nc, cx, cy, cz);
+      __syncwarp();
+      build_segments(S, d, R, cx, cy, cz, lane);
+      __syncwarp();
+      cached = cell;
+    }
+    // ---- phase A: the owned pairs within the cutoff 1
+#pragma unroll 1
+    for (int g = 0; g < nseg; g++) {
+      const int tb = S.tb[g], te = S.te[g];
+      if (tb >= te) continue;
+      const int code = S.code[g];
+      int b[2 * REACH];
+#pragma unroll
+      for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
+      const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
+      const float by = pi.y - (float)dy * csy, bz = pi.z - (float)dz * csz;
+      for (int t0 = tb; t0 < te; t0 += 32) {
+        const int t = t0 + lane;
+        bool in1 = false, near = false;
+        int ddx = 0;
+        if (t < te && t != s) {
+          const float4 pj = __ldg(d.posf + t);
+          ddx = frame_step<REACH>(t, b);
+          if (owns(fx0 + ddx, VERLET ? d.okey[t] : pj.x, ki, t, s)) {
+            const float dr2 =
+                dist2((pi.x - (float)(fx0 + ddx) * csx) - pj.x, by - pj.y, bz - pj.z);
+            in1 = dr2 < 1.0f;
+            near = fabsf(dr2 - 1.0f) <= kGuard;
+          }
+        }
+        if (__any_sync(0xffffffffu, near)) {
+          if (near) in1 = exact_dr2(d, R, si, d.perm[t]) < 1.0;
+        }
         const uint32_t mask = __ballot_sync(0xffffffffu, in1);
         if (in1) {
           const int pos = nl + __popc(mask & lt_mask);
-          if (pos < kNbrCap) out[pos] = e;
+          if (pos < kNbrCap) L[pos] = make_entry(t, fx0 + ddx, dy, dz);
         }
         nl += __popc(mask);
       }
-      nw = (int)nv;
-      fits = nl <= kNbrCap;
-    } else {
-      const int cell = (int)d.scell[s];
-      if (cell != cached) {
-        int cx, cy, cz;
-        cell_xyz(cell - R->cell_off, R->nc, cx, cy, cz);
-        __syncwarp();
-        build_segments(S, d, R, cx, cy, cz, lane);
-        __syncwarp();
-        cached = cell;
+    }
+    __syncwarp();
+    const bool fits = nl <= kNbrCap;
+    // ---- phase B: density weights
+    if (fits) {
+      for (int k0 = 0; k0 < nl; k0 += 32) {
+        const int k = k0 + lane;
+        const bool valid = k < nl;
+        int t = s, dx = 0, dy = 0, dz = 0;
+        if (valid) read_entry(L[k], t, dx, dy, dz);
+        test(valid, t, dx, dy, dz, valid ? __ldg(d.posf + t) : pi, true);
       }
-      // ---- phase A: the owned pairs within the cutoff 1
+    } else {
+      // a lane takes at most nseg + nl / 32 weights below 2^23 each
+      if (nl > kDensPairsMax && lane == 0) atomicCAS(d.err, 0, kErrDensPairs);
 #pragma unroll 1
       for (int g = 0; g < nseg; g++) {
         const int tb = S.tb[g], te = S.te[g];
@@ -156,240 +286,39 @@ __global__ void __launch_bounds__(kRowBlock, (MODE != kDensSweep && (REACH == 2 
 #pragma unroll
         for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
         const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
-        const float by = pi.y - (float)dy * csy, bz = pi.z - (float)dz * csz;
         for (int t0 = tb; t0 < te; t0 += 32) {
           const int t = t0 + lane;
-          bool in1 = false, near = false;
-          int ddx = 0;
-          if (t < te && t != s) {
-            const float4 pj = __ldg(d.posf + t);
-            ddx = frame_step<REACH>(t, b);
-            if (owns(fx0 + ddx, VERLET ? d.okey[t] : pj.x, ki, t, s)) {
-              const float ex = (pi.x - (float)(fx0 + ddx) * csx) - pj.x, ey = by - pj.y,
-                          ez = bz - pj.z;
-              const float dr2 = ex * ex + ey * ey + ez * ez;
-              in1 = dr2 < 1.0f;
-              near = fabsf(dr2 - 1.0f) <= kGuard;
-            }
-          }
-          if (__any_sync(0xffffffffu, near)) {
-            if (near) in1 = exact_dr2(d, R, si, d.perm[t]) < 1.0;
-          }
-          const uint32_t mask = __ballot_sync(0xffffffffu, in1);
-          if (in1) {
-            const int pos = nl + __popc(mask & lt_mask);
-            if (pos < kNbrCap) L[pos] = make_entry(t, fx0 + ddx, dy, dz);
-          }
-          nl += __popc(mask);
-        }
-      }
-      __syncwarp();
-      fits = nl <= kNbrCap;
-      nw = nl;
-      // ---- phase B: density weights
-      if (fits) {
-        for (int k0 = 0; k0 < nl; k0 += 32) {
-          const int k = k0 + lane;
-          const bool valid = k < nl;
-          int t = s, dx = 0, dy = 0, dz = 0;
-          if (valid) read_entry(L[k], t, dx, dy, dz);
-          test(valid, t, dx, dy, dz, valid ? __ldg(d.posf + t) : pi, true);
-        }
-      } else {
-        // a lane takes at most nseg + nl / 32 weights below 2^23 each
-        if (nl > kDensPairsMax && lane == 0) atomicCAS(d.err, 0, kErrDensPairs);
-#pragma unroll 1
-        for (int g = 0; g < nseg; g++) {
-          const int tb = S.tb[g], te = S.te[g];
-          if (tb >= te) continue;
-          const int code = S.code[g];
-          int b[2 * REACH];
-#pragma unroll
-          for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
-          const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
-          for (int t0 = tb; t0 < te; t0 += 32) {
-            const int t = t0 + lane;
-            const int dx = fx0 + frame_step<REACH>(t, b);
-            const float4 pj = t < te ? __ldg(d.posf + t) : pi;
-            const bool valid =
-                t < te && t != s && owns(dx, VERLET ? d.okey[t] : pj.x, ki, t, s);
-            test(valid, valid ? t : s, dx, dy, dz, pj, false);
-          }
+          const int dx = fx0 + frame_step<REACH>(t, b);
+          const float4 pj = t < te ? __ldg(d.posf + t) : pi;
+          const bool valid = t < te && t != s && owns(dx, VERLET ? d.okey[t] : pj.x, ki, t, s);
+          test(valid, valid ? t : s, dx, dy, dz, pj, false);
         }
       }
     }
     __syncwarp();
-    if (swept && fits) {  // list out for pass 2, coalesced
+    if (fits) {  // list out for pass 2, coalesced
       uint32_t* out = d.nbl + (size_t)s * kNbrCap;
       for (int k = lane; k < nl; k += 32) out[k] = L[k];
     }
-    // each weight is below 2^23, so up to 512 weighted pairs total below
-    // 2^32 (nw bounds them: the kept list's length, or the pairs in range)
-    unsigned long long a0, a1, a2;
-    if (nw <= 512) {
-      a0 = __reduce_add_sync(0xffffffffu, q0);
-      a1 = __reduce_add_sync(0xffffffffu, q1);
-      a2 = __reduce_add_sync(0xffffffffu, q2);
-    } else {
-      a0 = q0, a1 = q1, a2 = q2;
+    unsigned long long a0 = q0, a1 = q1, a2 = q2;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+      a2 += __shfl_xor_sync(0xffffffffu, a2, o);
     }
     if (MARKS) hit = __any_sync(0xffffffffu, hit);
     if (lane == 0) {
-      unsigned long long* q = d.dsum + 4 * (size_t)s;
-      if (a0) atomicAdd(q, a0);
-      if (a1) atomicAdd(q + 1, a1);
-      if (a2) atomicAdd(q + 2, a2);
+      if (a0) atomicAdd(d.dsum + s, a0);
+      if (a1) atomicAdd(d.dsum + d.dstride + s, a1);
+      if (a2) atomicAdd(d.dsum + 2 * d.dstride + s, a2);
       d.nbn[s] = fits ? (uint16_t)nl : (uint16_t)kNbrFallback;
       d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
       if (MARKS && hit) d.phit[s] = 1;
     }
     __syncwarp();
-  };
-  if constexpr (MODE == kDensKeptOver) {
-    // the few rows whose kept list did not fit: lane k tests row s0 + k
-    uint32_t rows = __ballot_sync(0xffffffffu, s0 + lane < s_end && d.vn[s0 + lane] == kNbrFallback);
-    while (rows) {
-      row(s0 + __ffs(rows) - 1);
-      rows &= rows - 1;
-    }
-  } else {
-    for (int s = s0; s < s_end; s++)
-      if (MODE == kDensSweep || d.vn[s] != kNbrFallback) row(s);
   }
 }
-
-// Pass 1 over the kept lists with LP lanes per particle (LP 4, 8 or 16; 32 is
-// k_density_f32's kDensKept form): for systems whose kept lists are short
-// (a liquid at density 6 keeps ~20 owned candidates per particle), one warp
-// per particle leaves most lanes idle and repeats the per-particle work (its
-// row, the totals of its weights, its counts) for every particle. The warp
-// sorts its 32 rows by kept-list length (as pass 2 does) and takes them
-// 32 / LP at a time. Per candidate it does what k_density_f32 does over a
-// kept list, and the pass-2 list comes out in the same order, so every LP
-// gives the same densities and lists bit for bit. Rows whose kept list
-// overflowed are left to kDensKeptOver.
-template <int REACH, bool MARKS, int LP>
-__global__ void __launch_bounds__(kRowBlock, 8) k_density_kept_lp(DevState d) {
-  constexpr int G = 32 / LP;  // particles per warp at a time
-  const int r = d.blk_rep[blockIdx.x];
-  const RepDev* R = d.reps + r;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int h = lane / LP, sl = lane % LP;
-  const int s0 = d.blk_row[blockIdx.x] + 32 * wid;
-  const int s_end = min(s0 + 32, R->row_off + R->n);
-  if (s0 >= s_end) return;
-  const bool warren = R->form == IDPD_FORM_WARREN_K;
-  const float cutd2 = R->wrd * R->wrd;  // density cutoff^2 (1 unless Warren)
-  const double cutd2d = (double)R->wrd * (double)R->wrd;
-  const float inv_rd = R->winv_rd, wnorm = R->wnorm, pre = R->dens_prescale;
-  const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
-  const bool prec = MARKS && R->prec_on;
-  const uint32_t gmask = (LP == 32 ? 0xffffffffu : ((1u << LP) - 1u)) << (LP * h);
-  const uint32_t group_lt = ((1u << lane) - 1u) & gmask;
-  // the chunk's rows sorted by kept-list length (rows past the end and
-  // overflowed lists count 0): key = length << 5 | row - s0
-  uint32_t key;
-  {
-    const int sk = s0 + lane;
-    const uint32_t c = sk < s_end ? (uint32_t)d.vn[sk] : 0u;
-    key = ((c != kNbrFallback ? c : 0u) << 5) | (uint32_t)lane;
-    key = warp_sort_asc(key, lane);
-  }
-  for (int i2 = 0; i2 < 32; i2 += G) {
-    const int s2 = s0 + (int)(__shfl_sync(0xffffffffu, key, i2 + h) & 31u);
-    const uint32_t nv0 = s2 < s_end ? (uint32_t)d.vn[s2] : kNbrFallback;
-    const bool act = nv0 != kNbrFallback;
-    if (!__any_sync(0xffffffffu, act)) continue;
-    const int s = s2 < s_end ? s2 : s0;
-    const int nv = act ? (int)nv0 : 0;
-    int nmax = nv;  // rounds of the warp: the longest list of its groups
-#pragma unroll
-    for (int o = LP; o < 32; o <<= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-    const float4 pi = d.posf[s];
-    const uint32_t si = d.perm[s], pri = fbits(pi.w);
-    int nl = 0;  // owned pairs within the cutoff
-    bool hit = false;
-    uint32_t q0 = 0, q1 = 0, q2 = 0;
-    const uint32_t* vl = d.vl + (size_t)s * kVerletCap;
-    uint32_t* out = d.nbl + (size_t)s * kNbrCap;
-    uint32_t e_next = sl < nv ? vl[sl] : 0u;  // one round ahead
-    for (int k0 = 0; k0 < nmax; k0 += LP) {
-      const int k = k0 + sl;
-      const bool valid = k < nv;
-      const uint32_t e = e_next;
-      if (k + LP < nv) e_next = vl[k + LP];
-      int t, dx, dy, dz;
-      read_entry(e, t, dx, dy, dz);
-      if (!valid) t = s;
-      const float4 pj = __ldg(d.posf + t);
-      const float ex = (pi.x - (float)dx * csx) - pj.x;
-      const float ey = (pi.y - (float)dy * csy) - pj.y;
-      const float ez = (pi.z - (float)dz * csz) - pj.z;
-      const float dr2 = ex * ex + ey * ey + ez * ez;
-      bool in1 = valid && dr2 < 1.0f;
-      bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
-      const bool near1 = valid && fabsf(dr2 - 1.0f) <= kGuard;
-      const bool near2 = valid && ((warren && fabsf(dr2 - cutd2) <= kGuard) || dr2 < 1.0e-10f);
-      // rare: the FP64 decisions of the reference near the cutoffs and at
-      // coincident positions
-      if (__any_sync(0xffffffffu, near1 || near2)) {
-        if (near1 || near2) {
-          const double e2 = exact_dr2(d, R, si, d.perm[t]);
-          if (near1) in1 = e2 < 1.0;
-          ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
-        }
-      }
-      const uint32_t prj = fbits(pj.w);
-      if (ind) {
-        const uint32_t w = dens_weight(dr2, warren, inv_rd, wnorm, pre);
-        add_weight(q0, q1, q2, prj, w);
-        atomicAdd(d.dsum + 4 * (size_t)t + (pri & 3u), (unsigned long long)w);
-      }
-      if (MARKS && prec && in1) {
-        hit |= pri == R->prec_from && prj == R->prec_near;
-        if (prj == R->prec_from && pri == R->prec_near) d.phit[t] = 1;
-      }
-      const uint32_t mask = __ballot_sync(0xffffffffu, in1);
-      if (in1) {
-        const int pos = nl + __popc(mask & group_lt);
-        if (pos < kNbrCap) out[pos] = e;
-      }
-      nl += __popc(mask & gmask);
-    }
-    // the totals of each group's lanes: a kept list holds at most kVerletCap
-    // (512) candidates, each weight is below 2^23, so a total is below 2^32
-    uint32_t a0 = 0, a1 = 0, a2 = 0;
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      const uint32_t t0 = __reduce_add_sync(0xffffffffu, h == g ? q0 : 0u);
-      const uint32_t t1 = __reduce_add_sync(0xffffffffu, h == g ? q1 : 0u);
-      const uint32_t t2 = __reduce_add_sync(0xffffffffu, h == g ? q2 : 0u);
-      if (h == g) {
-        a0 = t0;
-        a1 = t1;
-        a2 = t2;
-      }
-    }
-    if (MARKS) hit = (__ballot_sync(0xffffffffu, hit) & gmask) != 0u;
-    if (sl == 0 && act) {
-      unsigned long long* q = d.dsum + 4 * (size_t)s;
-      if (a0) atomicAdd(q, (unsigned long long)a0);
-      if (a1) atomicAdd(q + 1, (unsigned long long)a1);
-      if (a2) atomicAdd(q + 2, (unsigned long long)a2);
-      d.nbn[s] = nl <= kNbrCap ? (uint16_t)nl : (uint16_t)kNbrFallback;
-      d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
-      if (MARKS && hit) d.phit[s] = 1;
-    }
-    __syncwarp();
-  }
-}
-static_assert((long long)kVerletCap * (1ll << 23) <= (1ll << 32), "32-bit totals of pass 1");
 
 // The FP32 densities of pass 1 from its fixed-point sums (and the fixed-point
 // densities of the fine-grained API); the sums are zeroed for the next pass.
@@ -398,8 +327,8 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize(DevState d) {
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
   if (s >= R->row_off + R->n) return;
-  unsigned long long* q = d.dsum + 4 * (size_t)s;
-  const long long a0 = (long long)q[0], a1 = (long long)q[1], a2 = (long long)q[2];
+  unsigned long long *q0 = d.dsum + s, *q1 = q0 + d.dstride, *q2 = q1 + d.dstride;
+  const long long a0 = (long long)*q0, a1 = (long long)*q1, a2 = (long long)*q2;
   const float u = R->dens_unscale_f;
   d.densf[s] = make_float4(fix_to_float(a0, u), fix_to_float(a1, u), fix_to_float(a2, u), 0.0f);
   if (d.dqx) {
@@ -407,43 +336,105 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize(DevState d) {
     d.dqy[s] = a1;
     d.dqz[s] = a2;
   }
-  q[0] = q[1] = q[2] = 0ull;
+  *q0 = *q1 = *q2 = 0ull;
 }
 
-// The kept lists (rebuild steps only). The particles of one cell share its
-// stencil of neighbour segments and, per candidate, the frame offset, so a
-// warp takes one cell at a time and up to 32 of its particles at once: each
-// lane loads one candidate, every particle of the batch is tested against
-// the 32 candidates (one ballot per particle), and the lanes whose candidate
-// is in range append it to that particle's list in one coalesced store. A
-// candidate is kept when closer than 1 + skin in FP32 (with a margin: the
-// list only has to hold every pair that can come within the cutoff before
-// the next rebuild). Only the candidates the particle owns are kept (owns()
-// on the cell-local x of the build, kept in okey): the stencil's -x third is
-// never queued. Each warp builds the lists of exactly its 32-row chunk, one
-// cell's share of the chunk at a time (a cell split between chunks has its
-// stencil set up by each), so the warps of a CTA carry equal numbers of
-// particles. Also records each row's delta_sumr for the displacement test.
-template <int REACH>
-__global__ void __launch_bounds__(kRowBlock) k_verlet_build(DevState d) {
-  __shared__ SegTable seg[kWarps];
+// The forward half of a cell's stencil as one range of candidates: per (dy, dz) row of
+// search cells the run from the particle's own frame cell column to the stencil's +x
+// end (the -x frame column is never owned), its part beyond the box edge apart. A
+// candidate's frame offset in x is 0 or 1.
+struct HalfStencil {
+  int tb[kMaxSeg];    // first row
+  int end[kMaxSeg];   // candidates up to and including this part
+  int fwd[kMaxSeg];   // first row whose x offset is 1
+  int dyz[kMaxSeg];   // frame offsets: dy + 1 | (dz + 1) << 2
+};
+
+// Lane k < (2m+1)^2 sets up row k (two parts); returns the number of candidates.
+__device__ __forceinline__ int half_stencil(HalfStencil& S, const DevState& d, const RepDev* R,
+                                            int cx, int cy, int cz, int lane) {
+  const int m = R->reach, w = 2 * m + 1, rs = R->rshift;
+  const int nx = R->nc[0], ny = R->nc[1], nz = R->nc[2];
+  int n0 = 0, n1 = 0, b0 = 0, b1 = 0, f0 = 0x7fffffff, dyz = 0;
+  if (lane < w * w) {
+    const int dz = lane / w - m, dy = lane % w - m;
+    const int qz = cz + dz, wz = qz < 0 ? qz + nz : (qz >= nz ? qz - nz : qz);
+    const int qy = cy + dy, wy = qy < 0 ? qy + ny : (qy >= ny ? qy - ny : qy);
+    const int* start = d.cell_start + R->cell_off + (wz * ny + wy) * nx;
+    const int lo = cx & ~(m - 1), hi = cx + m;  // lo: first search cell of the frame cell
+    b0 = start[lo];
+    n0 = start[min(hi, nx - 1) + 1] - b0;
+    if (lo + m < nx) f0 = start[lo + m];
+    if (hi >= nx) {  // beyond the edge: the next frame cell
+      b1 = start[0];
+      n1 = start[hi - nx + 1] - b1;
+    }
+    dyz = ((qy >> rs) - (cy >> rs) + 1) | ((qz >> rs) - (cz >> rs) + 1) << 2;
+  }
+  int end = n0 + n1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += v;
+  }
+  if (lane < w * w) {
+    S.tb[2 * lane] = b0;
+    S.end[2 * lane] = end - n1;
+    S.fwd[2 * lane] = f0;
+    S.tb[2 * lane + 1] = b1;
+    S.end[2 * lane + 1] = end;
+    S.fwd[2 * lane + 1] = b1;
+    S.dyz[2 * lane] = S.dyz[2 * lane + 1] = dyz;
+  }
+  return __shfl_sync(0xffffffffu, end, 31);
+}
+
+// The lists from the cells. KEPT: the kept lists (rebuild steps only), every owned
+// candidate closer than 1 + skin in FP32 (with a margin: the list only has to hold
+// every pair that can come within the cutoff before the next rebuild); it also keeps
+// the cell-local x of the build (okey) and each row's delta_sumr for the displacement
+// test. Else (no kept lists, every step): the owned pairs within the cutoff, decisions
+// near it re-taken in FP64, straight into the lists of pass 2.
+//
+// The particles of one cell share its candidates and, per candidate, the frame
+// offset, so a warp takes one cell at a time and up to 32 of its particles at once:
+// each lane holds one candidate, every particle of the batch is tested against the 32
+// (one ballot per particle), and the lanes whose candidate is in range append it to
+// that particle's list in one coalesced store. The candidates of all the stencil's rows
+// are numbered through, so that each load round has 32 of them (by segment, a round
+// held a liquid's 26 to 40 in one or two loads); those farther than 1 + skin from the
+// batch's bounding box (about a quarter) are dropped and the others queued into full
+// rounds. Each warp builds the lists of its own chunk of `rows` rows, one cell's share of
+// it at a time (a cell split between chunks is set up by each).
+//
+// What bounds it: instruction issue of the tests. Kept lists, per rebuild: 984k-bead
+// membrane 742 -> 620 us, 998k-particle liquid 441 -> 329 us, 8k beads 105 -> 27 us.
+// Without kept lists it replaces a sweep of each particle's own 27 cells by one warp
+// (pass 1 in all: 400k-particle liquid 766 -> 194 us, 131k-bead membrane 543 -> 171 us, 31k
+// beads with solvent 397 -> 66 us, 3k particles 206 -> 30 us); its pairs' lists are read
+// at 8 lanes per particle, whatever the tuning's lanes for kept lists.
+template <bool KEPT>
+__global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) {
+  __shared__ HalfStencil seg[kWarps];
   __shared__ float4 bpos[kWarps][32];
   __shared__ float4 qpos[kWarps][64];
   __shared__ uint32_t qent[kWarps][64];
-  if (!d.vdev->rebuild) return;
+  if (KEPT && !d.vdev->rebuild) return;
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  SegTable& S = seg[wid];
+  HalfStencil& S = seg[wid];
   float4* P = bpos[wid];
   float4* QX = qpos[wid];
   uint32_t* QE = qent[wid];
+  uint32_t* lists = KEPT ? d.vl : d.nbl;
+  constexpr int cap = KEPT ? kVerletCap : kNbrCap;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const int s0 = d.blk_row[blockIdx.x] + 32 * wid;
-  const int s_end = min(s0 + 32, R->row_off + R->n);
-  const float rv2 = d.vdev->rv2;
+  const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
+  const int s_end = min(s0 + rows, R->row_off + R->n);
+  const float prune2 = KEPT ? d.vdev->rv2 : 1.0f + 1.0e-4f;
+  const float rv2 = KEPT ? prune2 : 1.0f;
   const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
-  constexpr int nseg = 2 * (2 * REACH + 1) * (2 * REACH + 1);
   // the chunk's rows cell by cell: [cs, ce) are the chunk's rows of one cell
   for (int cs = s0; cs < s_end;) {
     const int cell = (int)d.scell[cs];
@@ -451,16 +442,13 @@ __global__ void __launch_bounds__(kRowBlock) k_verlet_build(DevState d) {
     int cx, cy, cz;
     cell_xyz(cell - R->cell_off, R->nc, cx, cy, cz);
     __syncwarp();
-    build_segments(S, d, R, cx, cy, cz, lane);
+    const int total = half_stencil(S, d, R, cx, cy, cz, lane);
     for (int b0 = cs; b0 < ce; b0 += 32) {
       const int nb = min(32, ce - b0);
       const int me = b0 + lane;  // the lane's particle (lane < nb)
       __syncwarp();
       const float4 pm = lane < nb ? d.posf[me] : d.posf[b0];
       P[lane] = pm;
-      // the batch's bounding box: a candidate farther than 1 + skin from it
-      // is no candidate of any particle of the batch (about a quarter of the
-      // 27-cell stencil)
       float lox = pm.x, hix = pm.x, loy = pm.y, hiy = pm.y, loz = pm.z, hiz = pm.z;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -478,74 +466,75 @@ __global__ void __launch_bounds__(kRowBlock) k_verlet_build(DevState d) {
       // the lanes whose candidate is in range of particle k write it to k's
       // list, consecutive lanes to consecutive slots
       auto round = [&](float qx, float qy, float qz, uint32_t e, int t) {
-        const bool fwd = ((e >> kRowBits) & 3u) == 2u;  // frame offset +1: owned by all
+        // owns(): a candidate of the next frame column is owned by all, else qx is its
+        // cell-local x (a particle never owns itself)
+        const float qk = ((e >> kRowBits) & 3u) == 2u ? 3.0e38f : qx;
 #pragma unroll 4
         for (int k = 0; k < nb; k++) {
           const float4 pk = P[k];
-          const float ex = pk.x - qx, ey = pk.y - qy, ez = pk.z - qz;
-          // owns(): qx is the candidate's cell-local x when its offset is 0
-          // (a particle never owns itself); predicate logic, no branches
-          const bool own = fwd | (qx > pk.x) | ((qx == pk.x) & (t > b0 + k));
-          const bool in = (ex * ex + ey * ey + ez * ez < rv2) & own;
+          const float dr2 = dist2(pk.x - qx, pk.y - qy, pk.z - qz);
+          const bool own = (qk > pk.x) | ((qk == pk.x) & (t > b0 + k));
+          bool in = (dr2 < rv2) & own;
+          if (!KEPT) {
+            const bool near = (fabsf(dr2 - 1.0f) <= kGuard) & own;
+            if (__any_sync(0xffffffffu, near)) {
+              if (near) in = exact_dr2(d, R, d.perm[b0 + k], d.perm[t]) < 1.0;
+            }
+          }
           const uint32_t m = __ballot_sync(0xffffffffu, in);
           const int base = __shfl_sync(0xffffffffu, cnt, k);
           const int pos = base + __popc(m & lt_mask);
-          if (in && pos < kVerletCap) d.vl[(size_t)(b0 + k) * kVerletCap + pos] = e;
+          if (in && pos < cap) lists[(size_t)(b0 + k) * cap + pos] = e;
           if (lane == k) cnt += __popc(m);
         }
       };
-#pragma unroll 1
-      for (int g = 0; g < nseg; g++) {
-        const int tb = S.tb[g], te = S.te[g];
-        if (tb >= te) continue;
-        const int code = S.code[g];
-        int b[2 * REACH];
-#pragma unroll
-        for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
-        const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
-        for (int t0 = tb; t0 < te; t0 += 32) {
-          const int t = t0 + lane;
-          bool keep = false;
-          float qx = 0.0f, qy = 0.0f, qz = 0.0f;
-          uint32_t e = 0;
-          if (t < te) {
-            // the candidate in the frame of the cell's particles
-            const float4 pj = __ldg(d.posf + t);
-            const int fx = fx0 + frame_step<REACH>(t, b);
-            qx = fmaf((float)fx, csx, pj.x);
-            qy = fmaf((float)dy, csy, pj.y);
-            qz = fmaf((float)dz, csz, pj.z);
-            e = make_entry(t, fx, dy, dz);
-            const float ox = fmaxf(fmaxf(lox - qx, qx - hix), 0.0f);
-            const float oy = fmaxf(fmaxf(loy - qy, qy - hiy), 0.0f);
-            const float oz = fmaxf(fmaxf(loz - qz, qz - hiz), 0.0f);
-            keep = fx >= 0 && ox * ox + oy * oy + oz * oz < rv2;
+      int g = 0, gb = 0;  // the lane's part of the stencil, candidates before it
+      for (int k0 = 0; k0 < total; k0 += 32) {
+        const int c = k0 + lane;
+        bool keep = false;
+        float qx = 0.0f, qy = 0.0f, qz = 0.0f;
+        uint32_t e = 0;
+        int t = 0;
+        if (c < total) {
+          while (c >= S.end[g]) gb = S.end[g++];
+          t = S.tb[g] + (c - gb);
+          // the candidate in the frame of the cell's particles
+          const float4 pj = __ldg(d.posf + t);
+          const int fx = t >= S.fwd[g], dyz = S.dyz[g];
+          const int dy = (dyz & 3) - 1, dz = (dyz >> 2) - 1;
+          qx = fmaf((float)fx, csx, pj.x);
+          qy = fmaf((float)dy, csy, pj.y);
+          qz = fmaf((float)dz, csz, pj.z);
+          e = make_entry(t, fx, dy, dz);
+          const float ox = fmaxf(fmaxf(lox - qx, qx - hix), 0.0f);
+          const float oy = fmaxf(fmaxf(loy - qy, qy - hiy), 0.0f);
+          const float oz = fmaxf(fmaxf(loz - qz, qz - hiz), 0.0f);
+          keep = ox * ox + oy * oy + oz * oz < prune2;
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int at = qn + __popc(mask & lt_mask);
+          QX[at] = make_float4(qx, qy, qz, __int_as_float(t));
+          QE[at] = e;
+        }
+        qn += __popc(mask);
+        if (qn >= 32) {
+          __syncwarp();
+          const float4 q = QX[lane];
+          const uint32_t qe = QE[lane];
+          __syncwarp();
+          if (lane < qn - 32) {
+            QX[lane] = QX[32 + lane];
+            QE[lane] = QE[32 + lane];
           }
-          const uint32_t mask = __ballot_sync(0xffffffffu, keep);
-          if (keep) {
-            const int at = qn + __popc(mask & lt_mask);
-            QX[at] = make_float4(qx, qy, qz, __int_as_float(t));
-            QE[at] = e;
-          }
-          qn += __popc(mask);
-          if (qn >= 32) {
-            __syncwarp();
-            const float4 q = QX[lane];
-            const uint32_t qe = QE[lane];
-            __syncwarp();
-            if (lane < qn - 32) {
-              QX[lane] = QX[32 + lane];
-              QE[lane] = QE[32 + lane];
-            }
-            __syncwarp();
-            qn -= 32;
-            round(q.x, q.y, q.z, qe, __float_as_int(q.w));
-          }
+          __syncwarp();
+          qn -= 32;
+          round(q.x, q.y, q.z, qe, __float_as_int(q.w));
         }
       }
       __syncwarp();
       if (qn > 0) {  // the last, partial round (absent lanes far away)
-        float4 q = make_float4(1.0e30f, 0.0f, 0.0f, __int_as_float(-1));
+        float4 q = make_float4(1.0e18f, 0.0f, 0.0f, __int_as_float(-1));
         uint32_t qe = 0;
         if (lane < qn) {
           q = QX[lane];
@@ -555,26 +544,24 @@ __global__ void __launch_bounds__(kRowBlock) k_verlet_build(DevState d) {
       }
       __syncwarp();
       if (lane < nb) {
-        d.vn[me] = cnt <= kVerletCap ? (uint16_t)cnt : (uint16_t)kNbrFallback;
-        d.okey[me] = pm.x;
-        const uint32_t i = d.perm[me];
-        d.drx[me] = d.dsx[i];
-        d.dry[me] = d.dsy[i];
-        d.drz[me] = d.dsz[i];
+        (KEPT ? d.vn : d.nbn)[me] = cnt <= cap ? (uint16_t)cnt : (uint16_t)kNbrFallback;
+        if (KEPT) {
+          d.okey[me] = pm.x;
+          const uint32_t i = d.perm[me];
+          d.drx[me] = d.dsx[i];
+          d.dry[me] = d.dsy[i];
+          d.drz[me] = d.dsz[i];
+        }
       }
     }
     cs = ce;
   }
 }
 
-void launch_verlet_build(const DevState& d, int nblk, int reach, cudaStream_t st) {
-  if (nblk == 0) return;
-  if (reach == 2)
-    k_verlet_build<2><<<nblk, kRowBlock, 0, st>>>(d);
-  else
-    k_verlet_build<1><<<nblk, kRowBlock, 0, st>>>(d);
+void launch_verlet_build(const DevState& d, int nblk, cudaStream_t st) {
+  const int rows = build_rows(nblk);
+  if (nblk > 0) k_pair_build<true><<<dim3(nblk, 32 / rows), kRowBlock, 0, st>>>(d, rows);
 }
-
 
 // Plain FP64 pass 1 of one sorted row: FP64 positions of the storage rows,
 // FP64 sums. Returns the row's ordered pairs within the cutoff 1.
@@ -634,31 +621,45 @@ __global__ void __launch_bounds__(kRowBlock) k_density_f64(DevState d) {
   if (s < R->row_off + R->n) d.npair[s] = density_f64_row(d, r, s, R);
 }
 
-template <int REACH, bool MARKS>
-void launch_density_reach(const DevState& d, int nblk, bool verlet, int lanes, cudaStream_t st) {
-  constexpr size_t sm = dens_sweep_smem_bytes();
-  if (verlet) {
-    if (lanes == 4)
-      k_density_kept_lp<REACH, MARKS, 4><<<nblk, kRowBlock, 0, st>>>(d);
-    else if (lanes == 8)
-      k_density_kept_lp<REACH, MARKS, 8><<<nblk, kRowBlock, 0, st>>>(d);
-    else if (lanes == 16)
-      k_density_kept_lp<REACH, MARKS, 16><<<nblk, kRowBlock, 0, st>>>(d);
-    else
-      k_density_f32<REACH, kDensKept, MARKS><<<nblk, kRowBlock, 0, st>>>(d);
-    k_density_f32<REACH, kDensKeptOver, MARKS><<<nblk, kRowBlock, sm, st>>>(d);
-  } else {
-    k_density_f32<REACH, kDensSweep, MARKS><<<nblk, kRowBlock, sm, st>>>(d);
+template <bool MARKS, bool WARREN, bool KNOWN>
+void launch_density_lists(const DevState& d, int nblk, int lanes, cudaStream_t st) {
+  const int rows = chunk_rows(nblk, lanes);
+  const dim3 grid(nblk, 32 / rows);
+  if (lanes == 4)
+    k_density_list<MARKS, WARREN, KNOWN, 4><<<grid, kRowBlock, 0, st>>>(d, rows);
+  else if (lanes == 8)
+    k_density_list<MARKS, WARREN, KNOWN, 8><<<grid, kRowBlock, 0, st>>>(d, rows);
+  else if (lanes == 16)
+    k_density_list<MARKS, WARREN, KNOWN, 16><<<grid, kRowBlock, 0, st>>>(d, rows);
+  else
+    k_density_list<MARKS, WARREN, KNOWN, 32><<<grid, kRowBlock, 0, st>>>(d, rows);
+}
+
+template <int REACH, bool VERLET, bool MARKS>
+void launch_density_f32(const DevState& d, int nblk, int lanes, int form_mask, cudaStream_t st) {
+  if (!VERLET) {
+    const int rows = build_rows(nblk);
+    k_pair_build<false><<<dim3(nblk, 32 / rows), kRowBlock, 0, st>>>(d, rows);
+    lanes = 8;
   }
+  if (form_mask & (1 << IDPD_FORM_WARREN_K))
+    launch_density_lists<MARKS, true, !VERLET>(d, nblk, lanes, st);
+  if (form_mask & ~(1 << IDPD_FORM_WARREN_K))
+    launch_density_lists<MARKS, false, !VERLET>(d, nblk, lanes, st);
+  k_density_over<REACH, VERLET, MARKS><<<nblk, kRowBlock, dens_sweep_smem_bytes(), st>>>(d);
 }
 
 template <bool MARKS>
 void launch_density_f32(const DevState& d, int nblk, int reach, bool verlet, int lanes,
-                        cudaStream_t st) {
-  if (reach == 2)
-    launch_density_reach<2, MARKS>(d, nblk, verlet, lanes, st);
+                        int form_mask, cudaStream_t st) {
+  if (reach == 2 && verlet)
+    launch_density_f32<2, true, MARKS>(d, nblk, lanes, form_mask, st);
+  else if (reach == 2)
+    launch_density_f32<2, false, MARKS>(d, nblk, lanes, form_mask, st);
+  else if (verlet)
+    launch_density_f32<1, true, MARKS>(d, nblk, lanes, form_mask, st);
   else
-    launch_density_reach<1, MARKS>(d, nblk, verlet, lanes, st);
+    launch_density_f32<1, false, MARKS>(d, nblk, lanes, form_mask, st);
 }
 
 // The reference's pair expression in FP64 (nbdf_calculator.hpp:84-132): the
@@ -831,7 +832,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_kept64(DevState d) {
         q0 += prj == 0 ? qw : 0ll;
         q1 += prj == 1 ? qw : 0ll;
         q2 += prj == 2 ? qw : 0ll;
-        atomicAdd(d.dsum + 4 * (size_t)t + (pri & 3u), (unsigned long long)qw);
+        atomicAdd(d.dsum + (pri & 3u) * d.dstride + t, (unsigned long long)qw);
       }
       const uint32_t m = __ballot_sync(0xffffffffu, in1);
       if (in1) {
@@ -867,10 +868,9 @@ __global__ void __launch_bounds__(kRowBlock) k_density_kept64(DevState d) {
     q1 = warp_sum_ll(q1);
     q2 = warp_sum_ll(q2);
     if (lane == 0) {
-      unsigned long long* q = d.dsum + 4 * (size_t)s;
-      if (q0) atomicAdd(q, (unsigned long long)q0);
-      if (q1) atomicAdd(q + 1, (unsigned long long)q1);
-      if (q2) atomicAdd(q + 2, (unsigned long long)q2);
+      if (q0) atomicAdd(d.dsum + s, (unsigned long long)q0);
+      if (q1) atomicAdd(d.dsum + d.dstride + s, (unsigned long long)q1);
+      if (q2) atomicAdd(d.dsum + 2 * d.dstride + s, (unsigned long long)q2);
       d.nbn[s] = nl <= kNbrCap ? (uint16_t)nl : (uint16_t)kNbrFallback;
       d.npair[s] = 2u * (uint32_t)nl;
     }
@@ -885,10 +885,10 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize64(DevState d) {
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
   if (s >= R->row_off + R->n) return;
-  unsigned long long* q = d.dsum + 4 * (size_t)s;
-  const double a0 = (double)(long long)q[0] * kDensUnscale,
-               a1 = (double)(long long)q[1] * kDensUnscale,
-               a2 = (double)(long long)q[2] * kDensUnscale;
+  unsigned long long *q0 = d.dsum + s, *q1 = q0 + d.dstride, *q2 = q1 + d.dstride;
+  const double a0 = (double)(long long)*q0 * kDensUnscale,
+               a1 = (double)(long long)*q1 * kDensUnscale,
+               a2 = (double)(long long)*q2 * kDensUnscale;
   d.dens64[3 * s] = a0;
   d.dens64[3 * s + 1] = a1;
   d.dens64[3 * s + 2] = a2;
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize64(DevState d) {
     d.dqy[s] = __double2ll_rn(a1 / R->dens_unscale);
     d.dqz[s] = __double2ll_rn(a2 / R->dens_unscale);
   }
-  q[0] = q[1] = q[2] = 0ull;
+  *q0 = *q1 = *q2 = 0ull;
 }
 
 // Pass 2: over the pass-1 list (or, when it overflowed, the owned pairs
@@ -1044,7 +1044,7 @@ void launch_force_fp64(const DevState& d, int nblk, int mode, bool with_press, b
 }
 
 void launch_density(const DevState& d, int nblk, int mode, int reach, bool verlet, bool marks,
-                    size_t rows, cudaStream_t st, int lanes) {
+                    size_t rows, int form_mask, cudaStream_t st, int lanes) {
   if (nblk == 0) return;
   if (mode == kPairsF64) {
     k_density_f64<<<nblk, kRowBlock, 0, st>>>(d);
@@ -1060,9 +1060,9 @@ void launch_density(const DevState& d, int nblk, int mode, int reach, bool verle
   }
   if (marks) {
     cudaMemsetAsync(d.phit, 0, rows, st);
-    launch_density_f32<true>(d, nblk, reach, verlet, lanes, st);
+    launch_density_f32<true>(d, nblk, reach, verlet, lanes, form_mask, st);
   } else {
-    launch_density_f32<false>(d, nblk, reach, verlet, lanes, st);
+    launch_density_f32<false>(d, nblk, reach, verlet, lanes, form_mask, st);
   }
   k_dens_finalize<<<nblk, kRowBlock, 0, st>>>(d);
 }

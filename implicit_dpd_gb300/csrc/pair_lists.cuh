@@ -169,6 +169,25 @@ __device__ __forceinline__ void read_entry(uint32_t e, int& t, int& dx, int& dy,
   dz = (int)((e >> (kRowBits + 4)) & 3u) - 1;
 }
 
+// Frame-cell offsets (dx cs_x, dy cs_y, dz cs_z) of the 64 codes of a list
+// entry's top bits (dx + 1 | (dy + 1) << 2 | (dz + 1) << 4): one shared load
+// gives the shift of the other particle's cell-local coordinates. Each
+// product is exact (dx in {-1, 0, 1}), so (x_i - off) - x_j rounds as the
+// fused x_i - dx cs - x_j does.
+// The code kOffNone, of no entry, stands for no candidate: its offset is so far that the
+// squared distance is beyond every cutoff.
+struct OffTable {
+  float4 o[64];
+};
+constexpr uint32_t kOffNone = 63u;
+
+__device__ __forceinline__ void fill_off_table(OffTable& T, const RepDev& R, int c) {
+  const float dx = (float)((c & 3) - 1), dy = (float)(((c >> 2) & 3) - 1),
+              dz = (float)(((c >> 4) & 3) - 1);
+  T.o[c] = make_float4(c == (int)kOffNone ? 1.0e18f : dx * R.cs_f[0], dy * R.cs_f[1],
+                       dz * R.cs_f[2], 0.0f);
+}
+
 template <int REACH>
 __device__ __forceinline__ int frame_step(int t, const int* b) {
   int k = 0;
@@ -183,6 +202,41 @@ __device__ __forceinline__ void add_weight(uint32_t& q0, uint32_t& q1, uint32_t&
   q0 += pr == 0 ? v : 0u;
   q1 += pr == 1 ? v : 0u;
   q2 += pr == 2 ? v : 0u;
+}
+
+// Rows of one warp's chunk in the passes over lists with lp lanes per particle (32 at
+// most, at least one group of 32 / lp). Whole 32-row chunks leave a small system on a
+// few SMs, and a mid-sized one with a last wave that runs as long as its longest lists,
+// so the chunk is halved while the launch has fewer than kListWarps warps (five waves
+// of the 4,864 a GB300 holds at 64 registers), but not below two groups, whose setup
+// (the sort of the rows, the tables) is then a large part of the warp's work, unless
+// even one wave is not full. Measured at 32 / 16 / 8 / 4 / 2 rows, us. Pass 2,
+// membranes at 16 lanes: 984k beads 888 / 880 / 900 / 968 / 1098, 250k 283 / 254 / 247 /
+// 254 / 274, 131k 168 / 157 / 145 / 143 / 154, 62k 117 / 87 / 85 / 80 / 82, 8k 98 / 59 / 39
+// / 28 / 27; liquids at 4 lanes, 998k 213 / 227 / 266, 200k 59 / 57 / 61, 24k 24 / 20 / 18.
+// Pass 1, membranes at 8 lanes: 984k 407 / 406 / 428 / 488, 131k 84 / 83 / 75 / 77, 30k
+// 52 / 38 / 32 / 33; liquids at 4 lanes, 998k 173 / 179 / 194, 577k 89 / 83 / 86, 24k 24 /
+// 21 / 19.
+constexpr int kListWarps = 24000, kWaveWarps = 4864;
+inline int chunk_rows(int nblk, int lp) {
+  const int g = 32 / lp;
+  const long long n = (long long)nblk * kRowBlock;
+  int rows = 32;
+  while (rows > 2 * g && n < (long long)rows * kListWarps) rows >>= 1;
+  if (rows == 2 * g && n < (long long)rows * kWaveWarps) rows = g;
+  return rows;
+}
+
+// The same for the list build, whose cost per cell and chunk (the stencil, the loads of
+// its candidates) is shared by the chunk's particles: halved, down to 2 rows, only while
+// the launch does not fill one wave. Measured at 32 / 16 / 8 / 4 / 2 rows, us: membranes,
+// 984k beads 620 / 639 / 740 / 963, 131k 141 / 127 / 124 / 144, 62k 121 / 79 / 76 / 84, 30k 98 /
+// 60 / 47 / 49, 8k 78 / 56 / 38 / 31 / 27; liquids, 998k 329 / 361 / 449, 200k 92 / 87 / 98, 24k
+// 38 / 27 / 21 / 25.
+inline int build_rows(int nblk) {
+  int rows = 32;
+  while (rows > 2 && (long long)nblk * kRowBlock < (long long)rows * kWaveWarps) rows >>= 1;
+  return rows;
 }
 
 // Visits every neighbour cell within the stencil of the given reach

@@ -10,9 +10,9 @@ namespace idpd {
 // mantissa of 1 + w * pre (w * pre in [0, 1]).
 __device__ __forceinline__ uint32_t dens_weight(float dr2, bool warren, float inv_rd, float wnorm,
                                                 float pre) {
-  const float dr = dr2 * rsqrt_approx(dr2);
-  float w = warren ? 1.0f - dr * inv_rd : 1.0f - dr;
-  w = warren ? wnorm * (w * w) : w * w;
+  const float dr = __fmul_rn(dr2, rsqrt_approx(dr2));
+  float w = warren ? __fsub_rn(1.0f, __fmul_rn(dr, inv_rd)) : 1.0f - dr;
+  w = warren ? __fmul_rn(wnorm, __fmul_rn(w, w)) : __fmul_rn(w, w);
   return (uint32_t)(__float_as_int(fmaf(w, pre, 1.0f)) - 0x3f800000);
 }
 

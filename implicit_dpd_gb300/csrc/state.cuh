@@ -49,7 +49,8 @@ struct DevState {
   long long *dqx, *dqy, *dqz;  // partial densities in RepDev::dens_unscale units (fine-grained API only)
   double* dens64;              // [3N] partial densities of the FP64 arms (sorted order)
   double* svel;                // [4N] FP64 velocity per sorted row (FP64 engine-algorithm arm)
-  unsigned long long* dsum;    // [4N] pass-1 partial densities by property, fixed point (zero between passes)
+  unsigned long long* dsum;    // [4][dstride] pass-1 partial densities by property, fixed point (zero between passes)
+  size_t dstride;              // rows of one property's sums
   // ---- topology
   uint32_t* topol;  // [4 * total molecules] storage rows
   float* cf_bend;   // [total molecules]
@@ -180,12 +181,12 @@ struct PairTuning {
 // precursor marks, zeroed first over rows, the buffer's capacity).
 // (lanes: lanes per particle of the kept-list pass, 8, 16 or 32)
 void launch_density(const DevState& d, int nblk, int mode, int reach, bool verlet, bool marks,
-                    size_t rows, cudaStream_t st, int lanes = 32);
+                    size_t rows, int form_mask, cudaStream_t st, int lanes = 32);
 // Precursor conversion after the force pass (marks: the FP32 pass 1 left its
 // marks; else the cells are swept).
 void launch_precursor(const DevState& d, int nblk, bool marks, cudaStream_t st);
 // The kept lists of every particle (when this step rebuilds).
-void launch_verlet_build(const DevState& d, int nblk, int reach, cudaStream_t st);
+void launch_verlet_build(const DevState& d, int nblk, cudaStream_t st);
 // Pass 2 (kept: pass 1 ran over the kept lists; rows: the capacity of the
 // force sums, which the FP32 pass zeroes first, since its terms arrive by
 // atomic add).
