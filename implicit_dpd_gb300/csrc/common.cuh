@@ -87,6 +87,14 @@ struct BlockMap {
 
 __device__ __forceinline__ int sar(int x, int s) { return x >> s; }
 
+// First statement of the step's kernels: lets the next kernel of the stream be set up
+// while this one runs, and waits for the kernels before it (both do nothing in a launch
+// without the programmatic attribute).
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Approximate reciprocal square root, division and cosine without the steps
 // that keep subnormal operands (none occurs where they are used): rsqrt of 0 is
 // infinite, and for normal operands the results are rsqrtf's, __fdividef's and

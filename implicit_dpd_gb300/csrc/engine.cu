@@ -310,6 +310,7 @@ int ensure_capacity(idpd_handle* h, int rows, int ncell, int nblk, int namp) {
     AL(s->orig, cap); AL(s->key, cap);
   }
   AL(d.loc, cap);
+  d.arrival = o.key;  // the sort and the reorder never run at once
   AL(h->xfer, 9 * (size_t)cap);
   AL(d.slot, cap);
   AL(d.cell_cnt, cc);
@@ -695,50 +696,60 @@ int pair_mode(const idpd_handle* h) {
 // Cell list over the current positions (no drift).
 void enqueue_cells(idpd_handle* h, bool drift) {
   h->vl_dirty = true;
-  launch_drift_bin(h->d, h->nblk, drift, h->st);
-  launch_scan(h->d, h->ncell_tot, h->R - 1, h->st);
-  launch_scatter_sort_pack(h->d, h->nblk, h->ncell_tot, true, h->st);
+  launch_drift_bin(h->d, h->nblk, drift, h->R, StepConds{}, h->st);
+  launch_scan(h->d, h->ncell_tot, h->R - 1, {h->st, true});
+  launch_scatter_sort_pack(h->d, h->nblk, 0, {h->st, true});
 }
 
 // Work that most steps skip goes, in a captured step, into the body of an IF
-// node: begin_if adds the node after the kernel that sets its condition
-// (cond launches it) and starts capturing the body on h->cst; the caller
-// enqueues the work on the returned stream; end_if ends the body. When the
-// stream is not capturing (a step enqueued directly), the work goes to h->st
-// and its kernels skip themselves, as they do inside the body too.
+// node whose condition the step's first kernels set: step_conds makes the
+// conditions (before those kernels are captured), begin_if adds the node and
+// starts capturing the body on h->cst; the caller enqueues the work on the
+// returned stream; end_if ends the body. When the stream is not capturing (a
+// step enqueued directly), the work goes to h->st and its kernels skip
+// themselves, as they do inside the body too.
+StepConds step_conds(idpd_handle* h, bool verlet) {
+  StepConds c{};
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t g;
+  if ((h->flags & IDPD_CFG_PLAIN_GRAPHS) ||
+      cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, nullptr, nullptr, nullptr) != cudaSuccess ||
+      cs != cudaStreamCaptureStatusActive)
+    return c;
+  c.on = cudaGraphConditionalHandleCreate(&c.cm, g, 0, cudaGraphCondAssignDefault) ==
+             cudaSuccess &&
+         (!verlet || cudaGraphConditionalHandleCreate(&c.rebuild, g, 0,
+                                                      cudaGraphCondAssignDefault) == cudaSuccess);
+  return c;
+}
+
+// first: the stream of the body's first launch (it has no kernel before it in a body).
 struct IfScope {
-  cudaStream_t st;
+  Chain first;
   bool body;
 };
-template <class Cond>
-IfScope begin_if(idpd_handle* h, Cond&& cond) {
+IfScope begin_if(idpd_handle* h, const StepConds& c, cudaGraphConditionalHandle ch) {
+  const IfScope direct{{h->st, true}, false};
   cudaStreamCaptureStatus cs;
   cudaGraph_t g;
   const cudaGraphNode_t* deps = nullptr;
   const cudaGraphEdgeData* edges = nullptr;
   size_t nd = 0;
-  if ((h->flags & IDPD_CFG_PLAIN_GRAPHS) ||
-      cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, &deps, &edges, &nd) != cudaSuccess ||
-      cs != cudaStreamCaptureStatusActive)
-    return {h->st, false};
-  cudaGraphConditionalHandle ch;
-  if (cudaGraphConditionalHandleCreate(&ch, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
-    return {h->st, false};
-  cond(ch);
-  if (cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, &deps, &edges, &nd) != cudaSuccess)
-    return {h->st, false};
+  if (!c.on ||
+      cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, &deps, &edges, &nd) != cudaSuccess)
+    return direct;
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = ch;
   cp.conditional.type = cudaGraphCondTypeIf;
   cp.conditional.size = 1;
   cudaGraphNode_t node;
-  if (cudaGraphAddNode(&node, g, deps, edges, nd, &cp) != cudaSuccess) return {h->st, false};
+  if (cudaGraphAddNode(&node, g, deps, edges, nd, &cp) != cudaSuccess) return direct;
   cudaStreamUpdateCaptureDependencies(h->st, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
   if (cudaStreamBeginCaptureToGraph(h->cst, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                     cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-    return {h->st, false};  // an empty body: the kernels follow on h->st
-  return {h->cst, true};
+    return {{h->st, false}, false};  // an empty body: the kernels follow on h->st
+  return {{h->cst, false}, true};
 }
 
 void end_if(idpd_handle* h, const IfScope& s) {
@@ -749,59 +760,59 @@ void end_if(idpd_handle* h, const IfScope& s) {
 
 // One MD step; `observe` adds the per-particle virial to the pair pass and
 // the observation kernels (the records are written only for replicas whose
-// step counter is due).
-void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr) {
+// step counter is due); loop.left is set inside the K-step loop graph.
+void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr,
+                  const LoopTail& loop = LoopTail{}) {
   const int mode = pair_mode(h);
   DevState d = h->d;  // the step writes no fine-grained side outputs
   d.dqx = d.dqy = d.dqz = nullptr;
+  const Chain st{h->st, true};
+  // the first kernel, and a kernel behind an event, a memory node or an IF node,
+  // has no kernel right before it
+  const Chain head{h->st, false};
+  const Chain after_drift = drift_done ? head : st;
   const bool verlet = d.vdev && h->tune.skin > 0.0f && mode != kPairsF64;
+  const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
+  const int zero = kZeroForce | (observe ? kZeroVirial : 0) | (marks ? kZeroMarks : 0);
+  const StepConds conds = step_conds(h, verlet);
   if (verlet) {  // cells and lists only on rebuild steps
     const int* gate = &d.vdev->rebuild;
-    launch_drift_disp(d, h->nblk, h->st);
+    launch_drift_disp(d, h->nblk, head);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
-    launch_vl_decide(d, h->st);
-    const auto rebuild = [&](cudaGraphConditionalHandle c) { launch_cond_flag(c, gate, h->st); };
-    IfScope c = begin_if(h, rebuild);
-    launch_bin_gated(d, h->nblk, c.st);
-    launch_scan(d, h->ncell_tot, h->R - 1, c.st, gate);
-    launch_scatter_sort(d, h->nblk, h->ncell_tot, true, c.st, gate);
+    launch_vl_decide(d, h->R, conds, after_drift);
+    const IfScope c = begin_if(h, conds, conds.rebuild);
+    const Chain body{c.first.st, true};
+    launch_bin_gated(d, h->nblk, c.first);
+    launch_scan(d, h->ncell_tot, h->R - 1, body, gate);
+    launch_scatter_sort_pack(d, h->nblk, zero, body, gate);
+    launch_verlet_build(d, h->nblk, body);
     end_if(h, c);
-    launch_pack(d, h->nblk, h->st, gate);  // every step: the positions changed
-    c = begin_if(h, rebuild);
-    launch_verlet_build(d, h->nblk, c.st);
-    end_if(h, c);
+    launch_pack(d, h->nblk, zero, conds.on ? head : st, gate);  // the positions changed
   } else {
-    launch_drift_bin(d, h->nblk, true, h->st);
+    launch_drift_bin(d, h->nblk, true, h->R, conds, head);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
-    launch_scan(d, h->ncell_tot, h->R - 1, h->st);
-    launch_scatter_sort_pack(d, h->nblk, h->ncell_tot, true, h->st);
+    launch_scan(d, h->ncell_tot, h->R - 1, after_drift);
+    launch_scatter_sort_pack(d, h->nblk, zero, st);
   }
-  const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
-  launch_density(d, h->nblk, mode, h->tune.reach, verlet, marks, h->cap,
-                 form_mask(h), h->st, h->tune.dlanes);
-  launch_force(d, h->nblk, mode, observe, verlet, h->tune, form_mask(h), h->cap, h->st);
+  launch_density(d, h->nblk, mode, h->tune.reach, verlet, marks, h->cap, form_mask(h), st,
+                 h->tune.dlanes, true);
+  launch_force(d, h->nblk, mode, observe, verlet, h->tune, form_mask(h), h->cap, st, true);
   if (h->prec_any) {
     d.prec_count = h->prec_dev;
-    launch_precursor(d, h->nblk, marks, h->st);
+    launch_precursor(d, h->nblk, marks, st);
   }
-  launch_bonded_kick(d, h->nblk, true, h->st);
+  launch_bonded_kick(d, h->nblk, true, st);
   if (observe) launch_observe_bonds(d, h->obs_buf, h->n_amp_tot, h->amp_rep, h->st);
   {
-    IfScope c = begin_if(h, [&](cudaGraphConditionalHandle ch) {
-      launch_cond_cm(ch, d.rep_time, h->R, h->st);
-    });
-    launch_cmdrift(d, h->nblk, h->R, false, c.st);
+    const IfScope c = begin_if(h, conds, conds.cm);
+    launch_cmdrift(d, h->nblk, h->R, false, c.first);
     end_if(h, c);
   }
   if (h->chem_on)
     launch_chem(d, h->chem_buf, h->reps_h[0].nblk, h->chem_cfg.n_core, h->chem_amp_cap, false,
                 h->st);
   if (observe) launch_observe(d, h->obs_buf, h->nblk, h->n_amp_tot, h->amp_rep, h->R, h->st);
-  if (h->chem_on) {
-    launch_time_advance(d, h->R, h->st, &h->chem->stop_now);
-  } else {
-    launch_time_advance(d, h->R, h->st);
-  }
+  launch_step_tail(d, h->R, h->chem_on ? &h->chem->stop_now : nullptr, loop, head);
 }
 
 int enqueue_reorder(idpd_handle* h) {
@@ -1333,7 +1344,7 @@ int idpd_drift(idpd_handle* h) {
   cudaSetDevice(h->device);
   int rc = commit(h);
   if (rc) return rc;
-  launch_drift_bin(h->d, h->nblk, true, h->st);
+  launch_drift_bin(h->d, h->nblk, true, h->R, StepConds{}, h->st);
   // the arrival slots of this binning are not used: reset the cell counts
   CK(cudaMemsetAsync(h->d.cell_cnt, 0, sizeof(int) * h->ncell_tot, h->st));
   h->density_valid = false;
@@ -1414,7 +1425,7 @@ int idpd_remove_cmdrift(idpd_handle* h) {
 }
 
 // The loop graph: a WHILE conditional node whose body is the captured step
-// followed by k_loop_tail. Returns false (and leaves no graph) where the
+// (its last kernel sets the loop's condition). Returns false (and leaves no graph) where the
 // driver refuses any part of it; the steps then go one launch each.
 bool build_loop_graph(idpd_handle* h) {
   cudaGraph_t g = nullptr;
@@ -1432,8 +1443,8 @@ bool build_loop_graph(idpd_handle* h) {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       if (cudaStreamBeginCaptureToGraph(h->st, body, nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        enqueue_step(h, false);
-        launch_loop_tail(cond, h->loop_left, h->chem_on ? &h->chem->stopped : nullptr, h->st);
+        enqueue_step(h, false, nullptr,
+                     LoopTail{cond, h->loop_left, h->chem_on ? &h->chem->stopped : nullptr});
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(h->st, &body);
         ok = le == cudaSuccess && ce == cudaSuccess &&
@@ -1796,15 +1807,16 @@ int idpd_profile_step(idpd_handle* h, char* names, size_t names_len, float* ms, 
   CK(cudaEventRecord(ev[0], h->st));
   if (verlet) {
     launch_drift_disp(d, h->nblk, h->st);
-    launch_vl_decide(d, h->st);
-    launch_bin_gated(d, h->nblk, h->st);
+    launch_vl_decide(d, h->R, StepConds{}, {h->st, true});
+    launch_bin_gated(d, h->nblk, {h->st, true});
   } else {
-    launch_drift_bin(d, h->nblk, true, h->st);
+    launch_drift_bin(d, h->nblk, true, h->R, StepConds{}, h->st);
   }
   CK(cudaEventRecord(ev[1], h->st));
   launch_scan(d, h->ncell_tot, h->R - 1, h->st, gate);
   CK(cudaEventRecord(ev[2], h->st));
-  launch_scatter_sort_pack(d, h->nblk, h->ncell_tot, true, h->st, gate);
+  launch_scatter_sort_pack(d, h->nblk, kZeroForce, h->st, gate);
+  if (verlet) launch_pack(d, h->nblk, kZeroForce, {h->st, true}, gate);
   CK(cudaEventRecord(ev[3], h->st));
   if (verlet) launch_verlet_build(d, h->nblk, h->st);
   CK(cudaEventRecord(ev[4], h->st));
@@ -1812,13 +1824,13 @@ int idpd_profile_step(idpd_handle* h, char* names, size_t names_len, float* ms, 
   launch_density(d, h->nblk, mode, h->tune.reach, verlet, false, h->cap, form_mask(h), h->st,
                  h->tune.dlanes);
   CK(cudaEventRecord(ev[5], h->st));
-  launch_force(d, h->nblk, mode, false, verlet, h->tune, form_mask(h), h->cap, h->st);
+  launch_force(d, h->nblk, mode, false, verlet, h->tune, form_mask(h), h->cap, h->st, true);
   CK(cudaEventRecord(ev[6], h->st));
   launch_bonded_kick(d, h->nblk, true, h->st);
   CK(cudaEventRecord(ev[7], h->st));
   launch_cmdrift(d, h->nblk, h->R, false, h->st);
   CK(cudaEventRecord(ev[8], h->st));
-  launch_time_advance(d, h->R, h->st);
+  launch_step_tail(d, h->R, nullptr, LoopTail{}, h->st);
   CK(cudaEventRecord(ev[9], h->st));
   CK(cudaEventSynchronize(ev[9]));
   std::string all;

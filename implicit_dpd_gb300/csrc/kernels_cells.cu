@@ -57,8 +57,20 @@ __device__ __forceinline__ void drift_row(const DevState& d, const RepDev* R, in
   }
 }
 
+// Whether the centre-of-mass drift removal is due for some replica, into the condition of
+// its IF node; the whole block takes part.
+__device__ __forceinline__ void set_cm_cond(const StepConds& c, const uint32_t* rep_time, int R) {
+  int any = 0;
+  for (int r = threadIdx.x; r < R; r += blockDim.x) any |= (rep_time[r] % kCmCorr) == 0u;
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) cudaGraphSetConditional(c.cm, any ? 1u : 0u);
+}
+
 // One thread per storage row: optional drift, then cell index and arrival slot.
-__global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drift) {
+__global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drift, int nrep,
+                                                         StepConds conds) {
+  chain_begin();
+  if (conds.on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -78,6 +90,7 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
 // unwrapped) into the rebuild record.
 __global__ void __launch_bounds__(kRowBlock) k_drift_disp(DevState d) {
   __shared__ float wmax[kRowBlock / 32];
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -103,17 +116,23 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_disp(DevState d) {
   }
 }
 
-__global__ void k_vl_decide(VerletDev* v) {
-  if (threadIdx.x != 0) return;
-  const int rb = v->force || __uint_as_float(v->maxd2) > v->thr2;
-  v->rebuild = rb;
-  v->force = 0;
-  v->maxd2 = 0u;
-  v->rebuilds += (unsigned)rb;
+__global__ void __launch_bounds__(256) k_vl_decide(VerletDev* v, const uint32_t* rep_time,
+                                                   int nrep, StepConds conds) {
+  chain_begin();
+  if (threadIdx.x == 0) {
+    const int rb = v->force || __uint_as_float(v->maxd2) > v->thr2;
+    v->rebuild = rb;
+    v->force = 0;
+    v->maxd2 = 0u;
+    v->rebuilds += (unsigned)rb;
+    if (conds.on) cudaGraphSetConditional(conds.rebuild, rb ? 1u : 0u);
+  }
+  if (conds.on) set_cm_cond(conds, rep_time, nrep);
 }
 
 // The binning of k_drift_bin on a rebuild step (positions already drifted).
 __global__ void __launch_bounds__(kRowBlock) k_bin_gated(DevState d) {
+  chain_begin();
   if (!d.vdev->rebuild) return;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
@@ -127,14 +146,16 @@ __global__ void __launch_bounds__(kRowBlock) k_bin_gated(DevState d) {
   d.slot[i] = (uint32_t)atomicAdd(&d.cell_cnt[key], 1);
 }
 
-void launch_drift_disp(const DevState& d, int nblk, cudaStream_t st) {
-  if (nblk > 0) k_drift_disp<<<nblk, kRowBlock, 0, st>>>(d);
+void launch_drift_disp(const DevState& d, int nblk, const Chain& st) {
+  if (nblk > 0) launch(st, k_drift_disp, nblk, kRowBlock, 0, d);
 }
 
-void launch_vl_decide(const DevState& d, cudaStream_t st) { k_vl_decide<<<1, 32, 0, st>>>(d.vdev); }
+void launch_vl_decide(const DevState& d, int R, const StepConds& c, const Chain& st) {
+  launch(st, k_vl_decide, 1, 256, 0, d.vdev, d.rep_time, R, c);
+}
 
-void launch_bin_gated(const DevState& d, int nblk, cudaStream_t st) {
-  if (nblk > 0) k_bin_gated<<<nblk, kRowBlock, 0, st>>>(d);
+void launch_bin_gated(const DevState& d, int nblk, const Chain& st) {
+  if (nblk > 0) launch(st, k_bin_gated, nblk, kRowBlock, 0, d);
 }
 
 // ---------------------------------------------------------------- scan
@@ -170,11 +191,9 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   return res;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* cnt, int* start, int* part,
-                                                             int ncell, const int* gate) {
-  __shared__ int ws[33];
-  if (gate && !*gate) return;
-  const int base = blockIdx.x * kScanTile + threadIdx.x * kScanPerThread;
+// One tile's exclusive scan into start and its total; returns the total.
+__device__ __forceinline__ int scan_tile(const int* cnt, int* start, int base, int ncell, int carry,
+                                         int* ws) {
   int c[kScanPerThread];
   int sum = 0;
 #pragma unroll
@@ -183,37 +202,60 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* cnt, int
     sum += c[k];
   }
   int total;
-  int run = block_exclusive_scan(sum, ws, total);
+  int run = carry + block_exclusive_scan(sum, ws, total);
 #pragma unroll
   for (int k = 0; k < kScanPerThread; k++) {
     if (base + k < ncell) start[base + k] = run;
     run += c[k];
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = total;
+  return total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_parts(int* part, int nparts,
+// Exclusive scan of the cell counts. A block per tile of 4,096 cells writes its tile's scan
+// and total (k_scan_tiles); then each block adds the totals before its tile
+// (k_scan_finish). Up to kScanOneBlock cells (four tiles) one block does it all: one
+// launch instead of two, about as long as each of them.
+constexpr int kScanOneBlock = 4 * kScanTile;
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(int* cnt, int* start, int ncell,
+                                                             int n_tot, const RepDev* last,
                                                              const int* gate) {
   __shared__ int ws[33];
+  chain_begin();
   if (gate && !*gate) return;
   int carry = 0;
-  for (int b = 0; b < nparts; b += kScanThreads) {
-    const int i = b + threadIdx.x;
-    const int v = i < nparts ? part[i] : 0;
-    int total;
-    const int ex = block_exclusive_scan(v, ws, total);
-    if (i < nparts) part[i] = ex + carry;
-    carry += total;
+  for (int b = 0; b < ncell; b += kScanTile) {
+    const int base = b + threadIdx.x * kScanPerThread;
+    carry += scan_tile(cnt, start, base, ncell, carry, ws);
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; k++)
+      if (base + k < ncell) cnt[base + k] = 0;  // ready for the next binning
   }
+  if (threadIdx.x == 0) start[ncell] = last ? last->row_off + last->n : n_tot;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* cnt, int* start, int* part,
+                                                             int ncell, const int* gate) {
+  __shared__ int ws[33];
+  chain_begin();
+  if (gate && !*gate) return;
+  const int total = scan_tile(cnt, start, blockIdx.x * kScanTile + threadIdx.x * kScanPerThread,
+                              ncell, 0, ws);
+  if (threadIdx.x == 0) part[blockIdx.x] = total;
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_finish(int* cnt, int* start, const int* part,
                                                               int ncell, int n_tot,
                                                               const RepDev* last,
                                                               const int* gate) {
+  __shared__ int ws[33];
+  chain_begin();
   if (gate && !*gate) return;
+  int before = 0;
+  for (int p = threadIdx.x; p < blockIdx.x; p += kScanThreads) before += part[p];
+  int off;
+  block_exclusive_scan(before, ws, off);
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanPerThread;
-  const int off = part[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kScanPerThread; k++) {
     if (base + k < ncell) {
@@ -224,28 +266,38 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_finish(int* cnt, int* sta
   if (blockIdx.x == 0 && threadIdx.x == 0) start[ncell] = last ? last->row_off + last->n : n_tot;
 }
 
-void launch_scan(const DevState& d, int ncell_tot, int last_rep, cudaStream_t st,
+static void launch_scan_of(int* cnt, int* start, int* part, int ncell, int n_tot,
+                           const RepDev* last, const int* gate, const Chain& st) {
+  if (ncell <= kScanOneBlock) {
+    launch(st, k_scan_small, 1, kScanThreads, 0, cnt, start, ncell, n_tot, last, gate);
+    return;
+  }
+  const int nb = (ncell + kScanTile - 1) / kScanTile;
+  launch(st, k_scan_tiles, nb, kScanThreads, 0, cnt, start, part, ncell, gate);
+  launch(Chain(st.st, true), k_scan_finish, nb, kScanThreads, 0, cnt, start, part, ncell, n_tot,
+         last, gate);
+}
+
+void launch_scan(const DevState& d, int ncell_tot, int last_rep, const Chain& st,
                  const int* gate) {
-  const int nb = (ncell_tot + kScanTile - 1) / kScanTile;
-  k_scan_tiles<<<nb, kScanThreads, 0, st>>>(d.cell_cnt, d.cell_start, d.scan_part, ncell_tot, gate);
-  k_scan_parts<<<1, kScanThreads, 0, st>>>(d.scan_part, nb, gate);
-  k_scan_finish<<<nb, kScanThreads, 0, st>>>(d.cell_cnt, d.cell_start, d.scan_part, ncell_tot, 0,
-                                             d.reps + last_rep, gate);
+  launch_scan_of(d.cell_cnt, d.cell_start, d.scan_part, ncell_tot, 0, d.reps + last_rep, gate, st);
 }
 
 // ------------------------------------------------- scatter / sort / pack
 __global__ void __launch_bounds__(kRowBlock) k_scatter(DevState d, const int* gate) {
+  chain_begin();
   if (gate && !*gate) return;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
   if (i >= R->row_off + R->n) return;
   const uint32_t s = (uint32_t)d.cell_start[d.key[i]] + d.slot[i];
-  d.perm[s] = (uint32_t)i;
+  d.arrival[s] = (uint32_t)i;
 }
 
 // Rows of one cell in ascending storage row: the order a stable counting
-// sort gives, independent of the arrival order of the atomics. A warp per
+// sort gives, independent of the arrival order of the atomics (rows given as x y z
+// triples; the step's rows are placed by k_sort_pack). A warp per
 // cell: each of up to 128 rows finds its place by counting the smaller rows
 // (rows are distinct); a larger cell is sorted by one lane in place.
 __device__ __forceinline__ void sort_cell(uint32_t* perm, int b, int e, int lane) {
@@ -293,8 +345,7 @@ constexpr int kSortWarps = 8;
 constexpr int kSortBlocks = 1216;  // 8 per SM of a GB300; the cells are strided over them
 
 __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort(uint32_t* perm, const int* start,
-                                                               int ncell, const int* gate) {
-  if (gate && !*gate) return;
+                                                               int ncell) {
   const int lane = threadIdx.x & 31;
   for (int c = blockIdx.x * kSortWarps + (threadIdx.x >> 5); c < ncell; c += gridDim.x * kSortWarps)
     sort_cell(perm, start[c], start[c + 1], lane);
@@ -311,23 +362,10 @@ __device__ __forceinline__ double cell_offset(double x, double o, double L) {
   return v;
 }
 
-// One thread per sorted slot: FP32 cell-local position, velocity and ids.
-// gate (may be null): when it reads 0 the slots keep their rows and cells
-// of the last rebuild.
-__global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, const int* gate) {
-  const int r = d.blk_rep[blockIdx.x];
-  const int s = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (s >= R->row_off + R->n) return;
-  const uint32_t i = d.perm[s];
-  uint32_t key;
-  if (!gate || *gate) {
-    d.rank[i] = (uint32_t)s;
-    key = d.key[i];
-    d.scell[s] = key;
-  } else {
-    key = d.scell[s];
-  }
+// The FP32 copies of storage row i at sorted slot s, in cell key: cell-local position,
+// velocity and ids; zero: kZero* bits of what the passes after it add to.
+__device__ __forceinline__ void pack_row(const DevState& d, const RepDev* R, uint32_t i, int s,
+                                         uint32_t key, int zero) {
   int cx, cy, cz;
   cell_xyz((int)key - R->cell_off, R->nc, cx, cy, cz);
   cx >>= R->rshift;  // frame cell
@@ -348,19 +386,62 @@ __global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, const int* gate)
     v[1] = d.vy[i];
     v[2] = d.vz[i];
   }
+  const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (zero & kZeroForce) {
+    float4* f = reinterpret_cast<float4*>(d.fq + 4 * (size_t)s);
+    f[0] = z;
+    f[1] = z;
+  }
+  if (zero & kZeroVirial) {
+    float4* f = reinterpret_cast<float4*>(d.pq + 4 * (size_t)s);
+    f[0] = z;
+    f[1] = z;
+  }
+  if (zero & kZeroMarks) d.phit[s] = 0;
+}
+
+// One thread per arrival slot: the row's place in its cell, the order of ascending storage
+// rows that a stable counting sort gives, is the number of smaller rows in the cell (the
+// cell's rows are the neighbouring threads', so the reads are broadcasts), and its FP32
+// copies are written there. One kernel instead of a sort by cell (a warp each) and a
+// pass over the sorted rows.
+__global__ void __launch_bounds__(kRowBlock) k_sort_pack(DevState d, int zero, const int* gate) {
+  chain_begin();
+  if (gate && !*gate) return;
+  const int r = d.blk_rep[blockIdx.x];
+  const int k = d.blk_row[blockIdx.x] + threadIdx.x;
+  const RepDev* R = d.reps + r;
+  if (k >= R->row_off + R->n) return;
+  const uint32_t i = d.arrival[k], key = d.key[i];
+  const int b = d.cell_start[key], e = d.cell_start[key + 1];
+  int s = b;
+  for (int q = b; q < e; q++) s += d.arrival[q] < i;
+  d.perm[s] = i;
+  d.rank[i] = (uint32_t)s;
+  d.scell[s] = key;
+  pack_row(d, R, i, s, key, zero);
+}
+
+// One thread per sorted slot, for steps that keep the slots' rows and cells of the last
+// rebuild (packed, may be null: device flag; when set k_sort_pack wrote the copies).
+__global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, int zero, const int* packed) {
+  chain_begin();
+  if (packed && *packed) return;
+  const int r = d.blk_rep[blockIdx.x];
+  const int s = d.blk_row[blockIdx.x] + threadIdx.x;
+  const RepDev* R = d.reps + r;
+  if (s >= R->row_off + R->n) return;
+  pack_row(d, R, d.perm[s], s, d.scell[s], zero);
 }
 
 void launch_scan_raw(int* cnt, int* start, int* part, int ncell, int n_tot, cudaStream_t st) {
-  const int nb = (ncell + kScanTile - 1) / kScanTile;
-  k_scan_tiles<<<nb, kScanThreads, 0, st>>>(cnt, start, part, ncell, nullptr);
-  k_scan_parts<<<1, kScanThreads, 0, st>>>(part, nb, nullptr);
-  k_scan_finish<<<nb, kScanThreads, 0, st>>>(cnt, start, part, ncell, n_tot, nullptr, nullptr);
+  launch_scan_of(cnt, start, part, ncell, n_tot, nullptr, nullptr, st);
 }
 
 void launch_cell_sort_raw(uint32_t* perm, const int* start, int ncell, cudaStream_t st) {
   if (ncell > 0)
     k_cell_sort<<<std::min((ncell + kSortWarps - 1) / kSortWarps, kSortBlocks), 32 * kSortWarps,
-                  0, st>>>(perm, start, ncell, nullptr);
+                  0, st>>>(perm, start, ncell);
 }
 
 // Cell index and arrival slot of rows given as x y z triples (one grid, no
@@ -398,28 +479,20 @@ void launch_scatter_rows(const uint32_t* cell, const uint32_t* slot, const int* 
   if (n > 0) k_scatter_rows<<<(n + 255) / 256, 256, 0, st>>>(cell, slot, start, n, perm);
 }
 
-void launch_drift_bin(const DevState& d, int nblk, bool do_drift, cudaStream_t st) {
+void launch_drift_bin(const DevState& d, int nblk, bool do_drift, int R, const StepConds& c,
+                      const Chain& st) {
+  if (nblk > 0) launch(st, k_drift_bin, nblk, kRowBlock, 0, d, do_drift ? 1 : 0, R, c);
+}
+
+void launch_scatter_sort_pack(const DevState& d, int nblk, int zero, const Chain& st,
+                              const int* gate) {
   if (nblk == 0) return;
-  k_drift_bin<<<nblk, kRowBlock, 0, st>>>(d, do_drift ? 1 : 0);
+  launch(st, k_scatter, nblk, kRowBlock, 0, d, gate);
+  launch(Chain(st.st, true), k_sort_pack, nblk, kRowBlock, 0, d, zero, gate);
 }
 
-void launch_scatter_sort(const DevState& d, int nblk, int ncell_tot, bool stable, cudaStream_t st,
-                         const int* gate) {
-  if (nblk == 0) return;
-  k_scatter<<<nblk, kRowBlock, 0, st>>>(d, gate);
-  if (stable)
-    k_cell_sort<<<std::min((ncell_tot + kSortWarps - 1) / kSortWarps, kSortBlocks),
-                  32 * kSortWarps, 0, st>>>(d.perm, d.cell_start, ncell_tot, gate);
-}
-
-void launch_pack(const DevState& d, int nblk, cudaStream_t st, const int* gate) {
-  if (nblk > 0) k_pack<<<nblk, kRowBlock, 0, st>>>(d, gate);
-}
-
-void launch_scatter_sort_pack(const DevState& d, int nblk, int ncell_tot, bool stable,
-                              cudaStream_t st, const int* gate) {
-  launch_scatter_sort(d, nblk, ncell_tot, stable, st, gate);
-  launch_pack(d, nblk, st, gate);
+void launch_pack(const DevState& d, int nblk, int zero, const Chain& st, const int* packed) {
+  if (nblk > 0) launch(st, k_pack, nblk, kRowBlock, 0, d, zero, packed);
 }
 
 // ------------------------------------------------------------- reorder

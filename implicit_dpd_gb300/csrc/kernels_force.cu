@@ -476,6 +476,7 @@ __device__ __forceinline__ void force_walk_rows(const DevState& d, int kept, int
 template <bool PRESS, int FORM, int LP>
 __global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk, int rows) {
   extern __shared__ __align__(16) unsigned char force_smem[];
+  chain_begin();
   ForceBlockSmem* BS = reinterpret_cast<ForceBlockSmem*>(force_smem);
   const int fb = blockDim.x >> 7;  // 128-row blocks of this CTA
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -501,6 +502,7 @@ template <int REACH, bool PRESS, int FORM>
 __global__ void __launch_bounds__(kRowBlock) k_force_walk(DevState d, int kept, int nblk) {
   __shared__ ForceBlockSmem B;
   __shared__ ForceWarpSmem W[kWarps];
+  chain_begin();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int rb = blockIdx.x;
   const int r = d.blk_rep[rb];
@@ -515,17 +517,16 @@ __global__ void __launch_bounds__(kRowBlock) k_force_walk(DevState d, int kept, 
 // row blocks per CTA); the observation steps (PRESS) run 16 lanes, one row
 // block per CTA.
 template <int REACH, int FORM, bool PRESS, int LP>
-void launch_force_kernel(const DevState& d, int nblk, int kept, int fb, cudaStream_t st) {
+void launch_force_kernel(const DevState& d, int nblk, int kept, int fb, const Chain& st) {
   const int rows = chunk_rows(nblk, LP);
-  k_force_f32<PRESS, FORM, LP>
-      <<<dim3((nblk + fb - 1) / fb, 32 / rows), kRowBlock * fb, force_smem_bytes(fb), st>>>(d, nblk,
-                                                                                        rows);
-  k_force_walk<REACH, PRESS, FORM><<<nblk, kRowBlock, 0, st>>>(d, kept, nblk);
+  launch(st, k_force_f32<PRESS, FORM, LP>, dim3((nblk + fb - 1) / fb, 32 / rows), kRowBlock * fb,
+         force_smem_bytes(fb), d, nblk, rows);
+  launch(Chain(st.st, true), k_force_walk<REACH, PRESS, FORM>, nblk, kRowBlock, 0, d, kept, nblk);
 }
 
 template <int FORM, bool PRESS, int LP>
 void launch_force_shape(const DevState& d, int nblk, int reach, int kept, int fb,
-                        cudaStream_t st) {
+                        const Chain& st) {
   if (reach == 2)
     launch_force_kernel<2, FORM, PRESS, LP>(d, nblk, kept, fb, st);
   else
@@ -534,13 +535,11 @@ void launch_force_shape(const DevState& d, int nblk, int reach, int kept, int fb
 
 template <int FORM>
 void launch_force_form(const DevState& d, int nblk, bool with_press, const PairTuning& tu,
-                       int kept, cudaStream_t st) {
-  if (with_press) {
-    launch_force_shape<FORM, true, 16>(d, nblk, tu.reach, kept, 1, st);
-    return;
-  }
+                       int kept, Chain& st) {
   const int fb = tu.fblk == 2 || tu.fblk == 4 ? tu.fblk : 1;
-  if (tu.lanes == 4)
+  if (with_press)
+    launch_force_shape<FORM, true, 16>(d, nblk, tu.reach, kept, 1, st);
+  else if (tu.lanes == 4)
     launch_force_shape<FORM, false, 4>(d, nblk, tu.reach, kept, fb, st);
   else if (tu.lanes == 8)
     launch_force_shape<FORM, false, 8>(d, nblk, tu.reach, kept, fb, st);
@@ -548,25 +547,28 @@ void launch_force_form(const DevState& d, int nblk, bool with_press, const PairT
     launch_force_shape<FORM, false, 32>(d, nblk, tu.reach, kept, fb, st);
   else
     launch_force_shape<FORM, false, 16>(d, nblk, tu.reach, kept, fb, st);
+  st.chained = true;
 }
 
 void launch_force(const DevState& d, int nblk, int mode, bool with_press, bool kept,
-                  const PairTuning& tu, int form_mask, size_t rows, cudaStream_t st) {
+                  const PairTuning& tu, int form_mask, size_t rows, const Chain& st, bool zeroed) {
   if (nblk == 0) return;
-  if (mode != kPairsF64) {
-    cudaMemsetAsync(d.fq, 0, 4 * rows * sizeof(long long), st);
-    if (with_press) cudaMemsetAsync(d.pq, 0, 4 * rows * sizeof(long long), st);
+  Chain c = st;
+  if (mode != kPairsF64 && !zeroed) {
+    cudaMemsetAsync(d.fq, 0, 4 * rows * sizeof(long long), st.st);
+    if (with_press) cudaMemsetAsync(d.pq, 0, 4 * rows * sizeof(long long), st.st);
+    c.chained = false;
   }
   if (mode != kPairsF32) {
-    launch_force_fp64(d, nblk, mode, with_press, kept, st);
+    launch_force_fp64(d, nblk, mode, with_press, kept, c);
     return;
   }
   if (form_mask & (1 << IDPD_FORM_MDPD_K))
-    launch_force_form<IDPD_FORM_MDPD_K>(d, nblk, with_press, tu, kept ? 1 : 0, st);
+    launch_force_form<IDPD_FORM_MDPD_K>(d, nblk, with_press, tu, kept ? 1 : 0, c);
   if (form_mask & (1 << IDPD_FORM_PAIRWISE_K))
-    launch_force_form<IDPD_FORM_PAIRWISE_K>(d, nblk, with_press, tu, kept ? 1 : 0, st);
+    launch_force_form<IDPD_FORM_PAIRWISE_K>(d, nblk, with_press, tu, kept ? 1 : 0, c);
   if (form_mask & (1 << IDPD_FORM_WARREN_K))
-    launch_force_form<IDPD_FORM_WARREN_K>(d, nblk, with_press, tu, kept ? 1 : 0, st);
+    launch_force_form<IDPD_FORM_WARREN_K>(d, nblk, with_press, tu, kept ? 1 : 0, c);
 }
 
 }  // namespace idpd

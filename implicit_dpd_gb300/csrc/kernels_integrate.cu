@@ -80,6 +80,7 @@ __device__ __forceinline__ void chain_forces(const float3 p[4], float cf_s, floa
 // kick: vel = vel_buf + dt/2 acc (vel holds vel_buf after the drift).
 template <bool KICK>
 __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -122,12 +123,9 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
   }
 }
 
-void launch_bonded_kick(const DevState& d, int nblk, bool kick, cudaStream_t st) {
+void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st) {
   if (nblk == 0) return;
-  if (kick)
-    k_bonded_kick<true><<<nblk, kRowBlock, 0, st>>>(d);
-  else
-    k_bonded_kick<false><<<nblk, kRowBlock, 0, st>>>(d);
+  launch(st, kick ? k_bonded_kick<true> : k_bonded_kick<false>, nblk, kRowBlock, 0, d);
 }
 
 // Fine-grained ForceBonded::CalcListedForce: one thread per molecule adds
@@ -227,6 +225,7 @@ __device__ __forceinline__ bool cm_due(const DevState& d, int r, int force_now) 
 
 __global__ void __launch_bounds__(kRowBlock) k_cm_partial(DevState d, int force_now) {
   __shared__ long long sh[3][kRowBlock / 32];
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   if (!cm_due(d, r, force_now)) return;
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
@@ -258,6 +257,7 @@ __global__ void __launch_bounds__(kRowBlock) k_cm_partial(DevState d, int force_
 constexpr int kCmThreads = 256;
 __global__ void __launch_bounds__(kCmThreads) k_cm_finalize(DevState d, int force_now) {
   __shared__ long long sh[3][kCmThreads / 32];
+  chain_begin();
   const int r = blockIdx.x;
   if (!cm_due(d, r, force_now)) return;
   const RepDev* R = d.reps + r;
@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(kCmThreads) k_cm_finalize(DevState d, int forc
 }
 
 __global__ void __launch_bounds__(kRowBlock) k_cm_apply(DevState d, int force_now) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   if (!cm_due(d, r, force_now)) return;
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
@@ -292,66 +293,40 @@ __global__ void __launch_bounds__(kRowBlock) k_cm_apply(DevState d, int force_no
   d.vz[i] = __dsub_rn(d.vz[i], d.rep_mean[3 * r + 2]);
 }
 
-void launch_cmdrift(const DevState& d, int nblk, int R, bool force_now, cudaStream_t st) {
+void launch_cmdrift(const DevState& d, int nblk, int R, bool force_now, const Chain& st) {
   if (nblk == 0) return;
-  k_cm_partial<<<nblk, kRowBlock, 0, st>>>(d, force_now ? 1 : 0);
-  k_cm_finalize<<<R, kCmThreads, 0, st>>>(d, force_now ? 1 : 0);
-  k_cm_apply<<<nblk, kRowBlock, 0, st>>>(d, force_now ? 1 : 0);
-}
-
-__global__ void k_time_advance(uint32_t* t, int R, const int* skip) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (skip && *skip) return;
-  if (r < R) t[r] += 1u;
-}
-
-void launch_time_advance(const DevState& d, int R, cudaStream_t st, const int* skip) {
-  k_time_advance<<<(R + 127) / 128, 128, 0, st>>>(d.rep_time, R, skip);
+  const int f = force_now ? 1 : 0;
+  launch(st, k_cm_partial, nblk, kRowBlock, 0, d, f);
+  launch(Chain(st.st, true), k_cm_finalize, R, kCmThreads, 0, d, f);
+  launch(Chain(st.st, true), k_cm_apply, nblk, kRowBlock, 0, d, f);
 }
 
 // ------------------------------------------- K steps in one graph launch
 // The step repeated on the device by a WHILE conditional node: the count of
-// steps left is set before the launch; the last node of each step takes one
-// off and keeps the loop going while steps are left and, with the reaction
-// enabled, while the reaction has not stopped the run (stop: its flag).
+// steps left is set before the launch; the last kernel of each step, which also
+// advances the step counters, takes one off and keeps the loop going while steps
+// are left and, with the reaction enabled, while the reaction has not stopped the
+// run (stop: its flag).
 __global__ void k_loop_set(int* left, int n) { *left = n; }
 
-__global__ void k_loop_tail(cudaGraphConditionalHandle cond, int* left, const int* stop) {
-  const int l = *left - 1;
-  *left = l;
-  cudaGraphSetConditional(cond, (l > 0 && !(stop && *stop)) ? 1u : 0u);
+__global__ void __launch_bounds__(256) k_step_tail(uint32_t* t, int R, const int* skip,
+                                                   LoopTail loop) {
+  chain_begin();
+  if (!(skip && *skip))
+    for (int r = threadIdx.x; r < R; r += blockDim.x) t[r] += 1u;
+  if (loop.left && threadIdx.x == 0) {
+    const int l = *loop.left - 1;
+    *loop.left = l;
+    cudaGraphSetConditional(loop.cond, (l > 0 && !(loop.stop && *loop.stop)) ? 1u : 0u);
+  }
+}
+
+void launch_step_tail(const DevState& d, int R, const int* skip, const LoopTail& loop,
+                      const Chain& st) {
+  launch(st, k_step_tail, 1, 256, 0, d.rep_time, R, skip, loop);
 }
 
 void launch_loop_set(int* left, int n, cudaStream_t st) { k_loop_set<<<1, 1, 0, st>>>(left, n); }
-
-// IF nodes of a captured step: work that most steps skip (the cell and list
-// rebuild, the centre-of-mass drift removal every kCmCorr steps) sits in a
-// conditional body whose condition one thread sets from the device state,
-// so that a step without it launches none of its kernels.
-__global__ void k_cond_flag(cudaGraphConditionalHandle cond, const int* flag) {
-  cudaGraphSetConditional(cond, *flag ? 1u : 0u);
-}
-
-__global__ void k_cond_cm(cudaGraphConditionalHandle cond, const uint32_t* rep_time, int R) {
-  int any = 0;
-  for (int r = threadIdx.x; r < R; r += blockDim.x) any |= (rep_time[r] % kCmCorr) == 0u;
-  any = __syncthreads_or(any);
-  if (threadIdx.x == 0) cudaGraphSetConditional(cond, any ? 1u : 0u);
-}
-
-void launch_cond_flag(cudaGraphConditionalHandle cond, const int* flag, cudaStream_t st) {
-  k_cond_flag<<<1, 1, 0, st>>>(cond, flag);
-}
-
-void launch_cond_cm(cudaGraphConditionalHandle cond, const uint32_t* rep_time, int R,
-                    cudaStream_t st) {
-  k_cond_cm<<<1, 256, 0, st>>>(cond, rep_time, R);
-}
-
-void launch_loop_tail(cudaGraphConditionalHandle cond, int* left, const int* stop,
-                      cudaStream_t st) {
-  k_loop_tail<<<1, 1, 0, st>>>(cond, left, stop);
-}
 
 // ----------------------------------------------------------- utilities
 __global__ void k_saru_test(int n, const uint32_t* s1, const uint32_t* s2, const uint32_t* s3,

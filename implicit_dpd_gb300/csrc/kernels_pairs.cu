@@ -48,6 +48,7 @@ template <bool MARKS, bool WARREN, bool KNOWN, int LP>
 __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int rows) {
   constexpr int G = 32 / LP;  // particles per warp at a time
   __shared__ OffTable OT;
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   if ((R->form == IDPD_FORM_WARREN_K) != WARREN) return;
@@ -162,6 +163,7 @@ constexpr size_t dens_sweep_smem_bytes() {
 template <int REACH, bool VERLET, bool MARKS>
 __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d) {
   extern __shared__ __align__(16) unsigned char dens_smem[];
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -323,6 +325,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d) {
 // The FP32 densities of pass 1 from its fixed-point sums (and the fixed-point
 // densities of the fine-grained API); the sums are zeroed for the next pass.
 __global__ void __launch_bounds__(kRowBlock) k_dens_finalize(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -419,6 +422,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   __shared__ float4 bpos[kWarps][32];
   __shared__ float4 qpos[kWarps][64];
   __shared__ uint32_t qent[kWarps][64];
+  chain_begin();
   if (KEPT && !d.vdev->rebuild) return;
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
@@ -558,9 +562,9 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   }
 }
 
-void launch_verlet_build(const DevState& d, int nblk, cudaStream_t st) {
+void launch_verlet_build(const DevState& d, int nblk, const Chain& st) {
   const int rows = build_rows(nblk);
-  if (nblk > 0) k_pair_build<true><<<dim3(nblk, 32 / rows), kRowBlock, 0, st>>>(d, rows);
+  if (nblk > 0) launch(st, k_pair_build<true>, dim3(nblk, 32 / rows), kRowBlock, 0, d, rows);
 }
 
 // Plain FP64 pass 1 of one sorted row: FP64 positions of the storage rows,
@@ -615,6 +619,7 @@ __device__ __forceinline__ unsigned int density_f64_row(const DevState& d, int r
 }
 
 __global__ void __launch_bounds__(kRowBlock) k_density_f64(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -622,36 +627,37 @@ __global__ void __launch_bounds__(kRowBlock) k_density_f64(DevState d) {
 }
 
 template <bool MARKS, bool WARREN, bool KNOWN>
-void launch_density_lists(const DevState& d, int nblk, int lanes, cudaStream_t st) {
+void launch_density_lists(const DevState& d, int nblk, int lanes, const Chain& st) {
   const int rows = chunk_rows(nblk, lanes);
-  const dim3 grid(nblk, 32 / rows);
-  if (lanes == 4)
-    k_density_list<MARKS, WARREN, KNOWN, 4><<<grid, kRowBlock, 0, st>>>(d, rows);
-  else if (lanes == 8)
-    k_density_list<MARKS, WARREN, KNOWN, 8><<<grid, kRowBlock, 0, st>>>(d, rows);
-  else if (lanes == 16)
-    k_density_list<MARKS, WARREN, KNOWN, 16><<<grid, kRowBlock, 0, st>>>(d, rows);
-  else
-    k_density_list<MARKS, WARREN, KNOWN, 32><<<grid, kRowBlock, 0, st>>>(d, rows);
+  void (*k)(DevState, int) = lanes == 4    ? k_density_list<MARKS, WARREN, KNOWN, 4>
+                             : lanes == 8  ? k_density_list<MARKS, WARREN, KNOWN, 8>
+                             : lanes == 16 ? k_density_list<MARKS, WARREN, KNOWN, 16>
+                                           : k_density_list<MARKS, WARREN, KNOWN, 32>;
+  launch(st, k, dim3(nblk, 32 / rows), kRowBlock, 0, d, rows);
 }
 
 template <int REACH, bool VERLET, bool MARKS>
-void launch_density_f32(const DevState& d, int nblk, int lanes, int form_mask, cudaStream_t st) {
+void launch_density_f32(const DevState& d, int nblk, int lanes, int form_mask, Chain st) {
   if (!VERLET) {
     const int rows = build_rows(nblk);
-    k_pair_build<false><<<dim3(nblk, 32 / rows), kRowBlock, 0, st>>>(d, rows);
+    launch(st, k_pair_build<false>, dim3(nblk, 32 / rows), kRowBlock, 0, d, rows);
+    st.chained = true;
     lanes = 8;
   }
-  if (form_mask & (1 << IDPD_FORM_WARREN_K))
+  if (form_mask & (1 << IDPD_FORM_WARREN_K)) {
     launch_density_lists<MARKS, true, !VERLET>(d, nblk, lanes, st);
-  if (form_mask & ~(1 << IDPD_FORM_WARREN_K))
+    st.chained = true;
+  }
+  if (form_mask & ~(1 << IDPD_FORM_WARREN_K)) {
     launch_density_lists<MARKS, false, !VERLET>(d, nblk, lanes, st);
-  k_density_over<REACH, VERLET, MARKS><<<nblk, kRowBlock, dens_sweep_smem_bytes(), st>>>(d);
+    st.chained = true;
+  }
+  launch(st, k_density_over<REACH, VERLET, MARKS>, nblk, kRowBlock, dens_sweep_smem_bytes(), d);
 }
 
 template <bool MARKS>
 void launch_density_f32(const DevState& d, int nblk, int reach, bool verlet, int lanes,
-                        int form_mask, cudaStream_t st) {
+                        int form_mask, const Chain& st) {
   if (reach == 2 && verlet)
     launch_density_f32<2, true, MARKS>(d, nblk, lanes, form_mask, st);
   else if (reach == 2)
@@ -702,6 +708,7 @@ __device__ __forceinline__ double pair_cf64(const RepTab64* T, int form, uint32_
 // stored in the engine's fixed point.
 template <bool PRESS>
 __global__ void __launch_bounds__(kRowBlock) k_force_f64(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -777,6 +784,7 @@ constexpr double kBand64 = 1.0e-10;
 // the list of pass 2.
 template <bool VERLET>
 __global__ void __launch_bounds__(kRowBlock) k_density_kept64(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   const RepTab64* T = d.tab64 + r;
@@ -881,6 +889,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_kept64(DevState d) {
 // The FP64 densities of k_density_kept64 from its 2^-40 fixed-point sums
 // (zeroed for the next pass).
 __global__ void __launch_bounds__(kRowBlock) k_dens_finalize64(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -907,6 +916,7 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize64(DevState d) {
 // virial a e e to both). The sums start at zero (launch_force).
 template <bool PRESS, bool VERLET>
 __global__ void __launch_bounds__(kRowBlock) k_force_kept64(DevState d) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   const RepTab64* T = d.tab64 + r;
@@ -1026,45 +1036,36 @@ void launch_sum_pairs(const uint32_t* npair, int row0, int n, unsigned long long
 }
 
 void launch_force_fp64(const DevState& d, int nblk, int mode, bool with_press, bool kept,
-                       cudaStream_t st) {
-  if (mode == kPairsF64Kept) {
-    if (with_press && kept)
-      k_force_kept64<true, true><<<nblk, kRowBlock, 0, st>>>(d);
-    else if (with_press)
-      k_force_kept64<true, false><<<nblk, kRowBlock, 0, st>>>(d);
-    else if (kept)
-      k_force_kept64<false, true><<<nblk, kRowBlock, 0, st>>>(d);
-    else
-      k_force_kept64<false, false><<<nblk, kRowBlock, 0, st>>>(d);
-  } else if (with_press) {
-    k_force_f64<true><<<nblk, kRowBlock, 0, st>>>(d);
-  } else {
-    k_force_f64<false><<<nblk, kRowBlock, 0, st>>>(d);
-  }
+                       const Chain& st) {
+  void (*k)(DevState);
+  if (mode == kPairsF64Kept)
+    k = with_press ? (kept ? k_force_kept64<true, true> : k_force_kept64<true, false>)
+                   : (kept ? k_force_kept64<false, true> : k_force_kept64<false, false>);
+  else
+    k = with_press ? k_force_f64<true> : k_force_f64<false>;
+  launch(st, k, nblk, kRowBlock, 0, d);
 }
 
 void launch_density(const DevState& d, int nblk, int mode, int reach, bool verlet, bool marks,
-                    size_t rows, int form_mask, cudaStream_t st, int lanes) {
+                    size_t rows, int form_mask, const Chain& st, int lanes, bool zeroed) {
   if (nblk == 0) return;
   if (mode == kPairsF64) {
-    k_density_f64<<<nblk, kRowBlock, 0, st>>>(d);
+    launch(st, k_density_f64, nblk, kRowBlock, 0, d);
     return;
   }
   if (mode == kPairsF64Kept) {
-    if (verlet)
-      k_density_kept64<true><<<nblk, kRowBlock, 0, st>>>(d);
-    else
-      k_density_kept64<false><<<nblk, kRowBlock, 0, st>>>(d);
-    k_dens_finalize64<<<nblk, kRowBlock, 0, st>>>(d);
+    launch(st, verlet ? k_density_kept64<true> : k_density_kept64<false>, nblk, kRowBlock, 0, d);
+    launch(Chain(st.st, true), k_dens_finalize64, nblk, kRowBlock, 0, d);
     return;
   }
   if (marks) {
-    cudaMemsetAsync(d.phit, 0, rows, st);
-    launch_density_f32<true>(d, nblk, reach, verlet, lanes, form_mask, st);
+    if (!zeroed) cudaMemsetAsync(d.phit, 0, rows, st.st);
+    launch_density_f32<true>(d, nblk, reach, verlet, lanes, form_mask,
+                             zeroed ? st : Chain(st.st));
   } else {
     launch_density_f32<false>(d, nblk, reach, verlet, lanes, form_mask, st);
   }
-  k_dens_finalize<<<nblk, kRowBlock, 0, st>>>(d);
+  launch(Chain(st.st, true), k_dens_finalize, nblk, kRowBlock, 0, d);
 }
 
 // ------------------------------------------- precursor conversion
@@ -1075,6 +1076,7 @@ void launch_density(const DevState& d, int nblk, int mode, int reach, bool verle
 // 322-333); properties change in the FP64 rows, so the pair passes see them
 // from the next step's packing on.
 __global__ void __launch_bounds__(kRowBlock) k_precursor(DevState d, int marks) {
+  chain_begin();
   const int r = d.blk_rep[blockIdx.x];
   const RepDev* R = d.reps + r;
   if (!R->prec_on) return;
@@ -1107,8 +1109,8 @@ __global__ void __launch_bounds__(kRowBlock) k_precursor(DevState d, int marks) 
   }
 }
 
-void launch_precursor(const DevState& d, int nblk, bool marks, cudaStream_t st) {
-  if (nblk > 0) k_precursor<<<nblk, kRowBlock, 0, st>>>(d, marks ? 1 : 0);
+void launch_precursor(const DevState& d, int nblk, bool marks, const Chain& st) {
+  if (nblk > 0) launch(st, k_precursor, nblk, kRowBlock, 0, d, marks ? 1 : 0);
 }
 
 // -------------------------------------------- neighbour centre of mass

@@ -33,6 +33,7 @@ struct DevState {
   // ---- cell build (per step)
   uint32_t* key;   // global cell of storage row
   uint32_t* slot;  // arrival slot inside the cell
+  uint32_t* arrival;  // rows grouped by cell in arrival order (shares the reorder's key scratch)
   int* cell_cnt;   // [ncell_tot]
   int* cell_start; // [ncell_tot + 1]
   int* scan_part;  // block partial sums of the scan
@@ -123,31 +124,61 @@ constexpr int kRowBlock = 128;  // rows per block of row-block launches
 constexpr int kNbrCap = 512;    // neighbour-list slots per particle
 constexpr int kVerletCap = 512;  // kept-list slots per particle
 
+// Where a launch goes. chained: its kernel may be set up while the kernel before it in
+// the stream still runs (programmatic stream serialization; it waits for it in
+// chain_begin). Only a kernel whose predecessor in the stream is a kernel may be
+// chained, and only one that begins with chain_begin.
+struct Chain {
+  cudaStream_t st;
+  bool chained;
+  Chain(cudaStream_t s, bool c = false) : st(s), chained(c) {}
+};
+template <class... KArgs, class... Args>
+inline void launch(const Chain& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                   Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = c.chained ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Conditions of the IF nodes of a captured step, set by the step's first kernels: the
+// rebuild of cells and lists, and the centre-of-mass drift removal, due for some replica.
+struct StepConds {
+  cudaGraphConditionalHandle rebuild, cm;
+  int on;  // 0: the step holds no IF nodes
+};
+
+// What the pack zeroes for the passes that follow (their terms arrive by atomic add or
+// as marks).
+enum : int { kZeroForce = 1, kZeroVirial = 2, kZeroMarks = 4 };
+
 // kernels_cells.cu
-void launch_drift_bin(const DevState& d, int nblk, bool do_drift, cudaStream_t st);
+void launch_drift_bin(const DevState& d, int nblk, bool do_drift, int R, const StepConds& c,
+                      const Chain& st);
 // start[ncell_tot] = reps[last_rep].row_off + reps[last_rep].n, read on the
 // device (the particle count can grow on the device).
-void launch_scan(const DevState& d, int ncell_tot, int last_rep, cudaStream_t st,
+void launch_scan(const DevState& d, int ncell_tot, int last_rep, const Chain& st,
                  const int* gate = nullptr);
 // Steps with kept lists: drift plus the largest displacement since the last
 // rebuild, the rebuild decision, and the binning of rebuild steps.
-void launch_drift_disp(const DevState& d, int nblk, cudaStream_t st);
-void launch_vl_decide(const DevState& d, cudaStream_t st);
-void launch_bin_gated(const DevState& d, int nblk, cudaStream_t st);
-// gate (may be null): device flag; when 0 the sort is skipped and the pack
-// keeps each slot's cell of the last rebuild.
-void launch_scatter_sort_pack(const DevState& d, int nblk, int ncell_tot, bool stable,
-                              cudaStream_t st, const int* gate = nullptr);
-// The two halves of launch_scatter_sort_pack: rows to sorted slots and the
-// stable order within cells; the FP32 copies of the pair passes.
-void launch_scatter_sort(const DevState& d, int nblk, int ncell_tot, bool stable, cudaStream_t st,
-                         const int* gate = nullptr);
-void launch_pack(const DevState& d, int nblk, cudaStream_t st, const int* gate = nullptr);
-// Conditions of the IF nodes of a captured step: the rebuild flag, and
-// whether the centre-of-mass drift removal is due for some replica.
-void launch_cond_flag(cudaGraphConditionalHandle cond, const int* flag, cudaStream_t st);
-void launch_cond_cm(cudaGraphConditionalHandle cond, const uint32_t* rep_time, int R,
-                    cudaStream_t st);
+void launch_drift_disp(const DevState& d, int nblk, const Chain& st);
+void launch_vl_decide(const DevState& d, int R, const StepConds& c, const Chain& st);
+void launch_bin_gated(const DevState& d, int nblk, const Chain& st);
+// Rows to sorted slots in the stable order within cells, and their FP32 copies
+// (gate, may be null: device flag; when 0 nothing is done). zero: kZero* bits.
+void launch_scatter_sort_pack(const DevState& d, int nblk, int zero, const Chain& st,
+                              const int* gate = nullptr);
+// The FP32 copies of a step that keeps its cells (packed: device flag; when set
+// the step's launch_scatter_sort_pack has written them).
+void launch_pack(const DevState& d, int nblk, int zero, const Chain& st, const int* packed);
 void launch_reorder(const DevState& d, const DevState& o, int nblk, int n_topol,
                     cudaStream_t st);
 void launch_update_loc(const DevState& d, int nblk, cudaStream_t st);
@@ -180,25 +211,28 @@ struct PairTuning {
 // Pass 1 and its densities (verlet: over the kept lists; marks: also the
 // precursor marks, zeroed first over rows, the buffer's capacity).
 // (lanes: lanes per particle of the kept-list pass, 8, 16 or 32)
+// zeroed: the pack has zeroed the marks.
 void launch_density(const DevState& d, int nblk, int mode, int reach, bool verlet, bool marks,
-                    size_t rows, int form_mask, cudaStream_t st, int lanes = 32);
+                    size_t rows, int form_mask, const Chain& st, int lanes = 32,
+                    bool zeroed = false);
 // Precursor conversion after the force pass (marks: the FP32 pass 1 left its
 // marks; else the cells are swept).
-void launch_precursor(const DevState& d, int nblk, bool marks, cudaStream_t st);
+void launch_precursor(const DevState& d, int nblk, bool marks, const Chain& st);
 // The kept lists of every particle (when this step rebuilds).
-void launch_verlet_build(const DevState& d, int nblk, cudaStream_t st);
+void launch_verlet_build(const DevState& d, int nblk, const Chain& st);
 // Pass 2 (kept: pass 1 ran over the kept lists; rows: the capacity of the
-// force sums, which the FP32 pass zeroes first, since its terms arrive by
-// atomic add).
+// force sums, which are zeroed first, since their terms arrive by atomic add,
+// unless the pack has done it).
 void launch_force(const DevState& d, int nblk, int mode, bool with_press, bool kept,
-                  const PairTuning& tu, int form_mask, size_t rows, cudaStream_t st);
+                  const PairTuning& tu, int form_mask, size_t rows, const Chain& st,
+                  bool zeroed = false);
 void launch_com(const DevState& d, int nblk, double* cm_out, uint32_t* cnt_out, cudaStream_t st);
 // The sum of npair over rows [row0, row0 + n) into *out (device), zeroed first.
 void launch_sum_pairs(const uint32_t* npair, int row0, int n, unsigned long long* out,
                       cudaStream_t st);
 // The FP64 pass-2 kernels (plain and engine algorithm), launched by launch_force.
 void launch_force_fp64(const DevState& d, int nblk, int mode, bool with_press, bool kept,
-                       cudaStream_t st);
+                       const Chain& st);
 
 // kernels_chem.cu: one RandomChemEvent (LOCAL_CHEM_EVENT form) on replica 0.
 // force: run regardless of Parameter::time >= beg_chem (fine-grained call).
@@ -255,19 +289,24 @@ int walk_retrieve(WalkState* s, int kind, int tag, int n_walk, const int32_t* ni
                   void* const* result, std::string& err);
 
 // kernels_integrate.cu
-void launch_bonded_kick(const DevState& d, int nblk, bool kick, cudaStream_t st);
+void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st);
 void launch_bonded_fine(const DevState& d, int n_amp_tot, const int* amp_rep, double* vir_part,
                         cudaStream_t st);
 void launch_kick_only(const DevState& d, int nblk, cudaStream_t st);
 void launch_fq_to_acc(const DevState& d, int nblk, double* press_out, cudaStream_t st);
-void launch_cmdrift(const DevState& d, int nblk, int R, bool force_now, cudaStream_t st);
-// skip (may be null): device flag that, when set, leaves the step counter
-// unchanged (the reference breaks out of its loop before time++).
-void launch_time_advance(const DevState& d, int R, cudaStream_t st, const int* skip = nullptr);
-// The K-step loop graph: the count of steps, and the last node of each step.
+void launch_cmdrift(const DevState& d, int nblk, int R, bool force_now, const Chain& st);
+// The step's last kernel: Parameter::time++ per replica (skip, may be null: device flag
+// that, when set, leaves the step counters unchanged: the reference breaks out of its
+// loop before time++) and, inside the K-step loop graph, the loop's condition.
+struct LoopTail {
+  cudaGraphConditionalHandle cond;
+  int* left;        // steps left; null outside the loop graph
+  const int* stop;  // may be null: device flag that ends the loop
+};
+void launch_step_tail(const DevState& d, int R, const int* skip, const LoopTail& loop,
+                      const Chain& st);
+// The loop graph's count of steps.
 void launch_loop_set(int* left, int n, cudaStream_t st);
-void launch_loop_tail(cudaGraphConditionalHandle cond, int* left, const int* stop,
-                      cudaStream_t st);
 void launch_saru_test(int n, const uint32_t* s1, const uint32_t* s2, const uint32_t* s3, int draws,
                       uint32_t* out_u, float* out_n, cudaStream_t st);
 void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n, cudaStream_t st);
