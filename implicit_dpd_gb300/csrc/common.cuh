@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp64_int.cuh"
+
 namespace idpd {
 
 // Compile-time constants of the reference model (parameter.hpp:189-205).
@@ -41,6 +43,7 @@ constexpr float kGuard = 8.0e-6f;
 // reference's FP64 tables; geometry is kept in FP64 for the exact paths.
 struct RepDev {
   double box[3];
+  double half_box[3];
   double ibox[3];    // 1 / box (Parameter::ibox_leng)
   double inv_cs[3];  // search cells per unit length (nc / box)
   double cs[3];      // frame cell side (box / nf): cell-local coordinates refer to it
@@ -55,7 +58,7 @@ struct RepDev {
   int n;             // rows in use
   int blk_off;       // first block of the replica in row-block launches
   int nblk;
-  double dt;
+  double dt, half_dt;
   float cf_c[9], cf_g[9], cf_r[9], cf_m[27];
   float wa, wb, wrd, winv_rd, wnorm;  // Warren form
   float cf_s;
@@ -278,6 +281,12 @@ __device__ __forceinline__ double fix_to_double(long long q, double unscale) {
   const double magic = 6755399441055744.0;  // 1.5 * 2^52
   const double v = __longlong_as_double(q + __double_as_longlong(magic)) - magic;
   return v * unscale;
+}
+
+// The pair and bonded force of fixed-point sum q.
+__device__ __forceinline__ double force_of(long long q) {
+  if ((unsigned long long)(q + (1ll << 51)) < (1ull << 52)) return scale_force(q);
+  return plain_mul(fix_to_double(q, 1.0), kForceUnscale);
 }
 
 // Float with bits reinterpreted as a uint32 payload (prop / id in .w lanes).

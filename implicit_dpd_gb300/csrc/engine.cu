@@ -218,6 +218,7 @@ void fill_repdev(RepDev& R, const idpd_params& p, int reach, float skin) {
   R.rshift = reach == 2 ? 1 : 0;
   for (int k = 0; k < 3; k++) {
     R.box[k] = p.box[k];
+    R.half_box[k] = 0.5 * p.box[k];
     R.ibox[k] = 1.0 / p.box[k];
     R.nf[k] = (int)(p.box[k] / cut);
     R.nc[k] = R.nf[k] * reach;
@@ -228,6 +229,7 @@ void fill_repdev(RepDev& R, const idpd_params& p, int reach, float skin) {
   }
   R.ncell = R.nc[0] * R.nc[1] * R.nc[2];
   R.dt = p.dt;
+  R.half_dt = 0.5 * p.dt;
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) {
       R.cf_c[3 * i + j] = (float)p.cf_c[i][j];

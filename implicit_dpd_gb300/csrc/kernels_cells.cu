@@ -15,46 +15,46 @@ namespace idpd {
 __device__ __forceinline__ double wrap_pbc(double t, double L, double iL, long long hi_bits) {
   const long long b = __double_as_longlong(t);
   if (b >= 0 && b < hi_bits) return t;
-  const double f = floor(__dmul_rn(t, iL));
-  return __dsub_rn(t, __dmul_rn(f, L));
+  const double f = floor(plain_mul(t, iL));
+  return plain_add(t, -plain_mul(f, L));
 }
 
 __device__ __forceinline__ int cell_coord(double x, double inv_cs, int nc) {
-  int c = __double2int_rz(__dmul_rn(x, inv_cs));
-  c = c < 0 ? 0 : c;
+  int c = to_int(mul_f64(x, inv_cs));  // x >= 0 (or -0)
   return c >= nc ? nc - 1 : c;
 }
 
-// drift_and_predict of one storage row (driftkick.hpp:6-27); x, y, z hold
-// the row's position on entry and the new one on return.
-__device__ __forceinline__ void drift_row(const DevState& d, const RepDev* R, int i, double& x,
-                                          double& y, double& z) {
-  {
-    const double dt = R->dt;
-    const double h = __dmul_rn(0.5, dt);
-    double p[3] = {x, y, z};
-    double* vv[3] = {d.vx, d.vy, d.vz};
-    double* aa[3] = {d.ax, d.ay, d.az};
-    double* ds[3] = {d.dsx, d.dsy, d.dsz};
+// drift_and_predict of one storage row (driftkick.hpp:6-27); p holds the row's position
+// on entry and the new one on return, ds its new delta_sumr.
+__device__ __forceinline__ void drift_row(const DevState& d, const RepDev* R, int i, double p[3],
+                                          double ds[3]) {
+  const double dt = R->dt, h = R->half_dt;
+  double v[3] = {d.vx[i], d.vy[i], d.vz[i]};
+  const double a[3] = {d.ax[i], d.ay[i], d.az[i]};
+  ds[0] = d.dsx[i];
+  ds[1] = d.dsy[i];
+  ds[2] = d.dsz[i];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const double vp = __dadd_rn(vv[k][i], __dmul_rn(h, aa[k][i]));
-      const double dr = __dmul_rn(dt, vp);
-      const double t = __dadd_rn(p[k], dr);
-      ds[k][i] = __dadd_rn(ds[k][i], dr);
-      // hi = L (1 - 2^-50): below it t / L rounds below 1 and floor() is 0.
-      const double L = R->box[k];
-      const long long hi = __double_as_longlong(L) - 4;
-      p[k] = wrap_pbc(t, L, R->ibox[k], hi);
-      vv[k][i] = vp;
-    }
-    x = p[0];
-    y = p[1];
-    z = p[2];
-    d.px[i] = x;
-    d.py[i] = y;
-    d.pz[i] = z;
+  for (int k = 0; k < 3; k++) {
+    v[k] = add_f64(v[k], mul_f64(a[k], h));
+    const double dr = mul_f64(v[k], dt);
+    const double t = __dadd_rn(p[k], dr);
+    ds[k] = add_f64(ds[k], dr);
+    // hi = L (1 - 2^-50): below it t / L rounds below 1 and floor() is 0.
+    const double L = R->box[k];
+    const long long hi = __double_as_longlong(L) - 4;
+    p[k] = wrap_pbc(t, L, R->ibox[k], hi);
   }
+  d.vx[i] = v[0]; d.vy[i] = v[1]; d.vz[i] = v[2];
+  d.dsx[i] = ds[0]; d.dsy[i] = ds[1]; d.dsz[i] = ds[2];
+  d.px[i] = p[0]; d.py[i] = p[1]; d.pz[i] = p[2];
+}
+
+// a - b as a float, to about 2^-32 (far beyond any skin where that cannot be told).
+__device__ __forceinline__ float diff_f32(double a, double b) {
+  const long long q = to_fix(a) - to_fix(b);
+  const bool ok = in_fix(a) && in_fix(b) && q == (long long)(int)q;
+  return ok ? __int2float_rn((int)q) * 2.3283064365386963e-10f : 1.0e3f;
 }
 
 // Whether the centre-of-mass drift removal is due for some replica, into the condition of
@@ -75,11 +75,11 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
   if (i >= R->row_off + R->n) return;
-  double x = d.px[i], y = d.py[i], z = d.pz[i];
-  if (do_drift) drift_row(d, R, i, x, y, z);
-  const int cx = cell_coord(x, R->inv_cs[0], R->nc[0]);
-  const int cy = cell_coord(y, R->inv_cs[1], R->nc[1]);
-  const int cz = cell_coord(z, R->inv_cs[2], R->nc[2]);
+  double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
+  if (do_drift) drift_row(d, R, i, p, ds);
+  const int cx = cell_coord(p[0], R->inv_cs[0], R->nc[0]);
+  const int cy = cell_coord(p[1], R->inv_cs[1], R->nc[1]);
+  const int cz = cell_coord(p[2], R->inv_cs[2], R->nc[2]);
   const uint32_t key = (uint32_t)(R->cell_off + (cz * R->nc[1] + cy) * R->nc[0] + cx);
   d.key[i] = key;
   d.slot[i] = (uint32_t)atomicAdd(&d.cell_cnt[key], 1);
@@ -87,8 +87,16 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
 
 // Steps that keep the neighbour lists: drift, and the largest squared
 // displacement since the last rebuild (delta_sumr accumulates every drift,
-// unwrapped) into the rebuild record.
-__global__ void __launch_bounds__(kRowBlock) k_drift_disp(DevState d) {
+// unwrapped) into the rebuild record. The displacement only has to fall on the right
+// side of the threshold: it is taken in FP32, and again in FP64 close to it.
+//
+// What bounds the elementwise kernels (this one, the pack, the kick): at 10^6 particles
+// the FP64 unit (74 - 80 % busy, DRAM 11 - 19 %), so their products, conversions and
+// comparisons, and six of the drift's nine sums, run in integer instructions
+// (fp64_int.cuh); the sums left to the unit run beside them (all nine on it 59 us, six
+// 52, none 56). 998k particles, us in a launch list: drift 75 -> 52, pack 61 -> 27, kick
+// 31 -> 21; with the bonded forces of 984k beads 73 -> 52, 60 -> 34, 45 -> 41.
+__global__ void __launch_bounds__(kRowBlock, 8) k_drift_disp(DevState d) {
   __shared__ float wmax[kRowBlock / 32];
   chain_begin();
   const int r = d.blk_rep[blockIdx.x];
@@ -96,11 +104,19 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_disp(DevState d) {
   const RepDev* R = d.reps + r;
   float m = 0.0f;
   if (i < R->row_off + R->n) {
-    double x = d.px[i], y = d.py[i], z = d.pz[i];
-    drift_row(d, R, i, x, y, z);
     const uint32_t s = d.rank[i];
-    const double ex = d.dsx[i] - d.drx[s], ey = d.dsy[i] - d.dry[s], ez = d.dsz[i] - d.drz[s];
-    m = (float)(ex * ex + ey * ey + ez * ez);
+    const double r0[3] = {d.drx[s], d.dry[s], d.drz[s]};
+    double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
+    drift_row(d, R, i, p, ds);
+    const float fx = diff_f32(ds[0], r0[0]), fy = diff_f32(ds[1], r0[1]),
+                fz = diff_f32(ds[2], r0[2]);
+    m = fx * fx + fy * fy + fz * fz;
+    const float thr2 = d.vdev->thr2;
+    if (fabsf(m - thr2) < 1.0e-3f * thr2) {
+      const double ex = plain_add(ds[0], -r0[0]), ey = plain_add(ds[1], -r0[1]),
+                   ez = plain_add(ds[2], -r0[2]);
+      m = plain_f32(ex * ex + ey * ey + ez * ez);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -355,10 +371,9 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort(uint32_t* perm, c
 // to the cell (a particle that crossed the box edge since the cells were
 // built keeps its old cell). For a particle inside its cell, x - o is exact
 // in FP64 (Sterbenz: x lies in [o, 2o] or o = 0).
-__device__ __forceinline__ double cell_offset(double x, double o, double L) {
+__device__ __forceinline__ double cell_offset(double x, double o, double L, double half) {
   double v = __dsub_rn(x, o);
-  if (v > 0.5 * L) v = __dsub_rn(v, L);
-  else if (v < -0.5 * L) v = __dadd_rn(v, L);
+  if (abs_above(v, half)) v = plain_add(v, f64_bits(v) >> 63 ? L : -L);
   return v;
 }
 
@@ -373,13 +388,13 @@ __device__ __forceinline__ void pack_row(const DevState& d, const RepDev* R, uin
   cz >>= R->rshift;
   // the float split keeps 48 bits for the near-cutoff pair terms
   float lx, ly, lz, ex, ey, ez;
-  split_double(cell_offset(d.px[i], __dmul_rn((double)cx, R->cs[0]), R->box[0]), lx, ex);
-  split_double(cell_offset(d.py[i], __dmul_rn((double)cy, R->cs[1]), R->box[1]), ly, ey);
-  split_double(cell_offset(d.pz[i], __dmul_rn((double)cz, R->cs[2]), R->box[2]), lz, ez);
+  split_double(cell_offset(d.px[i], mul_int_f64(cx, R->cs[0]), R->box[0], R->half_box[0]), lx, ex);
+  split_double(cell_offset(d.py[i], mul_int_f64(cy, R->cs[1]), R->box[1], R->half_box[1]), ly, ey);
+  split_double(cell_offset(d.pz[i], mul_int_f64(cz, R->cs[2]), R->box[2], R->half_box[2]), lz, ez);
   d.posf[s] = make_float4(lx, ly, lz, __uint_as_float(d.prop[i]));
   d.poslo[s] = make_float4(ex, ey, ez, 0.0f);
-  d.velf[s] = make_float4(__double2float_rn(d.vx[i]), __double2float_rn(d.vy[i]),
-                          __double2float_rn(d.vz[i]), __uint_as_float(d.id[i]));
+  d.velf[s] = make_float4(to_f32(d.vx[i]), to_f32(d.vy[i]), to_f32(d.vz[i]),
+                          __uint_as_float(d.id[i]));
   if (d.svel) {  // FP64 engine-algorithm arm
     double* v = d.svel + 4 * (size_t)s;
     v[0] = d.vx[i];

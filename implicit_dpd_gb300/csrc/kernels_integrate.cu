@@ -88,6 +88,12 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
   const int s = (int)d.rank[i];
   const long long* fs = d.fq + 4 * (size_t)s;
   long long f[3] = {fs[0], fs[1], fs[2]};
+  double v[3];
+  if (KICK) {
+    v[0] = d.vx[i];
+    v[1] = d.vy[i];
+    v[2] = d.vz[i];
+  }
   const uint32_t a = d.amp_id[i];
   if (a != kNone && R->n_amp > 0) {
     const int u = (int)d.unit[i];
@@ -110,16 +116,15 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
     f[1] += fix_force(fu.y);
     f[2] += fix_force(fu.z);
   }
-  const double acx = fix_to_double(f[0], kForceUnscale), acy = fix_to_double(f[1], kForceUnscale),
-               acz = fix_to_double(f[2], kForceUnscale);
+  const double acx = force_of(f[0]), acy = force_of(f[1]), acz = force_of(f[2]);
   d.ax[i] = acx;
   d.ay[i] = acy;
   d.az[i] = acz;
   if (KICK) {
-    const double h = __dmul_rn(R->dt, 0.5);
-    d.vx[i] = __dadd_rn(d.vx[i], __dmul_rn(h, acx));
-    d.vy[i] = __dadd_rn(d.vy[i], __dmul_rn(h, acy));
-    d.vz[i] = __dadd_rn(d.vz[i], __dmul_rn(h, acz));
+    const double h = R->half_dt;
+    d.vx[i] = __dadd_rn(v[0], mul_f64(acx, h));
+    d.vy[i] = __dadd_rn(v[1], mul_f64(acy, h));
+    d.vz[i] = __dadd_rn(v[2], mul_f64(acz, h));
   }
 }
 
