@@ -267,6 +267,19 @@ __device__ __forceinline__ void fix_force_parts(float v, int& hi, int& lo) {
   lo = __float_as_int(fmaf(r, 67108864.0f, magic)) - __float_as_int(magic);
 }
 
+// fix_force for |v| < 65536. The bits of the second sum are 602 2^21 + lo, so the low part
+// goes in as it stands and 602 comes off the high part.
+__device__ __forceinline__ long long fix_force_small(float v) {
+  const float magic = 12582912.0f;  // 1.5 * 2^23: bits 0x4B400000 = 602 * 2^21
+  const float a = fmaf(v, 32.0f, magic);
+  const float r = fmaf(-(a - magic), 0.03125f, v);
+  const uint32_t lo = __float_as_uint(fmaf(r, 67108864.0f, magic));
+  long long x;
+  asm("mad.wide.s32 %0, %1, 2097152, %2;"
+      : "=l"(x) : "r"(__float_as_int(a) - (0x4B400000 + 602)), "l"((long long)(unsigned long long)lo));
+  return x;
+}
+
 __device__ __forceinline__ long long fix_force(float v) {
   if (!(fabsf(v) < 65536.0f)) return fix_from_float(v, kForceBits);
   int hi, lo;

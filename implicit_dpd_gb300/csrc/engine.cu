@@ -337,6 +337,7 @@ int ensure_capacity(idpd_handle* h, int rows, int ncell, int nblk, int namp) {
   AL(h->loop_left, 1);
   AL(d.rep_mean, 3 * h->R);
   AL(d.err, 1);
+  AL(d.overflow, 2);
   AL(h->amp_rep, ac);
   if (h->flags & (IDPD_CFG_FP64_PAIRS | IDPD_CFG_FP64_KEPT)) { AL(d.dens64, 3 * (size_t)cap); }
   if (h->flags & IDPD_CFG_FP64_KEPT) { AL(d.svel, 4 * (size_t)cap); }

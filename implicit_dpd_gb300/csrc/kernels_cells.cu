@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
                                                          StepConds conds) {
   chain_begin();
   if (conds.on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
 __global__ void __launch_bounds__(kRowBlock, 8) k_drift_disp(DevState d) {
   __shared__ float wmax[kRowBlock / 32];
   chain_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -235,7 +237,7 @@ constexpr int kScanOneBlock = 4 * kScanTile;
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_small(int* cnt, int* start, int ncell,
                                                              int n_tot, const RepDev* last,
-                                                             const int* gate) {
+                                                             const int* gate, int* overflow) {
   __shared__ int ws[33];
   chain_begin();
   if (gate && !*gate) return;
@@ -247,7 +249,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_small(int* cnt, int* star
     for (int k = 0; k < kScanPerThread; k++)
       if (base + k < ncell) cnt[base + k] = 0;  // ready for the next binning
   }
-  if (threadIdx.x == 0) start[ncell] = last ? last->row_off + last->n : n_tot;
+  if (threadIdx.x == 0) {
+    start[ncell] = last ? last->row_off + last->n : n_tot;
+    if (overflow) *overflow = 0;  // of the lists built next
+  }
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* cnt, int* start, int* part,
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* cnt, int
 __global__ void __launch_bounds__(kScanThreads) k_scan_finish(int* cnt, int* start, const int* part,
                                                               int ncell, int n_tot,
                                                               const RepDev* last,
-                                                              const int* gate) {
+                                                              const int* gate, int* overflow) {
   __shared__ int ws[33];
   chain_begin();
   if (gate && !*gate) return;
@@ -279,24 +284,28 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_finish(int* cnt, int* sta
       cnt[base + k] = 0;  // ready for the next binning
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) start[ncell] = last ? last->row_off + last->n : n_tot;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    start[ncell] = last ? last->row_off + last->n : n_tot;
+    if (overflow) *overflow = 0;  // of the lists built next
+  }
 }
 
 static void launch_scan_of(int* cnt, int* start, int* part, int ncell, int n_tot,
-                           const RepDev* last, const int* gate, const Chain& st) {
+                           const RepDev* last, const int* gate, int* overflow, const Chain& st) {
   if (ncell <= kScanOneBlock) {
-    launch(st, k_scan_small, 1, kScanThreads, 0, cnt, start, ncell, n_tot, last, gate);
+    launch(st, k_scan_small, 1, kScanThreads, 0, cnt, start, ncell, n_tot, last, gate, overflow);
     return;
   }
   const int nb = (ncell + kScanTile - 1) / kScanTile;
   launch(st, k_scan_tiles, nb, kScanThreads, 0, cnt, start, part, ncell, gate);
   launch(Chain(st.st, true), k_scan_finish, nb, kScanThreads, 0, cnt, start, part, ncell, n_tot,
-         last, gate);
+         last, gate, overflow);
 }
 
 void launch_scan(const DevState& d, int ncell_tot, int last_rep, const Chain& st,
                  const int* gate) {
-  launch_scan_of(d.cell_cnt, d.cell_start, d.scan_part, ncell_tot, 0, d.reps + last_rep, gate, st);
+  launch_scan_of(d.cell_cnt, d.cell_start, d.scan_part, ncell_tot, 0, d.reps + last_rep, gate,
+                 d.overflow, st);
 }
 
 // ------------------------------------------------- scatter / sort / pack
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, int zero, const 
 }
 
 void launch_scan_raw(int* cnt, int* start, int* part, int ncell, int n_tot, cudaStream_t st) {
-  launch_scan_of(cnt, start, part, ncell, n_tot, nullptr, nullptr, st);
+  launch_scan_of(cnt, start, part, ncell, n_tot, nullptr, nullptr, nullptr, st);
 }
 
 void launch_cell_sort_raw(uint32_t* perm, const int* start, int ncell, cudaStream_t st) {

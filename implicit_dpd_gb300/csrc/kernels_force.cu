@@ -1,6 +1,8 @@
 // Pass 2 of the FP32 engine, CalcForceEpEpDPD::operator()
 // (nbdf_calculator.hpp:63-145) with each pair taken once, by the particle
 // that owns it, over the pass-1 lists; and the dispatch of every pass-2 arm.
+#include <algorithm>
+
 #include "pair_lists.cuh"
 
 namespace idpd {
@@ -110,9 +112,7 @@ __device__ __forceinline__ void quad_both(const float w[4], const int t[4], int 
     if (BIG) {
       x = fix_force(w[j]);
     } else {
-      int h, l;
-      fix_force_parts(w[j], h, l);
-      x = mad_wide(h, 1 << 21, (long long)l);
+      x = fix_force_small(w[j]);
     }
     S = VIRIAL ? S + x : S - x;
     red_add_if(j < lim, sums + 4 * (size_t)t[j], x);
@@ -496,21 +496,25 @@ __global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk, int
 }
 
 // Pass 2 of the particles whose list overflowed (force_walk_rows), one warp
-// per 32-row chunk, 128-row blocks per CTA; a chunk without such a particle
-// costs one read of its list lengths.
+// per 32-row chunk; a few CTAs per SM stride over the row blocks and leave at once
+// when no list did.
 template <int REACH, bool PRESS, int FORM>
 __global__ void __launch_bounds__(kRowBlock) k_force_walk(DevState d, int kept, int nblk) {
   __shared__ ForceBlockSmem B;
   __shared__ ForceWarpSmem W[kWarps];
   chain_begin();
+  if (!d.overflow[1]) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int rb = blockIdx.x;
-  const int r = d.blk_rep[rb];
-  const RepDev* R = d.reps + r;
-  if (threadIdx.x < 9) fill_pair_table(B.T, *R, threadIdx.x);
-  __syncthreads();
-  if (R->form != FORM) return;
-  force_walk_rows<REACH, PRESS, FORM>(d, kept, d.blk_row[rb] + 32 * wid, r, R, B.T, W[wid], lane);
+  for (int rb = blockIdx.x; rb < nblk; rb += gridDim.x) {
+    const int r = d.blk_rep[rb];
+    const RepDev* R = d.reps + r;
+    __syncthreads();
+    if (threadIdx.x < 9) fill_pair_table(B.T, *R, threadIdx.x);
+    __syncthreads();
+    if (R->form == FORM)
+      force_walk_rows<REACH, PRESS, FORM>(d, kept, d.blk_row[rb] + 32 * wid, r, R, B.T, W[wid],
+                                          lane);
+  }
 }
 
 // Pass 2 of one pair form: the shape of the tuning (lanes per particle,
@@ -521,7 +525,8 @@ void launch_force_kernel(const DevState& d, int nblk, int kept, int fb, const Ch
   const int rows = chunk_rows(nblk, LP);
   launch(st, k_force_f32<PRESS, FORM, LP>, dim3((nblk + fb - 1) / fb, 32 / rows), kRowBlock * fb,
          force_smem_bytes(fb), d, nblk, rows);
-  launch(Chain(st.st, true), k_force_walk<REACH, PRESS, FORM>, nblk, kRowBlock, 0, d, kept, nblk);
+  launch(Chain(st.st, true), k_force_walk<REACH, PRESS, FORM>, std::min(nblk, kRareBlocks),
+         kRowBlock, 0, d, kept, nblk);
 }
 
 template <int FORM, bool PRESS, int LP>

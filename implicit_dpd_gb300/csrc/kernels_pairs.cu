@@ -140,7 +140,10 @@ __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int 
                reinterpret_cast<long long*>(d.dsum + (sl < 3 ? sl : 0) * d.dstride + s), (long long)q);
     if (MARKS) hit = (__ballot_sync(0xffffffffu, hit) & gmask) != 0u;
     if (sl == 0 && act) {
-      if (!KNOWN) d.nbn[s] = nl <= kNbrCap ? (uint16_t)nl : (uint16_t)kNbrFallback;
+      if (!KNOWN) {
+        d.nbn[s] = nl <= kNbrCap ? (uint16_t)nl : (uint16_t)kNbrFallback;
+        if (nl > kNbrCap) d.overflow[1] = 1;
+      }
       d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
       if (MARKS && hit) d.phit[s] = 1;
     }
@@ -155,130 +158,86 @@ static_assert((long long)kVerletCap * (1ll << 23) <= (1ll << 32) &&
 // pairs within the cutoff 1 to a list in shared memory; phase B takes the density
 // weights from that list with every lane busy and copies the list out for pass 2 (a
 // particle whose list overflows takes its weights during a second sweep). Shared
-// memory: per warp the neighbour segments and the list (dens_sweep_smem_bytes).
+// memory: per warp the neighbour segments and the list (dens_sweep_smem_bytes). A few
+// CTAs per SM stride over the row blocks and leave at once when the build had no such
+// list: with a CTA per row block, reading the list lengths, the empty pass took 12 us
+// at 10^6 particles (and pass 2's walk of its overflowed lists 16).
 constexpr size_t dens_sweep_smem_bytes() {
   return kWarps * (sizeof(SegTable) + kNbrCap * sizeof(uint32_t));
 }
 
 template <int REACH, bool VERLET, bool MARKS>
-__global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d) {
+__global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk) {
   extern __shared__ __align__(16) unsigned char dens_smem[];
   chain_begin();
-  const int r = d.blk_rep[blockIdx.x];
-  const RepDev* R = d.reps + r;
+  if (!d.overflow[0]) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   SegTable& S = reinterpret_cast<SegTable*>(dens_smem)[wid];
   uint32_t* L = reinterpret_cast<uint32_t*>(dens_smem + kWarps * sizeof(SegTable)) + wid * kNbrCap;
-  const int s0 = d.blk_row[blockIdx.x] + 32 * wid;
-  const int s_end = min(s0 + 32, R->row_off + R->n);
-  const uint16_t* len = VERLET ? d.vn : d.nbn;
-  uint32_t todo = __ballot_sync(0xffffffffu, s0 + lane < s_end && len[s0 + lane] == kNbrFallback);
-  const bool warren = R->form == IDPD_FORM_WARREN_K;
-  const float cutd2 = R->wrd * R->wrd;  // density cutoff^2 (1 unless Warren)
-  const double cutd2d = (double)R->wrd * (double)R->wrd;
-  const float inv_rd = R->winv_rd, wnorm = R->wnorm, pre = R->dens_prescale;
-  const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
-  const bool prec = MARKS && R->prec_on;
-  constexpr int nseg = 2 * (2 * REACH + 1) * (2 * REACH + 1);
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  int cached = -1;
-  for (; todo; todo &= todo - 1) {
-    const int s = s0 + __ffs(todo) - 1;
-    const float4 pi = d.posf[s];
-    const uint32_t si = d.perm[s], pri = fbits(pi.w);
-    const float ki = VERLET ? d.okey[s] : pi.x;  // the ownership key of the step
-    int nl = 0;  // owned pairs within the cutoff
-    bool hit = false;
-    uint32_t q0 = 0, q1 = 0, q2 = 0;
-    // weight of one owned candidate, to both particles; called by every lane
-    // together (valid = false for lanes without one) so that the rare FP64
-    // recheck is warp-uniform
-    auto test = [&](bool valid, int t, int dx, int dy, int dz, float4 pj, bool list_known) {
-      const float ex = (pi.x - (float)dx * csx) - pj.x;
-      const float ey = (pi.y - (float)dy * csy) - pj.y;
-      const float ez = (pi.z - (float)dz * csz) - pj.z;
-      const float dr2 = dist2(ex, ey, ez);
-      bool in1 = valid && (list_known || dr2 < 1.0f);
-      bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
-      const bool near1 = valid && !list_known && fabsf(dr2 - 1.0f) <= kGuard;
-      const bool near2 = valid && ((warren && fabsf(dr2 - cutd2) <= kGuard) || dr2 < 1.0e-10f);
-      if (__any_sync(0xffffffffu, near1 || near2)) {
-        if (near1 || near2) {
-          const double e2 = exact_dr2(d, R, si, d.perm[t]);
-          if (near1) in1 = e2 < 1.0;
-          ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
-        }
-      }
-      const uint32_t prj = fbits(pj.w);
-      if (ind) {
-        const uint32_t w = dens_weight(dr2, warren, inv_rd, wnorm, pre);
-        add_weight(q0, q1, q2, prj, w);
-        atomicAdd(d.dsum + (pri & 3u) * d.dstride + t, (unsigned long long)w);
-      }
-      if (MARKS && prec && in1) {
-        hit |= pri == R->prec_from && prj == R->prec_near;
-        if (prj == R->prec_from && pri == R->prec_near) d.phit[t] = 1;
-      }
-    };
-    const int cell = (int)d.scell[s];
-    if (cell != cached) {
-      int cx, cy, cz;
-      cell_xyz(cell - R->cell_off, R->nc, cx, cy, cz);
-      __syncwarp();
-      build_segments(S, d, R, cx, cy, cz, lane);
-      __syncwarp();
-      cached = cell;
-    }
-    // ---- phase A: the owned pairs within the cutoff 1
-#pragma unroll 1
-    for (int g = 0; g < nseg; g++) {
-      const int tb = S.tb[g], te = S.te[g];
-      if (tb >= te) continue;
-      const int code = S.code[g];
-      int b[2 * REACH];
-#pragma unroll
-      for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
-      const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
-      const float by = pi.y - (float)dy * csy, bz = pi.z - (float)dz * csz;
-      for (int t0 = tb; t0 < te; t0 += 32) {
-        const int t = t0 + lane;
-        bool in1 = false, near = false;
-        int ddx = 0;
-        if (t < te && t != s) {
-          const float4 pj = __ldg(d.posf + t);
-          ddx = frame_step<REACH>(t, b);
-          if (owns(fx0 + ddx, VERLET ? d.okey[t] : pj.x, ki, t, s)) {
-            const float dr2 =
-                dist2((pi.x - (float)(fx0 + ddx) * csx) - pj.x, by - pj.y, bz - pj.z);
-            in1 = dr2 < 1.0f;
-            near = fabsf(dr2 - 1.0f) <= kGuard;
+  for (int rb = blockIdx.x; rb < nblk; rb += gridDim.x) {
+    const int r = d.blk_rep[rb];
+    const RepDev* R = d.reps + r;
+    const int s0 = d.blk_row[rb] + 32 * wid;
+    const int s_end = min(s0 + 32, R->row_off + R->n);
+    const uint16_t* len = VERLET ? d.vn : d.nbn;
+    uint32_t todo = __ballot_sync(0xffffffffu, s0 + lane < s_end && len[s0 + lane] == kNbrFallback);
+    const bool warren = R->form == IDPD_FORM_WARREN_K;
+    const float cutd2 = R->wrd * R->wrd;  // density cutoff^2 (1 unless Warren)
+    const double cutd2d = (double)R->wrd * (double)R->wrd;
+    const float inv_rd = R->winv_rd, wnorm = R->wnorm, pre = R->dens_prescale;
+    const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
+    const bool prec = MARKS && R->prec_on;
+    constexpr int nseg = 2 * (2 * REACH + 1) * (2 * REACH + 1);
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    int cached = -1;
+    for (; todo; todo &= todo - 1) {
+      const int s = s0 + __ffs(todo) - 1;
+      const float4 pi = d.posf[s];
+      const uint32_t si = d.perm[s], pri = fbits(pi.w);
+      const float ki = VERLET ? d.okey[s] : pi.x;  // the ownership key of the step
+      int nl = 0;  // owned pairs within the cutoff
+      bool hit = false;
+      uint32_t q0 = 0, q1 = 0, q2 = 0;
+      // weight of one owned candidate, to both particles; called by every lane
+      // together (valid = false for lanes without one) so that the rare FP64
+      // recheck is warp-uniform
+      auto test = [&](bool valid, int t, int dx, int dy, int dz, float4 pj, bool list_known) {
+        const float ex = (pi.x - (float)dx * csx) - pj.x;
+        const float ey = (pi.y - (float)dy * csy) - pj.y;
+        const float ez = (pi.z - (float)dz * csz) - pj.z;
+        const float dr2 = dist2(ex, ey, ez);
+        bool in1 = valid && (list_known || dr2 < 1.0f);
+        bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
+        const bool near1 = valid && !list_known && fabsf(dr2 - 1.0f) <= kGuard;
+        const bool near2 = valid && ((warren && fabsf(dr2 - cutd2) <= kGuard) || dr2 < 1.0e-10f);
+        if (__any_sync(0xffffffffu, near1 || near2)) {
+          if (near1 || near2) {
+            const double e2 = exact_dr2(d, R, si, d.perm[t]);
+            if (near1) in1 = e2 < 1.0;
+            ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
           }
         }
-        if (__any_sync(0xffffffffu, near)) {
-          if (near) in1 = exact_dr2(d, R, si, d.perm[t]) < 1.0;
+        const uint32_t prj = fbits(pj.w);
+        if (ind) {
+          const uint32_t w = dens_weight(dr2, warren, inv_rd, wnorm, pre);
+          add_weight(q0, q1, q2, prj, w);
+          atomicAdd(d.dsum + (pri & 3u) * d.dstride + t, (unsigned long long)w);
         }
-        const uint32_t mask = __ballot_sync(0xffffffffu, in1);
-        if (in1) {
-          const int pos = nl + __popc(mask & lt_mask);
-          if (pos < kNbrCap) L[pos] = make_entry(t, fx0 + ddx, dy, dz);
+        if (MARKS && prec && in1) {
+          hit |= pri == R->prec_from && prj == R->prec_near;
+          if (prj == R->prec_from && pri == R->prec_near) d.phit[t] = 1;
         }
-        nl += __popc(mask);
+      };
+      const int cell = (int)d.scell[s];
+      if (cell != cached) {
+        int cx, cy, cz;
+        cell_xyz(cell - R->cell_off, R->nc, cx, cy, cz);
+        __syncwarp();
+        build_segments(S, d, R, cx, cy, cz, lane);
+        __syncwarp();
+        cached = cell;
       }
-    }
-    __syncwarp();
-    const bool fits = nl <= kNbrCap;
-    // ---- phase B: density weights
-    if (fits) {
-      for (int k0 = 0; k0 < nl; k0 += 32) {
-        const int k = k0 + lane;
-        const bool valid = k < nl;
-        int t = s, dx = 0, dy = 0, dz = 0;
-        if (valid) read_entry(L[k], t, dx, dy, dz);
-        test(valid, t, dx, dy, dz, valid ? __ldg(d.posf + t) : pi, true);
-      }
-    } else {
-      // a lane takes at most nseg + nl / 32 weights below 2^23 each
-      if (nl > kDensPairsMax && lane == 0) atomicCAS(d.err, 0, kErrDensPairs);
+      // ---- phase A: the owned pairs within the cutoff 1
 #pragma unroll 1
       for (int g = 0; g < nseg; g++) {
         const int tb = S.tb[g], te = S.te[g];
@@ -288,37 +247,88 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d) {
 #pragma unroll
         for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
         const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
+        const float by = pi.y - (float)dy * csy, bz = pi.z - (float)dz * csz;
         for (int t0 = tb; t0 < te; t0 += 32) {
           const int t = t0 + lane;
-          const int dx = fx0 + frame_step<REACH>(t, b);
-          const float4 pj = t < te ? __ldg(d.posf + t) : pi;
-          const bool valid = t < te && t != s && owns(dx, VERLET ? d.okey[t] : pj.x, ki, t, s);
-          test(valid, valid ? t : s, dx, dy, dz, pj, false);
+          bool in1 = false, near = false;
+          int ddx = 0;
+          if (t < te && t != s) {
+            const float4 pj = __ldg(d.posf + t);
+            ddx = frame_step<REACH>(t, b);
+            if (owns(fx0 + ddx, VERLET ? d.okey[t] : pj.x, ki, t, s)) {
+              const float dr2 =
+                  dist2((pi.x - (float)(fx0 + ddx) * csx) - pj.x, by - pj.y, bz - pj.z);
+              in1 = dr2 < 1.0f;
+              near = fabsf(dr2 - 1.0f) <= kGuard;
+            }
+          }
+          if (__any_sync(0xffffffffu, near)) {
+            if (near) in1 = exact_dr2(d, R, si, d.perm[t]) < 1.0;
+          }
+          const uint32_t mask = __ballot_sync(0xffffffffu, in1);
+          if (in1) {
+            const int pos = nl + __popc(mask & lt_mask);
+            if (pos < kNbrCap) L[pos] = make_entry(t, fx0 + ddx, dy, dz);
+          }
+          nl += __popc(mask);
         }
       }
-    }
-    __syncwarp();
-    if (fits) {  // list out for pass 2, coalesced
-      uint32_t* out = d.nbl + (size_t)s * kNbrCap;
-      for (int k = lane; k < nl; k += 32) out[k] = L[k];
-    }
-    unsigned long long a0 = q0, a1 = q1, a2 = q2;
+      __syncwarp();
+      const bool fits = nl <= kNbrCap;
+      // ---- phase B: density weights
+      if (fits) {
+        for (int k0 = 0; k0 < nl; k0 += 32) {
+          const int k = k0 + lane;
+          const bool valid = k < nl;
+          int t = s, dx = 0, dy = 0, dz = 0;
+          if (valid) read_entry(L[k], t, dx, dy, dz);
+          test(valid, t, dx, dy, dz, valid ? __ldg(d.posf + t) : pi, true);
+        }
+      } else {
+        // a lane takes at most nseg + nl / 32 weights below 2^23 each
+        if (nl > kDensPairsMax && lane == 0) atomicCAS(d.err, 0, kErrDensPairs);
+#pragma unroll 1
+        for (int g = 0; g < nseg; g++) {
+          const int tb = S.tb[g], te = S.te[g];
+          if (tb >= te) continue;
+          const int code = S.code[g];
+          int b[2 * REACH];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-      a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-      a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+          for (int q = 0; q < 2 * REACH; q++) b[q] = S.bnd[g][q];
+          const int fx0 = (code & 7) - 4, dy = ((code >> 3) & 7) - 4, dz = ((code >> 6) & 7) - 4;
+          for (int t0 = tb; t0 < te; t0 += 32) {
+            const int t = t0 + lane;
+            const int dx = fx0 + frame_step<REACH>(t, b);
+            const float4 pj = t < te ? __ldg(d.posf + t) : pi;
+            const bool valid = t < te && t != s && owns(dx, VERLET ? d.okey[t] : pj.x, ki, t, s);
+            test(valid, valid ? t : s, dx, dy, dz, pj, false);
+          }
+        }
+      }
+      __syncwarp();
+      if (fits) {  // list out for pass 2, coalesced
+        uint32_t* out = d.nbl + (size_t)s * kNbrCap;
+        for (int k = lane; k < nl; k += 32) out[k] = L[k];
+      }
+      unsigned long long a0 = q0, a1 = q1, a2 = q2;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+      }
+      if (MARKS) hit = __any_sync(0xffffffffu, hit);
+      if (lane == 0) {
+        if (a0) atomicAdd(d.dsum + s, a0);
+        if (a1) atomicAdd(d.dsum + d.dstride + s, a1);
+        if (a2) atomicAdd(d.dsum + 2 * d.dstride + s, a2);
+        d.nbn[s] = fits ? (uint16_t)nl : (uint16_t)kNbrFallback;
+        if (!fits) d.overflow[1] = 1;
+        d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
+        if (MARKS && hit) d.phit[s] = 1;
+      }
+      __syncwarp();
     }
-    if (MARKS) hit = __any_sync(0xffffffffu, hit);
-    if (lane == 0) {
-      if (a0) atomicAdd(d.dsum + s, a0);
-      if (a1) atomicAdd(d.dsum + d.dstride + s, a1);
-      if (a2) atomicAdd(d.dsum + 2 * d.dstride + s, a2);
-      d.nbn[s] = fits ? (uint16_t)nl : (uint16_t)kNbrFallback;
-      d.npair[s] = 2u * (uint32_t)nl;  // ordered pairs: each owned pair counts twice
-      if (MARKS && hit) d.phit[s] = 1;
-    }
-    __syncwarp();
   }
 }
 
@@ -549,6 +559,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
       __syncwarp();
       if (lane < nb) {
         (KEPT ? d.vn : d.nbn)[me] = cnt <= cap ? (uint16_t)cnt : (uint16_t)kNbrFallback;
+        if (cnt > cap) d.overflow[0] = 1;
         if (KEPT) {
           d.okey[me] = pm.x;
           const uint32_t i = d.perm[me];
@@ -652,7 +663,8 @@ void launch_density_f32(const DevState& d, int nblk, int lanes, int form_mask, C
     launch_density_lists<MARKS, false, !VERLET>(d, nblk, lanes, st);
     st.chained = true;
   }
-  launch(st, k_density_over<REACH, VERLET, MARKS>, nblk, kRowBlock, dens_sweep_smem_bytes(), d);
+  launch(st, k_density_over<REACH, VERLET, MARKS>, std::min(nblk, kRareBlocks), kRowBlock,
+         dens_sweep_smem_bytes(), d, nblk);
 }
 
 template <bool MARKS>

@@ -239,6 +239,9 @@ inline int build_rows(int nblk) {
   return rows;
 }
 
+// CTAs of the passes over rows whose lists overflowed (8 per SM).
+constexpr int kRareBlocks = 1216;
+
 // Visits every neighbour cell within the stencil of the given reach
 // (plain FP64 kernels and the centre-of-mass pass).
 template <class F>
@@ -266,13 +269,6 @@ __device__ __forceinline__ void red_add(long long* p, long long v) {
 __device__ __forceinline__ void red_add_if(bool p, long long* a, long long v) {
   asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p red.global.add.u64 [%0], %1;\n}\n"
                ::"l"(a), "l"(v), "r"((int)p) : "memory");
-}
-
-// a b + c in 64 bits.
-__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
-  long long d;
-  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-  return d;
 }
 
 }  // namespace idpd
