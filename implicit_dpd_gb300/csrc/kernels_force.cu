@@ -100,23 +100,26 @@ __device__ __forceinline__ void quad_components(float x, float y, float z, int c
 // same for both, +x) and the sum of the other particle of pair j, row t[j], x by
 // atomic add. The three lanes of a quad that hold x, y and z address one row at a
 // time, so a row's three adds leave the SM as one access of its 32-byte sector.
-// BIG: some term of the warp may reach +-65536 (the bit-level conversion).
-// lim: pairs of the quad that exist (0 on the lane without a component); sums
-// points at component c of row 0.
-template <bool VIRIAL, bool BIG>
+// The terms are below 65536. lim: pairs of the quad that exist (0 on the lane without a
+// component); sums points at component c of row 0.
+template <bool VIRIAL>
 __device__ __forceinline__ void quad_both(const float w[4], const int t[4], int lim,
                                           long long* sums, long long& S) {
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    long long x;
-    if (BIG) {
-      x = fix_force(w[j]);
-    } else {
-      x = fix_force_small(w[j]);
-    }
+    const long long x = fix_force_small(w[j]);
     S = VIRIAL ? S + x : S - x;
     red_add_if(j < lim, sums + 4 * (size_t)t[j], x);
   }
+}
+
+// A term too large for the fast conversion (or none at all: NaN), one lane on its own:
+// v goes to the other particle's sum, -v (VIRIAL: v) to the owner's.
+template <bool VIRIAL>
+__device__ __forceinline__ void big_both(float v, long long* owner, long long* other) {
+  const long long x = fix_force(v);
+  red_add(other, x);
+  red_add(owner, VIRIAL ? x : -x);
 }
 
 // One owned pair of a pass-1 list (fast path of pass 2), given the other
@@ -175,11 +178,11 @@ __device__ __forceinline__ bool pair_terms(const DevState& d, const RepDev* R, c
   float ex = (I.pi.x - (float)dx * R->cs_f[0]) - pj.x;
   float ey = (I.pi.y - (float)dy * R->cs_f[1]) - pj.y;
   float ez = (I.pi.z - (float)dz * R->cs_f[2]) - pj.z;
-  float dr2 = ex * ex + ey * ey + ez * ez;
+  float dr2 = dist2(ex, ey, ez);
   if (dr2 < kCloseCut2) {
     close_pair_vector(I.pi, __ldg(d.poslo + I.row), pj, __ldg(d.poslo + t), dx, dy, dz, R, ex, ey,
                       ez);
-    dr2 = ex * ex + ey * ey + ez * ez;
+    dr2 = dist2(ex, ey, ez);
   }
   const float inv_dr = rsqrt_approx(dr2);
   const float dr = dr2 * inv_dr;
@@ -187,7 +190,7 @@ __device__ __forceinline__ bool pair_terms(const DevState& d, const RepDev* R, c
   if (dr2 > kNearCut2)  // admitted pairs have 1 - r >= 0 up to ~1e-13
     w = fmaxf(near_cut_w(I.pi, __ldg(d.poslo + I.row), pj, __ldg(d.poslo + t), dx, dy, dz, R, dr),
               0.0f);
-  const float a = pair_cf<FORM, PRESS>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
+  const float a = pair_cf<FORM, false>(T, R, I.pri, fbits(pj.w), dr, inv_dr, w, ex, ey, ez, I.vi, vj,
                                 I.di, dj, I.idi, idj, I.seed);
   if (!isfinite(a)) atomicCAS(d.err, 0, kErrNonFinite);
   g[0] = a * ex;
@@ -283,7 +286,8 @@ size_t force_smem_bytes(int fb) { return (size_t)fb * sizeof(ForceBlockSmem); }
 // L1 76 % busy. With the terms turned inside each quad of lanes (quad_components), one
 // instruction adds x, y and z of eight rows in eight sectors: a third of the sectors,
 // atomic unit 16 %, long-scoreboard stalls 4.3 -> 2.4 per issue, L1 hit rate 22 -> 39 %;
-// 984k-bead membrane 976 -> 836 us, 998k-particle liquid 248 -> 207 us. A register cap
+// 984k-bead membrane 976 -> 836 us, 998k-particle liquid 248 -> 207 us (786 and 174 with
+// the cheaper conversion and with large terms taken out of the common path). A register cap
 // of 72 or 92 instead of 64 (7 or 5 CTAs per SM) gave 852 and 935 us on that membrane.
 //
 // Pass 2 over the rows s0 .. s0 + rows - 1 of replica r (one warp's chunk, rows
@@ -325,29 +329,34 @@ __device__ __forceinline__ void force_rows(const DevState& d, int s0, int rows, 
       if (k + LP < nu) e_next = __ldg(list + k + LP);
       const int t = (int)(e & kRowMask);
       float ex, ey, ez;
-      const float an = owned_pair<PRESS, FORM>(d, R, T, OT, I, e, valid, __ldg(d.posf + t),
+      float an = owned_pair<PRESS, FORM>(d, R, T, OT, I, e, valid, __ldg(d.posf + t),
                                         __ldg(d.velf + t), __ldg(d.densf + t), ex, ey, ez);
+      // |e| <= 1 up to rounding: below this no component reaches 65536
+      const bool big = !(fabsf(an) < 60000.0f);
+      if (__any_sync(0xffffffffu, big)) {
+        if (big) {
+          if (!isfinite(an)) atomicCAS(d.err, 0, kErrNonFinite);
+          const float g[3] = {an * ex, an * ey, an * ez}, x[3] = {ex, ey, ez};
+#pragma unroll
+          for (int q = 0; q < 3; q++) {
+            big_both<false>(g[q], d.fq + 4 * (size_t)s + q, d.fq + 4 * (size_t)t + q);
+            if (PRESS)
+              big_both<true>(-g[q] * x[q], d.pq + 4 * (size_t)s + q, d.pq + 4 * (size_t)t + q);
+          }
+          an = 0.0f;
+        }
+      }
       const float gx = an * ex, gy = an * ey, gz = an * ez;
       int tq[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) tq[j] = __shfl_sync(0xffffffffu, t, j, 4);
       const int lim = c < 3 ? nu - (k - c) : 0;
-      // |e| <= 1 up to rounding: below this no component reaches 65536
-      const bool big = __any_sync(0xffffffffu, !(fabsf(an) < 60000.0f));
       float w[4];
       quad_components(gx, gy, gz, c, w);
-      if (!big) {
-        quad_both<false, false>(w, tq, lim, d.fq + c, F);
-      } else {
-        if (!isfinite(an)) atomicCAS(d.err, 0, kErrNonFinite);
-        quad_both<false, true>(w, tq, lim, d.fq + c, F);
-      }
+      quad_both<false>(w, tq, lim, d.fq + c, F);
       if (PRESS) {  // the virial a e e, the same for both particles
         quad_components(-gx * ex, -gy * ey, -gz * ez, c, w);
-        if (!big)
-          quad_both<true, false>(w, tq, lim, d.pq + c, V);
-        else
-          quad_both<true, true>(w, tq, lim, d.pq + c, V);
+        quad_both<true>(w, tq, lim, d.pq + c, V);
       }
     }
     F = group_total<LP>(F);
