@@ -326,13 +326,17 @@ class Engine:
                                             C.cast(pj, C.c_void_p), _p(nj)), "dispatch_walks")
 
     def retrieve_walks(self, kind, tag=0):
-        """RetrieveKernel: one record array of WALK_DTYPES[kind][2] per walk."""
+        """RetrieveKernel: one record array of WALK_DTYPES[kind][2] per walk, all
+        slices of one array, walk after walk."""
         ni = self._walk_ni
-        out = [np.zeros(int(k), WALK_DTYPES[kind][2]) for k in ni]
-        ptrs = (C.c_void_p * max(len(out), 1))(*[a.ctypes.data for a in out])
-        self._ck(self.L.idpd_retrieve_walks(self.h, kind, tag, len(out), _p(ni),
-                                            C.cast(ptrs, C.c_void_p)), "retrieve_walks")
-        return out
+        ends = np.cumsum(ni, dtype=np.int64)
+        total = int(ends[-1]) if len(ni) else 0
+        rec = np.zeros(total, WALK_DTYPES[kind][2])
+        ptr = rec.ctypes.data + (ends - ni) * rec.itemsize if len(ni) else np.zeros(1, np.int64)
+        ptr = np.ascontiguousarray(ptr, np.uintp)
+        self._ck(self.L.idpd_retrieve_walks(self.h, kind, tag, len(ni), _p(ni), _p(ptr)),
+                 "retrieve_walks")
+        return [rec[e - k:e] for e, k in zip(ends.tolist(), ni.tolist())]
 
     def set_tuning(self, reach, skin=None, lanes=None, blocks=None, dens_lanes=None):
         """reach 1 or 2; skin > 0 keeps the neighbour lists between rebuilds;
