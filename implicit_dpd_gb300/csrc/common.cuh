@@ -287,6 +287,17 @@ __device__ __forceinline__ long long fix_force(float v) {
   return ((long long)hi << 21) + (long long)lo;
 }
 
+// fix_from_float(v, 40) for |v| < 8: a float from 2^-17 on is a multiple of 2^-40, and its
+// two parts (2^-19 and the rest) are exact.
+__device__ __forceinline__ long long fix_pos(float v) {
+  if (fabsf(v) < 7.62939453125e-6f) return fix_from_float(v, kPosBits);
+  const float magic = 12582912.0f;  // 1.5 * 2^23: bits 602 * 2^21
+  const float a = fmaf(v, 524288.0f, magic);
+  const float r = fmaf(-(a - magic), 1.9073486328125e-6f, v);
+  const uint32_t lo = __float_as_uint(fmaf(r, 1099511627776.0f, magic));
+  return ((long long)(__float_as_int(a) - (0x4B400000 + 602)) << 21) + (long long)(unsigned long long)lo;
+}
+
 // Fixed-point sum to double, exactly for |q| < 2^51: the integer is added
 // into the mantissa of 1.5 * 2^52 and the bias removed with one FP64 add
 // (an int64-to-double conversion is a slower FP64-pipe instruction).

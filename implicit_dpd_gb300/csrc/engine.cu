@@ -1275,68 +1275,52 @@ int idpd_download_aux(idpd_handle* h, int32_t r, double* density, double* press,
   const RepDev& R = h->reps_h[r];
   const int n = R.n;
   if (n == 0) return IDPD_OK;
-  std::vector<uint32_t> orig(n), perm(n);
-  CK(cudaMemcpyAsync(orig.data(), h->d.orig + R.row_off, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  auto scatter3 = [&](const std::vector<double>& src, double* out, int w) {
-    for (int q = 0; q < n; q++)
-      for (int k = 0; k < w; k++)
-        out[(size_t)w * (orig[q] - (uint32_t)R.row_off) + k] = src[(size_t)w * q + k];
+  // each field is gathered into upload order on the device, host buffers through the
+  // staging buffer (9 n doubles: a field's first use of a part waits for its last copy)
+  double* stage = h->xfer;
+  auto gather = [&](double* out, int width, auto&& launch_into) -> int {
+    double* view = static_cast<double*>(const_cast<void*>(device_view(out)));
+    if (stage + (size_t)width * n > h->xfer + 9 * (size_t)n) stage = h->xfer;
+    double* to = view ? view : stage;
+    launch_into(to);
+    CK(cudaGetLastError());
+    if (view) return IDPD_OK;
+    stage += (size_t)width * n;
+    CK(cudaMemcpyAsync(out, to, sizeof(double) * width * n, cudaMemcpyDeviceToHost, h->st));
+    return IDPD_OK;
   };
-  if (density && h->density_valid && h->d.dens64 && pair_mode(h) != kPairsF32) {
-    // the FP64 arms: their FP64 densities (sorted order), unrounded
-    std::vector<double> ds(3 * (size_t)n);
-    CK(cudaMemcpyAsync(perm.data(), h->d.perm + R.row_off, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemcpyAsync(ds.data(), h->d.dens64 + 3 * (size_t)R.row_off, sizeof(double) * 3 * n,
-                       cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    std::vector<double> byrow(3 * (size_t)n);
-    for (int sidx = 0; sidx < n; sidx++) {
-      const int row = (int)perm[sidx] - R.row_off;
-      for (int k = 0; k < 3; k++) byrow[3 * (size_t)row + k] = ds[3 * (size_t)sidx + k];
-    }
-    scatter3(byrow, density, 3);
-  } else if (density) {
-    if (!h->density_valid || !h->d.dqx) return fail(h, IDPD_ERR_STATE, "run idpd_density first");
-    std::vector<long long> q[3];
-    const long long* src[3] = {h->d.dqx, h->d.dqy, h->d.dqz};
-    CK(cudaMemcpyAsync(perm.data(), h->d.perm + R.row_off, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, h->st));
-    for (int k = 0; k < 3; k++) {
-      q[k].resize(n);
-      CK(cudaMemcpyAsync(q[k].data(), src[k] + R.row_off, sizeof(long long) * n, cudaMemcpyDeviceToHost, h->st));
-    }
-    CK(cudaStreamSynchronize(h->st));
-    std::vector<double> byrow(3 * (size_t)n);
-    for (int sidx = 0; sidx < n; sidx++) {
-      const int row = (int)perm[sidx] - R.row_off;
-      for (int k = 0; k < 3; k++) byrow[3 * (size_t)row + k] = (double)q[k][sidx] * R.dens_unscale;
-    }
-    scatter3(byrow, density, 3);
+  const DevState& d = h->d;
+  int rc = IDPD_OK;
+  if (density) {
+    const bool f64 = d.dens64 && pair_mode(h) != kPairsF32;  // the FP64 arms' own, unrounded
+    if (!h->density_valid || (!f64 && !d.dqx))
+      return fail(h, IDPD_ERR_STATE, "run idpd_density first");
+    rc = gather(density, 3, [&](double* to) {
+      launch_gather_density(d, f64 ? d.dens64 : nullptr, R.dens_unscale, R.row_off, to, n, h->st);
+    });
+    if (rc) return rc;
   }
   if (press) {
     if (!h->press64) return fail(h, IDPD_ERR_STATE, "run idpd_force first");
-    std::vector<double> b(3 * (size_t)n);
-    CK(cudaMemcpyAsync(b.data(), h->press64 + 3 * (size_t)R.row_off, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    scatter3(b, press, 3);
+    rc = gather(press, 3, [&](double* to) {
+      launch_gather_records(h->press64, 3, d.loc, R.row_off, to, n, h->st);
+    });
+    if (rc) return rc;
   }
   if (nei_cm) {
     if (!h->cm64) return fail(h, IDPD_ERR_STATE, "run idpd_density first");
-    std::vector<double> b(6 * (size_t)n);
-    CK(cudaMemcpyAsync(b.data(), h->cm64 + 6 * (size_t)R.row_off, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    scatter3(b, nei_cm, 6);
+    rc = gather(nei_cm, 6, [&](double* to) {
+      launch_gather_records(h->cm64, 6, d.loc, R.row_off, to, n, h->st);
+    });
+    if (rc) return rc;
   }
   if (delta_sumr) {
-    std::vector<double> b(3 * (size_t)n), t(n);
-    const double* src[3] = {h->d.dsx, h->d.dsy, h->d.dsz};
-    for (int k = 0; k < 3; k++) {
-      CK(cudaMemcpyAsync(t.data(), src[k] + R.row_off, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
-      CK(cudaStreamSynchronize(h->st));
-      for (int q = 0; q < n; q++) b[3 * (size_t)q + k] = t[q];
-    }
-    scatter3(b, delta_sumr, 3);
+    rc = gather(delta_sumr, 3, [&](double* to) {
+      launch_soa_to_aos(d.dsx, d.dsy, d.dsz, d.loc, R.row_off, to, n, h->st);
+    });
+    if (rc) return rc;
   }
+  CK(cudaStreamSynchronize(h->st));
   return IDPD_OK;
 }
 

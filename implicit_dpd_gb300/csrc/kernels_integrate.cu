@@ -434,6 +434,48 @@ void launch_soa_to_aos(const double* x, const double* y, const double* z, const 
   k_soa_to_aos<<<(n + 255) / 256, 256, 0, st>>>(x, y, z, loc, row0, aos, n);
 }
 
+// Derived fields of one replica's rows in upload order (device, managed or staging
+// memory). Densities of sorted slots, from FP64 (d64) or from fixed point (q, in units of
+// unscale); W-component records of storage rows.
+__global__ void k_gather_density(DevState d, const double* d64, double unscale, int row0,
+                                 double* out, int n) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint32_t s = d.rank[d.loc[row0 + k]];
+  double v[3];
+  if (d64) {
+    for (int c = 0; c < 3; c++) v[c] = d64[3 * (size_t)s + c];
+  } else {
+    v[0] = __dmul_rn((double)d.dqx[s], unscale);
+    v[1] = __dmul_rn((double)d.dqy[s], unscale);
+    v[2] = __dmul_rn((double)d.dqz[s], unscale);
+  }
+  for (int c = 0; c < 3; c++) out[3 * (size_t)k + c] = v[c];
+}
+
+void launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
+                           double* out, int n, cudaStream_t st) {
+  if (n > 0) k_gather_density<<<(n + 255) / 256, 256, 0, st>>>(d, d64, unscale, row0, out, n);
+}
+
+template <int W>
+__global__ void k_gather_records(const double* rec, const uint32_t* loc, int row0, double* out,
+                                 int n) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n * W) return;
+  out[k] = rec[(size_t)W * loc[row0 + k / W] + k % W];
+}
+
+void launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
+                           double* out, int n, cudaStream_t st) {
+  if (n == 0) return;
+  const int b = (n * width + 255) / 256;
+  if (width == 6)
+    k_gather_records<6><<<b, 256, 0, st>>>(rec, loc, row0, out, n);
+  else
+    k_gather_records<3><<<b, 256, 0, st>>>(rec, loc, row0, out, n);
+}
+
 // The four u32 fields of rows row0 .. row0 + n - 1 in upload order (loc maps
 // upload rows to storage rows): out[f * n + k] = field f of upload row k.
 __global__ void k_gather_u32x4(const uint32_t* a, const uint32_t* b, const uint32_t* c,

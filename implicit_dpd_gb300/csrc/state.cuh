@@ -316,6 +316,10 @@ void launch_set_dynamics(const DevState& d, const double* pos, const double* vel
                          double box2, bool kept, cudaStream_t st);
 void launch_soa_to_aos(const double* x, const double* y, const double* z, const uint32_t* loc,
                        int row0, double* aos, int n, cudaStream_t st);
+void launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
+                           double* out, int n, cudaStream_t st);
+void launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
+                           double* out, int n, cudaStream_t st);
 void launch_gather_u32x4(const uint32_t* a, const uint32_t* b, const uint32_t* c,
                          const uint32_t* e, const uint32_t* loc, int row0, uint32_t* out, int n,
                          cudaStream_t st);
