@@ -91,7 +91,12 @@ struct idpd_handle {
   int* obs_count = nullptr;
   ObsBuffers obs_buf{};                 // per-layout scratch (null until needed)
   cudaGraphExec_t graph_obs = nullptr;  // the step with the observation
-  // K steps in one launch: the step inside a WHILE conditional node
+  cudaGraphExec_t graph_cm = nullptr;   // the step with the drift removal
+  cudaGraphExec_t graph_run = nullptr;  // kRunSteps plain steps
+  std::vector<uint32_t> time_h;  // Parameter::time per replica, as rep_time on the device
+  bool time_known = false;       // (not after steps with the reaction, which may stop)
+  int* err_host = nullptr;       // pinned copy of the device's error word
+  // steps with the reaction in one launch: the step inside a WHILE conditional node
   cudaGraphExec_t graph_loop = nullptr;
   cudaStream_t cst = nullptr;  // captures the bodies of the step's IF nodes
   int* loop_left = nullptr;  // device count of the loop's steps left
@@ -148,19 +153,17 @@ int dalloc(idpd_handle* h, T** p, size_t count) {
   return IDPD_OK;
 }
 
+void invalidate_graph(idpd_handle* h) {
+  for (cudaGraphExec_t* g :
+       {&h->graph_loop, &h->graph, &h->graph_obs, &h->graph_cm, &h->graph_run})
+    if (*g) {
+      cudaGraphExecDestroy(*g);
+      *g = nullptr;
+    }
+}
+
 void free_all(idpd_handle* h) {
-  if (h->graph_loop) {
-    cudaGraphExecDestroy(h->graph_loop);
-    h->graph_loop = nullptr;
-  }
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
-  if (h->graph_obs) {
-    cudaGraphExecDestroy(h->graph_obs);
-    h->graph_obs = nullptr;
-  }
+  invalidate_graph(h);
   h->obs_buf.part = nullptr;
   h->obs_buf.mvir = h->obs_buf.mdif = nullptr;
   for (void* p : h->allocs) cudaFree(p);
@@ -174,21 +177,6 @@ void free_all(idpd_handle* h) {
   h->chem_buf = ChemBuffers{h->chem, nullptr, nullptr, nullptr, nullptr};
   h->chem_buf_total = h->chem_buf_tcap = 0;
   h->cap = h->ncell_cap = h->nblk_cap = h->n_amp_cap = 0;
-}
-
-void invalidate_graph(idpd_handle* h) {
-  if (h->graph_loop) {
-    cudaGraphExecDestroy(h->graph_loop);
-    h->graph_loop = nullptr;
-  }
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
-  if (h->graph_obs) {
-    cudaGraphExecDestroy(h->graph_obs);
-    h->graph_obs = nullptr;
-  }
 }
 
 int check_params(idpd_handle* h, const idpd_params* p) {
@@ -591,6 +579,8 @@ int commit(idpd_handle* h) {
       CK(cudaMemcpyAsync(h->amp_rep, amp_rep.data(), sizeof(int) * amp, cudaMemcpyHostToDevice, h->st));
     }
     CK(cudaMemcpyAsync(d.rep_time, time.data(), sizeof(uint32_t) * h->R, cudaMemcpyHostToDevice, h->st));
+    h->time_h = time;
+    h->time_known = true;
     if (h->chem_on) {
       int rc2 = chem_layout(h);
       if (rc2) return rc2;
@@ -674,10 +664,32 @@ int retune_cells(idpd_handle* h) {
   return IDPD_OK;
 }
 
-int check_device_error(idpd_handle* h) {
-  int e = 0;
-  CK(cudaMemcpyAsync(&e, h->d.err, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+// The step counters of the replicas.
+int host_times(idpd_handle* h) {
+  if (h->time_known) return IDPD_OK;
+  h->time_h.resize(h->R);
+  CK(cudaMemcpyAsync(h->time_h.data(), h->d.rep_time, sizeof(uint32_t) * h->R,
+                     cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
+  h->time_known = true;
+  return IDPD_OK;
+}
+
+// Queues the copy of the error word, for check_device_error after the stream was waited for.
+int queue_error_copy(idpd_handle* h) {
+  if (!h->err_host) CK(cudaMallocHost((void**)&h->err_host, sizeof(int)));
+  CK(cudaMemcpyAsync(h->err_host, h->d.err, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+  return IDPD_OK;
+}
+
+int check_device_error(idpd_handle* h, bool copied = false) {
+  int e = 0;
+  if (copied) {
+    e = *h->err_host;
+  } else {
+    CK(cudaMemcpyAsync(&e, h->d.err, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaStreamSynchronize(h->st));
+  }
   if (e == 0) return IDPD_OK;
   CK(cudaMemsetAsync(h->d.err, 0, sizeof(int), h->st));
   switch (e) {
@@ -711,7 +723,7 @@ void enqueue_cells(idpd_handle* h, bool drift) {
 // returned stream; end_if ends the body. When the stream is not capturing (a
 // step enqueued directly), the work goes to h->st and its kernels skip
 // themselves, as they do inside the body too.
-StepConds step_conds(idpd_handle* h, bool verlet) {
+StepConds step_conds(idpd_handle* h, bool rebuild, bool cm) {
   StepConds c{};
   cudaStreamCaptureStatus cs;
   cudaGraph_t g;
@@ -719,10 +731,11 @@ StepConds step_conds(idpd_handle* h, bool verlet) {
       cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, nullptr, nullptr, nullptr) != cudaSuccess ||
       cs != cudaStreamCaptureStatusActive)
     return c;
-  c.on = cudaGraphConditionalHandleCreate(&c.cm, g, 0, cudaGraphCondAssignDefault) ==
-             cudaSuccess &&
-         (!verlet || cudaGraphConditionalHandleCreate(&c.rebuild, g, 0,
-                                                      cudaGraphCondAssignDefault) == cudaSuccess);
+  // (a handle without its node makes the graph invalid: only those in use)
+  c.on = rebuild && cudaGraphConditionalHandleCreate(&c.rebuild, g, 0,
+                                                     cudaGraphCondAssignDefault) == cudaSuccess;
+  c.cm_on = cm && cudaGraphConditionalHandleCreate(&c.cm, g, 0, cudaGraphCondAssignDefault) ==
+                      cudaSuccess;
   return c;
 }
 
@@ -731,14 +744,14 @@ struct IfScope {
   Chain first;
   bool body;
 };
-IfScope begin_if(idpd_handle* h, const StepConds& c, cudaGraphConditionalHandle ch) {
+IfScope begin_if(idpd_handle* h, bool on, cudaGraphConditionalHandle ch) {
   const IfScope direct{{h->st, true}, false};
   cudaStreamCaptureStatus cs;
   cudaGraph_t g;
   const cudaGraphNode_t* deps = nullptr;
   const cudaGraphEdgeData* edges = nullptr;
   size_t nd = 0;
-  if (!c.on ||
+  if (!on ||
       cudaStreamGetCaptureInfo(h->st, &cs, nullptr, &g, &deps, &edges, &nd) != cudaSuccess)
     return direct;
   cudaGraphNodeParams cp = {};
@@ -761,11 +774,17 @@ void end_if(idpd_handle* h, const IfScope& s) {
   cudaStreamEndCapture(h->cst, &body);
 }
 
+// The centre-of-mass drift removal of a step, every kCmCorr steps: left out (the host
+// knows that no replica is due), its kernels (which skip the replicas that are not), or
+// an IF node around them (in the loop graph, whose steps the host does not tell apart).
+enum CmForm { kCmNone, kCmKernels, kCmIfNode };
+
 // One MD step; `observe` adds the per-particle virial to the pair pass and
 // the observation kernels (the records are written only for replicas whose
-// step counter is due); loop.left is set inside the K-step loop graph.
-void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr,
-                  const LoopTail& loop = LoopTail{}) {
+// step counter is due); loop.left is set inside the K-step loop graph; chained: a step's
+// last kernel is right before it in the stream.
+void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_done = nullptr,
+                  const LoopTail& loop = LoopTail{}, bool chained = false) {
   const int mode = pair_mode(h);
   DevState d = h->d;  // the step writes no fine-grained side outputs
   d.dqx = d.dqy = d.dqz = nullptr;
@@ -777,13 +796,14 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
   const bool verlet = d.vdev && h->tune.skin > 0.0f && mode != kPairsF64;
   const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
   const int zero = kZeroForce | (observe ? kZeroVirial : 0) | (marks ? kZeroMarks : 0);
-  const StepConds conds = step_conds(h, verlet);
+  const StepConds conds = step_conds(h, verlet, cm == kCmIfNode);
+  const Chain first{h->st, chained};
   if (verlet) {  // cells and lists only on rebuild steps
     const int* gate = &d.vdev->rebuild;
-    launch_drift_disp(d, h->nblk, head);
+    launch_drift_disp(d, h->nblk, first);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
     launch_vl_decide(d, h->R, conds, after_drift);
-    const IfScope c = begin_if(h, conds, conds.rebuild);
+    const IfScope c = begin_if(h, conds.on, conds.rebuild);
     const Chain body{c.first.st, true};
     launch_bin_gated(d, h->nblk, c.first);
     launch_scan(d, h->ncell_tot, h->R - 1, body, gate);
@@ -792,7 +812,7 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
     end_if(h, c);
     launch_pack(d, h->nblk, zero, conds.on ? head : st, gate);  // the positions changed
   } else {
-    launch_drift_bin(d, h->nblk, true, h->R, conds, head);
+    launch_drift_bin(d, h->nblk, true, h->R, conds, first);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
     launch_scan(d, h->ncell_tot, h->R - 1, after_drift);
     launch_scatter_sort_pack(d, h->nblk, zero, st);
@@ -806,8 +826,8 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
   }
   launch_bonded_kick(d, h->nblk, true, st);
   if (observe) launch_observe_bonds(d, h->obs_buf, h->n_amp_tot, h->amp_rep, h->st);
-  {
-    const IfScope c = begin_if(h, conds, conds.cm);
+  if (cm != kCmNone) {
+    const IfScope c = begin_if(h, conds.cm_on, conds.cm);
     launch_cmdrift(d, h->nblk, h->R, false, c.first);
     end_if(h, c);
   }
@@ -815,7 +835,8 @@ void enqueue_step(idpd_handle* h, bool observe, cudaEvent_t drift_done = nullptr
     launch_chem(d, h->chem_buf, h->reps_h[0].nblk, h->chem_cfg.n_core, h->chem_amp_cap, false,
                 h->st);
   if (observe) launch_observe(d, h->obs_buf, h->nblk, h->n_amp_tot, h->amp_rep, h->R, h->st);
-  launch_step_tail(d, h->R, h->chem_on ? &h->chem->stop_now : nullptr, loop, head);
+  launch_step_tail(d, h->R, h->chem_on ? &h->chem->stop_now : nullptr, loop,
+                   conds.cm_on ? head : st);
 }
 
 int enqueue_reorder(idpd_handle* h) {
@@ -983,6 +1004,7 @@ int idpd_destroy(idpd_handle* h) {
   if (h->obs_count) cudaFree(h->obs_count);
   if (h->prec_dev) cudaFree(h->prec_dev);
   if (h->chem_flag_host) cudaFreeHost(h->chem_flag_host);
+  if (h->err_host) cudaFreeHost(h->err_host);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->st) cudaStreamDestroy(h->st);
@@ -1016,6 +1038,7 @@ int idpd_set_params(idpd_handle* h, int32_t r, const idpd_params* p) {
     cudaSetDevice(h->device);
     CK(cudaMemcpyAsync(h->d.rep_time + r, &p->time, sizeof(uint32_t), cudaMemcpyHostToDevice, h->st));
     CK(cudaStreamSynchronize(h->st));
+    if (h->time_known) h->time_h[r] = p->time;
   }
   return IDPD_OK;
 }
@@ -1411,8 +1434,36 @@ int idpd_remove_cmdrift(idpd_handle* h) {
   return check_device_error(h);
 }
 
-// The loop graph: a WHILE conditional node whose body is the captured step
-// (its last kernel sets the loop's condition). Returns false (and leaves no graph) where the
+// Steps of one launch of graph_run. A step inside a WHILE node, whose first kernel waits for
+// the node, costs up to 5 us more than one in a plain graph (3k particles 42.8 us against
+// 38.5, 24k 47.7 against 46.9, 1M 503 against 497), so runs of steps without the reaction go
+// out eight at a time.
+constexpr int kRunSteps = 8;
+
+// Captures nsteps steps into *ge (if it is not there yet).
+int build_graph(idpd_handle* h, cudaGraphExec_t* ge, int nsteps, bool observe, CmForm cm) {
+  if (*ge) return IDPD_OK;
+  cudaGraph_t g;
+  CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
+  for (int k = 0; k < nsteps; k++)
+    enqueue_step(h, observe, cm, nullptr, LoopTail{}, k > 0);
+  const cudaError_t launch_err = cudaGetLastError();  // a launch refused during capture
+  const cudaError_t cap_err = cudaStreamEndCapture(h->st, &g);
+  if (cap_err != cudaSuccess || launch_err != cudaSuccess)
+    return fail(h, IDPD_ERR_CUDA, "step capture: %s (first launch error: %s)",
+                cudaGetErrorString(cap_err), cudaGetErrorString(launch_err));
+  const cudaError_t e = cudaGraphInstantiate(ge, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    *ge = nullptr;
+    return fail(h, IDPD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
+  }
+  return IDPD_OK;
+}
+
+// The loop graph, for steps with the reaction: a WHILE conditional node whose body is the
+// captured step (its last kernel sets the loop's condition, so that the loop can end after
+// a step whose event stopped the run). Returns false (and leaves no graph) where the
 // driver refuses any part of it; the steps then go one launch each.
 bool build_loop_graph(idpd_handle* h) {
   cudaGraph_t g = nullptr;
@@ -1430,7 +1481,7 @@ bool build_loop_graph(idpd_handle* h) {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       if (cudaStreamBeginCaptureToGraph(h->st, body, nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        enqueue_step(h, false, nullptr,
+        enqueue_step(h, false, kCmIfNode, nullptr,
                      LoopTail{cond, h->loop_left, h->chem_on ? &h->chem->stopped : nullptr});
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(h->st, &body);
@@ -1457,56 +1508,49 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   if (h->chem_on && h->chem_stopped)
     return fail(h, IDPD_ERR_STATE, "the reaction reached max_amp_num: the run has ended");
   if ((rc = ensure_verlet_ready(h)) || (rc = ensure_phit(h))) return rc;
-  std::vector<uint32_t> time;  // step counters, to pick the steps that observe
-  if (h->obs_period > 0) {
-    if ((rc = ensure_obs(h))) return rc;
-    time.resize(h->R);
-    CK(cudaMemcpyAsync(time.data(), h->d.rep_time, sizeof(uint32_t) * h->R, cudaMemcpyDeviceToHost,
-                       h->st));
-    CK(cudaStreamSynchronize(h->st));
-  }
-  for (int variant = 0; variant < (h->obs_period > 0 ? 2 : 1); variant++) {
-    cudaGraphExec_t& ge = variant ? h->graph_obs : h->graph;
-    if (ge) continue;
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(h, variant == 1);
-    const cudaError_t launch_err = cudaGetLastError();  // a launch refused during capture
-    const cudaError_t cap_err = cudaStreamEndCapture(h->st, &g);
-    if (cap_err != cudaSuccess || launch_err != cudaSuccess)
-      return fail(h, IDPD_ERR_CUDA, "step capture: %s (first launch error: %s)",
-                  cudaGetErrorString(cap_err), cudaGetErrorString(launch_err));
-    cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return fail(h, IDPD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
-  }
-  const bool loop = nsteps > 1 && !(h->flags & IDPD_CFG_PLAIN_GRAPHS) && !h->loop_failed;
+  if (h->obs_period > 0 && (rc = ensure_obs(h))) return rc;
+  if ((rc = host_times(h))) return rc;
+  // with the reaction, and in the plain form, the drift removal's kernels are in every step
+  const bool plain = h->flags & IDPD_CFG_PLAIN_GRAPHS;
+  const bool every_cm = h->chem_on || plain;
+  if ((rc = build_graph(h, &h->graph, 1, false, every_cm ? kCmKernels : kCmNone))) return rc;
+  const bool loop = h->chem_on && nsteps > 1 && !plain && !h->loop_failed;
   if (loop && !h->graph_loop && !build_loop_graph(h)) h->loop_failed = true;
   const bool use_loop = loop && h->graph_loop;
-  // whether the step `ahead` steps from now observes: some replica's step
-  // counter is then a multiple of the period
-  auto observes = [&](int ahead) {
-    for (uint32_t t : time)
-      if (((t + (uint32_t)ahead) % (uint32_t)h->obs_period) == 0u) return true;
+  const bool use_run = !every_cm && nsteps > 1;
+  if (use_run && (rc = build_graph(h, &h->graph_run, kRunSteps, false, kCmNone))) return rc;
+  // whether some replica's step counter is a multiple of `period`, `ahead` steps from now
+  auto due = [&](int period, int ahead) {
+    for (uint32_t t : h->time_h)
+      if (((t + (uint32_t)ahead) % (uint32_t)period) == 0u) return true;
     return false;
   };
+  auto observes = [&](int ahead) { return h->obs_period > 0 && due(h->obs_period, ahead); };
+  auto removes = [&](int ahead) { return !every_cm && due((int)kCmCorr, ahead); };
   CK(cudaEventRecord(h->ev0, h->st));
   for (int k = 0; k < nsteps;) {
-    // an observing step is one launch of the observation graph; a run of
-    // other steps up to the next storage reorder is one launch of the loop
-    const bool obs = !time.empty() && observes(0);
+    // a step that observes or removes the drift is one launch of its graph; the steps up to
+    // the next of these, or the next storage reorder, go out kRunSteps at a time (with the
+    // reaction, as one launch of the loop)
+    const bool obs = observes(0), cm = removes(0);
     int c = 1;
-    if (!obs && use_loop) {
-      const int room = std::max(h->sort_period - h->steps_since_sort, 1);
-      while (k + c < nsteps && c < room && !(!time.empty() && observes(c))) c++;
+    if (!obs && !cm && (use_loop || use_run)) {
+      const int room = std::min(nsteps - k, std::max(h->sort_period - h->steps_since_sort, 1));
+      const int most = use_loop ? room : kRunSteps;
+      while (c < room && c < most && !observes(c) && !removes(c)) c++;
+      if (use_run && c < kRunSteps) c = 1;
     }
-    if (c > 1) {
+    if (c > 1 && use_loop) {
       launch_loop_set(h->loop_left, c, h->st);
       CK(cudaGraphLaunch(h->graph_loop, h->st));
+    } else if (c > 1) {
+      CK(cudaGraphLaunch(h->graph_run, h->st));
     } else {
-      CK(cudaGraphLaunch(obs ? h->graph_obs : h->graph, h->st));
+      cudaGraphExec_t* ge = obs ? &h->graph_obs : (cm ? &h->graph_cm : &h->graph);
+      if ((rc = build_graph(h, ge, 1, obs, kCmKernels))) return rc;
+      CK(cudaGraphLaunch(*ge, h->st));
     }
-    for (uint32_t& t : time) t += (uint32_t)c;
+    for (uint32_t& t : h->time_h) t += (uint32_t)c;
     k += c;
     h->steps_since_sort += c;
     if (h->steps_since_sort >= h->sort_period) {
@@ -1523,12 +1567,14 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
       }
     }
   }
+  if (h->chem_on) h->time_known = false;  // a stopped step does not count
   CK(cudaEventRecord(h->ev1, h->st));
-  CK(cudaEventSynchronize(h->ev1));
+  if ((rc = queue_error_copy(h))) return rc;
+  CK(cudaStreamSynchronize(h->st));
   CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
   h->density_valid = false;
   if ((rc = sync_counts(h))) return rc;
-  return check_device_error(h);
+  return check_device_error(h, true);
 }
 
 // One step on host arrays: the rows in as idpd_set_dynamics, one step as
@@ -1554,21 +1600,20 @@ int idpd_step_host(idpd_handle* h, int32_t r, double* pos, double* vel, double* 
   if (h->n_tot == 0) return IDPD_OK;
   h->pairs_valid = true;
   if ((rc = ensure_verlet_ready(h)) || (rc = ensure_phit(h))) return rc;
-  bool observe = false;
-  if (h->obs_period > 0) {
-    if ((rc = ensure_obs(h))) return rc;
-    std::vector<uint32_t> time(h->R);
-    CK(cudaMemcpyAsync(time.data(), h->d.rep_time, sizeof(uint32_t) * h->R, cudaMemcpyDeviceToHost,
-                       h->st));
-    CK(cudaStreamSynchronize(h->st));
-    for (uint32_t t : time) observe = observe || (t % (uint32_t)h->obs_period) == 0u;
+  bool observe = false, cm = false;
+  if (h->obs_period > 0 && (rc = ensure_obs(h))) return rc;
+  if ((rc = host_times(h))) return rc;
+  for (uint32_t t : h->time_h) {
+    observe = observe || (h->obs_period > 0 && (t % (uint32_t)h->obs_period) == 0u);
+    cm = cm || (t % kCmCorr) == 0u;
   }
   if ((rc = ensure_xst(h))) return rc;
   const RepDev& R = h->reps_h[r];
   const size_t n = (size_t)R.n;
   const DevState& d = h->d;
   CK(cudaEventRecord(h->ev0, h->st));
-  enqueue_step(h, observe, h->x_drift);
+  enqueue_step(h, observe, cm ? kCmKernels : kCmNone, h->x_drift);
+  for (uint32_t& t : h->time_h) t++;
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) return fail(h, IDPD_ERR_CUDA, "step launch: %s", cudaGetErrorString(le));
   CK(cudaEventRecord(h->ev1, h->st));
@@ -1591,10 +1636,11 @@ int idpd_step_host(idpd_handle* h, int32_t r, double* pos, double* vel, double* 
     if ((rc = enqueue_reorder(h))) return rc;
     h->steps_since_sort = 0;
   }
+  if ((rc = queue_error_copy(h))) return rc;
   CK(cudaStreamSynchronize(h->st));
   CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
   h->density_valid = false;
-  return check_device_error(h);
+  return check_device_error(h, true);
 }
 
 int idpd_sync(idpd_handle* h) {
@@ -1818,6 +1864,7 @@ int idpd_profile_step(idpd_handle* h, char* names, size_t names_len, float* ms, 
   launch_cmdrift(d, h->nblk, h->R, false, h->st);
   CK(cudaEventRecord(ev[8], h->st));
   launch_step_tail(d, h->R, nullptr, LoopTail{}, h->st);
+  for (uint32_t& t : h->time_h) t++;
   CK(cudaEventRecord(ev[9], h->st));
   CK(cudaEventSynchronize(ev[9]));
   std::string all;

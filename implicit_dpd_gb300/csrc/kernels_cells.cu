@@ -70,7 +70,7 @@ __device__ __forceinline__ void set_cm_cond(const StepConds& c, const uint32_t* 
 __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drift, int nrep,
                                                          StepConds conds) {
   chain_begin();
-  if (conds.on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
+  if (conds.cm_on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
   if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) k_vl_decide(VerletDev* v, const uint32_t*
     v->rebuilds += (unsigned)rb;
     if (conds.on) cudaGraphSetConditional(conds.rebuild, rb ? 1u : 0u);
   }
-  if (conds.on) set_cm_cond(conds, rep_time, nrep);
+  if (conds.cm_on) set_cm_cond(conds, rep_time, nrep);
 }
 
 // The binning of k_drift_bin on a rebuild step (positions already drifted).

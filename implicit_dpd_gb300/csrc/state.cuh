@@ -151,10 +151,11 @@ inline void launch(const Chain& c, void (*kernel)(KArgs...), dim3 grid, dim3 blo
 }
 
 // Conditions of the IF nodes of a captured step, set by the step's first kernels: the
-// rebuild of cells and lists, and the centre-of-mass drift removal, due for some replica.
+// rebuild of cells and lists, and (inside the loop graph) the centre-of-mass drift
+// removal, due for some replica.
 struct StepConds {
   cudaGraphConditionalHandle rebuild, cm;
-  int on;  // 0: the step holds no IF nodes
+  int on, cm_on;  // 0: the step holds no such node
 };
 
 // What the pack zeroes for the passes that follow (their terms arrive by atomic add or
