@@ -774,6 +774,14 @@ void end_if(idpd_handle* h, const IfScope& s) {
   cudaStreamEndCapture(h->cst, &body);
 }
 
+// Up to kGateRows rows the kernels of a rebuild are in every step and skip themselves where
+// there is none; above, they are in an IF node. The node costs 4 to 6 us a step; the
+// kernels' empty blocks, which grow with the rows, less than that up to 400k rows and more
+// at 1M. Us per step with the node and without: 8k membrane 53.7 and 50.2, 24k liquid 47.0
+// and 41.3, 131k membrane 263.6 and 256.4, 200k liquid 141.8 and 136.7, 400k liquid 234.3
+// and 232.2, 500k membrane the same, 1M liquid 504 and 515.
+constexpr int kGateRows = 400000;
+
 // The centre-of-mass drift removal of a step, every kCmCorr steps: left out (the host
 // knows that no replica is due), its kernels (which skip the replicas that are not), or
 // an IF node around them (in the loop graph, whose steps the host does not tell apart).
@@ -796,7 +804,7 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
   const bool verlet = d.vdev && h->tune.skin > 0.0f && mode != kPairsF64;
   const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
   const int zero = kZeroForce | (observe ? kZeroVirial : 0) | (marks ? kZeroMarks : 0);
-  const StepConds conds = step_conds(h, verlet, cm == kCmIfNode);
+  const StepConds conds = step_conds(h, verlet && h->n_tot > kGateRows, cm == kCmIfNode);
   const Chain first{h->st, chained};
   if (verlet) {  // cells and lists only on rebuild steps
     const int* gate = &d.vdev->rebuild;
@@ -810,7 +818,7 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
     launch_scatter_sort_pack(d, h->nblk, zero, body, gate);
     launch_verlet_build(d, h->nblk, body);
     end_if(h, c);
-    launch_pack(d, h->nblk, zero, conds.on ? head : st, gate);  // the positions changed
+    if (conds.on) launch_pack(d, h->nblk, zero, head, gate);
   } else {
     launch_drift_bin(d, h->nblk, true, h->R, conds, first);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
@@ -824,7 +832,9 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
     d.prec_count = h->prec_dev;
     launch_precursor(d, h->nblk, marks, st);
   }
-  launch_bonded_kick(d, h->nblk, true, st);
+  const bool tail = observe || cm != kCmNone || h->chem_on || loop.left;
+  launch_bonded_kick(d, h->nblk, true, st, tail ? 0 : h->R);
+  if (!tail) return;
   if (observe) launch_observe_bonds(d, h->obs_buf, h->n_amp_tot, h->amp_rep, h->st);
   if (cm != kCmNone) {
     const IfScope c = begin_if(h, conds.cm_on, conds.cm);
@@ -1849,7 +1859,6 @@ int idpd_profile_step(idpd_handle* h, char* names, size_t names_len, float* ms, 
   launch_scan(d, h->ncell_tot, h->R - 1, h->st, gate);
   CK(cudaEventRecord(ev[2], h->st));
   launch_scatter_sort_pack(d, h->nblk, kZeroForce, h->st, gate);
-  if (verlet) launch_pack(d, h->nblk, kZeroForce, {h->st, true}, gate);
   CK(cudaEventRecord(ev[3], h->st));
   if (verlet) launch_verlet_build(d, h->nblk, h->st);
   CK(cudaEventRecord(ev[4], h->st));

@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(kRowBlock, 8) k_drift_disp(DevState d) {
   }
 }
 
+// (Taken by the drift's last block instead, behind a counter, it was no faster below 400k
+// rows, and at 1M the drift grew by 5 us.)
 __global__ void __launch_bounds__(256) k_vl_decide(VerletDev* v, const uint32_t* rep_time,
                                                    int nrep, StepConds conds) {
   chain_begin();
@@ -428,14 +430,19 @@ __device__ __forceinline__ void pack_row(const DevState& d, const RepDev* R, uin
 // rows that a stable counting sort gives, is the number of smaller rows in the cell (the
 // cell's rows are the neighbouring threads', so the reads are broadcasts), and its FP32
 // copies are written there. One kernel instead of a sort by cell (a warp each) and a
-// pass over the sorted rows.
+// pass over the sorted rows. gate (may be null): device flag; when 0 the slots keep the
+// rows and cells of the last rebuild, and only the copies are written.
 __global__ void __launch_bounds__(kRowBlock) k_sort_pack(DevState d, int zero, const int* gate) {
   chain_begin();
-  if (gate && !*gate) return;
+  const bool sort = !gate || *gate;
   const int r = d.blk_rep[blockIdx.x];
   const int k = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
   if (k >= R->row_off + R->n) return;
+  if (!sort) {
+    pack_row(d, R, d.perm[k], k, d.scell[k], zero);
+    return;
+  }
   const uint32_t i = d.arrival[k], key = d.key[i];
   const int b = d.cell_start[key], e = d.cell_start[key + 1];
   int s = b;
@@ -446,11 +453,11 @@ __global__ void __launch_bounds__(kRowBlock) k_sort_pack(DevState d, int zero, c
   pack_row(d, R, i, s, key, zero);
 }
 
-// One thread per sorted slot, for steps that keep the slots' rows and cells of the last
-// rebuild (packed, may be null: device flag; when set k_sort_pack wrote the copies).
+// The copies alone, in a step whose rebuild is in an IF node (packed: device flag; when set
+// k_sort_pack wrote them there).
 __global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, int zero, const int* packed) {
   chain_begin();
-  if (packed && *packed) return;
+  if (*packed) return;
   const int r = d.blk_rep[blockIdx.x];
   const int s = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;

@@ -78,9 +78,13 @@ __device__ __forceinline__ void chain_forces(const float3 p[4], float cf_s, floa
 // One thread per storage row: pair force + bonded force on this bead (the
 // chain is re-evaluated per bead, no scatter), acc written in FP64, then
 // kick: vel = vel_buf + dt/2 acc (vel holds vel_buf after the drift).
+// advance: where nothing after it in the step reads or holds the step counters, the
+// first block advances them (their number; a kernel of its own for it took 1.5 us).
 template <bool KICK>
-__global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
+__global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advance) {
   chain_begin();
+  if (KICK && blockIdx.x == 0)
+    for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
   const int r = d.blk_rep[blockIdx.x];
   const int i = d.blk_row[blockIdx.x] + threadIdx.x;
   const RepDev* R = d.reps + r;
@@ -128,9 +132,9 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d) {
   }
 }
 
-void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st) {
+void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st, int advance) {
   if (nblk == 0) return;
-  launch(st, kick ? k_bonded_kick<true> : k_bonded_kick<false>, nblk, kRowBlock, 0, d);
+  launch(st, kick ? k_bonded_kick<true> : k_bonded_kick<false>, nblk, kRowBlock, 0, d, advance);
 }
 
 // Fine-grained ForceBonded::CalcListedForce: one thread per molecule adds

@@ -175,11 +175,12 @@ void launch_drift_disp(const DevState& d, int nblk, const Chain& st);
 void launch_vl_decide(const DevState& d, int R, const StepConds& c, const Chain& st);
 void launch_bin_gated(const DevState& d, int nblk, const Chain& st);
 // Rows to sorted slots in the stable order within cells, and their FP32 copies
-// (gate, may be null: device flag; when 0 nothing is done). zero: kZero* bits.
+// (gate, may be null: device flag; when 0 the slots stay and only the copies are written).
+// zero: kZero* bits.
 void launch_scatter_sort_pack(const DevState& d, int nblk, int zero, const Chain& st,
                               const int* gate = nullptr);
-// The FP32 copies of a step that keeps its cells (packed: device flag; when set
-// the step's launch_scatter_sort_pack has written them).
+// The FP32 copies of a step that keeps its cells, after an IF node with the rebuild (packed:
+// device flag; when set the launch_scatter_sort_pack in it has written them).
 void launch_pack(const DevState& d, int nblk, int zero, const Chain& st, const int* packed);
 void launch_reorder(const DevState& d, const DevState& o, int nblk, int n_topol,
                     cudaStream_t st);
@@ -291,7 +292,8 @@ int walk_retrieve(WalkState* s, int kind, int tag, int n_walk, const int32_t* ni
                   void* const* result, std::string& err);
 
 // kernels_integrate.cu
-void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st);
+// advance: the step counters of R replicas too (0: launch_step_tail does it).
+void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st, int advance = 0);
 void launch_bonded_fine(const DevState& d, int n_amp_tot, const int* amp_rep, double* vir_part,
                         cudaStream_t st);
 void launch_kick_only(const DevState& d, int nblk, cudaStream_t st);

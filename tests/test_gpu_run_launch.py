@@ -8,8 +8,9 @@ import numpy as np
 import pytest
 
 from helpers import mdpd_params, mixed_system
-from implicit_dpd_gb300.abi import CFG_PLAIN_GRAPHS
-from implicit_dpd_gb300.engine import Engine
+from implicit_dpd_gb300 import configs
+from implicit_dpd_gb300.abi import CFG_PLAIN_GRAPHS, FORM_WARREN
+from implicit_dpd_gb300.engine import Engine, derive_params
 
 pytestmark = pytest.mark.gpu
 
@@ -53,6 +54,32 @@ def test_runs_of_steps_equal_single_steps(skin, times, period):
     for x, y in zip(oa, ob):
         for k in x:
             assert np.array_equal(np.asarray(x[k]), np.asarray(y[k])), k
+
+
+@pytest.mark.parametrize("rho", [5.9, 6.0])
+def test_rebuild_in_an_if_node_or_in_every_step(rho):
+    # 396,716 rows, below the line where the rebuild's kernels go into an IF node, and
+    # 403,440, above it; against one launch per step, which has no such node
+    box = np.array([41.0, 41.0, 40.0])
+    st = configs.liquid(box, rho, seed=71)
+    q = derive_params(configs.run_param(box, dt=0.005, cf_r=3.0))
+    q.seed, q.time, q.form = 5, 95, FORM_WARREN
+    q.warren_a, q.warren_b, q.warren_rd = -40.0, 25.0, 0.75
+
+    def run(flags):
+        e = Engine(flags=flags)
+        e.set_params(q)
+        e.upload(st)
+        e.set_tuning(1, 0.2)
+        e.step(20)
+        out, n = e.download(), e.list_rebuilds()
+        e.close()
+        return out, n
+
+    (a, na), (b, nb) = run(0), run(CFG_PLAIN_GRAPHS)
+    assert na == nb and 1 < na < 20  # steps with and without a rebuild
+    for k in ("pos", "vel", "acc", "id"):
+        assert np.array_equal(a[k], b[k]), k
 
 
 def test_host_array_steps_remove_the_drift_when_due():
