@@ -69,13 +69,13 @@ __device__ __forceinline__ void set_cm_cond(const StepConds& c, const uint32_t* 
 // One thread per storage row: optional drift, then cell index and arrival slot.
 __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drift, int nrep,
                                                          StepConds conds) {
-  chain_begin();
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
   if (conds.cm_on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
   if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
-  const int r = d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (i >= R->row_off + R->n) return;
+  if (i >= end) return;
   double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
   if (do_drift) drift_row(d, R, i, p, ds);
   const int cx = cell_coord(p[0], R->inv_cs[0], R->nc[0]);
@@ -99,13 +99,13 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
 // 31 -> 21; with the bonded forces of 984k beads 73 -> 52, 60 -> 34, 45 -> 41.
 __global__ void __launch_bounds__(kRowBlock, 8) k_drift_disp(DevState d) {
   __shared__ float wmax[kRowBlock / 32];
-  chain_begin();
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
-  const int r = d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
   float m = 0.0f;
-  if (i < R->row_off + R->n) {
+  if (i < end) {
     const uint32_t s = d.rank[i];
     const double r0[3] = {d.drx[s], d.dry[s], d.drz[s]};
     double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
@@ -152,12 +152,11 @@ __global__ void __launch_bounds__(256) k_vl_decide(VerletDev* v, const uint32_t*
 
 // The binning of k_drift_bin on a rebuild step (positions already drifted).
 __global__ void __launch_bounds__(kRowBlock) k_bin_gated(DevState d) {
-  chain_begin();
-  if (!d.vdev->rebuild) return;
-  const int r = d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (i >= R->row_off + R->n) return;
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
+  if (!d.vdev->rebuild || i >= end) return;
   const int cx = cell_coord(d.px[i], R->inv_cs[0], R->nc[0]);
   const int cy = cell_coord(d.py[i], R->inv_cs[1], R->nc[1]);
   const int cz = cell_coord(d.pz[i], R->inv_cs[2], R->nc[2]);
@@ -312,12 +311,11 @@ void launch_scan(const DevState& d, int ncell_tot, int last_rep, const Chain& st
 
 // ------------------------------------------------- scatter / sort / pack
 __global__ void __launch_bounds__(kRowBlock) k_scatter(DevState d, const int* gate) {
-  chain_begin();
-  if (gate && !*gate) return;
-  const int r = d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (i >= R->row_off + R->n) return;
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
+  if ((gate && !*gate) || i >= end) return;
   const uint32_t s = (uint32_t)d.cell_start[d.key[i]] + d.slot[i];
   d.arrival[s] = (uint32_t)i;
 }
@@ -433,12 +431,12 @@ __device__ __forceinline__ void pack_row(const DevState& d, const RepDev* R, uin
 // pass over the sorted rows. gate (may be null): device flag; when 0 the slots keep the
 // rows and cells of the last rebuild, and only the copies are written.
 __global__ void __launch_bounds__(kRowBlock) k_sort_pack(DevState d, int zero, const int* gate) {
-  chain_begin();
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int k = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
   const bool sort = !gate || *gate;
-  const int r = d.blk_rep[blockIdx.x];
-  const int k = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (k >= R->row_off + R->n) return;
+  if (k >= end) return;
   if (!sort) {
     pack_row(d, R, d.perm[k], k, d.scell[k], zero);
     return;
@@ -456,12 +454,11 @@ __global__ void __launch_bounds__(kRowBlock) k_sort_pack(DevState d, int zero, c
 // The copies alone, in a step whose rebuild is in an IF node (packed: device flag; when set
 // k_sort_pack wrote them there).
 __global__ void __launch_bounds__(kRowBlock) k_pack(DevState d, int zero, const int* packed) {
-  chain_begin();
-  if (*packed) return;
-  const int r = d.blk_rep[blockIdx.x];
-  const int s = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (s >= R->row_off + R->n) return;
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int s = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
+  if (*packed || s >= end) return;
   pack_row(d, R, d.perm[s], s, d.scell[s], zero);
 }
 

@@ -485,7 +485,7 @@ __device__ __forceinline__ void force_walk_rows(const DevState& d, int kept, int
 template <bool PRESS, int FORM, int LP>
 __global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk, int rows) {
   extern __shared__ __align__(16) unsigned char force_smem[];
-  chain_begin();
+  chain_launch();
   ForceBlockSmem* BS = reinterpret_cast<ForceBlockSmem*>(force_smem);
   const int fb = blockDim.x >> 7;  // 128-row blocks of this CTA
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -499,8 +499,11 @@ __global__ void __launch_bounds__(1024, 1) k_force_f32(DevState d, int nblk, int
     if (tb < 64) fill_off_table(BS[rbl].OT, *R, tb);
   }
   __syncthreads();
-  if (rb >= nblk || R->form != FORM) return;
-  force_rows<PRESS, FORM, LP>(d, d.blk_row[rb] + 32 * (wid % kWarps) + rows * blockIdx.y,
+  const bool mine = rb < nblk && R->form == FORM;
+  const int row0 = mine ? d.blk_row[rb] : 0;
+  chain_wait();
+  if (!mine) return;
+  force_rows<PRESS, FORM, LP>(d, row0 + 32 * (wid % kWarps) + rows * blockIdx.y,
                                      rows, r, R, BS[rbl].T, BS[rbl].OT, lane);
 }
 

@@ -82,13 +82,13 @@ __device__ __forceinline__ void chain_forces(const float3 p[4], float cf_s, floa
 // first block advances them (their number; a kernel of its own for it took 1.5 us).
 template <bool KICK>
 __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advance) {
-  chain_begin();
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
   if (KICK && blockIdx.x == 0)
     for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
-  const int r = d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (i >= R->row_off + R->n) return;
+  if (i >= end) return;
   const int s = (int)d.rank[i];
   const long long* fs = d.fq + 4 * (size_t)s;
   long long f[3] = {fs[0], fs[1], fs[2]};

@@ -48,20 +48,20 @@ template <bool MARKS, bool WARREN, bool KNOWN, int LP>
 __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int rows) {
   constexpr int G = 32 / LP;  // particles per warp at a time
   __shared__ OffTable OT;
-  chain_begin();
-  const int r = d.blk_rep[blockIdx.x];
-  const RepDev* R = d.reps + r;
-  if ((R->form == IDPD_FORM_WARREN_K) != WARREN) return;
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
   if (threadIdx.x < 64) fill_off_table(OT, *R, threadIdx.x);
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int h = lane / LP, sl = lane % LP;
   const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
   const int nrow = min(rows, R->row_off + R->n - s0);
-  if (nrow <= 0) return;
   const float cutd2 = WARREN ? R->wrd * R->wrd : 1.0f;  // density cutoff^2
   const float inv_rd = R->winv_rd, wnorm = R->wnorm, pre = R->dens_prescale;
   const bool prec = MARKS && R->prec_on;
+  const bool other_form = (R->form == IDPD_FORM_WARREN_K) != WARREN;
+  chain_wait();
+  if (other_form || nrow <= 0) return;
   const uint32_t gmask = (LP == 32 ? 0xffffffffu : ((1u << LP) - 1u)) << (LP * h);
   const uint32_t group_lt = ((1u << lane) - 1u) & gmask;
   const uint16_t* len = KNOWN ? d.nbn : d.vn;
@@ -335,14 +335,14 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
 // The FP32 densities of pass 1 from its fixed-point sums (and the fixed-point
 // densities of the fine-grained API); the sums are zeroed for the next pass.
 __global__ void __launch_bounds__(kRowBlock) k_dens_finalize(DevState d) {
-  chain_begin();
-  const int r = d.blk_rep[blockIdx.x];
-  const int s = d.blk_row[blockIdx.x] + threadIdx.x;
-  const RepDev* R = d.reps + r;
-  if (s >= R->row_off + R->n) return;
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int s = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  const float u = R->dens_unscale_f;
+  chain_wait();
+  if (s >= end) return;
   unsigned long long *q0 = d.dsum + s, *q1 = q0 + d.dstride, *q2 = q1 + d.dstride;
   const long long a0 = (long long)*q0, a1 = (long long)*q1, a2 = (long long)*q2;
-  const float u = R->dens_unscale_f;
   d.densf[s] = make_float4(fix_to_float(a0, u), fix_to_float(a1, u), fix_to_float(a2, u), 0.0f);
   if (d.dqx) {
     d.dqx[s] = a0;
@@ -432,10 +432,12 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   __shared__ float4 bpos[kWarps][32];
   __shared__ float4 qpos[kWarps][64];
   __shared__ uint32_t qent[kWarps][64];
-  chain_begin();
-  if (KEPT && !d.vdev->rebuild) return;
-  const int r = d.blk_rep[blockIdx.x];
-  const RepDev* R = d.reps + r;
+  chain_launch();
+  if (KEPT) {  // (the constants' loads held over the wait cost rebuilds 2 %)
+    chain_wait();
+    if (!d.vdev->rebuild) return;
+  }
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   HalfStencil& S = seg[wid];
   float4* P = bpos[wid];
@@ -446,9 +448,10 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   const uint32_t lt_mask = (1u << lane) - 1u;
   const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
   const int s_end = min(s0 + rows, R->row_off + R->n);
+  const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
+  if (!KEPT) chain_wait();
   const float prune2 = KEPT ? d.vdev->rv2 : 1.0f + 1.0e-4f;
   const float rv2 = KEPT ? prune2 : 1.0f;
-  const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
   // the chunk's rows cell by cell: [cs, ce) are the chunk's rows of one cell
   for (int cs = s0; cs < s_end;) {
     const int cell = (int)d.scell[cs];

@@ -127,8 +127,8 @@ constexpr int kVerletCap = 512;  // kept-list slots per particle
 
 // Where a launch goes. chained: its kernel may be set up while the kernel before it in
 // the stream still runs (programmatic stream serialization; it waits for it in
-// chain_begin). Only a kernel whose predecessor in the stream is a kernel may be
-// chained, and only one that begins with chain_begin.
+// chain_wait). Only a kernel whose predecessor in the stream is a kernel may be
+// chained, and only one that begins with chain_launch and comes to chain_wait.
 struct Chain {
   cudaStream_t st;
   bool chained;
