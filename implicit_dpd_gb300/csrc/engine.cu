@@ -1225,23 +1225,32 @@ struct RowTriple {
   int slot;  // staging slot in h->xfer (3 n doubles each)
 };
 
-// Gathers the triples into upload order on the step's stream and copies the
-// host ones back on the exchange stream, so that each gather after the first
-// runs under the previous copy; the step's stream then waits for the copies.
-int gather_rows_out(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) {
+// Takes the triples to upload order on the step's stream: those for device or managed
+// memory in one launch, each of those for host memory to the staging buffer, copied back on
+// the exchange stream, so that each after the first runs under the previous copy; the
+// step's stream then waits for the copies.
+int rows_to_caller(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) {
   const size_t n = (size_t)R.n;
-  bool copied = false;
+  RowFields direct{};
+  bool any = false, copied = false;
   for (int k = 0; k < nf; k++) {
     if (!f[k].out) continue;
     double* view = static_cast<double*>(const_cast<void*>(device_view(f[k].out)));
-    double* tmp = view ? view : h->xfer + 3 * n * f[k].slot;
-    launch_soa_to_aos(f[k].x, f[k].y, f[k].z, h->d.loc, R.row_off, tmp, (int)n, h->st);
-    if (view) continue;
+    if (view) {
+      direct.set(k, f[k].x, f[k].y, f[k].z, view);
+      any = true;
+      continue;
+    }
+    double* tmp = h->xfer + 3 * n * f[k].slot;
+    RowFields one{};
+    one.set(0, f[k].x, f[k].y, f[k].z, tmp);
+    launch_rows_out(one, h->d.orig, R.row_off, (int)n, h->st);
     CK(cudaEventRecord(h->x_mid, h->st));
     CK(cudaStreamWaitEvent(h->xst, h->x_mid, 0));
     CK(cudaMemcpyAsync(f[k].out, tmp, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->xst));
     copied = true;
   }
+  if (any) launch_rows_out(direct, h->d.orig, R.row_off, (int)n, h->st);
   if (copied) {
     CK(cudaEventRecord(h->x_done, h->xst));
     CK(cudaStreamWaitEvent(h->st, h->x_done, 0));
@@ -1280,13 +1289,14 @@ int idpd_download_state(idpd_handle* h, int32_t r, double* pos, double* vel, dou
   const RowTriple f3[3] = {{d.px, d.py, d.pz, pos, 0}, {d.vx, d.vy, d.vz, vel, 1},
                            {d.ax, d.ay, d.az, acc, 2}};
   int rc = ensure_xst(h);
-  if (!rc) rc = gather_rows_out(h, R, f3, 3);
+  if (!rc) rc = rows_to_caller(h, R, f3, 3);
   if (rc) return rc;
   const uint32_t* uf[4] = {d.id, d.prop, d.amp_id, d.unit};
   uint32_t* uo[4] = {id, prop, amp_id, unit};
-  std::vector<uint32_t> orig(n), tmpu(n);
-  bool need_u = id || prop || amp_id || unit;
-  if (need_u) {
+  std::vector<uint32_t> orig, tmpu;
+  if (id || prop || amp_id || unit) {
+    orig.resize(n);
+    tmpu.resize(n);
     CK(cudaMemcpyAsync(orig.data(), d.orig + R.row_off, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
   }
@@ -1349,7 +1359,9 @@ int idpd_download_aux(idpd_handle* h, int32_t r, double* density, double* press,
   }
   if (delta_sumr) {
     rc = gather(delta_sumr, 3, [&](double* to) {
-      launch_soa_to_aos(d.dsx, d.dsy, d.dsz, d.loc, R.row_off, to, n, h->st);
+      RowFields f{};
+      f.set(0, d.dsx, d.dsy, d.dsz, to);
+      launch_rows_out(f, d.orig, R.row_off, n, h->st);
     });
     if (rc) return rc;
   }
@@ -1632,14 +1644,16 @@ int idpd_step_host(idpd_handle* h, int32_t r, double* pos, double* vel, double* 
   {
     double* view = static_cast<double*>(const_cast<void*>(device_view(pos)));
     double* tmp = view ? view : h->xfer;
-    launch_soa_to_aos(d.px, d.py, d.pz, d.loc, R.row_off, tmp, (int)n, h->xst);
+    RowFields f{};
+    f.set(0, d.px, d.py, d.pz, tmp);
+    launch_rows_out(f, d.orig, R.row_off, (int)n, h->xst);
     if (!view) CK(cudaMemcpyAsync(pos, tmp, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->xst));
   }
   // velocities and accelerations after the kick, the second gather under the
   // first copy; the step's stream then waits for every copy (a reorder
   // permutes the storage rows: not while they are read)
   const RowTriple f2[2] = {{d.vx, d.vy, d.vz, vel, 1}, {d.ax, d.ay, d.az, acc, 2}};
-  if ((rc = gather_rows_out(h, R, f2, 2))) return rc;
+  if ((rc = rows_to_caller(h, R, f2, 2))) return rc;
   CK(cudaEventRecord(h->x_done, h->xst));
   CK(cudaStreamWaitEvent(h->st, h->x_done, 0));
   if (++h->steps_since_sort >= h->sort_period) {
@@ -1760,9 +1774,11 @@ int idpd_dump_xyz_async(idpd_handle* h, int32_t replica, const char* path, int32
   uint32_t* u32 = reinterpret_cast<uint32_t*>(h->dump_dev + 16 + 9 * sizeof(double) * (size_t)n);
   CK(cudaMemcpyAsync(h->dump_dev, d.rep_time + replica, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                      h->st));
-  launch_soa_to_aos(d.px, d.py, d.pz, d.loc, R.row_off, f64, n, h->st);
-  launch_soa_to_aos(d.vx, d.vy, d.vz, d.loc, R.row_off, f64 + 3 * (size_t)n, n, h->st);
-  launch_soa_to_aos(d.ax, d.ay, d.az, d.loc, R.row_off, f64 + 6 * (size_t)n, n, h->st);
+  RowFields f{};
+  f.set(0, d.px, d.py, d.pz, f64);
+  f.set(1, d.vx, d.vy, d.vz, f64 + 3 * (size_t)n);
+  f.set(2, d.ax, d.ay, d.az, f64 + 6 * (size_t)n);
+  launch_rows_out(f, d.orig, R.row_off, n, h->st);
   launch_gather_u32x4(d.id, d.prop, d.amp_id, d.unit, d.loc, R.row_off, u32, n, h->st);
   CK(cudaGetLastError());
   CK(cudaEventRecord(h->dump_ready, h->st));

@@ -419,23 +419,29 @@ void launch_set_dynamics(const DevState& d, const double* pos, const double* vel
                                                   kept ? 1 : 0);
 }
 
-// Storage rows of one replica back to upload order, three doubles per row:
-// output row k comes from storage row loc[row0 + k], so the writes (to device
-// memory or straight to page-locked host memory) are in order.
-__global__ void k_soa_to_aos(const double* x, const double* y, const double* z,
-                             const uint32_t* loc, int row0, double* aos, int n) {
+// Storage rows of one replica back to upload order, three doubles per row of each field:
+// storage row row0 + k goes to output row orig[row0 + k] - row0. The reads are in order and
+// the rows' writes meet in L2; reading by output row takes a 32-byte sector for each
+// number. The three fields of 984k rows to device buffers, with one launch for all: 185 ->
+// 85 us per call.
+__global__ void __launch_bounds__(256) k_rows_out(RowFields f, const uint32_t* orig, int row0,
+                                                  int n) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const uint32_t i = loc[row0 + k];
-  aos[3 * (size_t)k] = x[i];
-  aos[3 * (size_t)k + 1] = y[i];
-  aos[3 * (size_t)k + 2] = z[i];
+  const size_t i = (size_t)row0 + k;
+  const size_t at = 3 * (size_t)(orig[i] - (uint32_t)row0);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    if (!f.out[c]) continue;
+    const double x = f.x[c][i], y = f.y[c][i], z = f.z[c][i];
+    f.out[c][at] = x;
+    f.out[c][at + 1] = y;
+    f.out[c][at + 2] = z;
+  }
 }
 
-void launch_soa_to_aos(const double* x, const double* y, const double* z, const uint32_t* loc,
-                       int row0, double* aos, int n, cudaStream_t st) {
-  if (n == 0) return;
-  k_soa_to_aos<<<(n + 255) / 256, 256, 0, st>>>(x, y, z, loc, row0, aos, n);
+void launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n, cudaStream_t st) {
+  if (n > 0) k_rows_out<<<(n + 255) / 256, 256, 0, st>>>(f, orig, row0, n);
 }
 
 // Derived fields of one replica's rows in upload order (device, managed or staging

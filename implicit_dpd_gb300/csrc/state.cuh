@@ -317,8 +317,19 @@ void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n
 void launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
                          const double* acc, int row0, int n, double box0, double box1,
                          double box2, bool kept, cudaStream_t st);
-void launch_soa_to_aos(const double* x, const double* y, const double* z, const uint32_t* loc,
-                       int row0, double* aos, int n, cudaStream_t st);
+// Up to three fields (x, y, z arrays in storage order) to rows in upload order, each three
+// doubles (out null: not this one).
+struct RowFields {
+  const double *x[3], *y[3], *z[3];
+  double* out[3];
+  void set(int c, const double* fx, const double* fy, const double* fz, double* o) {
+    x[c] = fx;
+    y[c] = fy;
+    z[c] = fz;
+    out[c] = o;
+  }
+};
+void launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n, cudaStream_t st);
 void launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
                            double* out, int n, cudaStream_t st);
 void launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
