@@ -851,18 +851,6 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
 
 int enqueue_reorder(idpd_handle* h) {
   launch_reorder(h->d, h->o, h->nblk, 4 * h->n_amp_tot, h->st);
-  const size_t n = (size_t)h->n_tot;
-  DevState& d = h->d;
-  DevState& o = h->o;
-  double* dd[12] = {d.px, d.py, d.pz, d.vx, d.vy, d.vz, d.ax, d.ay, d.az, d.dsx, d.dsy, d.dsz};
-  double* od[12] = {o.px, o.py, o.pz, o.vx, o.vy, o.vz, o.ax, o.ay, o.az, o.dsx, o.dsy, o.dsz};
-  for (int k = 0; k < 12; k++)
-    CK(cudaMemcpyAsync(dd[k], od[k], sizeof(double) * n, cudaMemcpyDeviceToDevice, h->st));
-  uint32_t* du[6] = {d.id, d.prop, d.amp_id, d.unit, d.orig, d.key};
-  uint32_t* ou[6] = {o.id, o.prop, o.amp_id, o.unit, o.orig, o.key};
-  for (int k = 0; k < 6; k++)
-    CK(cudaMemcpyAsync(du[k], ou[k], sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->st));
-  launch_update_loc(h->d, h->nblk, h->st);
   return IDPD_OK;
 }
 

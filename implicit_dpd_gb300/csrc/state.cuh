@@ -184,7 +184,6 @@ void launch_scatter_sort_pack(const DevState& d, int nblk, int zero, const Chain
 void launch_pack(const DevState& d, int nblk, int zero, const Chain& st, const int* packed);
 void launch_reorder(const DevState& d, const DevState& o, int nblk, int n_topol,
                     cudaStream_t st);
-void launch_update_loc(const DevState& d, int nblk, cudaStream_t st);
 // Counting-sort pieces on raw arrays: exclusive scan of cnt into start
 // (start[ncell] = n_tot, cnt cleared; part holds ncell / 4096 + 1 ints) and
 // the per-cell ascending order of perm.
