@@ -357,10 +357,13 @@ __global__ void __launch_bounds__(kRowBlock) k_dens_finalize(DevState d) {
 // end (the -x frame column is never owned), its part beyond the box edge apart. A
 // candidate's frame offset in x is 0 or 1.
 struct HalfStencil {
-  int tb[kMaxSeg];    // first row
-  int end[kMaxSeg];   // candidates up to and including this part
-  int fwd[kMaxSeg];   // first row whose x offset is 1
-  int dyz[kMaxSeg];   // frame offsets: dy + 1 | (dz + 1) << 2
+  struct alignas(16) Part {
+    int shift;      // row - candidate number
+    int end;        // candidates up to and including this part
+    int fwd;        // first row whose x offset is 1
+    uint32_t code;  // the frame offsets y and z of a list entry
+    float oy, oz;   // the same in length
+  } part[kMaxSeg];
 };
 
 // Lane k < (2m+1)^2 sets up row k (two parts); returns the number of candidates.
@@ -368,7 +371,7 @@ __device__ __forceinline__ int half_stencil(HalfStencil& S, const DevState& d, c
                                             int cx, int cy, int cz, int lane) {
   const int m = R->reach, w = 2 * m + 1, rs = R->rshift;
   const int nx = R->nc[0], ny = R->nc[1], nz = R->nc[2];
-  int n0 = 0, n1 = 0, b0 = 0, b1 = 0, f0 = 0x7fffffff, dyz = 0;
+  int n0 = 0, n1 = 0, b0 = 0, b1 = 0, f0 = 0x7fffffff, fy = 0, fz = 0;
   if (lane < w * w) {
     const int dz = lane / w - m, dy = lane % w - m;
     const int qz = cz + dz, wz = qz < 0 ? qz + nz : (qz >= nz ? qz - nz : qz);
@@ -382,7 +385,8 @@ __device__ __forceinline__ int half_stencil(HalfStencil& S, const DevState& d, c
       b1 = start[0];
       n1 = start[hi - nx + 1] - b1;
     }
-    dyz = ((qy >> rs) - (cy >> rs) + 1) | ((qz >> rs) - (cz >> rs) + 1) << 2;
+    fy = (qy >> rs) - (cy >> rs);
+    fz = (qz >> rs) - (cz >> rs);
   }
   int end = n0 + n1;
 #pragma unroll
@@ -391,16 +395,26 @@ __device__ __forceinline__ int half_stencil(HalfStencil& S, const DevState& d, c
     if (lane >= o) end += v;
   }
   if (lane < w * w) {
-    S.tb[2 * lane] = b0;
-    S.end[2 * lane] = end - n1;
-    S.fwd[2 * lane] = f0;
-    S.tb[2 * lane + 1] = b1;
-    S.end[2 * lane + 1] = end;
-    S.fwd[2 * lane + 1] = b1;
-    S.dyz[2 * lane] = S.dyz[2 * lane + 1] = dyz;
+    const uint32_t code = make_entry(0, -1, fy, fz);
+    const float oy = (float)fy * R->cs_f[1], oz = (float)fz * R->cs_f[2];
+    S.part[2 * lane] = {b0 - (end - n1 - n0), end - n1, f0, code, oy, oz};
+    S.part[2 * lane + 1] = {b1 - (end - n1), end, b1, code, oy, oz};
   }
   return __shfl_sync(0xffffffffu, end, 31);
 }
+
+// Two particles of a batch, as the packed FP32 instructions take them, and the lengths of
+// their lists so far: xy = (x, x', y, y'), zn = (z, z', length, length').
+struct BatchPair {
+  float4 xy, zn;
+  __device__ __forceinline__ void set(int which, float x, float y, float z) {
+    (&xy.x)[which] = x;
+    (&xy.z)[which] = y;
+    (&zn.x)[which] = z;
+    (&zn.z)[which] = __int_as_float(0);
+  }
+  __device__ __forceinline__ int length(int which) const { return __float_as_int((&zn.z)[which]); }
+};
 
 // The lists from the cells. KEPT: the kept lists (rebuild steps only), every owned
 // candidate closer than 1 + skin in FP32 (with a margin: the list only has to hold
@@ -420,16 +434,22 @@ __device__ __forceinline__ int half_stencil(HalfStencil& S, const DevState& d, c
 // rounds. Each warp builds the lists of its own chunk of `rows` rows, one cell's share of
 // it at a time (a cell split between chunks is set up by each).
 //
-// What bounds it: instruction issue of the tests. Kept lists, per rebuild: 984k-bead
-// membrane 742 -> 620 us, 998k-particle liquid 441 -> 329 us, 8k beads 105 -> 27 us.
+// What bounds it: instruction issue of the tests, about 25 instructions per particle and 32
+// candidates. Two particles are tested together, so that the distances take the packed
+// FP32 instructions, each rounded as the scalar one (984k-bead membrane 620 -> 531 us per
+// rebuild, 998k-particle liquid 329 -> 298, 131k beads without kept lists 163 -> 152 us of
+// pass 1). Fewer registers (a cap for 10 or 12 CTAs per SM) cost 6 and 12 %, loads of the
+// next candidates one round ahead 5 %, a cell's candidates shared by the CTA's warps 3 to
+// 20 % below 100k rows. Kept lists, per rebuild, against a sweep of each particle's cells:
+// 984k beads 742 us, the liquid 441, 8k beads 105 (now 27).
 // Without kept lists it replaces a sweep of each particle's own 27 cells by one warp
-// (pass 1 in all: 400k-particle liquid 766 -> 194 us, 131k-bead membrane 543 -> 171 us, 31k
-// beads with solvent 397 -> 66 us, 3k particles 206 -> 30 us); its pairs' lists are read
+// (pass 1 in all: 400k-particle liquid 766 -> 173 us, 131k-bead membrane 543 -> 152 us, 31k
+// beads with solvent 397 -> 55 us, 3k particles 206 -> 20 us); its pairs' lists are read
 // at 8 lanes per particle, whatever the tuning's lanes for kept lists.
 template <bool KEPT>
 __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) {
   __shared__ HalfStencil seg[kWarps];
-  __shared__ float4 bpos[kWarps][32];
+  __shared__ BatchPair batch[kWarps][16];
   __shared__ float4 qpos[kWarps][64];
   __shared__ uint32_t qent[kWarps][64];
   chain_launch();
@@ -440,7 +460,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   HalfStencil& S = seg[wid];
-  float4* P = bpos[wid];
+  BatchPair* P = batch[wid];
   float4* QX = qpos[wid];
   uint32_t* QE = qent[wid];
   uint32_t* lists = KEPT ? d.vl : d.nbl;
@@ -448,7 +468,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   const uint32_t lt_mask = (1u << lane) - 1u;
   const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
   const int s_end = min(s0 + rows, R->row_off + R->n);
-  const float csx = R->cs_f[0], csy = R->cs_f[1], csz = R->cs_f[2];
+  const float csx = R->cs_f[0];
   if (!KEPT) chain_wait();
   const float prune2 = KEPT ? d.vdev->rv2 : 1.0f + 1.0e-4f;
   const float rv2 = KEPT ? prune2 : 1.0f;
@@ -465,7 +485,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
       const int me = b0 + lane;  // the lane's particle (lane < nb)
       __syncwarp();
       const float4 pm = lane < nb ? d.posf[me] : d.posf[b0];
-      P[lane] = pm;
+      P[lane >> 1].set(lane & 1, lane < nb ? pm.x : 1.0e18f, pm.y, pm.z);
       float lox = pm.x, hix = pm.x, loy = pm.y, hiy = pm.y, loz = pm.z, hiz = pm.z;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -477,35 +497,48 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
         hiz = fmaxf(hiz, __shfl_xor_sync(0xffffffffu, hiz, o));
       }
       __syncwarp();
-      int cnt = 0;  // the list length of the lane's particle
-      int qn = 0;   // candidates queued for the next full round
-      // tests the 32 queued candidates against every particle of the batch:
-      // the lanes whose candidate is in range of particle k write it to k's
+      int qn = 0;  // candidates queued for the next full round
+      // tests the 32 queued candidates against every particle of the batch, two at a
+      // time: the lanes whose candidate is in range of a particle write it to its
       // list, consecutive lanes to consecutive slots
       auto round = [&](float qx, float qy, float qz, uint32_t e, int t) {
         // owns(): a candidate of the next frame column is owned by all, else qx is its
         // cell-local x (a particle never owns itself)
         const float qk = ((e >> kRowBits) & 3u) == 2u ? 3.0e38f : qx;
-#pragma unroll 4
-        for (int k = 0; k < nb; k++) {
-          const float4 pk = P[k];
-          const float dr2 = dist2(pk.x - qx, pk.y - qy, pk.z - qz);
-          const bool own = (qk > pk.x) | ((qk == pk.x) & (t > b0 + k));
-          bool in = (dr2 < rv2) & own;
+        const f32x2 nx = pack2(-qx, -qx), ny = pack2(-qy, -qy), nz = pack2(-qz, -qz);
+#pragma unroll 1
+        for (int k = 0; k < nb; k += 2) {
+          const float4 xy = P[k >> 1].xy, zn = P[k >> 1].zn;
+          const f32x2 ex = add2(pack2(xy.x, xy.y), nx), ey = add2(pack2(xy.z, xy.w), ny),
+                      ez = add2(pack2(zn.x, zn.y), nz);
+          float d0, d1;  // dist2() of both
+          unpack2(fma2(ez, ez, fma2(ex, ex, mul2(ey, ey))), d0, d1);
+          const bool own0 = (qk > xy.x) | ((qk == xy.x) & (t > b0 + k));
+          const bool own1 = (qk > xy.y) | ((qk == xy.y) & (t > b0 + k + 1));
+          bool in0 = (d0 < rv2) & own0, in1 = (d1 < rv2) & own1;
           if (!KEPT) {
-            const bool near = (fabsf(dr2 - 1.0f) <= kGuard) & own;
-            if (__any_sync(0xffffffffu, near)) {
-              if (near) in = exact_dr2(d, R, d.perm[b0 + k], d.perm[t]) < 1.0;
+            const bool near0 = (fabsf(d0 - 1.0f) <= kGuard) & own0;
+            const bool near1 = (fabsf(d1 - 1.0f) <= kGuard) & own1;
+            if (__any_sync(0xffffffffu, near0 | near1)) {
+              if (near0) in0 = exact_dr2(d, R, d.perm[b0 + k], d.perm[t]) < 1.0;
+              if (near1) in1 = exact_dr2(d, R, d.perm[b0 + k + 1], d.perm[t]) < 1.0;
             }
           }
-          const uint32_t m = __ballot_sync(0xffffffffu, in);
-          const int base = __shfl_sync(0xffffffffu, cnt, k);
-          const int pos = base + __popc(m & lt_mask);
-          if (in && pos < cap) lists[(size_t)(b0 + k) * cap + pos] = e;
-          if (lane == k) cnt += __popc(m);
+          const uint32_t m0 = __ballot_sync(0xffffffffu, in0);
+          const uint32_t m1 = __ballot_sync(0xffffffffu, in1);
+          const int n0 = __float_as_int(zn.z), n1 = __float_as_int(zn.w);
+          const int at0 = n0 + __popc(m0 & lt_mask), at1 = n1 + __popc(m1 & lt_mask);
+          uint32_t* list = lists + (size_t)(b0 + k) * cap;
+          if (in0 && at0 < cap) list[at0] = e;
+          if (in1 && at1 < cap) list[cap + at1] = e;
+          if (lane == 0)
+            *reinterpret_cast<float2*>(&P[k >> 1].zn.z) =
+                make_float2(__int_as_float(n0 + __popc(m0)), __int_as_float(n1 + __popc(m1)));
         }
+        __syncwarp();
       };
-      int g = 0, gb = 0;  // the lane's part of the stencil, candidates before it
+      int g = 0;  // the lane's part of the stencil
+      HalfStencil::Part part = S.part[0];
       for (int k0 = 0; k0 < total; k0 += 32) {
         const int c = k0 + lane;
         bool keep = false;
@@ -513,16 +546,15 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
         uint32_t e = 0;
         int t = 0;
         if (c < total) {
-          while (c >= S.end[g]) gb = S.end[g++];
-          t = S.tb[g] + (c - gb);
+          while (c >= part.end) part = S.part[++g];
+          t = c + part.shift;
           // the candidate in the frame of the cell's particles
           const float4 pj = __ldg(d.posf + t);
-          const int fx = t >= S.fwd[g], dyz = S.dyz[g];
-          const int dy = (dyz & 3) - 1, dz = (dyz >> 2) - 1;
-          qx = fmaf((float)fx, csx, pj.x);
-          qy = fmaf((float)dy, csy, pj.y);
-          qz = fmaf((float)dz, csz, pj.z);
-          e = make_entry(t, fx, dy, dz);
+          const bool fx = t >= part.fwd;
+          qx = fx ? csx + pj.x : pj.x;
+          qy = part.oy + pj.y;
+          qz = part.oz + pj.z;
+          e = (uint32_t)t | part.code | (fx ? 2u : 1u) << kRowBits;
           const float ox = fmaxf(fmaxf(lox - qx, qx - hix), 0.0f);
           const float oy = fmaxf(fmaxf(loy - qy, qy - hiy), 0.0f);
           const float oz = fmaxf(fmaxf(loz - qz, qz - hiz), 0.0f);
@@ -561,6 +593,7 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
       }
       __syncwarp();
       if (lane < nb) {
+        const int cnt = P[lane >> 1].length(lane & 1);
         (KEPT ? d.vn : d.nbn)[me] = cnt <= cap ? (uint16_t)cnt : (uint16_t)kNbrFallback;
         if (cnt > cap) d.overflow[0] = 1;
         if (KEPT) {

@@ -229,13 +229,16 @@ inline int chunk_rows(int nblk, int lp) {
 
 // The same for the list build, whose cost per cell and chunk (the stencil, the loads of
 // its candidates) is shared by the chunk's particles: halved, down to 2 rows, only while
-// the launch does not fill one wave. Measured at 32 / 16 / 8 / 4 / 2 rows, us: membranes,
-// 984k beads 620 / 639 / 740 / 963, 131k 141 / 127 / 124 / 144, 62k 121 / 79 / 76 / 84, 30k 98 /
-// 60 / 47 / 49, 8k 78 / 56 / 38 / 31 / 27; liquids, 998k 329 / 361 / 449, 200k 92 / 87 / 98, 24k
-// 38 / 27 / 21 / 25.
+// the launch does not fill one wave, from 16 and 32 rows while it does not fill two (the
+// last wave's share of it). Measured, us per build at the rows left by this rule / at half as
+// many / at twice: membranes, 250k beads 175 / 190 / 200, 131k 110 / 124 / 112, 62k 66 / 74 / 80,
+// 30k 45 / 56 / 43, 8k 27 / - / 31; liquids, 400k 136 / 138 / -, 200k 81 / 98 / 86, 24k 25 / 29 / 21;
+// without kept lists, us of pass 1: 131k membrane 147 / - / 151, 50k liquid 41 / 45 / 40 (a
+// step at twice the rows 82 instead of 76), 31k mixed 55 / 61 / 51 (106 instead of 103).
 inline int build_rows(int nblk) {
+  const long long n = (long long)nblk * kRowBlock;
   int rows = 32;
-  while (rows > 2 && (long long)nblk * kRowBlock < (long long)rows * kWaveWarps) rows >>= 1;
+  while (rows > 2 && n < (long long)rows * kWaveWarps * (rows >= 16 ? 2 : 1)) rows >>= 1;
   return rows;
 }
 
