@@ -789,10 +789,11 @@ enum CmForm { kCmNone, kCmKernels, kCmIfNode };
 
 // One MD step; `observe` adds the per-particle virial to the pair pass and
 // the observation kernels (the records are written only for replicas whose
-// step counter is due); loop.left is set inside the K-step loop graph; chained: a step's
-// last kernel is right before it in the stream.
+// step counter is due); loop.left is set inside the K-step loop graph; after, before: a
+// step is right before, right after it in the same graph (their kick and drift are one
+// kernel).
 void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_done = nullptr,
-                  const LoopTail& loop = LoopTail{}, bool chained = false) {
+                  const LoopTail& loop = LoopTail{}, bool after = false, bool before = false) {
   const int mode = pair_mode(h);
   DevState d = h->d;  // the step writes no fine-grained side outputs
   d.dqx = d.dqy = d.dqz = nullptr;
@@ -805,10 +806,9 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
   const bool marks = mode == kPairsF32 && h->prec_any && d.phit;
   const int zero = kZeroForce | (observe ? kZeroVirial : 0) | (marks ? kZeroMarks : 0);
   const StepConds conds = step_conds(h, verlet && h->n_tot > kGateRows, cm == kCmIfNode);
-  const Chain first{h->st, chained};
   if (verlet) {  // cells and lists only on rebuild steps
     const int* gate = &d.vdev->rebuild;
-    launch_drift_disp(d, h->nblk, first);
+    if (!after) launch_drift_disp(d, h->nblk, head);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
     launch_vl_decide(d, h->R, conds, after_drift);
     const IfScope c = begin_if(h, conds.on, conds.rebuild);
@@ -820,7 +820,7 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
     end_if(h, c);
     if (conds.on) launch_pack(d, h->nblk, zero, head, gate);
   } else {
-    launch_drift_bin(d, h->nblk, true, h->R, conds, first);
+    if (!after) launch_drift_bin(d, h->nblk, true, h->R, conds, head);
     if (drift_done) cudaEventRecord(drift_done, h->st);  // positions final
     launch_scan(d, h->ncell_tot, h->R - 1, after_drift);
     launch_scatter_sort_pack(d, h->nblk, zero, st);
@@ -833,6 +833,10 @@ void enqueue_step(idpd_handle* h, bool observe, CmForm cm, cudaEvent_t drift_don
     launch_precursor(d, h->nblk, marks, st);
   }
   const bool tail = observe || cm != kCmNone || h->chem_on || loop.left;
+  if (before) {
+    launch_kick_drift(d, h->nblk, verlet, st, h->R);
+    return;
+  }
   launch_bonded_kick(d, h->nblk, true, st, tail ? 0 : h->R);
   if (!tail) return;
   if (observe) launch_observe_bonds(d, h->obs_buf, h->n_amp_tot, h->amp_rep, h->st);
@@ -1456,7 +1460,7 @@ int build_graph(idpd_handle* h, cudaGraphExec_t* ge, int nsteps, bool observe, C
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < nsteps; k++)
-    enqueue_step(h, observe, cm, nullptr, LoopTail{}, k > 0);
+    enqueue_step(h, observe, cm, nullptr, LoopTail{}, k > 0, k + 1 < nsteps);
   const cudaError_t launch_err = cudaGetLastError();  // a launch refused during capture
   const cudaError_t cap_err = cudaStreamEndCapture(h->st, &g);
   if (cap_err != cudaSuccess || launch_err != cudaSuccess)

@@ -4,58 +4,9 @@
 // performs drift_and_predict (driftkick.hpp:6-27) in the same pass.
 #include <algorithm>
 
-#include "state.cuh"
+#include "row_ops.cuh"
 
 namespace idpd {
-
-// Periodic wrap of driftkick.hpp:19-21, t - floor(t / L) L with the
-// reference's rounding. Rows that stay inside [0, hi) keep t unchanged
-// without touching the FP64 pipe (the sign bit and the bit pattern order of
-// non-negative doubles decide it); all others take the reference expression.
-__device__ __forceinline__ double wrap_pbc(double t, double L, double iL, long long hi_bits) {
-  const long long b = __double_as_longlong(t);
-  if (b >= 0 && b < hi_bits) return t;
-  const double f = floor(plain_mul(t, iL));
-  return plain_add(t, -plain_mul(f, L));
-}
-
-__device__ __forceinline__ int cell_coord(double x, double inv_cs, int nc) {
-  int c = to_int(mul_f64(x, inv_cs));  // x >= 0 (or -0)
-  return c >= nc ? nc - 1 : c;
-}
-
-// drift_and_predict of one storage row (driftkick.hpp:6-27); p holds the row's position
-// on entry and the new one on return, ds its new delta_sumr.
-__device__ __forceinline__ void drift_row(const DevState& d, const RepDev* R, int i, double p[3],
-                                          double ds[3]) {
-  const double dt = R->dt, h = R->half_dt;
-  double v[3] = {d.vx[i], d.vy[i], d.vz[i]};
-  const double a[3] = {d.ax[i], d.ay[i], d.az[i]};
-  ds[0] = d.dsx[i];
-  ds[1] = d.dsy[i];
-  ds[2] = d.dsz[i];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    v[k] = add_f64(v[k], mul_f64(a[k], h));
-    const double dr = mul_f64(v[k], dt);
-    const double t = __dadd_rn(p[k], dr);
-    ds[k] = add_f64(ds[k], dr);
-    // hi = L (1 - 2^-50): below it t / L rounds below 1 and floor() is 0.
-    const double L = R->box[k];
-    const long long hi = __double_as_longlong(L) - 4;
-    p[k] = wrap_pbc(t, L, R->ibox[k], hi);
-  }
-  d.vx[i] = v[0]; d.vy[i] = v[1]; d.vz[i] = v[2];
-  d.dsx[i] = ds[0]; d.dsy[i] = ds[1]; d.dsz[i] = ds[2];
-  d.px[i] = p[0]; d.py[i] = p[1]; d.pz[i] = p[2];
-}
-
-// a - b as a float, to about 2^-32 (far beyond any skin where that cannot be told).
-__device__ __forceinline__ float diff_f32(double a, double b) {
-  const long long q = to_fix(a) - to_fix(b);
-  const bool ok = in_fix(a) && in_fix(b) && q == (long long)(int)q;
-  return ok ? __int2float_rn((int)q) * 2.3283064365386963e-10f : 1.0e3f;
-}
 
 // Whether the centre-of-mass drift removal is due for some replica, into the condition of
 // its IF node; the whole block takes part.
@@ -78,18 +29,11 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
   if (i >= end) return;
   double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
   if (do_drift) drift_row(d, R, i, p, ds);
-  const int cx = cell_coord(p[0], R->inv_cs[0], R->nc[0]);
-  const int cy = cell_coord(p[1], R->inv_cs[1], R->nc[1]);
-  const int cz = cell_coord(p[2], R->inv_cs[2], R->nc[2]);
-  const uint32_t key = (uint32_t)(R->cell_off + (cz * R->nc[1] + cy) * R->nc[0] + cx);
-  d.key[i] = key;
-  d.slot[i] = (uint32_t)atomicAdd(&d.cell_cnt[key], 1);
+  bin_row(d, R, i, p);
 }
 
 // Steps that keep the neighbour lists: drift, and the largest squared
-// displacement since the last rebuild (delta_sumr accumulates every drift,
-// unwrapped) into the rebuild record. The displacement only has to fall on the right
-// side of the threshold: it is taken in FP32, and again in FP64 close to it.
+// displacement since the last rebuild into the rebuild record.
 //
 // What bounds the elementwise kernels (this one, the pack, the kick): at 10^6 particles
 // the FP64 unit (74 - 80 % busy, DRAM 11 - 19 %), so their products, conversions and
@@ -110,28 +54,9 @@ __global__ void __launch_bounds__(kRowBlock, 8) k_drift_disp(DevState d) {
     const double r0[3] = {d.drx[s], d.dry[s], d.drz[s]};
     double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
     drift_row(d, R, i, p, ds);
-    const float fx = diff_f32(ds[0], r0[0]), fy = diff_f32(ds[1], r0[1]),
-                fz = diff_f32(ds[2], r0[2]);
-    m = fx * fx + fy * fy + fz * fz;
-    const float thr2 = d.vdev->thr2;
-    if (fabsf(m - thr2) < 1.0e-3f * thr2) {
-      const double ex = plain_add(ds[0], -r0[0]), ey = plain_add(ds[1], -r0[1]),
-                   ez = plain_add(ds[2], -r0[2]);
-      m = plain_f32(ex * ex + ey * ey + ez * ez);
-    }
+    m = displacement2(d, ds, r0);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = 0.0f;
-    for (int w = 0; w < kRowBlock / 32; w++) b = fmaxf(b, wmax[w]);
-    // non-negative floats order like their bit patterns; the running maximum
-    // is read first, so only blocks that raise it take the (single-address) atomic
-    const unsigned int bb = __float_as_uint(b);
-    if (b > 0.0f && bb > *(volatile unsigned int*)&d.vdev->maxd2) atomicMax(&d.vdev->maxd2, bb);
-  }
+  note_displacement(d, m, wmax);
 }
 
 // (Taken by the drift's last block instead, behind a counter, it was no faster below 400k
@@ -157,12 +82,8 @@ __global__ void __launch_bounds__(kRowBlock) k_bin_gated(DevState d) {
   const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
   chain_wait();
   if (!d.vdev->rebuild || i >= end) return;
-  const int cx = cell_coord(d.px[i], R->inv_cs[0], R->nc[0]);
-  const int cy = cell_coord(d.py[i], R->inv_cs[1], R->nc[1]);
-  const int cz = cell_coord(d.pz[i], R->inv_cs[2], R->nc[2]);
-  const uint32_t key = (uint32_t)(R->cell_off + (cz * R->nc[1] + cy) * R->nc[0] + cx);
-  d.key[i] = key;
-  d.slot[i] = (uint32_t)atomicAdd(&d.cell_cnt[key], 1);
+  const double p[3] = {d.px[i], d.py[i], d.pz[i]};
+  bin_row(d, R, i, p);
 }
 
 void launch_drift_disp(const DevState& d, int nblk, const Chain& st) {

@@ -4,7 +4,7 @@
 //                                 bend :117-150, cf_spring parameter.hpp:713-716)
 //   kick                          driftkick.hpp:33-40
 //   remove_cmdrift_global         driftkick.hpp:43-54
-#include "state.cuh"
+#include "row_ops.cuh"
 
 namespace idpd {
 
@@ -75,29 +75,15 @@ __device__ __forceinline__ void chain_forces(const float3 p[4], float cf_s, floa
   if (vir) *vir = v;
 }
 
-// One thread per storage row: pair force + bonded force on this bead (the
-// chain is re-evaluated per bead, no scatter), acc written in FP64, then
-// kick: vel = vel_buf + dt/2 acc (vel holds vel_buf after the drift).
-// advance: where nothing after it in the step reads or holds the step counters, the
-// first block advances them (their number; a kernel of its own for it took 1.5 us).
-template <bool KICK>
-__global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advance) {
-  chain_launch();
-  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
-  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
-  chain_wait();
-  if (KICK && blockIdx.x == 0)
-    for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
-  if (i >= end) return;
+// Pair force + bonded force on the bead of storage row i (its chain is re-evaluated per
+// bead, no scatter), in fixed point.
+__device__ __forceinline__ void row_force(const DevState& d, const RepDev* R, int i,
+                                          long long f[3]) {
   const int s = (int)d.rank[i];
   const long long* fs = d.fq + 4 * (size_t)s;
-  long long f[3] = {fs[0], fs[1], fs[2]};
-  double v[3];
-  if (KICK) {
-    v[0] = d.vx[i];
-    v[1] = d.vy[i];
-    v[2] = d.vz[i];
-  }
+  f[0] = fs[0];
+  f[1] = fs[1];
+  f[2] = fs[2];
   const uint32_t a = d.amp_id[i];
   if (a != kNone && R->n_amp > 0) {
     const int u = (int)d.unit[i];
@@ -120,6 +106,29 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advan
     f[1] += fix_force(fu.y);
     f[2] += fix_force(fu.z);
   }
+}
+
+// One thread per storage row: the force on this bead, acc written in FP64, then
+// kick: vel = vel_buf + dt/2 acc (vel holds vel_buf after the drift).
+// advance: where nothing after it in the step reads or holds the step counters, the
+// first block advances them (their number; a kernel of its own for it took 1.5 us).
+template <bool KICK>
+__global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advance) {
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
+  if (KICK && blockIdx.x == 0)
+    for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
+  if (i >= end) return;
+  double v[3];
+  if (KICK) {
+    v[0] = d.vx[i];
+    v[1] = d.vy[i];
+    v[2] = d.vz[i];
+  }
+  long long f[3];
+  row_force(d, R, i, f);
   const double acx = force_of(f[0]), acy = force_of(f[1]), acz = force_of(f[2]);
   d.ax[i] = acx;
   d.ay[i] = acy;
@@ -130,6 +139,49 @@ __global__ void __launch_bounds__(kRowBlock) k_bonded_kick(DevState d, int advan
     d.vy[i] = __dadd_rn(v[1], mul_f64(acy, h));
     d.vz[i] = __dadd_rn(v[2], mul_f64(acz, h));
   }
+}
+
+// The kick of a step and the drift of the next in a run of steps with nothing between
+// them: k_bonded_kick and k_drift_disp (KEPT) or k_drift_bin on the same row, one launch
+// and one product by dt/2 less, without the acceleration's and the velocity's way through
+// memory (the acceleration of a run's last step is the one that is kept). Us per step:
+// 998k particles 489 -> 483, 984k beads 1415 -> 1410, 110k 225.6 -> 221.3, 24k 38.5 ->
+// 36.8, 3k 34.6 -> 33.9.
+template <bool KEPT>
+__global__ void __launch_bounds__(kRowBlock, 8) k_kick_drift(DevState d, int advance) {
+  __shared__ float wmax[kRowBlock / 32];
+  chain_launch();
+  const RepDev* R = d.reps + d.blk_rep[blockIdx.x];
+  const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
+  chain_wait();
+  if (blockIdx.x == 0) {
+    for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
+    if (threadIdx.x == 0) d.overflow[1] = 0;
+  }
+  float m = 0.0f;
+  if (i < end) {
+    long long f[3];
+    row_force(d, R, i, f);
+    const double h = R->half_dt;
+    const double kv[3] = {mul_f64(force_of(f[0]), h), mul_f64(force_of(f[1]), h),
+                          mul_f64(force_of(f[2]), h)};
+    double v[3] = {__dadd_rn(d.vx[i], kv[0]), __dadd_rn(d.vy[i], kv[1]), __dadd_rn(d.vz[i], kv[2])};
+    double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
+    drift_row(d, R, i, v, kv, p, ds);
+    if (KEPT) {
+      const uint32_t s = d.rank[i];
+      const double r0[3] = {d.drx[s], d.dry[s], d.drz[s]};
+      m = displacement2(d, ds, r0);
+    } else {
+      bin_row(d, R, i, p);
+    }
+  }
+  if (KEPT) note_displacement(d, m, wmax);
+}
+
+void launch_kick_drift(const DevState& d, int nblk, bool kept, const Chain& st, int advance) {
+  if (nblk > 0)
+    launch(st, kept ? k_kick_drift<true> : k_kick_drift<false>, nblk, kRowBlock, 0, d, advance);
 }
 
 void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st, int advance) {

@@ -293,6 +293,9 @@ int walk_retrieve(WalkState* s, int kind, int tag, int n_walk, const int32_t* ni
 // kernels_integrate.cu
 // advance: the step counters of R replicas too (0: launch_step_tail does it).
 void launch_bonded_kick(const DevState& d, int nblk, bool kick, const Chain& st, int advance = 0);
+// The kick, the step counters and the next step's drift (kept: with the displacement, else
+// with the binning).
+void launch_kick_drift(const DevState& d, int nblk, bool kept, const Chain& st, int advance);
 void launch_bonded_fine(const DevState& d, int n_amp_tot, const int* amp_rep, double* vir_part,
                         cudaStream_t st);
 void launch_kick_only(const DevState& d, int nblk, cudaStream_t st);
