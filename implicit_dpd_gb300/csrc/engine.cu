@@ -92,7 +92,7 @@ struct idpd_handle {
   ObsBuffers obs_buf{};                 // per-layout scratch (null until needed)
   cudaGraphExec_t graph_obs = nullptr;  // the step with the observation
   cudaGraphExec_t graph_cm = nullptr;   // the step with the drift removal
-  cudaGraphExec_t graph_run = nullptr;  // kRunSteps plain steps
+  cudaGraphExec_t graph_run[3] = {};    // kRunSteps[k] plain steps
   std::vector<uint32_t> time_h;  // Parameter::time per replica, as rep_time on the device
   bool time_known = false;       // (not after steps with the reaction, which may stop)
   int* err_host = nullptr;       // pinned copy of the device's error word
@@ -155,7 +155,8 @@ int dalloc(idpd_handle* h, T** p, size_t count) {
 
 void invalidate_graph(idpd_handle* h) {
   for (cudaGraphExec_t* g :
-       {&h->graph_loop, &h->graph, &h->graph_obs, &h->graph_cm, &h->graph_run})
+       {&h->graph_loop, &h->graph, &h->graph_obs, &h->graph_cm, &h->graph_run[0], &h->graph_run[1],
+        &h->graph_run[2]})
     if (*g) {
       cudaGraphExecDestroy(*g);
       *g = nullptr;
@@ -1448,11 +1449,11 @@ int idpd_remove_cmdrift(idpd_handle* h) {
   return check_device_error(h);
 }
 
-// Steps of one launch of graph_run. A step inside a WHILE node, whose first kernel waits for
+// Steps of one launch of each graph_run. A step inside a WHILE node, whose first kernel waits for
 // the node, costs up to 5 us more than one in a plain graph (3k particles 42.8 us against
 // 38.5, 24k 47.7 against 46.9, 1M 503 against 497), so runs of steps without the reaction go
-// out eight at a time.
-constexpr int kRunSteps = 8;
+// out eight at a time, and what is left of a run four and two at a time.
+constexpr int kRunSteps[3] = {8, 4, 2};
 
 // Captures nsteps steps into *ge (if it is not there yet).
 int build_graph(idpd_handle* h, cudaGraphExec_t* ge, int nsteps, bool observe, CmForm cm) {
@@ -1532,7 +1533,8 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   if (loop && !h->graph_loop && !build_loop_graph(h)) h->loop_failed = true;
   const bool use_loop = loop && h->graph_loop;
   const bool use_run = !every_cm && nsteps > 1;
-  if (use_run && (rc = build_graph(h, &h->graph_run, kRunSteps, false, kCmNone))) return rc;
+  for (int k = 0; k < 3 && use_run; k++)
+    if ((rc = build_graph(h, &h->graph_run[k], kRunSteps[k], false, kCmNone))) return rc;
   // whether some replica's step counter is a multiple of `period`, `ahead` steps from now
   auto due = [&](int period, int ahead) {
     for (uint32_t t : h->time_h)
@@ -1544,21 +1546,25 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   CK(cudaEventRecord(h->ev0, h->st));
   for (int k = 0; k < nsteps;) {
     // a step that observes or removes the drift is one launch of its graph; the steps up to
-    // the next of these, or the next storage reorder, go out kRunSteps at a time (with the
-    // reaction, as one launch of the loop)
+    // the next of these, or the next storage reorder, go out in runs (with the reaction, as
+    // one launch of the loop)
     const bool obs = observes(0), cm = removes(0);
-    int c = 1;
+    int c = 1, run = 3;
     if (!obs && !cm && (use_loop || use_run)) {
       const int room = std::min(nsteps - k, std::max(h->sort_period - h->steps_since_sort, 1));
-      const int most = use_loop ? room : kRunSteps;
+      const int most = use_loop ? room : kRunSteps[0];
       while (c < room && c < most && !observes(c) && !removes(c)) c++;
-      if (use_run && c < kRunSteps) c = 1;
+      if (use_run) {
+        run = 0;
+        while (run < 3 && kRunSteps[run] > c) run++;
+        c = run < 3 ? kRunSteps[run] : 1;
+      }
     }
     if (c > 1 && use_loop) {
       launch_loop_set(h->loop_left, c, h->st);
       CK(cudaGraphLaunch(h->graph_loop, h->st));
     } else if (c > 1) {
-      CK(cudaGraphLaunch(h->graph_run, h->st));
+      CK(cudaGraphLaunch(h->graph_run[run], h->st));
     } else {
       cudaGraphExec_t* ge = obs ? &h->graph_obs : (cm ? &h->graph_cm : &h->graph);
       if ((rc = build_graph(h, ge, 1, obs, kCmKernels))) return rc;
