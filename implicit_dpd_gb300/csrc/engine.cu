@@ -246,8 +246,7 @@ void fill_repdev(RepDev& R, const idpd_params& p, int reach, float skin) {
 
 // A caller buffer that lives in device or managed memory, which the kernels
 // read or write where it lies; null for host memory, which goes through the
-// staging buffer and a copy engine (page-locked memory read by the kernels
-// over the host link measured slower than the copies).
+// staging buffer and a copy engine unless link_view takes it.
 const void* device_view(const void* p) {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -256,6 +255,23 @@ const void* device_view(const void* p) {
   }
   if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) return p;
   return nullptr;
+}
+
+// A caller buffer of n doubles in page-locked host memory, which kernels read and write over
+// the host link in whole cache lines, as fast as a copy engine and without the staging
+// buffer's kernel behind it; null for any other, and for one that is not aligned or not
+// page-locked to its end.
+double* link_view(const double* p, size_t n) {
+  cudaPointerAttributes a{}, z{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&z, p + n - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  double* v = static_cast<double*>(a.devicePointer);
+  const bool ok = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && v &&
+                  z.devicePointer == v + (n - 1) && reinterpret_cast<uintptr_t>(v) % 8 == 0;
+  return ok ? v : nullptr;
 }
 
 // Bit f set when some replica uses pair-force form f.
@@ -1141,6 +1157,16 @@ int idpd_set_dynamics(idpd_handle* h, int32_t r, const double* pos, const double
   // copied to the staging buffer first
   const double* src[3] = {pos, vel, acc};
   const double* dev[3];
+  // with built kept lists the position change counts as displacement (the
+  // next step rebuilds when it is too large); else the lists are rebuilt
+  const bool kept = h->d.vdev && !h->vl_dirty && h->tune.skin > 0.0f;
+  for (int k = 0; k < 3; k++) dev[k] = link_view(src[k], 3 * n);
+  if (dev[0] && dev[1] && dev[2]) {
+    launch_set_dynamics_host(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1],
+                             R.box[2], kept, h->st);
+    h->density_valid = false;
+    return IDPD_OK;
+  }
   for (int k = 0; k < 3; k++) {
     dev[k] = static_cast<const double*>(device_view(src[k]));
     if (!dev[k]) {
@@ -1149,9 +1175,6 @@ int idpd_set_dynamics(idpd_handle* h, int32_t r, const double* pos, const double
       dev[k] = stage;
     }
   }
-  // with built kept lists the position change counts as displacement (the
-  // next step rebuilds when it is too large); else the lists are rebuilt
-  const bool kept = h->d.vdev && !h->vl_dirty && h->tune.skin > 0.0f;
   launch_set_dynamics(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1], R.box[2],
                       kept, h->st);
   h->density_valid = false;
@@ -1219,9 +1242,10 @@ struct RowTriple {
 };
 
 // Takes the triples to upload order on the step's stream: those for device or managed
-// memory in one launch, each of those for host memory to the staging buffer, copied back on
-// the exchange stream, so that each after the first runs under the previous copy; the
-// step's stream then waits for the copies.
+// memory in one launch, those for page-locked host memory over the link, each of those for
+// other host memory to the staging buffer, copied back on the exchange stream, so that
+// each after the first runs under the previous copy; the step's stream then waits for the
+// copies.
 int rows_to_caller(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) {
   const size_t n = (size_t)R.n;
   RowFields direct{};
@@ -1232,6 +1256,10 @@ int rows_to_caller(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) 
     if (view) {
       direct.set(k, f[k].x, f[k].y, f[k].z, view);
       any = true;
+      continue;
+    }
+    if (double* link = link_view(f[k].out, 3 * n)) {
+      launch_rows_host(f[k].x, f[k].y, f[k].z, h->d.loc, R.row_off, link, (int)n, h->st);
       continue;
     }
     double* tmp = h->xfer + 3 * n * f[k].slot;

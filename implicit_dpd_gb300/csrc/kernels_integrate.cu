@@ -471,6 +471,59 @@ void launch_set_dynamics(const DevState& d, const double* pos, const double* vel
                                                   kept ? 1 : 0);
 }
 
+// The same from page-locked host memory, read where it lies: a thread per number of the
+// arrays, so that the reads over the host link are whole cache lines (188 GB/s, a copy
+// engine's rate; a thread per row read 24-byte pieces and was slower than the copies), to
+// storage rows through loc. Four idpd_step_host calls of 131k beads 1590 -> 1499 us, of 20k
+// 590 -> 546, of 500k 4688 -> 4502, with k_rows_host below (five sixths of it here: three
+// copies and the kernel behind them were 63 us of 131k rows, this is 50).
+__global__ void __launch_bounds__(256) k_set_dynamics_host(DevState d, const double* pos,
+                                                           const double* vel, const double* acc,
+                                                           int row0, int n, double b0, double b1,
+                                                           double b2, int kept) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 3 * (size_t)n) return;
+  const double p = pos[e], v = vel[e], a = acc[e];
+  const int c = (int)(e % 3);
+  const uint32_t i = d.loc[row0 + (int)(e / 3)];
+  const double box = c == 0 ? b0 : (c == 1 ? b1 : b2);
+  if (!(p >= 0.0 && p <= box && isfinite(v) && isfinite(a))) atomicCAS(d.err, 0, kErrBadCell);
+  double* x = c == 0 ? d.px : (c == 1 ? d.py : d.pz);
+  if (kept) {
+    double t = p - x[i];
+    t = t > 0.5 * box ? t - box : (t < -0.5 * box ? t + box : t);
+    (c == 0 ? d.drx : (c == 1 ? d.dry : d.drz))[d.rank[i]] -= t;
+  }
+  x[i] = p;
+  (c == 0 ? d.vx : (c == 1 ? d.vy : d.vz))[i] = v;
+  (c == 0 ? d.ax : (c == 1 ? d.ay : d.az))[i] = a;
+}
+
+void launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
+                              const double* acc, int row0, int n, double box0, double box1,
+                              double box2, bool kept, cudaStream_t st) {
+  if (n > 0)
+    k_set_dynamics_host<<<(unsigned)((3 * (size_t)n + 255) / 256), 256, 0, st>>>(
+        d, pos, vel, acc, row0, n, box0, box1, box2, kept ? 1 : 0);
+}
+
+// A field to page-locked host memory, written where it lies: a thread per number, whole
+// cache lines over the host link.
+__global__ void __launch_bounds__(256) k_rows_host(const double* x, const double* y,
+                                                   const double* z, const uint32_t* loc, int row0,
+                                                   double* out, int n) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 3 * (size_t)n) return;
+  const int c = (int)(e % 3);
+  out[e] = (c == 0 ? x : (c == 1 ? y : z))[loc[row0 + (int)(e / 3)]];
+}
+
+void launch_rows_host(const double* x, const double* y, const double* z, const uint32_t* loc,
+                      int row0, double* out, int n, cudaStream_t st) {
+  if (n > 0)
+    k_rows_host<<<(unsigned)((3 * (size_t)n + 255) / 256), 256, 0, st>>>(x, y, z, loc, row0, out, n);
+}
+
 // Storage rows of one replica back to upload order, three doubles per row of each field:
 // storage row row0 + k goes to output row orig[row0 + k] - row0. The reads are in order and
 // the rows' writes meet in L2; reading by output row takes a 32-byte sector for each

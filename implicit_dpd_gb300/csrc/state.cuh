@@ -319,6 +319,11 @@ void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n
 void launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
                          const double* acc, int row0, int n, double box0, double box1,
                          double box2, bool kept, cudaStream_t st);
+void launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
+                              const double* acc, int row0, int n, double box0, double box1,
+                              double box2, bool kept, cudaStream_t st);
+void launch_rows_host(const double* x, const double* y, const double* z, const uint32_t* loc,
+                      int row0, double* out, int n, cudaStream_t st);
 // Up to three fields (x, y, z arrays in storage order) to rows in upload order, each three
 // doubles (out null: not this one).
 struct RowFields {
