@@ -43,7 +43,7 @@ METRIC = "particle-steps/s on 1 GB300: FP32+batched vs plain FP64 kernel at stat
 # reads the particle's posf (16 B) and writes its densf (16 B); the force pass
 # reads posf, velf, densf (3 x 16 B) and writes the fixed-point force (3 x 8 B).
 PAIR_KERNELS = {
-    "density": {"kernel": "k_density_f32", "bytes_per_particle": 32,
+    "density": {"kernel": "k_density_list", "bytes_per_particle": 32,
                 "profile": "density_membrane_1m.md"},
     "force": {"kernel": "k_force_f32", "bytes_per_particle": 72,
               "profile": "force_membrane_1m.md"},
@@ -54,20 +54,18 @@ STEP_BYTES_PER_PARTICLE = 176  # compulsory HBM bytes of one particle-step
 # (the Saru hash and draws) + 5 SFU (sqrt r, rcp, sqrt w, log, cos); the
 # density pass ~12 FP32 + 1 SFU.
 OPS_PER_ORDERED_PAIR = {"force": 134, "density": 13}
-# Kernels a captured step launches (the loop node repeats them): without kept
-# lists drift_bin, scan x3, scatter, cell_sort, pack, density, density
-# finalize, force, force walk, bonded_kick, the drift-removal condition, time,
-# the loop's tail; with kept lists drift_disp, rebuild decision, two rebuild
-# conditions, pack, density (kept lists, overflowed kept lists), density
-# finalize, force, force walk, bonded_kick, the drift-removal condition, time,
-# the loop's tail. A rebuild step adds the IF body of the cells and lists (bin,
-# scan x3, scatter, cell_sort, list build); a step whose replica counter is a
-# multiple of 100 adds the drift removal (3 kernels).
-KERNELS_PER_STEP = 15
-KERNELS_PER_KEPT_STEP = 14
-KERNELS_PER_REBUILD = 7
-KERNELS_PER_CM = 3
-KERNELS_PER_REORDER = 4        # gather, topology, identity, loc
+# Kernels a captured step launches: without kept lists drift_bin, scan x2, scatter,
+# sort_pack, pair_build, density over the lists, over the overflowed lists, density
+# finalize, force, force walk, bonded_kick; with kept lists (above 400,000 rows) drift_disp,
+# rebuild decision, pack, density x2, density finalize, force, force walk, bonded_kick.
+# A rebuild step adds the IF body of the cells and lists (bin, scan x2, scatter,
+# sort_pack, list build); a step whose replica counter is a multiple of 100 adds the
+# drift removal (3 kernels) and the step counters' kernel (else part of the kick).
+KERNELS_PER_STEP = 12
+KERNELS_PER_KEPT_STEP = 9
+KERNELS_PER_REBUILD = 6
+KERNELS_PER_CM = 4
+KERNELS_PER_REORDER = 3        # gather, topology, copy back
 
 
 def n_amp_for(box, layers):
@@ -623,7 +621,7 @@ def replicas_bench(steps=50, n_rep=256, device=0, rank=0, world=1, dist=None):
         upload(eb, k, k)
     eb.step(3)
     dist.barrier()
-    eb.step(steps)  # the steps in one graph launch (the step in a WHILE node)
+    eb.step(steps)  # eight steps per graph launch
     batched = n_tot * steps / (dist.max(eb.last_step_ms()) * 1e-3)
     # the same batch with one graph launch per step
     ep = Engine(n_replicas=len(mine), device=device, flags=CFG_PLAIN_GRAPHS)
@@ -668,8 +666,7 @@ def replicas_bench(steps=50, n_rep=256, device=0, rank=0, world=1, dist=None):
             "steps": steps, "tuning": tuned,
             "batched": batched, "batched_per_step_launch": per_step_launch,
             "one_at_a_time": one_at_a_time,
-            "launch": "batched: the steps of one idpd_step call in one graph launch (the "
-                      "captured step repeated by a conditional WHILE node on the device); "
+            "launch": "batched: the steps of one idpd_step call eight per graph launch; "
                       "batched_per_step_launch: one graph launch per step",
             "speedup": batched / one_at_a_time, "unit": "particle-steps/s",
             "launch_gaps": {"tuning": {"reach": reach, "skin": 0.0}, "graph_ms_per_step": graph_ms,
@@ -780,15 +777,16 @@ def pair_roofline(kernel_ms, pairs, n, clocks, device, which=None):
                                                  if traffic else None)}}
 
 
-def gpu_launches(steps, kept, rebuilds, t0, n_reorders):
+def gpu_launches(steps, kept, rebuilds, t0, n_reorders, loop=True):
     """The kernels the timed steps launch: per step those of the captured
-    step, the IF bodies that ran (rebuilds with kept lists, the drift removal
-    at step counters that are multiples of 100), one count kernel per launch
-    of the loop (split at each storage reorder) and the reorders' kernels."""
+    step, what the rebuilds (with kept lists) and the drift removal (at step
+    counters that are multiples of 100) add, the reorders' kernels and, where the
+    steps go out in the loop graph (with the reaction), one count kernel per
+    launch of it (split at each storage reorder)."""
     cm = sum(1 for t in range(t0, t0 + steps) if t % 100 == 0)
     per = KERNELS_PER_KEPT_STEP if kept else KERNELS_PER_STEP
     return (steps * per + (rebuilds * KERNELS_PER_REBUILD if kept else 0) + cm * KERNELS_PER_CM
-            + (n_reorders + 1) + n_reorders * KERNELS_PER_REORDER)
+            + (n_reorders + 1 if loop else 0) + n_reorders * KERNELS_PER_REORDER)
 
 
 def step_roofline(roofline, n, ms_per_step):
@@ -963,10 +961,8 @@ def run_engine(args, rank, world, local_rank):
            "kernel_ms": kernel_ms, "fp64_plain": fp64, "fp64_same_algorithm": fp64_same,
            "e2e": e2e, "cpu_baseline": cpu,
            "batched_replicas": batched, "reaction": reaction, "liquid": liquid,
-           # per step its kernels and the loop's tail node; per launch of the
-           # loop its count kernel (one launch, split at each reorder)
            "gpu_launches": gpu_launches(args.steps, reach["skin"] > 0, rebuilds, t0_step,
-                                        n_reorders),
+                                        n_reorders, loop=False),
            "force_error_bar": "max-particle relative force error <= 1e-5 vs FP64 (tests/test_gpu_parity.py)"}
     if rank == 0:
         print(json.dumps(out), flush=True)

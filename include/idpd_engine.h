@@ -113,12 +113,13 @@ typedef struct idpd_config {
 #define IDPD_CFG_FP64_KEPT 0x4
 /* Plain graphs: idpd_step(h, K) launches one graph per step, and the step's
  * graph holds no conditional nodes (every gated kernel is launched and skips
- * itself). By default the K steps go to the device in one launch, a graph
- * whose conditional WHILE node repeats the captured step K times (between
- * storage reorders and observing steps), and the step's rarely needed work
- * (the cell and list rebuild, the drift removal) sits in conditional IF
- * nodes. Results are the same either way; profilers that cannot trace the
- * kernels of graphs with conditional nodes need the plain form. */
+ * itself). By default the K steps go out eight per graph (with the reaction
+ * in one launch: a conditional WHILE node repeats the captured step), between
+ * storage reorders, observing steps and steps that remove the drift; the
+ * drift removal is in the graph of the steps that are due only, and above
+ * 400,000 rows the cell and list rebuild is in a conditional IF node. Results
+ * are the same either way; profilers that cannot trace the kernels of graphs
+ * with conditional nodes need the plain form. */
 #define IDPD_CFG_PLAIN_GRAPHS 0x8
 
 int idpd_create(const idpd_config* cfg, idpd_handle** out);
@@ -200,11 +201,12 @@ int idpd_remove_cmdrift(idpd_handle* h);
 
 /* nsteps iterations of the main loop body of src/main.cpp:166-184 (drift,
  * density, force, bonded, kick, centre-of-mass drift removal every 100 steps,
- * time += 1) for every replica, captured once into a CUDA graph. The steps up
- * to the next storage reorder or observing step go to the device in one
- * launch (the graph's conditional WHILE node repeats the step, and ends the
- * loop after a step whose reaction event stopped the run); an observing step
- * is one launch, and with IDPD_CFG_PLAIN_GRAPHS every step is.
+ * time += 1) for every replica, captured once into CUDA graphs. The steps up
+ * to the next storage reorder, observing step or step that removes the drift
+ * go to the device eight per launch, the rest one by one; with the reaction in
+ * one launch (the graph's conditional WHILE node repeats the step, and ends
+ * the loop after a step whose reaction event stopped the run). With
+ * IDPD_CFG_PLAIN_GRAPHS every step is a launch.
  * Per-particle press and nei_cm_pos are not produced by this path. */
 int idpd_step(idpd_handle* h, int32_t nsteps);
 /* Blocks until the handle's stream is idle; reports device-side errors. */
