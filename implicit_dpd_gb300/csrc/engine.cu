@@ -1045,6 +1045,8 @@ int idpd_set_params(idpd_handle* h, int32_t r, const idpd_params* p) {
   if (rc) return rc;
   const bool geom_changed = !h->params_set[r] ||
                             std::memcmp(h->params[r].box, p->box, sizeof(p->box)) != 0;
+  // the captured steps hold the pair passes of the forms present
+  if (h->params_set[r] && h->params[r].form != p->form) invalidate_graph(h);
   h->params[r] = *p;
   h->params_set[r] = 1;
   if (geom_changed && h->on_device) {

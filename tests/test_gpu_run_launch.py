@@ -7,7 +7,7 @@ set in between and across a step on host arrays."""
 import numpy as np
 import pytest
 
-from helpers import mdpd_params, mixed_system
+from helpers import mdpd_params, mixed_system, warren_params
 from implicit_dpd_gb300 import configs
 from implicit_dpd_gb300.abi import CFG_PLAIN_GRAPHS, FORM_WARREN
 from implicit_dpd_gb300.engine import Engine, derive_params
@@ -105,5 +105,32 @@ def test_host_array_steps_remove_the_drift_when_due():
 
     (a, ta), (b, tb) = run(True), run(False)
     assert ta == tb == 102
+    for k in ("pos", "vel", "acc"):
+        assert np.array_equal(a[k], b[k]), k
+
+
+def test_a_change_of_the_pair_form_between_steps():
+    # the captured steps hold one form's passes: after the change, as a fresh handle
+    box, st, n_amp = mixed_system(seed=91)
+
+    def engine(p, state):
+        e = Engine()
+        e.set_params(p)
+        e.upload(state)
+        e.build_topology(n_amp)
+        return e
+
+    e = engine(mdpd_params(box, time=3), st)
+    e.step(5)
+    mid = e.download()
+    q = warren_params(box, time=8)
+    e.set_params(q)
+    e.step(5)
+    a = e.download()
+    e.close()
+    e = engine(q, mid)
+    e.step(5)
+    b = e.download()
+    e.close()
     for k in ("pos", "vel", "acc"):
         assert np.array_equal(a[k], b[k]), k
