@@ -210,7 +210,8 @@ __device__ __forceinline__ void add_weight(uint32_t& q0, uint32_t& q1, uint32_t&
 // so the chunk is halved while the launch has fewer than kListWarps warps (five waves
 // of the 4,864 a GB300 holds at 64 registers), but not below two groups, whose setup
 // (the sort of the rows, the tables) is then a large part of the warp's work, unless
-// even one wave is not full. Measured at 32 / 16 / 8 / 4 / 2 rows, us. Pass 2,
+// not even two waves are full (one wave as the line: 31k mixed 101.4 us per step instead of
+// 100.1, 62k membrane 141.7 instead of 139.4, others the same; half a wave: 31k 105). Measured at 32 / 16 / 8 / 4 / 2 rows, us. Pass 2,
 // membranes at 16 lanes: 984k beads 888 / 880 / 900 / 968 / 1098, 250k 283 / 254 / 247 /
 // 254 / 274, 131k 168 / 157 / 145 / 143 / 154, 62k 117 / 87 / 85 / 80 / 82, 8k 98 / 59 / 39
 // / 28 / 27; liquids at 4 lanes, 998k 213 / 227 / 266, 200k 59 / 57 / 61, 24k 24 / 20 / 18.
@@ -223,7 +224,7 @@ inline int chunk_rows(int nblk, int lp) {
   const long long n = (long long)nblk * kRowBlock;
   int rows = 32;
   while (rows > 2 * g && n < (long long)rows * kListWarps) rows >>= 1;
-  if (rows == 2 * g && n < (long long)rows * kWaveWarps) rows = g;
+  if (rows == 2 * g && n < 2ll * rows * kWaveWarps) rows = g;
   return rows;
 }
 
