@@ -133,7 +133,7 @@ __device__ __forceinline__ float owned_pair(const DevState& d, const RepDev* R, 
                                             bool valid, float4 pj, float4 vj, float4 dj, float& ex,
                                             float& ey, float& ez) {
   const int t = (int)(e & kRowMask);
-  const float4 o = OT.o[e >> kRowBits];
+  const auto o = OT.at(e >> kRowBits);
   ex = (I.pi.x - o.x) - pj.x;
   ey = (I.pi.y - o.y) - pj.y;
   ez = (I.pi.z - o.z) - pj.z;

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int 
       e_next = k0 + LP + sl < nv ? list[k0 + LP + sl] : none;
       const int t = (int)(e & kRowMask);
       const float4 pj = __ldg(d.posf + t);
-      const float4 o = OT.o[e >> kRowBits];  // far away on a lane without a candidate
+      const auto o = OT.at(e >> kRowBits);  // far away on a lane without a candidate
       const float dr2 = dist2((pi.x - o.x) - pj.x, (pi.y - o.y) - pj.y, (pi.z - o.z) - pj.z);
       bool in1 = dr2 < (KNOWN ? 4.0f : 1.0f);
       bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
