@@ -359,7 +359,7 @@ typedef struct idpd_result_dpd { double acc[3], press[3]; } idpd_result_dpd;
 enum { IDPD_WALK_DENSITY = 0, IDPD_WALK_FORCE = 1 };
 
 /* DispatchKernel: copies the walks to the device and starts the pass; returns
- * without waiting. epi[w] / epj[w] point to n_epi[w] / n_epj[w] structs of the
+ * without waiting for it (the caller's records are its own again on return). epi[w] / epj[w] point to n_epi[w] / n_epj[w] structs of the
  * kind's EPI / EPJ type. One dispatch per kind may be in flight; tag is kept
  * for the matching retrieve. */
 int idpd_dispatch_walks(idpd_handle* h, int32_t kind, int32_t tag, int32_t n_walk,
