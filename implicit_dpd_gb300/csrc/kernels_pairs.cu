@@ -444,8 +444,7 @@ struct BatchPair {
 // 984k beads 742 us, the liquid 441, 8k beads 105 (now 27).
 // Without kept lists it replaces a sweep of each particle's own 27 cells by one warp
 // (pass 1 in all: 400k-particle liquid 766 -> 173 us, 131k-bead membrane 543 -> 152 us, 31k
-// beads with solvent 397 -> 55 us, 3k particles 206 -> 20 us); its pairs' lists are read
-// at 8 lanes per particle, whatever the tuning's lanes for kept lists.
+// beads with solvent 397 -> 55 us, 3k particles 206 -> 20 us).
 template <bool KEPT>
 __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) {
   __shared__ HalfStencil seg[kWarps];
@@ -689,7 +688,10 @@ void launch_density_f32(const DevState& d, int nblk, int lanes, int form_mask, C
     const int rows = build_rows(nblk);
     launch(st, k_pair_build<false>, dim3(nblk, 32 / rows), kRowBlock, 0, d, rows);
     st.chained = true;
-    lanes = 8;
+    // whatever the tuning's lanes for kept lists. Us per step at 16 / 8 / 4 lanes: liquids, 3k
+    // 32.9 / 33.5 / 34.4, 6k 36.5 / 37.2 / 37.2, 50k 74.9 / 73.3 / 72.9, 400k 324 / 311 / 304; 31k
+    // mixed 100.0 / 99.3 / 104.4, 131k membrane 279 / 277 / 281
+    lanes = nblk * kRowBlock < 16384 ? 16 : 8;
   }
   if (form_mask & (1 << IDPD_FORM_WARREN_K)) {
     launch_density_lists<MARKS, true, !VERLET>(d, nblk, lanes, st);
