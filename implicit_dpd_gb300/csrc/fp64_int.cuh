@@ -203,6 +203,19 @@ IDPD_HD int to_int(double x) {
   return (int)(((b & kMant) | kHidden) >> (52 - e));
 }
 
+// The cell of coordinate x on an axis of nc cells, inv_cs cells per unit length: the
+// truncated product, and the nearest cell for a coordinate outside the box, 0 for NaN (a run
+// that diverged, a caller's rows that are refused later), so that the result is always an
+// index below nc.
+IDPD_HD int cell_index(double x, double inv_cs, int nc) {
+  const double q = mul_f64(x, inv_cs);
+  const uint64_t b = f64_bits(q);
+  if (b >= 0x41E0000000000000ull)  // 2^31 and above, infinite, NaN, negative
+    return b <= 0x7FF0000000000000ull ? nc - 1 : 0;
+  const int c = to_int(q);
+  return c >= nc ? nc - 1 : c;
+}
+
 // |x| > y for y >= 0, x finite.
 IDPD_HD bool abs_above(double x, double y) { return (f64_bits(x) << 1) > (f64_bits(y) << 1); }
 

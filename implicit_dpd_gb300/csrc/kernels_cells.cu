@@ -464,9 +464,9 @@ __global__ void __launch_bounds__(256) k_bin_rows(const double* pos, int n, doub
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* p = pos + 3 * (size_t)i;
-  const int cx = cell_coord(p[0], ix, nx);
-  const int cy = cell_coord(p[1], iy, ny);
-  const int cz = cell_coord(p[2], iz, nz);
+  const int cx = cell_index(p[0], ix, nx);
+  const int cy = cell_index(p[1], iy, ny);
+  const int cz = cell_index(p[2], iz, nz);
   const uint32_t c = (uint32_t)((cz * ny + cy) * nx + cx);
   cell[i] = c;
   slot[i] = (uint32_t)atomicAdd(&cnt[c], 1);

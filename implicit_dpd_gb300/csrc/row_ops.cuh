@@ -17,11 +17,6 @@ __device__ __forceinline__ double wrap_pbc(double t, double L, double iL, long l
   return plain_add(t, -plain_mul(f, L));
 }
 
-__device__ __forceinline__ int cell_coord(double x, double inv_cs, int nc) {
-  int c = to_int(mul_f64(x, inv_cs));  // x >= 0 (or -0)
-  return c >= nc ? nc - 1 : c;
-}
-
 // drift_and_predict of one storage row (driftkick.hpp:6-27), from its velocity v and
 // kv = a dt/2; p holds the row's position on entry and the new one on return, ds its new
 // delta_sumr.
@@ -99,9 +94,9 @@ __device__ __forceinline__ void note_displacement(const DevState& d, float m, fl
 // Cell index and arrival slot of row i at position p.
 __device__ __forceinline__ void bin_row(const DevState& d, const RepDev* R, int i,
                                         const double p[3]) {
-  const int cx = cell_coord(p[0], R->inv_cs[0], R->nc[0]);
-  const int cy = cell_coord(p[1], R->inv_cs[1], R->nc[1]);
-  const int cz = cell_coord(p[2], R->inv_cs[2], R->nc[2]);
+  const int cx = cell_index(p[0], R->inv_cs[0], R->nc[0]);
+  const int cy = cell_index(p[1], R->inv_cs[1], R->nc[1]);
+  const int cz = cell_index(p[2], R->inv_cs[2], R->nc[2]);
   const uint32_t key = (uint32_t)(R->cell_off + (cz * R->nc[1] + cy) * R->nc[0] + cx);
   d.key[i] = key;
   d.slot[i] = (uint32_t)atomicAdd(&d.cell_cnt[key], 1);
