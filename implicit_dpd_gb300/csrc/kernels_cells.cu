@@ -25,7 +25,6 @@ __global__ void __launch_bounds__(kRowBlock) k_drift_bin(DevState d, int do_drif
   const int i = d.blk_row[blockIdx.x] + threadIdx.x, end = R->row_off + R->n;
   chain_wait();
   if (conds.cm_on && blockIdx.x == 0) set_cm_cond(conds, d.rep_time, nrep);
-  if (blockIdx.x == 0 && threadIdx.x == 0) d.overflow[1] = 0;
   if (i >= end) return;
   double p[3] = {d.px[i], d.py[i], d.pz[i]}, ds[3];
   if (do_drift) drift_row(d, R, i, p, ds);

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kRowBlock, 8) k_kick_drift(DevState d, int adv
   chain_wait();
   if (blockIdx.x == 0) {
     for (int t = threadIdx.x; t < advance; t += kRowBlock) d.rep_time[t] += 1u;
-    if (threadIdx.x == 0) d.overflow[1] = 0;
+    if (KEPT && threadIdx.x == 0) d.overflow[1] = 0;
   }
   float m = 0.0f;
   if (i < end) {

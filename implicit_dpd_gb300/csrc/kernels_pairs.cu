@@ -468,7 +468,10 @@ __global__ void __launch_bounds__(kRowBlock) k_pair_build(DevState d, int rows) 
   const int s0 = d.blk_row[blockIdx.x] + 32 * wid + rows * blockIdx.y;
   const int s_end = min(s0 + rows, R->row_off + R->n);
   const float csx = R->cs_f[0];
-  if (!KEPT) chain_wait();
+  if (!KEPT) {
+    chain_wait();
+    if (blockIdx.x + blockIdx.y == 0 && threadIdx.x == 0) d.overflow[1] = 0;
+  }
   const float prune2 = KEPT ? d.vdev->rv2 : 1.0f + 1.0e-4f;
   const float rv2 = KEPT ? prune2 : 1.0f;
   // the chunk's rows cell by cell: [cs, ce) are the chunk's rows of one cell

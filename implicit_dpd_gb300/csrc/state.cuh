@@ -67,7 +67,11 @@ struct DevState {
                      // counted by pass 1 (2 x the owned pairs in the once-per-pair passes)
   double* rep_mean;  // [R * 3]
   int* err;          // device error word (0 = ok)
-  int* overflow;     // [2] some list of the last build, some pass-2 list of the step did not fit
+  // [2] some list of the last build (cleared with its cells' scan), some pass-2 list did not
+  // fit. The second holds as long as the lists do, which outlive a new binning at the same
+  // positions: cleared where pass 1 comes next, by the drift of a step with kept lists
+  // and by the build of pass-2 lists.
+  int* overflow;
   unsigned long long* prec_count;  // [R] precursor conversions per replica
   uint8_t* phit;                   // [N] pass 1 took a pair of the conversion's properties
   // ---- neighbour lists kept between rebuilds (null when the skin is 0)
