@@ -2007,8 +2007,7 @@ int idpd_set_observe(idpd_handle* h, int32_t period, int32_t capacity) {
   cudaSetDevice(h->device);
   CK(cudaStreamSynchronize(h->st));
   if (period > 0 && capacity != h->obs_cap) {
-    if (h->walks) walk_destroy(h->walks);
-  if (h->obs_rec) cudaFree(h->obs_rec);
+    if (h->obs_rec) cudaFree(h->obs_rec);
     h->obs_rec = nullptr;
     CK(cudaMalloc((void**)&h->obs_rec, sizeof(idpd_observation) * (size_t)capacity));
     if (!h->obs_count) CK(cudaMalloc((void**)&h->obs_count, sizeof(int)));
