@@ -7,6 +7,7 @@
 // the FP64 positions in the reference's operation order. Pass 2 queues the
 // in-range pairs of a warp in shared memory and evaluates them 32 at a time;
 // sums are 64-bit fixed point as in the cell-list passes.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -48,15 +49,21 @@ __device__ __forceinline__ void split_local(const double* x, const double* ref, 
   lo.w = 0.0f;
 }
 
-// One walk's records in the caller's memory, and where they go in the raw buffer.
+// A piece of a walk's records in the caller's memory, and where it goes in the raw buffer.
 struct WalkSeg {
   const unsigned long long* src;
   unsigned long long dst, words;  // in 8-byte words
 };
 
+// Words of a piece at most. A CTA has 8 KB of loads in flight, 2.6 GB/s over the link, so a
+// walk of many records is shared by many: dispatches of 64 i and 500,000 j records of pass 2
+// (44 MB) with a CTA per walk and side 16.7 ms (the host's copy 2.2), in pieces 0.27 (the same at 1,024 to 8,192
+// words).
+constexpr size_t kSegWords = 2048;
+
 // The walks' records from the caller's host memory, read where they lie over the coherent
-// host link (devices that share the host's page tables): a CTA per walk and side, whole
-// cache lines. Both passes' dispatches of 1,345 walks (42 MB) 7.3 -> 5.4 ms, most of
+// host link (devices that share the host's page tables): a CTA per piece, whole cache
+// lines. Both passes' dispatches of 1,345 walks (42 MB) 7.3 -> 5.4 ms, most of
 // the rest in the caller's Python; before, the host copied every walk into a page-locked
 // buffer first, as it still does for unaligned records.
 __global__ void __launch_bounds__(256) k_walk_gather(const WalkSeg* seg, unsigned long long* raw) {
@@ -381,8 +388,12 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
   bool direct = s->coherent;
   for (int w = 0; w < n_walk && direct; w++)
     direct = (reinterpret_cast<uintptr_t>(epi[w]) | reinterpret_cast<uintptr_t>(epj[w])) % 8 == 0;
-  if ((direct ? grow(&K.h_seg, K.h_seg_cap, 2 * (size_t)n_walk, true) ||
-                    grow(&K.d_seg, K.d_seg_cap, 2 * (size_t)n_walk, false)
+  size_t nseg = 0;
+  for (int w = 0; w < n_walk && direct; w++)
+    nseg += (n_epi[w] * si / 8 + kSegWords - 1) / kSegWords +
+            (n_epj[w] * sj / 8 + kSegWords - 1) / kSegWords;
+  if ((direct ? grow(&K.h_seg, K.h_seg_cap, nseg, true) ||
+                    grow(&K.d_seg, K.d_seg_cap, nseg, false)
               : grow(&K.h_raw, K.h_raw_cap, raw, true)) ||
       grow(&K.d_raw, K.d_raw_cap, raw, false) ||
       grow(&K.h_int, K.h_int_cap, nint, true) || grow(&K.d_int, K.d_int_cap, nint, false) ||
@@ -403,12 +414,16 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
   int* walk_of_i = K.h_int;
   int* j_off = K.h_int + ni;
   long long oi = 0, oj = 0;
+  WalkSeg* seg = K.h_seg;
+  auto pieces = [&](const void* p, size_t words, size_t dst) {
+    const unsigned long long* src = static_cast<const unsigned long long*>(p);
+    for (size_t k = 0; k < words; k += kSegWords)
+      *seg++ = {src + k, dst + k, std::min(kSegWords, words - k)};
+  };
   for (int w = 0; w < n_walk; w++) {
     if (direct) {
-      K.h_seg[2 * w] = {static_cast<const unsigned long long*>(epi[w]), oi * si / 8,
-                        n_epi[w] * si / 8};
-      K.h_seg[2 * w + 1] = {static_cast<const unsigned long long*>(epj[w]),
-                            (ni * si + oj * sj) / 8, n_epj[w] * sj / 8};
+      pieces(epi[w], n_epi[w] * si / 8, oi * si / 8);
+      pieces(epj[w], n_epj[w] * sj / 8, (ni * si + oj * sj) / 8);
     } else {
       if (n_epi[w]) std::memcpy(hi + oi * si, epi[w], n_epi[w] * si);
       if (n_epj[w]) std::memcpy(hj + oj * sj, epj[w], n_epj[w] * sj);
@@ -424,10 +439,10 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
     oj += n_epj[w];
   }
   j_off[n_walk] = (int)oj;
-  if (direct && n_walk > 0) {
-    cudaMemcpyAsync(K.d_seg, K.h_seg, sizeof(WalkSeg) * 2 * n_walk, cudaMemcpyHostToDevice, s->rd);
-    k_walk_gather<<<2 * n_walk, 256, 0, s->rd>>>(K.d_seg,
-                                                 reinterpret_cast<unsigned long long*>(K.d_raw));
+  if (direct && nseg > 0) {
+    cudaMemcpyAsync(K.d_seg, K.h_seg, sizeof(WalkSeg) * nseg, cudaMemcpyHostToDevice, s->rd);
+    k_walk_gather<<<(unsigned)nseg, 256, 0, s->rd>>>(
+        K.d_seg, reinterpret_cast<unsigned long long*>(K.d_raw));
     cudaEventRecord(K.read, s->rd);
     cudaStreamWaitEvent(st, K.read, 0);
   } else if (!direct) {
@@ -486,7 +501,7 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
   K.ni = (int)ni;
   K.n_walk = n_walk;
   // the caller's arrays are its own again on return
-  if (direct && n_walk > 0 && cudaEventSynchronize(K.read) != cudaSuccess) {
+  if (direct && nseg > 0 && cudaEventSynchronize(K.read) != cudaSuccess) {
     err = "walk records could not be read";
     return IDPD_ERR_CUDA;
   }
