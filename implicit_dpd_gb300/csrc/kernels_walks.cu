@@ -57,8 +57,8 @@ struct WalkSeg {
 
 // Words of a piece at most. A CTA has 8 KB of loads in flight, 2.6 GB/s over the link, so a
 // walk of many records is shared by many: dispatches of 64 i and 500,000 j records of pass 2
-// (44 MB) with a CTA per walk and side 16.7 ms (the host's copy 2.2), in pieces 0.27 (the same at 1,024 to 8,192
-// words).
+// (44 MB) with a CTA per walk and side 16.7 ms (the host's copy 2.2), in pieces 0.27 (the
+// same at 1,024 to 8,192 words).
 constexpr size_t kSegWords = 2048;
 
 // The walks' records from the caller's host memory, read where they lie over the coherent
@@ -486,8 +486,13 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
       k_walk_density<<<nb, 32 * kWalkWarps, 0, st>>>(W, R);
     }
   }
+  // the caller's arrays are its own again on return, also on return with an error
+  auto caller_owns = [&] {
+    return !(direct && nseg > 0) || cudaStreamSynchronize(s->rd) == cudaSuccess;
+  };
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
+    caller_owns();
     err = std::string("walk launch: ") + cudaGetErrorString(e);
     return IDPD_ERR_CUDA;
   }
@@ -500,8 +505,7 @@ int walk_dispatch(WalkState* s, cudaStream_t st, const RepDev& R, const idpd_par
   K.tag = tag;
   K.ni = (int)ni;
   K.n_walk = n_walk;
-  // the caller's arrays are its own again on return
-  if (direct && nseg > 0 && cudaEventSynchronize(K.read) != cudaSuccess) {
+  if (!caller_owns()) {
     err = "walk records could not be read";
     return IDPD_ERR_CUDA;
   }
