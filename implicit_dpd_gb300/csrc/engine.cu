@@ -135,11 +135,15 @@ int fail(idpd_handle* h, int code, const char* fmt, ...) {
   return code;
 }
 
+// A failed call returns its error; the runtime's copy of it is cleared, or the next check of
+// a launch, the engine's or another library's, would report it again.
 #define CK(call)                                                                          \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                 \
       return fail(h, IDPD_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_));      \
+    }                                                                                     \
   } while (0)
 
 template <class T>
