@@ -1,6 +1,7 @@
 // Host side of the C ABI in include/idpd_engine.h: handle life cycle,
 // replica layout, uploads and downloads, the per-step launch sequence and its
 // CUDA graph.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -12,6 +13,7 @@
 #include <thread>
 #include <vector>
 
+#include "host_range.hpp"
 #include "idpd_engine.h"
 #include "state.cuh"
 
@@ -263,19 +265,37 @@ const void* device_view(const void* p) {
 
 // A caller buffer of n doubles in page-locked host memory, which kernels read and write over
 // the host link in whole cache lines, as fast as a copy engine and without the staging
-// buffer's kernel behind it; null for any other, and for one that is not aligned or not
-// page-locked to its end.
-double* link_view(const double* p, size_t n) {
-  cudaPointerAttributes a{}, z{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&z, p + n - 1) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  double* v = static_cast<double*>(a.devicePointer);
-  const bool ok = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && v &&
-                  z.devicePointer == v + (n - 1) && reinterpret_cast<uintptr_t>(v) % 8 == 0;
-  return ok ? v : nullptr;
+// buffer's kernel behind it; null for any other, and for one that link_address refuses. The
+// extent of the allocation is the driver's (a query of 0.05 us).
+double* link_view(const double* p, size_t n, bool write) {
+  using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault,
+                                         &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<Query>(f);
+  }();
+  if (!query) return nullptr;
+  unsigned type = 0, access = 0;
+  CUdeviceptr dev = 0, start = 0;
+  HostPointer a;
+  CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,
+                                 CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+  void* out[5] = {&type, &dev, &start, &a.size, &access};
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (query(5, what, out, at) != CUDA_SUCCESS) return nullptr;
+  a.page_locked = type == CU_MEMORYTYPE_HOST;
+  a.device = dev;
+  a.start = start;
+  a.writable = access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+  return reinterpret_cast<double*>(link_address(a, at, n * sizeof(double), write));
 }
 
 // Bit f set when some replica uses pair-force form f.
@@ -1166,7 +1186,7 @@ int idpd_set_dynamics(idpd_handle* h, int32_t r, const double* pos, const double
   // with built kept lists the position change counts as displacement (the
   // next step rebuilds when it is too large); else the lists are rebuilt
   const bool kept = h->d.vdev && !h->vl_dirty && h->tune.skin > 0.0f;
-  for (int k = 0; k < 3; k++) dev[k] = link_view(src[k], 3 * n);
+  for (int k = 0; k < 3; k++) dev[k] = link_view(src[k], 3 * n, false);
   if (dev[0] && dev[1] && dev[2]) {
     launch_set_dynamics_host(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1],
                              R.box[2], kept, h->st);
@@ -1264,7 +1284,7 @@ int rows_to_caller(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) 
       any = true;
       continue;
     }
-    if (double* link = link_view(f[k].out, 3 * n)) {
+    if (double* link = link_view(f[k].out, 3 * n, true)) {
       launch_rows_host(f[k].x, f[k].y, f[k].z, h->d.loc, R.row_off, link, (int)n, h->st);
       continue;
     }
