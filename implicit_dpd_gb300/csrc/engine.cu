@@ -1188,8 +1188,8 @@ int idpd_set_dynamics(idpd_handle* h, int32_t r, const double* pos, const double
   const bool kept = h->d.vdev && !h->vl_dirty && h->tune.skin > 0.0f;
   for (int k = 0; k < 3; k++) dev[k] = link_view(src[k], 3 * n, false);
   if (dev[0] && dev[1] && dev[2]) {
-    launch_set_dynamics_host(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1],
-                             R.box[2], kept, h->st);
+    CK(launch_set_dynamics_host(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1],
+                                R.box[2], kept, h->st));
     h->density_valid = false;
     return IDPD_OK;
   }
@@ -1201,8 +1201,8 @@ int idpd_set_dynamics(idpd_handle* h, int32_t r, const double* pos, const double
       dev[k] = stage;
     }
   }
-  launch_set_dynamics(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1], R.box[2],
-                      kept, h->st);
+  CK(launch_set_dynamics(h->d, dev[0], dev[1], dev[2], R.row_off, R.n, R.box[0], R.box[1],
+                         R.box[2], kept, h->st));
   h->density_valid = false;
   return IDPD_OK;
 }
@@ -1285,19 +1285,19 @@ int rows_to_caller(idpd_handle* h, const RepDev& R, const RowTriple* f, int nf) 
       continue;
     }
     if (double* link = link_view(f[k].out, 3 * n, true)) {
-      launch_rows_host(f[k].x, f[k].y, f[k].z, h->d.loc, R.row_off, link, (int)n, h->st);
+      CK(launch_rows_host(f[k].x, f[k].y, f[k].z, h->d.loc, R.row_off, link, (int)n, h->st));
       continue;
     }
     double* tmp = h->xfer + 3 * n * f[k].slot;
     RowFields one{};
     one.set(0, f[k].x, f[k].y, f[k].z, tmp);
-    launch_rows_out(one, h->d.orig, R.row_off, (int)n, h->st);
+    CK(launch_rows_out(one, h->d.orig, R.row_off, (int)n, h->st));
     CK(cudaEventRecord(h->x_mid, h->st));
     CK(cudaStreamWaitEvent(h->xst, h->x_mid, 0));
     CK(cudaMemcpyAsync(f[k].out, tmp, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->xst));
     copied = true;
   }
-  if (any) launch_rows_out(direct, h->d.orig, R.row_off, (int)n, h->st);
+  if (any) CK(launch_rows_out(direct, h->d.orig, R.row_off, (int)n, h->st));
   if (copied) {
     CK(cudaEventRecord(h->x_done, h->xst));
     CK(cudaStreamWaitEvent(h->st, h->x_done, 0));
@@ -1372,8 +1372,7 @@ int idpd_download_aux(idpd_handle* h, int32_t r, double* density, double* press,
     double* view = static_cast<double*>(const_cast<void*>(device_view(out)));
     if (stage + (size_t)width * n > h->xfer + 9 * (size_t)n) stage = h->xfer;
     double* to = view ? view : stage;
-    launch_into(to);
-    CK(cudaGetLastError());
+    CK(launch_into(to));
     if (view) return IDPD_OK;
     stage += (size_t)width * n;
     CK(cudaMemcpyAsync(out, to, sizeof(double) * width * n, cudaMemcpyDeviceToHost, h->st));
@@ -1386,21 +1385,21 @@ int idpd_download_aux(idpd_handle* h, int32_t r, double* density, double* press,
     if (!h->density_valid || (!f64 && !d.dqx))
       return fail(h, IDPD_ERR_STATE, "run idpd_density first");
     rc = gather(density, 3, [&](double* to) {
-      launch_gather_density(d, f64 ? d.dens64 : nullptr, R.dens_unscale, R.row_off, to, n, h->st);
+      return launch_gather_density(d, f64 ? d.dens64 : nullptr, R.dens_unscale, R.row_off, to, n, h->st);
     });
     if (rc) return rc;
   }
   if (press) {
     if (!h->press64) return fail(h, IDPD_ERR_STATE, "run idpd_force first");
     rc = gather(press, 3, [&](double* to) {
-      launch_gather_records(h->press64, 3, d.loc, R.row_off, to, n, h->st);
+      return launch_gather_records(h->press64, 3, d.loc, R.row_off, to, n, h->st);
     });
     if (rc) return rc;
   }
   if (nei_cm) {
     if (!h->cm64) return fail(h, IDPD_ERR_STATE, "run idpd_density first");
     rc = gather(nei_cm, 6, [&](double* to) {
-      launch_gather_records(h->cm64, 6, d.loc, R.row_off, to, n, h->st);
+      return launch_gather_records(h->cm64, 6, d.loc, R.row_off, to, n, h->st);
     });
     if (rc) return rc;
   }
@@ -1408,7 +1407,7 @@ int idpd_download_aux(idpd_handle* h, int32_t r, double* density, double* press,
     rc = gather(delta_sumr, 3, [&](double* to) {
       RowFields f{};
       f.set(0, d.dsx, d.dsy, d.dsz, to);
-      launch_rows_out(f, d.orig, R.row_off, n, h->st);
+      return launch_rows_out(f, d.orig, R.row_off, n, h->st);
     });
     if (rc) return rc;
   }
@@ -1698,7 +1697,7 @@ int idpd_step_host(idpd_handle* h, int32_t r, double* pos, double* vel, double* 
     double* tmp = view ? view : h->xfer;
     RowFields f{};
     f.set(0, d.px, d.py, d.pz, tmp);
-    launch_rows_out(f, d.orig, R.row_off, (int)n, h->xst);
+    CK(launch_rows_out(f, d.orig, R.row_off, (int)n, h->xst));
     if (!view) CK(cudaMemcpyAsync(pos, tmp, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->xst));
   }
   // velocities and accelerations after the kick, the second gather under the
@@ -1830,7 +1829,7 @@ int idpd_dump_xyz_async(idpd_handle* h, int32_t replica, const char* path, int32
   f.set(0, d.px, d.py, d.pz, f64);
   f.set(1, d.vx, d.vy, d.vz, f64 + 3 * (size_t)n);
   f.set(2, d.ax, d.ay, d.az, f64 + 6 * (size_t)n);
-  launch_rows_out(f, d.orig, R.row_off, n, h->st);
+  CK(launch_rows_out(f, d.orig, R.row_off, n, h->st));
   launch_gather_u32x4(d.id, d.prop, d.amp_id, d.unit, d.loc, R.row_off, u32, n, h->st);
   CK(cudaGetLastError());
   CK(cudaEventRecord(h->dump_ready, h->st));

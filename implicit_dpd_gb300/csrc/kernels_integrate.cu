@@ -463,12 +463,12 @@ __global__ void k_set_dynamics(DevState d, const double* pos, const double* vel,
   d.ax[i] = a[0]; d.ay[i] = a[1]; d.az[i] = a[2];
 }
 
-void launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
-                         const double* acc, int row0, int n, double box0, double box1,
-                         double box2, bool kept, cudaStream_t st) {
-  if (n == 0) return;
-  k_set_dynamics<<<(n + 255) / 256, 256, 0, st>>>(d, pos, vel, acc, row0, n, box0, box1, box2,
-                                                  kept ? 1 : 0);
+cudaError_t launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
+                                const double* acc, int row0, int n, double box0, double box1,
+                                double box2, bool kept, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, k_set_dynamics, (n + 255) / 256, 256, 0, d, pos, vel, acc, row0, n, box0, box1,
+                box2, kept ? 1 : 0);
 }
 
 // The same from page-locked host memory, read where it lies: a thread per number of the
@@ -499,12 +499,12 @@ __global__ void __launch_bounds__(256) k_set_dynamics_host(DevState d, const dou
   (c == 0 ? d.ax : (c == 1 ? d.ay : d.az))[i] = a;
 }
 
-void launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
-                              const double* acc, int row0, int n, double box0, double box1,
-                              double box2, bool kept, cudaStream_t st) {
-  if (n > 0)
-    k_set_dynamics_host<<<(unsigned)((3 * (size_t)n + 255) / 256), 256, 0, st>>>(
-        d, pos, vel, acc, row0, n, box0, box1, box2, kept ? 1 : 0);
+cudaError_t launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
+                                     const double* acc, int row0, int n, double box0, double box1,
+                                     double box2, bool kept, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, k_set_dynamics_host, (unsigned)((3 * (size_t)n + 255) / 256), 256, 0, d, pos,
+                vel, acc, row0, n, box0, box1, box2, kept ? 1 : 0);
 }
 
 // A field to page-locked host memory, written where it lies: a thread per number, whole
@@ -518,10 +518,11 @@ __global__ void __launch_bounds__(256) k_rows_host(const double* x, const double
   out[e] = (c == 0 ? x : (c == 1 ? y : z))[loc[row0 + (int)(e / 3)]];
 }
 
-void launch_rows_host(const double* x, const double* y, const double* z, const uint32_t* loc,
-                      int row0, double* out, int n, cudaStream_t st) {
-  if (n > 0)
-    k_rows_host<<<(unsigned)((3 * (size_t)n + 255) / 256), 256, 0, st>>>(x, y, z, loc, row0, out, n);
+cudaError_t launch_rows_host(const double* x, const double* y, const double* z,
+                             const uint32_t* loc, int row0, double* out, int n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, k_rows_host, (unsigned)((3 * (size_t)n + 255) / 256), 256, 0, x, y, z, loc,
+                row0, out, n);
 }
 
 // Storage rows of one replica back to upload order, three doubles per row of each field:
@@ -545,8 +546,10 @@ __global__ void __launch_bounds__(256) k_rows_out(RowFields f, const uint32_t* o
   }
 }
 
-void launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n, cudaStream_t st) {
-  if (n > 0) k_rows_out<<<(n + 255) / 256, 256, 0, st>>>(f, orig, row0, n);
+cudaError_t launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n,
+                            cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, k_rows_out, (n + 255) / 256, 256, 0, f, orig, row0, n);
 }
 
 // Derived fields of one replica's rows in upload order (device, managed or staging
@@ -568,9 +571,10 @@ __global__ void k_gather_density(DevState d, const double* d64, double unscale, 
   for (int c = 0; c < 3; c++) out[3 * (size_t)k + c] = v[c];
 }
 
-void launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
-                           double* out, int n, cudaStream_t st) {
-  if (n > 0) k_gather_density<<<(n + 255) / 256, 256, 0, st>>>(d, d64, unscale, row0, out, n);
+cudaError_t launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
+                                  double* out, int n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, k_gather_density, (n + 255) / 256, 256, 0, d, d64, unscale, row0, out, n);
 }
 
 template <int W>
@@ -581,14 +585,11 @@ __global__ void k_gather_records(const double* rec, const uint32_t* loc, int row
   out[k] = rec[(size_t)W * loc[row0 + k / W] + k % W];
 }
 
-void launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
-                           double* out, int n, cudaStream_t st) {
-  if (n == 0) return;
-  const int b = (n * width + 255) / 256;
-  if (width == 6)
-    k_gather_records<6><<<b, 256, 0, st>>>(rec, loc, row0, out, n);
-  else
-    k_gather_records<3><<<b, 256, 0, st>>>(rec, loc, row0, out, n);
+cudaError_t launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
+                                  double* out, int n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  return launch(st, width == 6 ? k_gather_records<6> : k_gather_records<3>,
+                (n * width + 255) / 256, 256, 0, rec, loc, row0, out, n);
 }
 
 // The four u32 fields of rows row0 .. row0 + n - 1 in upload order (loc maps

@@ -139,8 +139,8 @@ struct Chain {
   Chain(cudaStream_t s, bool c = false) : st(s), chained(c) {}
 };
 template <class... KArgs, class... Args>
-inline void launch(const Chain& c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                   Args... args) {
+inline cudaError_t launch(const Chain& c, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                          size_t smem, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -151,7 +151,7 @@ inline void launch(const Chain& c, void (*kernel)(KArgs...), dim3 grid, dim3 blo
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = c.chained ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 // Conditions of the IF nodes of a captured step, set by the step's first kernels: the
@@ -320,14 +320,15 @@ void launch_loop_set(int* left, int n, cudaStream_t st);
 void launch_saru_test(int n, const uint32_t* s1, const uint32_t* s2, const uint32_t* s3, int draws,
                       uint32_t* out_u, float* out_n, cudaStream_t st);
 void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n, cudaStream_t st);
-void launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
-                         const double* acc, int row0, int n, double box0, double box1,
-                         double box2, bool kept, cudaStream_t st);
-void launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
-                              const double* acc, int row0, int n, double box0, double box1,
-                              double box2, bool kept, cudaStream_t st);
-void launch_rows_host(const double* x, const double* y, const double* z, const uint32_t* loc,
-                      int row0, double* out, int n, cudaStream_t st);
+// The exchange with a caller's rows: the launches' own errors, for the caller.
+cudaError_t launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
+                                const double* acc, int row0, int n, double box0, double box1,
+                                double box2, bool kept, cudaStream_t st);
+cudaError_t launch_set_dynamics_host(const DevState& d, const double* pos, const double* vel,
+                                     const double* acc, int row0, int n, double box0, double box1,
+                                     double box2, bool kept, cudaStream_t st);
+cudaError_t launch_rows_host(const double* x, const double* y, const double* z,
+                             const uint32_t* loc, int row0, double* out, int n, cudaStream_t st);
 // Up to three fields (x, y, z arrays in storage order) to rows in upload order, each three
 // doubles (out null: not this one).
 struct RowFields {
@@ -340,11 +341,12 @@ struct RowFields {
     out[c] = o;
   }
 };
-void launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n, cudaStream_t st);
-void launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
-                           double* out, int n, cudaStream_t st);
-void launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
-                           double* out, int n, cudaStream_t st);
+cudaError_t launch_rows_out(const RowFields& f, const uint32_t* orig, int row0, int n,
+                            cudaStream_t st);
+cudaError_t launch_gather_density(const DevState& d, const double* d64, double unscale, int row0,
+                                  double* out, int n, cudaStream_t st);
+cudaError_t launch_gather_records(const double* rec, int width, const uint32_t* loc, int row0,
+                                  double* out, int n, cudaStream_t st);
 void launch_gather_u32x4(const uint32_t* a, const uint32_t* b, const uint32_t* c,
                          const uint32_t* e, const uint32_t* loc, int row0, uint32_t* out, int n,
                          cudaStream_t st);

@@ -42,3 +42,37 @@ def test_a_refused_copy_does_not_fail_the_next_call():
     finally:
         rt.cudaHostUnregister(part.ctypes.data)
     e.close()
+
+
+def test_an_error_left_by_another_library_is_not_the_exchange_calls():
+    import torch
+
+    box, st, n_amp = mixed_system(seed=83)
+    e = Engine()
+    e.set_params(mdpd_params(box, time=4))
+    e.upload(st)
+    e.build_topology(n_amp, [0])
+    e.density()
+    e.force()
+    want = e.download_aux(press=True, nei_cm=True, dsr=True), e.download()
+    rt = torch.cuda.cudart()
+
+    def refused():  # memory that is not registered: the runtime keeps the error
+        assert int(rt.cudaHostUnregister(st["pos"].ctypes.data)) != 0
+
+    refused()
+    aux = e.download_aux(press=True, nei_cm=True, dsr=True)
+    for k, v in want[0].items():
+        assert np.array_equal(aux[k], v, equal_nan=True), k
+    refused()
+    got = e.download()
+    for k in ("pos", "vel", "acc"):
+        assert np.array_equal(got[k], want[1][k]), k
+    refused()
+    e.set_dynamics(got["pos"], got["vel"], got["acc"])
+    e.sync()
+    e.close()
+    try:  # the error goes to its own library
+        torch.full((1,), 1.0, device="cuda")
+    except RuntimeError:
+        pass
