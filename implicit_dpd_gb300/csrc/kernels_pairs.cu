@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
       const float ki = VERLET ? d.okey[s] : pi.x;  // the ownership key of the step
       int nl = 0;  // owned pairs within the cutoff
       bool hit = false;
-      uint32_t q0 = 0, q1 = 0, q2 = 0;
+      // 64-bit sums: one lane can take every pair of a long second sweep
+      unsigned long long q0 = 0, q1 = 0, q2 = 0;
       // weight of one owned candidate, to both particles; called by every lane
       // together (valid = false for lanes without one) so that the rare FP64
       // recheck is warp-uniform
@@ -285,7 +286,6 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
           test(valid, t, dx, dy, dz, valid ? __ldg(d.posf + t) : pi, true);
         }
       } else {
-        // a lane takes at most nseg + nl / 32 weights below 2^23 each
         if (nl > kDensPairsMax && lane == 0) atomicCAS(d.err, 0, kErrDensPairs);
 #pragma unroll 1
         for (int g = 0; g < nseg; g++) {

@@ -202,8 +202,8 @@ __device__ __forceinline__ int frame_step(int t, const int* b) {
 }
 
 // Density weight of one in-range pair, accumulated by the candidate's property.
-__device__ __forceinline__ void add_weight(uint32_t& q0, uint32_t& q1, uint32_t& q2, uint32_t pr,
-                                           uint32_t v) {
+template <class Q>
+__device__ __forceinline__ void add_weight(Q& q0, Q& q1, Q& q2, uint32_t pr, uint32_t v) {
   q0 += pr == 0 ? v : 0u;
   q1 += pr == 1 ? v : 0u;
   q2 += pr == 2 ? v : 0u;

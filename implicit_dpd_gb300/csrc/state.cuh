@@ -97,8 +97,8 @@ struct VerletDev {
 // Error codes written by kernels into DevState::err.
 enum : int { kErrNone = 0, kErrCellOverflow = 1, kErrBadCell = 2, kErrListOverflow = 3,
              kErrNonFinite = 4, kErrComBox = 5, kErrChemCapacity = 6, kErrDensPairs = 7 };
-// Pairs within the cutoff of one particle that pass 1 can weigh (its lanes
-// keep 32-bit partial densities: (18 + kDensPairsMax / 32) * 2^23 < 2^32).
+// Pairs within the cutoff of one particle, its own share, beyond which pass 1 reports
+// kErrDensPairs (the pairs of a density far outside any use of the model).
 constexpr int kDensPairsMax = 15000;
 
 // Device state of ChemManager (chemmanager.hpp:3-282) for replica 0 of a
