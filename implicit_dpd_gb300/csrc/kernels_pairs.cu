@@ -109,6 +109,12 @@ __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int 
           const double cutd2d = WARREN ? (double)R->wrd * (double)R->wrd : 1.0;
           if (near1) in1 = e2 < 1.0;
           ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
+          if (ind && dr2 < 1.0e-10f) {
+            ind = false;
+            const uint32_t w = dens_weight(close_dr2(e2), WARREN, inv_rd, wnorm, pre);
+            add_weight(q0, q1, q2, fbits(pj.w), w);
+            atomicAdd(other + t, (unsigned long long)w);
+          }
         }
       }
       const uint32_t prj = fbits(pj.w);
@@ -206,7 +212,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
         const float ex = (pi.x - (float)dx * csx) - pj.x;
         const float ey = (pi.y - (float)dy * csy) - pj.y;
         const float ez = (pi.z - (float)dz * csz) - pj.z;
-        const float dr2 = dist2(ex, ey, ez);
+        float dr2 = dist2(ex, ey, ez);
         bool in1 = valid && (list_known || dr2 < 1.0f);
         bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
         const bool near1 = valid && !list_known && fabsf(dr2 - 1.0f) <= kGuard;
@@ -216,6 +222,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
             const double e2 = exact_dr2(d, R, si, d.perm[t]);
             if (near1) in1 = e2 < 1.0;
             ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
+            if (near2 && dr2 < 1.0e-10f) dr2 = close_dr2(e2);
           }
         }
         const uint32_t prj = fbits(pj.w);

@@ -16,6 +16,11 @@ __device__ __forceinline__ uint32_t dens_weight(float dr2, bool warren, float in
   return (uint32_t)(__float_as_int(fmaf(w, pre, 1.0f)) - 0x3f800000);
 }
 
+// The squared distance that dens_weight takes for two particles closer than 1e-5, from their
+// FP64 distance e2: their FP32 coordinates may coincide, and 0 has no reciprocal root.
+// From 1e-7 on, which leaves the weight below 2^23.
+__device__ __forceinline__ float close_dr2(double e2) { return fmaxf((float)e2, 1.0e-14f); }
+
 // The replica's FP32 coefficients per property pair k = 3 prop_i + prop_j,
 // packed so that one pair reads two shared-memory words: a = (cf_c, cf_r,
 // cf_g, cf_m[k][0]), b = (cf_m[k][1], cf_m[k][2]).
