@@ -1577,10 +1577,12 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
     return fail(h, IDPD_ERR_STATE, "the reaction reached max_amp_num: the run has ended");
   if ((rc = ensure_verlet_ready(h)) || (rc = ensure_phit(h))) return rc;
   if (h->obs_period > 0 && (rc = ensure_obs(h))) return rc;
-  if ((rc = host_times(h))) return rc;
-  // with the reaction, and in the plain form, the drift removal's kernels are in every step
+  // with the reaction, and in the plain form, the drift removal's kernels are in every step, and
+  // only observations ask for the counters (their copy and wait 10 us a call)
   const bool plain = h->flags & IDPD_CFG_PLAIN_GRAPHS;
   const bool every_cm = h->chem_on || plain;
+  if ((h->obs_period > 0 || !every_cm) && (rc = host_times(h))) return rc;
+  if (h->chem_on) h->time_known = false;  // after this call: a stopped step does not count
   if ((rc = build_graph(h, &h->graph, 1, false, every_cm ? kCmKernels : kCmNone))) return rc;
   const bool loop = h->chem_on && nsteps > 1 && !plain && !h->loop_failed;
   if (loop && !h->graph_loop && !build_loop_graph(h)) h->loop_failed = true;
@@ -1640,7 +1642,6 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
       }
     }
   }
-  if (h->chem_on) h->time_known = false;  // a stopped step does not count
   CK(cudaEventRecord(h->ev1, h->st));
   if ((rc = queue_error_copy(h))) return rc;
   CK(cudaStreamSynchronize(h->st));
