@@ -95,6 +95,7 @@ struct idpd_handle {
   cudaGraphExec_t graph_obs = nullptr;  // the step with the observation
   cudaGraphExec_t graph_cm = nullptr;   // the step with the drift removal
   cudaGraphExec_t graph_run[3] = {};    // kRunSteps[k] plain steps
+  bool run_wanted[3] = {};              // some call had use for it
   std::vector<uint32_t> time_h;  // Parameter::time per replica, as rep_time on the device
   bool time_known = false;       // (not after steps with the reaction, which may stop)
   int* err_host = nullptr;       // pinned copy of the device's error word
@@ -167,6 +168,7 @@ void invalidate_graph(idpd_handle* h) {
       cudaGraphExecDestroy(*g);
       *g = nullptr;
     }
+  std::fill(h->run_wanted, h->run_wanted + 3, false);
 }
 
 void free_all(idpd_handle* h) {
@@ -1506,6 +1508,11 @@ int idpd_remove_cmdrift(idpd_handle* h) {
 // the node, costs up to 5 us more than one in a plain graph (3k particles 42.8 us against
 // 38.5, 24k 47.7 against 46.9, 1M 503 against 497), so runs of steps without the reaction go
 // out eight at a time, and what is left of a run four and two at a time.
+//
+// A run is captured when a call first needs it (14 steps in three runs cost 370 us, whatever
+// the length asked for: two steps after a change of the tuning 433 us, now 169): the shortest
+// at once, a longer one behind as many steps of the call that are queued already, whose time
+// covers its capture, or when an earlier call had use for it.
 constexpr int kRunSteps[3] = {8, 4, 2};
 
 // Captures nsteps steps into *ge (if it is not there yet).
@@ -1583,13 +1590,10 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   const bool every_cm = h->chem_on || plain;
   if ((h->obs_period > 0 || !every_cm) && (rc = host_times(h))) return rc;
   if (h->chem_on) h->time_known = false;  // after this call: a stopped step does not count
-  if ((rc = build_graph(h, &h->graph, 1, false, every_cm ? kCmKernels : kCmNone))) return rc;
   const bool loop = h->chem_on && nsteps > 1 && !plain && !h->loop_failed;
   if (loop && !h->graph_loop && !build_loop_graph(h)) h->loop_failed = true;
   const bool use_loop = loop && h->graph_loop;
   const bool use_run = !every_cm && nsteps > 1;
-  for (int k = 0; k < 3 && use_run; k++)
-    if ((rc = build_graph(h, &h->graph_run[k], kRunSteps[k], false, kCmNone))) return rc;
   // whether some replica's step counter is a multiple of `period`, `ahead` steps from now
   auto due = [&](int period, int ahead) {
     for (uint32_t t : h->time_h)
@@ -1598,33 +1602,45 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   };
   auto observes = [&](int ahead) { return h->obs_period > 0 && due(h->obs_period, ahead); };
   auto removes = [&](int ahead) { return !every_cm && due((int)kCmCorr, ahead); };
+  // The launch that follows `sent` steps of the call: a step that observes or removes the drift
+  // is one launch of its graph; the steps up to the next of these, or the next storage
+  // reorder, go out in runs (with the reaction, as one launch of the loop).
+  struct Launch {
+    int steps;
+    cudaGraphExec_t* graph;
+    bool observe;
+    CmForm cm;
+  };
+  bool wanted[3];  // in earlier calls
+  std::copy(h->run_wanted, h->run_wanted + 3, wanted);
+  auto next = [&](int sent) -> Launch {
+    if (observes(0)) return {1, &h->graph_obs, true, kCmKernels};
+    if (removes(0)) return {1, &h->graph_cm, false, kCmKernels};
+    const int room =
+        std::min(nsteps - sent, std::max(h->sort_period - h->steps_since_sort, 1));
+    const int most = use_loop ? room : (use_run ? std::min(room, kRunSteps[0]) : 1);
+    int c = 1;
+    while (c < most && !observes(c) && !removes(c)) c++;
+    if (use_loop && c > 1) return {c, &h->graph_loop, false, kCmIfNode};
+    bool first = true;
+    for (int q = 0; q < 3 && use_run; q++) {
+      const int n = kRunSteps[q];
+      if (n > c) continue;
+      if (first) h->run_wanted[q] = true;
+      first = false;
+      if (h->graph_run[q] || q == 2 || sent >= n || wanted[q])
+        return {n, &h->graph_run[q], false, kCmNone};
+    }
+    return {1, &h->graph, false, every_cm ? kCmKernels : kCmNone};
+  };
+  auto ready = [&](const Launch& x) { return build_graph(h, x.graph, x.steps, x.observe, x.cm); };
+  Launch x = next(0);
+  if ((rc = ready(x))) return rc;
   CK(cudaEventRecord(h->ev0, h->st));
-  for (int k = 0; k < nsteps;) {
-    // a step that observes or removes the drift is one launch of its graph; the steps up to
-    // the next of these, or the next storage reorder, go out in runs (with the reaction, as
-    // one launch of the loop)
-    const bool obs = observes(0), cm = removes(0);
-    int c = 1, run = 3;
-    if (!obs && !cm && (use_loop || use_run)) {
-      const int room = std::min(nsteps - k, std::max(h->sort_period - h->steps_since_sort, 1));
-      const int most = use_loop ? room : kRunSteps[0];
-      while (c < room && c < most && !observes(c) && !removes(c)) c++;
-      if (use_run) {
-        run = 0;
-        while (run < 3 && kRunSteps[run] > c) run++;
-        c = run < 3 ? kRunSteps[run] : 1;
-      }
-    }
-    if (c > 1 && use_loop) {
-      launch_loop_set(h->loop_left, c, h->st);
-      CK(cudaGraphLaunch(h->graph_loop, h->st));
-    } else if (c > 1) {
-      CK(cudaGraphLaunch(h->graph_run[run], h->st));
-    } else {
-      cudaGraphExec_t* ge = obs ? &h->graph_obs : (cm ? &h->graph_cm : &h->graph);
-      if ((rc = build_graph(h, ge, 1, obs, kCmKernels))) return rc;
-      CK(cudaGraphLaunch(*ge, h->st));
-    }
+  for (int k = 0;;) {
+    const int c = x.steps;
+    if (x.graph == &h->graph_loop) launch_loop_set(h->loop_left, c, h->st);
+    CK(cudaGraphLaunch(*x.graph, h->st));
     for (uint32_t& t : h->time_h) t += (uint32_t)c;
     k += c;
     h->steps_since_sort += c;
@@ -1641,6 +1657,9 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
         break;
       }
     }
+    if (k >= nsteps) break;
+    x = next(k);
+    if ((rc = ready(x))) return rc;
   }
   CK(cudaEventRecord(h->ev1, h->st));
   if ((rc = queue_error_copy(h))) return rc;
