@@ -15,6 +15,7 @@
 // FP64 throughout, FP64 sums in cell order.
 #include <algorithm>
 
+#include "cell_reach.hpp"
 #include "pair_lists.cuh"
 
 namespace idpd {
@@ -1239,8 +1240,8 @@ __global__ void __launch_bounds__(kRowBlock) k_com(DevState d, double* cm, uint3
           // the cells of the row that come within rn_c, from cx - ml to cx + mr
           const float rem = sqrtf(rem2);
           const int c0 = cx - ((cx >> rs) << rs);
-          const int ml = min(m, c0 - (int)floorf((pi.x - rem) * inv_side));
-          const int mr = min(m, (int)floorf((pi.x + rem) * inv_side) - c0);
+          const int ml = cells_left(pi.x, rem, inv_side, c0, m);
+          const int mr = cells_right(pi.x, rem, inv_side, c0, m);
           const int wy = qy < 0 ? qy + ny : (qy >= ny ? qy - ny : qy);
           const int wz = qz < 0 ? qz + nz : (qz >= nz ? qz - nz : qz);
           const int c00 = R->cell_off + (wz * ny + wy) * nx;
