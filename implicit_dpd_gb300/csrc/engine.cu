@@ -1690,6 +1690,7 @@ int idpd_step_host(idpd_handle* h, int32_t r, double* pos, double* vel, double* 
     if ((rc = idpd_step(h, 1))) return rc;
     return idpd_download_state(h, r, pos, vel, acc, nullptr, nullptr, nullptr, nullptr);
   }
+  if ((rc = commit(h))) return rc;  // parameters set since the last step
   if (h->n_tot == 0) return IDPD_OK;
   h->pairs_valid = true;
   if ((rc = ensure_verlet_ready(h)) || (rc = ensure_phit(h))) return rc;
