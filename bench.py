@@ -54,18 +54,24 @@ STEP_BYTES_PER_PARTICLE = 176  # compulsory HBM bytes of one particle-step
 # (the Saru hash and draws) + 5 SFU (sqrt r, rcp, sqrt w, log, cos); the
 # density pass ~12 FP32 + 1 SFU.
 OPS_PER_ORDERED_PAIR = {"force": 134, "density": 13}
-# Kernels a captured step launches: without kept lists drift_bin, scan x2, scatter,
-# sort_pack, pair_build, density over the lists, over the overflowed lists, density
-# finalize, force, force walk, bonded_kick; with kept lists (above 400,000 rows) drift_disp,
-# rebuild decision, pack, density x2, density finalize, force, force walk, bonded_kick.
-# A rebuild step adds the IF body of the cells and lists (bin, scan x2, scatter,
-# sort_pack, list build); a step whose replica counter is a multiple of 100 adds the
-# drift removal (3 kernels) and the step counters' kernel (else part of the kick).
+# Kernels a captured step of more than 16,384 cells launches (the scan is one kernel less up
+# to there): without kept lists drift_bin, scan x2, scatter, sort_pack, pair_build, density over
+# the lists, over the overflowed lists, density finalize, force, force walk, bonded_kick; with
+# kept lists above 400,000 rows drift_disp, rebuild decision, pack, density x2, density
+# finalize, force, force walk, bonded_kick. There a rebuild step adds the IF body of the cells
+# and lists (bin, scan x2, scatter, sort_pack, list build); up to 400,000 rows these are in
+# every step, and the pack is sort_pack's. A step whose replica counter is a multiple of 100
+# adds the drift removal (3 kernels) and the step counters' kernel (else part of the kick). In
+# a run of steps without any of this between them the kick of each step but the last and
+# the drift of the next are one kernel.
 KERNELS_PER_STEP = 12
 KERNELS_PER_KEPT_STEP = 9
 KERNELS_PER_REBUILD = 6
 KERNELS_PER_CM = 4
 KERNELS_PER_REORDER = 3        # gather, topology, copy back
+ONE_SCAN_CELLS = 16384
+GATED_ROWS = 400_000
+RUNS = (8, 4, 2)               # steps per launch of idpd_step without the reaction
 
 
 def n_amp_for(box, layers):
@@ -789,6 +795,54 @@ def gpu_launches(steps, kept, rebuilds, t0, n_reorders, loop=True):
             + (n_reorders + 1 if loop else 0) + n_reorders * KERNELS_PER_REORDER)
 
 
+def grid_cells(box, tune):
+    """Search cells of a replica under a tuning (idpd_set_tuning)."""
+    return int(np.prod((np.asarray(box) / (1.0 + tune["skin"])).astype(int) * tune["reach"]))
+
+
+def step_runs(calls, t0, since_sort, sort_period=100):
+    """The launches of the last of several idpd_step calls (their step counts, the first one
+    after a change that dropped the captured steps) by the steps of each, and the storage
+    reorders between them: the engine's rule without the reaction and without observations.
+    t0: the step counter, since_sort: the steps since the last reorder, before the last call."""
+    captured, wanted = {2}, set()
+    time, since = t0 - sum(calls[:-1]), (since_sort - sum(calls[:-1])) % sort_period
+    for steps in calls:
+        earlier, runs, reorders, sent = set(wanted), [], 0, 0
+        while sent < steps:
+            n = 1
+            if time % 100 != 0 and steps > 1:
+                room = min(steps - sent, sort_period - since, RUNS[0])
+                while n < room and (time + n) % 100 != 0:
+                    n += 1
+                fitting = [r for r in RUNS if r <= n]
+                wanted.update(fitting[:1])
+                n = next((r for r in fitting if r in captured or sent >= r or r in earlier), 1)
+                captured.add(n)
+            runs.append(n)
+            sent += n
+            time += n
+            since += n
+            if since >= sort_period:
+                since, reorders = 0, reorders + 1
+    return runs, reorders
+
+
+def timed_launches(calls, kept, rows, cells, rebuilds, t0, since_sort, plain=False):
+    """The kernels that the last of the calls launches (step_runs; rebuilds: of that call)."""
+    runs, reorders = step_runs(calls, t0, since_sort)
+    steps, two_scans = calls[-1], cells > ONE_SCAN_CELLS
+    if kept and rows > GATED_ROWS and not plain:
+        n = gpu_launches(steps, True, rebuilds, t0, reorders, loop=False)
+        n -= 0 if two_scans else rebuilds
+    else:
+        per_step = KERNELS_PER_STEP + (2 if kept else 0) - (0 if two_scans else 1)
+        n = steps * per_step + reorders * KERNELS_PER_REORDER
+        n += KERNELS_PER_CM * (steps if plain else
+                               sum(1 for t in range(t0, t0 + steps) if t % 100 == 0))
+    return n if plain else n - sum(r - 1 for r in runs)
+
+
 def step_roofline(roofline, n, ms_per_step):
     """The step against the sum of its passes' lower-bound times: the two pair
     passes at the issue bound (their algorithmic lane operations per ordered
@@ -946,7 +1000,6 @@ def run_engine(args, rank, world, local_rank):
     if rank == 0 and world == 1 and not args.no_cpu:
         timed_state = e.download()
         cpu = cpu_baseline(timed_state, n_amp, rp, e.get_params().time)
-    n_reorders = args.steps // 100
     out = {"metric": METRIC, "value": value, "unit": "particle-steps/s", "n_gpus": world,
            "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms_max / args.steps,
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
@@ -961,8 +1014,9 @@ def run_engine(args, rank, world, local_rank):
            "kernel_ms": kernel_ms, "fp64_plain": fp64, "fp64_same_algorithm": fp64_same,
            "e2e": e2e, "cpu_baseline": cpu,
            "batched_replicas": batched, "reaction": reaction, "liquid": liquid,
-           "gpu_launches": gpu_launches(args.steps, reach["skin"] > 0, rebuilds, t0_step,
-                                        n_reorders, loop=False),
+           "gpu_launches": timed_launches([max(args.warmup, 3), args.steps], reach["skin"] > 0, n,
+                                          grid_cells(box, reach), rebuilds, t0_step,
+                                          (t0_step - 1) % 100, plain=GRAPH_FLAGS != 0),
            "force_error_bar": "max-particle relative force error <= 1e-5 vs FP64 (tests/test_gpu_parity.py)"}
     if rank == 0:
         print(json.dumps(out), flush=True)
