@@ -25,14 +25,10 @@ constexpr int IDPD_FORM_WARREN_K = 2;
 constexpr double kForceScale = 67108864.0;           // 2^26 per unit force
 constexpr double kForceUnscale = 1.0 / 67108864.0;
 constexpr double kDensScale = 1099511627776.0;        // 2^40 per unit density
-constexpr float kDensScaleF = 1099511627776.0f;
 constexpr double kDensUnscale = 1.0 / 1099511627776.0;
 constexpr double kPosScale = 1099511627776.0;         // 2^40: COM sums, delta_sumr
-constexpr float kPosScaleF = 1099511627776.0f;
 constexpr int kForceBits = 26;
-constexpr int kDensBits = 40;
 constexpr int kPosBits = 40;
-constexpr float kDensUnscaleF = 1.0f / 1099511627776.0f;
 
 // FP32 pair-set decisions within this band of a cutoff are re-taken in FP64
 // from the FP64 positions, exactly as the reference's FP64 test. The bound on
@@ -87,8 +83,6 @@ struct BlockMap {
   const int* rep;
   const int* row;
 };
-
-__device__ __forceinline__ int sar(int x, int s) { return x >> s; }
 
 // The step's kernels begin with chain_launch, which lets the next kernel of the stream be
 // set up while this one runs, and come to chain_wait, which waits for the kernels before

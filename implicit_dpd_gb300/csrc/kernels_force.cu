@@ -259,8 +259,6 @@ struct ForceWarpSmem {
   uint32_t qt[64], qc[64];
 };
 
-
-
 size_t force_smem_bytes(int fb) { return (size_t)fb * sizeof(ForceBlockSmem); }
 
 // Each pair is evaluated once, by the particle that owns it (owns()), and
@@ -302,7 +300,6 @@ __device__ __forceinline__ void force_rows(const DevState& d, int s0, int rows, 
   if (nrow <= 0) return;
   PairI I;
   I.seed = R->seed + d.rep_time[r];
-  constexpr uint32_t group_mask = LP == 32 ? 0xffffffffu : ((1u << LP) - 1u);
   // the chunk's rows sorted by the length of their lists (overflowed lists
   // count 0, lanes without a row come last): key = length << 5 | row - s0
   uint32_t key = 0xffffffffu;

@@ -410,19 +410,6 @@ void launch_saru_test(int n, const uint32_t* s1, const uint32_t* s2, const uint3
   k_saru_test<<<(n + 255) / 256, 256, 0, st>>>(n, s1, s2, s3, draws, out_u, out_n);
 }
 
-__global__ void k_aos_to_soa(const double* aos, double* x, double* y, double* z, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  x[i] = aos[3 * (size_t)i];
-  y[i] = aos[3 * (size_t)i + 1];
-  z[i] = aos[3 * (size_t)i + 2];
-}
-
-void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n, cudaStream_t st) {
-  if (n == 0) return;
-  k_aos_to_soa<<<(n + 255) / 256, 256, 0, st>>>(aos, x, y, z, n);
-}
-
 // Per-step host exchange: rows of one replica in upload order (pos, vel and
 // acc as three arrays of 3 doubles per row) into the storage rows; invalid
 // rows raise an error. The position change of a row counts, at its nearest

@@ -110,13 +110,6 @@ __device__ __forceinline__ void build_segments(SegTable& S, const DevState& d, c
   }
 }
 
-__device__ __forceinline__ int seg_dx(const SegTable& S, int g, int t) {
-  int dx = (S.code[g] & 7) - 4;
-#pragma unroll
-  for (int q = 0; q < 2 * kMaxReach; q++) dx += t >= S.bnd[g][q];
-  return dx;
-}
-
 struct PairCode {
   int dx, dy, dz, sx, sy, sz;
 };

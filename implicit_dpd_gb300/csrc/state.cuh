@@ -319,7 +319,6 @@ void launch_step_tail(const DevState& d, int R, const int* skip, const LoopTail&
 void launch_loop_set(int* left, int n, cudaStream_t st);
 void launch_saru_test(int n, const uint32_t* s1, const uint32_t* s2, const uint32_t* s3, int draws,
                       uint32_t* out_u, float* out_n, cudaStream_t st);
-void launch_aos_to_soa(const double* aos, double* x, double* y, double* z, int n, cudaStream_t st);
 // The exchange with a caller's rows: the launches' own errors, for the caller.
 cudaError_t launch_set_dynamics(const DevState& d, const double* pos, const double* vel,
                                 const double* acc, int row0, int n, double box0, double box1,
