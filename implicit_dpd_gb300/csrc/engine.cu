@@ -2050,11 +2050,13 @@ int idpd_set_observe(idpd_handle* h, int32_t period, int32_t capacity) {
     return fail(h, IDPD_ERR_INVALID_ARG, "period >= 0 and capacity >= 1 required");
   cudaSetDevice(h->device);
   CK(cudaStreamSynchronize(h->st));
+  if (period > 0 && !h->obs_count) CK(cudaMalloc((void**)&h->obs_count, sizeof(int)));
   if (period > 0 && capacity != h->obs_cap) {
+    // (the old buffer stays until there is a new one: captured steps write to it)
+    idpd_observation* rec = nullptr;
+    CK(cudaMalloc((void**)&rec, sizeof(idpd_observation) * (size_t)capacity));
     if (h->obs_rec) cudaFree(h->obs_rec);
-    h->obs_rec = nullptr;
-    CK(cudaMalloc((void**)&h->obs_rec, sizeof(idpd_observation) * (size_t)capacity));
-    if (!h->obs_count) CK(cudaMalloc((void**)&h->obs_count, sizeof(int)));
+    h->obs_rec = rec;
     h->obs_cap = capacity;
   }
   if (h->obs_count) CK(cudaMemsetAsync(h->obs_count, 0, sizeof(int), h->st));
