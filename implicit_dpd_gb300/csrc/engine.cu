@@ -160,6 +160,11 @@ int dalloc(idpd_handle* h, T** p, size_t count) {
   return IDPD_OK;
 }
 
+void dfree(idpd_handle* h, void* p) {
+  h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), p), h->allocs.end());
+  cudaFree(p);
+}
+
 void invalidate_graph(idpd_handle* h) {
   for (cudaGraphExec_t* g :
        {&h->graph_loop, &h->graph, &h->graph_obs, &h->graph_cm, &h->graph_run[0], &h->graph_run[1],
@@ -250,6 +255,18 @@ void fill_repdev(RepDev& R, const idpd_params& p, int reach, float skin) {
   R.dens_prescale = (float)std::ldexp(1.0, -k);
   R.dens_unscale = std::ldexp(1.0, k - 23);
   R.dens_unscale_f = (float)R.dens_unscale;
+}
+
+// The handle's search cells under a tuning, and whether they fit the 32-bit cell numbers.
+bool cells_fit(const std::vector<idpd_params>& params, int reach, float skin) {
+  const double cut = 1.0 + (double)skin;
+  double cells = 0.0;
+  for (const idpd_params& p : params) {
+    double c = 1.0;
+    for (int k = 0; k < 3; k++) c *= std::floor(p.box[k] / cut) * reach;
+    cells += c;
+  }
+  return cells < 2147483647.0;
 }
 
 // A caller buffer that lives in device or managed memory, which the kernels
@@ -534,6 +551,8 @@ int commit(idpd_handle* h) {
   for (int r = 0; r < h->R; r++)
     if (!h->params_set[r]) return fail(h, IDPD_ERR_STATE, "replica %d has no parameters", r);
   if (h->layout_dirty) {
+    if (!cells_fit(h->params, h->tune.reach, h->tune.skin))
+      return fail(h, IDPD_ERR_CAPACITY, "too many cells");
     h->pairs_valid = false;
     invalidate_graph(h);
     h->reps_h.assign(h->R, RepDev{});
@@ -561,7 +580,6 @@ int commit(idpd_handle* h) {
       amp += R.n_amp + extra_amp;
       if ((long long)row >= (1ll << 25))  // the sorted row of a list entry has 25 bits
         return fail(h, IDPD_ERR_CAPACITY, "more than 2^25 particle rows in one handle");
-      if ((long long)cell >= (1ll << 31) - 1) return fail(h, IDPD_ERR_CAPACITY, "too many cells");
     }
     h->n_tot = row;
     h->ncell_tot = cell;
@@ -666,41 +684,49 @@ int commit(idpd_handle* h) {
   return IDPD_OK;
 }
 
-// (Re)allocates only the cell arrays, keeping the particle arrays.
+// Cell arrays for ncell cells, keeping the particle arrays (and, when they cannot be
+// allocated, the present cell arrays).
 int realloc_cells(idpd_handle* h, int ncell) {
   DevState& d = h->d;
   if (ncell > h->ncell_cap) {
-    for (void* p : {(void*)d.cell_cnt, (void*)d.cell_start, (void*)d.scan_part}) {
-      h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), p), h->allocs.end());
-      cudaFree(p);
-    }
+    int *cnt = nullptr, *start = nullptr, *part = nullptr;
     int rc;
-    if ((rc = dalloc(h, &d.cell_cnt, ncell)) || (rc = dalloc(h, &d.cell_start, ncell + 1)) ||
-        (rc = dalloc(h, &d.scan_part, (ncell + 4095) / 4096 + 1)))
+    if ((rc = dalloc(h, &cnt, ncell)) || (rc = dalloc(h, &start, (size_t)ncell + 1)) ||
+        (rc = dalloc(h, &part, ((size_t)ncell + 4095) / 4096 + 1))) {
+      for (int* p : {cnt, start, part}) dfree(h, p);
       return rc;
+    }
+    for (int* p : {d.cell_cnt, d.cell_start, d.scan_part}) dfree(h, p);
+    d.cell_cnt = cnt;
+    d.cell_start = start;
+    d.scan_part = part;
     h->ncell_cap = ncell;
   }
-  CK(cudaMemsetAsync(d.cell_cnt, 0, sizeof(int) * h->ncell_cap, h->st));
+  CK(cudaMemsetAsync(d.cell_cnt, 0, sizeof(int) * (size_t)h->ncell_cap, h->st));
   return IDPD_OK;
 }
 
-// Applies a new cell reach to a committed layout: new cell grids and cell
+// Applies a new cell reach or skin to a committed layout: new cell grids and cell
 // offsets, same particle rows.
 int retune_cells(idpd_handle* h) {
-  invalidate_graph(h);
+  if (!cells_fit(h->params, h->tune.reach, h->tune.skin))
+    return fail(h, IDPD_ERR_CAPACITY, "too many cells");
+  std::vector<RepDev> reps = h->reps_h;
   int cell = 0;
   for (int r = 0; r < h->R; r++) {
-    RepDev& R = h->reps_h[r];
-    const RepDev keep = R;
+    RepDev& R = reps[r];
+    const RepDev& keep = h->reps_h[r];
     fill_rep(h, r, R);
     R.row_off = keep.row_off; R.n = keep.n; R.blk_off = keep.blk_off; R.nblk = keep.nblk;
     R.n_amp = keep.n_amp; R.amp_off = keep.amp_off;
     R.cell_off = cell;
     cell += R.ncell;
   }
-  h->ncell_tot = cell;
   int rc = realloc_cells(h, cell);
   if (rc) return rc;
+  invalidate_graph(h);
+  h->reps_h = reps;
+  h->ncell_tot = cell;
   CK(cudaMemcpyAsync(h->d.reps, h->reps_h.data(), sizeof(RepDev) * h->R, cudaMemcpyHostToDevice, h->st));
   CK(cudaStreamSynchronize(h->st));
   h->density_valid = false;
@@ -1773,6 +1799,7 @@ int idpd_set_tuning(idpd_handle* h, const idpd_tuning* t) {
   const int dlanes = t->density_lanes ? t->density_lanes : 32;
   if (lanes != h->tune.lanes || fblk != h->tune.fblk || dlanes != h->tune.dlanes)
     invalidate_graph(h);
+  const PairTuning before = h->tune;
   h->tune.dlanes = dlanes;
   h->tune.lanes = lanes;
   h->tune.fblk = fblk;
@@ -1780,7 +1807,10 @@ int idpd_set_tuning(idpd_handle* h, const idpd_tuning* t) {
   h->tune.skin = t->skin;
   if (changed && h->on_device && !h->layout_dirty) {
     int rc = retune_cells(h);
-    if (rc) return rc;
+    if (rc) {
+      h->tune = before;
+      return rc;
+    }
     h->vl_dirty = true;
     return ensure_verlet(h);
   }
