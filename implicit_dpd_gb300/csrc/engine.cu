@@ -154,10 +154,19 @@ int dalloc(idpd_handle* h, T** p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
-  if (e != cudaSuccess) return fail(h, IDPD_ERR_CUDA, "cudaMalloc(%zu B): %s", count * sizeof(T),
-                                    cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(h, IDPD_ERR_CUDA, "cudaMalloc(%zu B): %s", count * sizeof(T),
+                cudaGetErrorString(e));
+  }
   h->allocs.push_back((void*)*p);
   return IDPD_OK;
+}
+
+// One of a set of buffers, kept from an earlier try that did not get them all.
+template <class T>
+int dbuf(idpd_handle* h, T** p, size_t count) {
+  return *p ? IDPD_OK : dalloc(h, p, count);
 }
 
 void dfree(idpd_handle* h, void* p) {
@@ -418,10 +427,10 @@ int ensure_obs(idpd_handle* h) {
   int rc = ensure_press(h);
   if (rc) return rc;
   ObsBuffers& b = h->obs_buf;
-  if (!b.part) {
-    if ((rc = dalloc(h, &b.part, (size_t)h->nblk_cap)) ||
-        (rc = dalloc(h, &b.mvir, 3 * (size_t)h->n_amp_cap)) ||
-        (rc = dalloc(h, &b.mdif, (size_t)h->n_amp_cap)))
+  if (!b.mdif) {  // the last of them
+    if ((rc = dbuf(h, &b.part, (size_t)h->nblk_cap)) ||
+        (rc = dbuf(h, &b.mvir, 3 * (size_t)h->n_amp_cap)) ||
+        (rc = dbuf(h, &b.mdif, (size_t)h->n_amp_cap)))
       return rc;
     invalidate_graph(h);
   }
@@ -437,12 +446,12 @@ int ensure_obs(idpd_handle* h) {
 int ensure_verlet(idpd_handle* h) {
   if (h->tune.skin <= 0.0f) return IDPD_OK;
   DevState& d = h->d;
-  if (!d.vl) {
+  if (!d.vdev) {  // the last of them: the others may be there after a refused allocation
     int rc;
-    if ((rc = dalloc(h, &d.vl, (size_t)kVerletCap * h->cap)) || (rc = dalloc(h, &d.vn, h->cap)) ||
-        (rc = dalloc(h, &d.okey, h->cap)) ||
-        (rc = dalloc(h, &d.drx, h->cap)) || (rc = dalloc(h, &d.dry, h->cap)) ||
-        (rc = dalloc(h, &d.drz, h->cap)) || (rc = dalloc(h, &d.vdev, 1)))
+    if ((rc = dbuf(h, &d.vl, (size_t)kVerletCap * h->cap)) || (rc = dbuf(h, &d.vn, h->cap)) ||
+        (rc = dbuf(h, &d.okey, h->cap)) ||
+        (rc = dbuf(h, &d.drx, h->cap)) || (rc = dbuf(h, &d.dry, h->cap)) ||
+        (rc = dbuf(h, &d.drz, h->cap)) || (rc = dbuf(h, &d.vdev, 1)))
       return rc;
   }
   VerletDev v{};
@@ -471,7 +480,7 @@ int ensure_phit(idpd_handle* h) {
 // when cells were rebuilt outside the step.
 int ensure_verlet_ready(idpd_handle* h) {
   if (h->tune.skin <= 0.0f) return IDPD_OK;
-  if (!h->d.vl) return ensure_verlet(h);
+  if (!h->d.vdev) return ensure_verlet(h);
   if (h->vl_dirty) {
     static const int kOne = 1;
     CK(cudaMemcpyAsync(&h->d.vdev->force, &kOne, sizeof(int), cudaMemcpyHostToDevice, h->st));
@@ -481,16 +490,16 @@ int ensure_verlet_ready(idpd_handle* h) {
 }
 
 int ensure_aux(idpd_handle* h) {
-  if (h->press64) return IDPD_OK;
+  if (h->vir_part) return IDPD_OK;  // the last of them
   int rc = ensure_press(h);
   if (rc) return rc;
   DevState& d = h->d;
-  if ((rc = dalloc(h, &d.dqx, h->cap)) ||
-      (rc = dalloc(h, &d.dqy, h->cap)) || (rc = dalloc(h, &d.dqz, h->cap)) ||
-      (rc = dalloc(h, &h->press64, 3 * (size_t)h->cap)) ||
-      (rc = dalloc(h, &h->cm64, 6 * (size_t)h->cap)) ||
-      (rc = dalloc(h, &h->cm_cnt, 2 * (size_t)h->cap)) ||
-      (rc = dalloc(h, &h->vir_part, 3 * (size_t)h->n_amp_cap)))
+  if ((rc = dbuf(h, &d.dqx, h->cap)) ||
+      (rc = dbuf(h, &d.dqy, h->cap)) || (rc = dbuf(h, &d.dqz, h->cap)) ||
+      (rc = dbuf(h, &h->press64, 3 * (size_t)h->cap)) ||
+      (rc = dbuf(h, &h->cm64, 6 * (size_t)h->cap)) ||
+      (rc = dbuf(h, &h->cm_cnt, 2 * (size_t)h->cap)) ||
+      (rc = dbuf(h, &h->vir_part, 3 * (size_t)h->n_amp_cap)))
     return rc;
   invalidate_graph(h);  // DevState changed (aux pointers)
   return IDPD_OK;
@@ -511,11 +520,13 @@ int chem_layout(idpd_handle* h) {
   b.chem = h->chem;
   int rc = IDPD_OK;
   if ((size_t)total > h->chem_buf_total) {
+    h->chem_buf_total = 0;  // until both are there
     if ((rc = dalloc(h, &b.flags, (size_t)total))) return rc;
     if ((rc = dalloc(h, &b.chunk, (size_t)(total + 1023) / 1024))) return rc;
     h->chem_buf_total = (size_t)total;
   }
   if ((size_t)tcap > h->chem_buf_tcap) {
+    h->chem_buf_tcap = 0;
     if ((rc = dalloc(h, &b.targets, 2 * (size_t)tcap))) return rc;
     if ((rc = dalloc(h, &b.draws, 25 * (size_t)tcap))) return rc;
     h->chem_buf_tcap = (size_t)tcap;
