@@ -103,11 +103,14 @@ constexpr uint64_t kMant = 0xFFFFFFFFFFFFFull, kHidden = 0x10000000000000ull;
 // normal).
 IDPD_HD double mul_f64(double a, double b) {
   const uint64_t ab = f64_bits(a), bb = f64_bits(b);
-  const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52);
+  // a factor that is zero, subnormal, not finite or negative gets an exponent that no product
+  // takes (once for all its uses)
+  constexpr int kNoFactor = 8192;
+  const int fb = (int)(bb >> 52), eb = (uint32_t)(fb - 1) > 2045u ? kNoFactor : fb;
+  const int ea = (int)(ab >> 52) & 0x7ff;
   int e = ea + eb - 1022;
-  const bool plain_b = (uint32_t)(eb - 1) > 2045u;  // zero, subnormal, not finite, negative
-  if (plain_b || ea == 0 || ea == 0x7ff || e < 2 || e > 2045) {
-    if (!plain_b && (ab << 1) == 0) return a;  // a zero keeps its sign
+  if (ea == 0 || ea == 0x7ff || e < 2 || e > 2045) {
+    if ((ab << 1) == 0 && eb != kNoFactor) return a;  // a zero keeps its sign
     return plain_mul(a, b);
   }
   const uint64_t m = (ab & kMant) | kHidden, f = (bb & kMant) << 11 | 0x8000000000000000ull;
