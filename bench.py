@@ -817,7 +817,8 @@ def step_runs(calls, t0, since_sort, sort_period=100):
                     n += 1
                 fitting = [r for r in RUNS if r <= n]
                 wanted.update(fitting[:1])
-                n = next((r for r in fitting if r in captured or sent >= r or r in earlier), 1)
+                n = next((r for r in fitting if r in captured
+                          or (r == fitting[0] and (sent >= r or r in earlier))), 1)
                 captured.add(n)
             runs.append(n)
             sent += n

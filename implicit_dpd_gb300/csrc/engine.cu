@@ -1548,8 +1548,8 @@ int idpd_remove_cmdrift(idpd_handle* h) {
 //
 // A run is captured when a call first needs it (14 steps in three runs cost 370 us, whatever
 // the length asked for: two steps after a change of the tuning 433 us, now 169): the shortest
-// at once, a longer one behind as many steps of the call that are queued already, whose time
-// covers its capture, or when an earlier call had use for it.
+// at once; a longer one behind as many steps of the call that are queued already, as shorter
+// runs, whose time covers its capture, or when an earlier call had use for it.
 constexpr int kRunSteps[3] = {8, 4, 2};
 
 // Captures nsteps steps into *ge (if it is not there yet).
@@ -1659,14 +1659,13 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
     int c = 1;
     while (c < most && !observes(c) && !removes(c)) c++;
     if (use_loop && c > 1) return {c, &h->graph_loop, false, kCmIfNode};
-    bool first = true;
-    for (int q = 0; q < 3 && use_run; q++) {
+    int longest = 0;
+    while (longest < 3 && kRunSteps[longest] > c) longest++;
+    for (int q = longest; q < 3 && use_run; q++) {
       const int n = kRunSteps[q];
-      if (n > c) continue;
-      if (first) h->run_wanted[q] = true;
-      first = false;
-      if (h->graph_run[q] || q == 2 || sent >= n || wanted[q])
-        return {n, &h->graph_run[q], false, kCmNone};
+      const bool capture = q == longest && (sent >= n || wanted[q]);
+      if (q == longest) h->run_wanted[q] = true;
+      if (h->graph_run[q] || q == 2 || capture) return {n, &h->graph_run[q], false, kCmNone};
     }
     return {1, &h->graph, false, every_cm ? kCmKernels : kCmNone};
   };
