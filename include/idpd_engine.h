@@ -203,10 +203,10 @@ int idpd_remove_cmdrift(idpd_handle* h);
  * density, force, bonded, kick, centre-of-mass drift removal every 100 steps,
  * time += 1) for every replica, captured once into CUDA graphs. The steps up
  * to the next storage reorder, observing step or step that removes the drift
- * go to the device eight per launch, the rest one by one; with the reaction in
- * one launch (the graph's conditional WHILE node repeats the step, and ends
- * the loop after a step whose reaction event stopped the run). With
- * IDPD_CFG_PLAIN_GRAPHS every step is a launch.
+ * go to the device eight per launch, what is left of them four, two and one at a
+ * time; with the reaction in one launch (the graph's conditional WHILE node
+ * repeats the step, and ends the loop after a step whose reaction event stopped
+ * the run). With IDPD_CFG_PLAIN_GRAPHS every step is a launch.
  * Per-particle press and nei_cm_pos are not produced by this path. */
 int idpd_step(idpd_handle* h, int32_t nsteps);
 /* Blocks until the handle's stream is idle; reports device-side errors. */
