@@ -103,13 +103,19 @@ __device__ __forceinline__ void chain_begin() {
   chain_wait();
 }
 
-// Approximate reciprocal square root, division and cosine without the steps
-// that keep subnormal operands (none occurs where they are used): rsqrt of 0 is
-// infinite, and for normal operands the results are rsqrtf's, __fdividef's and
+// Approximate reciprocal square root, product, division and cosine without the steps
+// that keep subnormal operands: rsqrt of 0 and of those is infinite, 0 and those times it no
+// number, and for normal operands the results are rsqrtf's, __fmul_rn's, __fdividef's and
 // __cosf's.
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// a * b saturated to [0, 1], 0 for no number.
+__device__ __forceinline__ float mul_sat(float a, float b) {
+  float y;
+  asm("mul.rn.ftz.sat.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
   return y;
 }
 __device__ __forceinline__ float div_approx(float a, float b) {

@@ -110,12 +110,6 @@ __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int 
           const double cutd2d = WARREN ? (double)R->wrd * (double)R->wrd : 1.0;
           if (near1) in1 = e2 < 1.0;
           ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
-          if (ind && dr2 < 1.0e-10f) {
-            ind = false;
-            const uint32_t w = dens_weight(close_dr2(e2), WARREN, inv_rd, wnorm, pre);
-            add_weight(q0, q1, q2, fbits(pj.w), w);
-            atomicAdd(other + t, (unsigned long long)w);
-          }
         }
       }
       const uint32_t prj = fbits(pj.w);
@@ -134,8 +128,8 @@ __global__ void __launch_bounds__(kRowBlock, 10) k_density_list(DevState d, int 
       }
     }
     if (KNOWN) nl = nv;
-    // the totals of each group's lanes: a list holds at most 512 entries and each
-    // weight is below 2^23, so a total is below 2^32
+    // the totals of each group's lanes: a list holds at most 512 entries and each weight is
+    // below 2^23 (2^23 within 3e-8 of the particle, not for 512 partners), so a total fits 32 bits
 #pragma unroll
     for (int o = 1; o < LP; o <<= 1) {
       q0 += __shfl_xor_sync(0xffffffffu, q0, o);
@@ -213,7 +207,7 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
         const float ex = (pi.x - (float)dx * csx) - pj.x;
         const float ey = (pi.y - (float)dy * csy) - pj.y;
         const float ez = (pi.z - (float)dz * csz) - pj.z;
-        float dr2 = dist2(ex, ey, ez);
+        const float dr2 = dist2(ex, ey, ez);
         bool in1 = valid && (list_known || dr2 < 1.0f);
         bool ind = in1 && dr2 < cutd2 && dr2 >= 1.0e-10f;
         const bool near1 = valid && !list_known && fabsf(dr2 - 1.0f) <= kGuard;
@@ -223,7 +217,6 @@ __global__ void __launch_bounds__(kRowBlock) k_density_over(DevState d, int nblk
             const double e2 = exact_dr2(d, R, si, d.perm[t]);
             if (near1) in1 = e2 < 1.0;
             ind = in1 && (near2 ? (e2 < cutd2d && e2 != 0.0) : (dr2 < cutd2 && dr2 >= 1.0e-10f));
-            if (near2 && dr2 < 1.0e-10f) dr2 = close_dr2(e2);
           }
         }
         const uint32_t prj = fbits(pj.w);

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_walk_density(WalkDev w, Rep
     const int j = j0 + lane;
     const bool valid = j < je;
     const float4 pj = valid ? w.pj[j] : make_float4(1.0e18f, 0.0f, 0.0f, 0.0f);
-    float dr2 = walk_dist2(pi, pj);
+    const float dr2 = walk_dist2(pi, pj);
     bool in_b = valid && dr2 < kRnC2f && dr2 != 0.0f;
     bool in_1 = valid && dr2 < 1.0f && dr2 != 0.0f;
     bool in_d = in_1 && dr2 < cutd2;
@@ -162,7 +162,6 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_walk_density(WalkDev w, Rep
         in_b = e2 < kRnC2 && e2 != 0.0;
         in_1 = e2 < 1.0 && e2 != 0.0;
         in_d = in_1 && e2 < cutd2d;
-        if (dr2 < 1.0e-10f) dr2 = close_dr2(e2);
       }
     }
     if (!valid) continue;
