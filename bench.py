@@ -800,11 +800,12 @@ def grid_cells(box, tune):
     return int(np.prod((np.asarray(box) / (1.0 + tune["skin"])).astype(int) * tune["reach"]))
 
 
-def step_runs(calls, t0, since_sort, sort_period=100):
+def step_runs(calls, t0, since_sort, sort_period=100, step_ms=0.0):
     """The launches of the last of several idpd_step calls (their step counts, the first one
     after a change that dropped the captured steps) by the steps of each, and the storage
     reorders between them: the engine's rule without the reaction and without observations.
-    t0: the step counter, since_sort: the steps since the last reorder, before the last call."""
+    t0: the step counter, since_sort: the steps since the last reorder, before the last call;
+    step_ms: the time of a step (a call of 4 ms or more captures every run)."""
     captured, wanted = {2}, set()
     time, since = t0 - sum(calls[:-1]), (since_sort - sum(calls[:-1])) % sort_period
     for steps in calls:
@@ -826,12 +827,14 @@ def step_runs(calls, t0, since_sort, sort_period=100):
             since += n
             if since >= sort_period:
                 since, reorders = 0, reorders + 1
+        if steps > 1 and steps * step_ms >= 4.0:
+            captured.update(RUNS)
     return runs, reorders
 
 
-def timed_launches(calls, kept, rows, cells, rebuilds, t0, since_sort, plain=False):
+def timed_launches(calls, kept, rows, cells, rebuilds, t0, since_sort, plain=False, step_ms=0.0):
     """The kernels that the last of the calls launches (step_runs; rebuilds: of that call)."""
-    runs, reorders = step_runs(calls, t0, since_sort)
+    runs, reorders = step_runs(calls, t0, since_sort, step_ms=step_ms)
     steps, two_scans = calls[-1], cells > ONE_SCAN_CELLS
     if kept and rows > GATED_ROWS and not plain:
         n = gpu_launches(steps, True, rebuilds, t0, reorders, loop=False)
@@ -1017,7 +1020,8 @@ def run_engine(args, rank, world, local_rank):
            "batched_replicas": batched, "reaction": reaction, "liquid": liquid,
            "gpu_launches": timed_launches([max(args.warmup, 3), args.steps], reach["skin"] > 0, n,
                                           grid_cells(box, reach), rebuilds, t0_step,
-                                          (t0_step - 1) % 100, plain=GRAPH_FLAGS != 0),
+                                          (t0_step - 1) % 100, plain=GRAPH_FLAGS != 0,
+                                          step_ms=ms_max / args.steps),
            "force_error_bar": "max-particle relative force error <= 1e-5 vs FP64 (tests/test_gpu_parity.py)"}
     if rank == 0:
         print(json.dumps(out), flush=True)

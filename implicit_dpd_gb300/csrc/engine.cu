@@ -96,6 +96,7 @@ struct idpd_handle {
   cudaGraphExec_t graph_cm = nullptr;   // the step with the drift removal
   cudaGraphExec_t graph_run[3] = {};    // kRunSteps[k] plain steps
   bool run_wanted[3] = {};              // some call had use for it
+  double step_ms = 0.0;                 // of the last idpd_step call
   std::vector<uint32_t> time_h;  // Parameter::time per replica, as rep_time on the device
   bool time_known = false;       // (not after steps with the reaction, which may stop)
   int* err_host = nullptr;       // pinned copy of the device's error word
@@ -1549,8 +1550,12 @@ int idpd_remove_cmdrift(idpd_handle* h) {
 // A run is captured when a call first needs it (14 steps in three runs cost 370 us, whatever
 // the length asked for: two steps after a change of the tuning 433 us, now 169): the shortest
 // at once; a longer one behind as many steps of the call that are queued already, as shorter
-// runs, whose time covers its capture, or when an earlier call had use for it.
+// runs, whose time covers its capture, or when an earlier call had use for it. A call of
+// kRunsAtOnceMs or more, by the steps of the one before, captures what is missing while its
+// last steps run: the capture of a run with IF nodes waits for the device (984k beads, 20
+// steps after a warm-up of 5: 34.3 ms with a capture among them, 34.2 without).
 constexpr int kRunSteps[3] = {8, 4, 2};
+constexpr double kRunsAtOnceMs = 4.0;
 
 // Captures nsteps steps into *ge (if it is not there yet).
 int build_graph(idpd_handle* h, cudaGraphExec_t* ge, int nsteps, bool observe, CmForm cm) {
@@ -1699,8 +1704,14 @@ int idpd_step(idpd_handle* h, int32_t nsteps) {
   }
   CK(cudaEventRecord(h->ev1, h->st));
   if ((rc = queue_error_copy(h))) return rc;
+  for (int q = 0; q < 3 && use_run && nsteps * h->step_ms >= kRunsAtOnceMs; q++) {
+    if (h->graph_run[q]) continue;
+    if ((rc = build_graph(h, &h->graph_run[q], kRunSteps[q], false, kCmNone))) return rc;
+    CK(cudaGraphUpload(h->graph_run[q], h->st));
+  }
   CK(cudaStreamSynchronize(h->st));
   CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
+  h->step_ms = h->last_ms / nsteps;
   h->density_valid = false;
   if ((rc = sync_counts(h))) return rc;
   return check_device_error(h, true);

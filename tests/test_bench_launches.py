@@ -25,6 +25,12 @@ def test_runs_of_a_call(calls, t0, since, runs, reorders):
     assert bench.step_runs(calls, t0, since) == (runs, reorders)
 
 
+def test_runs_after_a_long_call():
+    assert bench.step_runs([5, 20], 6, 5, step_ms=1.7) == ([8, 8, 4], 0)
+    assert bench.step_runs([5], 6, 5, step_ms=1.7) == ([2, 2, 1], 0)
+    assert bench.step_runs([2, 20], 3, 2, step_ms=1.7) == ([2, 2, 2, 2, 8, 4], 0)
+
+
 def test_launches_of_a_call():
     # 984k beads, kept lists: 20 steps, 7 rebuilds, runs of 8, 8 and 4 with 17 fused pairs
     assert bench.timed_launches([40, 20], True, 984040, 92000, 7, 2571, 70) == 20 * 9 + 7 * 6 - 17
